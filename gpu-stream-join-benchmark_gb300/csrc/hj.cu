@@ -514,37 +514,118 @@ __global__ void __launch_bounds__(1024) part_scan_kernel(const uint32_t *__restr
     }
 }
 
-// One bucket of the join list with what its join reads before the tuples:
-// both sides' counts and run starts, the window, the window's radix bits, and
-// whether the window is radix-partitioned (its buckets may use a direct table).
+// One piece of the join list with what its join reads before the tuples: a
+// bucket's build run and (a piece of) its probe run, their sides, the window
+// and its radix bits.
 struct __align__(16) JoinItem {
-    uint32_t b, nR, nS, sR, sS, w, lg, direct;
+    uint32_t nB, nP, sB, sP;   // tuples and first position of the build run and of the probe piece
+    uint32_t w, lg, flags, pad;   // window; low key bits that all keys of the bucket share; kItem*
 };
 static_assert(sizeof(JoinItem) == 32, "two 16-byte words per join item");
+enum : uint32_t {
+    kItemModel = 1u,    // a learned bucket: a key range rather than a residue class
+    kItemSwap = 2u,     // built from the right side, probed by the left
+    kItemRaw = 4u,      // an unpartitioned window: positions index its sides' tuples
+    kItemHot = 8u       // a piece of a build run longer than its table
+};
+
+// A bucket's pieces: nb build pieces times np probe pieces, every pair of them
+// one item (count and checksum are sums over the pairs).
+struct JoinGrid {
+    uint32_t nb, np;
+    __host__ __device__ uint32_t items() const { return nb * np; }
+};
+
+// A bucket is cut into pieces of about `chunk` probe tuples, joined by
+// different CTAs; each builds the bucket's table again, so a piece has at least
+// as many probes as the build run.  A longer build run (cap: a table's slots)
+// is a hot key's or a low fan-out's: up to kHotRuns tables long it is joined in
+// one piece, whose refused keys are compacted in place (only one CTA may do
+// that); beyond, both runs are cut, into at most kHotSplit pieces each, or one
+// CTA would join millions of tuples alone (8 x 2^24, z = 1.5, one hot key in
+// the buckets: 6.1 ms).
+constexpr uint32_t kHotRuns = 8, kHotSplit = 16;
+__host__ __device__ __forceinline__ JoinGrid join_grid(uint32_t nB, uint32_t nP, uint32_t chunk, uint32_t cap) {
+    JoinGrid g{1, 1};
+    if (nB < cap) {
+        const uint32_t per = chunk > nB ? chunk : nB;
+        g.np = (uint32_t)(((uint64_t)nP + per / 2) / per);   // rounded: a piece is at most 1.5 chunks
+        if (g.np == 0) g.np = 1;
+    } else if (nB > kHotRuns * cap && nP > kHotRuns * cap) {
+        const uint32_t per = kHotRuns / 2 * cap, kb = nB / per, kp = nP / per;   // at least 2 of each
+        g.nb = kb < kHotSplit ? kb : kHotSplit;
+        g.np = kp < kHotSplit ? kp : kHotSplit;
+    }
+    return g;
+}
+
+// The most items a call can have: one per bucket and, by join_grid, at most one
+// more per chunk of probes and kHotSplit more per kHotRuns / 2 tables of a side.
+static inline uint64_t join_items_bound(uint64_t buckets, uint64_t tuples, uint32_t chunk, uint32_t cap) {
+    return buckets + tuples / chunk + tuples / (kHotRuns / 2 * cap) * kHotSplit;
+}
+
+// Item q of a bucket: its build piece and its probe piece.
+__device__ __forceinline__ void item_piece(JoinItem &ji, const JoinGrid &g, uint32_t q, uint32_t nB, uint32_t sB,
+                                           uint32_t nP, uint32_t sP) {
+    const uint32_t ib = q / g.np, ip = q - ib * g.np;
+    const uint32_t b0 = (uint32_t)((uint64_t)nB * ib / g.nb), p0 = (uint32_t)((uint64_t)nP * ip / g.np);
+    ji.sB = sB + b0;
+    ji.nB = (uint32_t)((uint64_t)nB * (ib + 1) / g.nb) - b0;
+    ji.sP = sP + p0;
+    ji.nP = (uint32_t)((uint64_t)nP * (ip + 1) / g.np) - p0;
+}
+
+// Whether a window needs no partitioning: its smaller side is one bucket, so
+// the join reads the tuples themselves.  Sides differ much in real batches (an
+// idle stream against a busy one), and partitioning the larger side into one
+// bucket would copy it for nothing.  With the fan-out by the smaller side, the
+// smaller side built and long runs cut, the bucket joins of the 1,024 windows
+// above went from 6.60 to 4.17 ms, their counting from 0.70 to 0.57 and their
+// scatter from 1.75 to 1.35.
+__host__ __device__ __forceinline__ bool raw_window(const WinPlan &wp) { return wp.raw != 0; }
 
 // Per window, one CTA: exclusive scan of the window's bucket counts on each
 // side, starting at the window's base in that side's partitioned array (the
 // tuples of the windows before it: baseL / baseR), giving the bucket starts
 // and scatter cursors; then every bucket with tuples on both sides is appended
-// to the join list (items, length *jn: nothing else can match).
+// to the join list (items, length *jn: nothing else can match), in pieces.
+// either: the join may build from either side, and builds from the smaller;
+// otherwise it builds from the left.
 __global__ void __launch_bounds__(1024)
 part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restrict__ baseL,
                      const uint32_t *__restrict__ baseR, const uint32_t *__restrict__ cnt,
                      uint32_t *__restrict__ start, uint32_t *__restrict__ cursor, uint32_t B,
                      const LearnedModel *__restrict__ models, JoinItem *__restrict__ items,
-                     uint32_t *__restrict__ jn) {
+                     uint32_t *__restrict__ jn, uint32_t chunk, uint32_t cap, bool either) {
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry_s;
     const uint32_t w = blockIdx.x;
     const WinPlan wp = wins[w];
+    if (raw_window(wp)) {   // its pieces, straight over the tuples
+        const uint32_t nL = (uint32_t)wp.n_left, nR = (uint32_t)wp.n_right;
+        const bool swap = either && nR < nL;
+        const uint32_t nB = swap ? nR : nL, nP = swap ? nL : nR;
+        const JoinGrid g = join_grid(nB, nP, chunk, cap);   // (the build side is below cap)
+        const uint32_t k = g.items();
+        if (threadIdx.x == 0) carry_s = atomicAdd(jn, k);
+        SJBG_BARRIER();
+        for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) {
+            JoinItem ji;
+            item_piece(ji, g, i, nB, 0u, nP, 0u);
+            ji.w = w; ji.lg = 0; ji.flags = kItemRaw | (swap ? kItemSwap : 0u); ji.pad = 0;
+            items[carry_s + i] = ji;
+        }
+        return;
+    }
     const uint32_t P = 1u << wp.log2_buckets, b0 = wp.bucket_base;
     constexpr uint32_t kItems = 4;
-    const uint32_t chunk = blockDim.x * kItems;
+    const uint32_t tchunk = blockDim.x * kItems;
     for (uint32_t side = 0; side < 2; side++) {
         const uint32_t lo = side * B + b0, hi = lo + P;
         if (threadIdx.x == 0) carry_s = side ? baseR[w] : baseL[w];
         SJBG_BARRIER();
-        for (uint32_t base = lo; base < hi; base += chunk) {
+        for (uint32_t base = lo; base < hi; base += tchunk) {
             uint32_t v[kItems], s = 0;
 #pragma unroll
             for (uint32_t k = 0; k < kItems; k++) {
@@ -579,20 +660,28 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
     }
     // join list: one reservation per warp of joinable buckets (the starts were
     // written by this CTA, before the scan's last barrier)
-    const uint32_t direct = (models ? model_of(wp, models) : nullptr) == nullptr ? 1u : 0u;
+    const bool model = models && model_of(wp, models) != nullptr;
     for (uint32_t i0 = 0; i0 < P; i0 += blockDim.x) {
         const uint32_t i = i0 + threadIdx.x, b = b0 + i;
-        const uint32_t nR = i < P ? cnt[b] : 0u, nS = i < P ? cnt[B + b] : 0u;
-        const bool ok = nR != 0u && nS != 0u;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, ok);
+        const uint32_t nL = i < P ? cnt[b] : 0u, nR = i < P ? cnt[B + b] : 0u;
+        const bool swap = either && nR < nL;
+        const uint32_t nB = swap ? nR : nL, nP = swap ? nL : nR;
+        const JoinGrid g = join_grid(nB, nP, chunk, cap);
+        const uint32_t k = (nL != 0u && nR != 0u) ? g.items() : 0u;
+        uint32_t tot;
+        const uint32_t ex = warp_excl_scan(k, &tot);
         uint32_t wbase = 0;
-        if (lane_id() == 0 && m) wbase = atomicAdd(jn, (uint32_t)__popc(m));
-        wbase = __shfl_sync(0xFFFFFFFFu, wbase, 0);
-        if (ok) {
+        if (lane_id() == 0 && tot) wbase = atomicAdd(jn, tot);
+        wbase = __shfl_sync(0xFFFFFFFFu, wbase, 0) + ex;
+        if (k) {
+            const uint32_t sL = start[b], sR = start[B + b];
             JoinItem ji;
-            ji.b = b; ji.nR = nR; ji.nS = nS; ji.sR = start[b]; ji.sS = start[B + b];
-            ji.w = w; ji.lg = wp.log2_buckets; ji.direct = direct;
-            items[wbase + __popc(m & ((1u << lane_id()) - 1u))] = ji;
+            ji.w = w; ji.lg = wp.log2_buckets; ji.pad = 0;
+            ji.flags = (model ? kItemModel : 0u) | (swap ? kItemSwap : 0u) | (g.nb > 1 ? kItemHot : 0u);
+            for (uint32_t q = 0; q < k; q++) {
+                item_piece(ji, g, q, nB, swap ? sR : sL, nP, swap ? sL : sR);
+                items[wbase + q] = ji;
+            }
         }
     }
 }
@@ -1011,7 +1100,7 @@ part_fine_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_t
 }
 
 // ------------------------------------------------------------------ 4. bucket join
-constexpr uint32_t kMaxProbe = 64;   // linear-probe bound of the count tables
+constexpr uint32_t kMaxProbe = 64;   // linear-probe bound of the count tables that may fill up
 
 // Count-table slots for buckets of about `target` left tuples (load <= 0.77).
 static inline uint32_t count_table_cap(uint32_t target) { return (target * 13u / 10u + 31u) & ~31u; }
@@ -1021,6 +1110,7 @@ struct CountTable {
     uint32_t *cnt;               // C + 1
     unsigned long long *sumf;    // C + 1
     uint32_t C;                  // slots (any size: the hash is scaled, not masked)
+    uint32_t max_probe;          // kMaxProbe, or C when the build run is shorter than the table (every key fits)
 };
 
 // Home slot of a key in a table of C slots: a 32-bit multiplicative hash scaled to [0, C).
@@ -1039,8 +1129,8 @@ __device__ __forceinline__ void ct_add_sum(unsigned long long *slot, unsigned lo
     atomicAdd(&w2[1], add_carry((uint32_t)(f >> 32), old, flo));
 }
 
-// Insert `c` tuples of `key` with fr-sum `f`.  A key that finds neither itself
-// nor a free slot within kMaxProbe slots is refused (false) and joined in a
+// Insert `c` tuples of `key` with hash sum `f`.  A key that finds neither itself
+// nor a free slot within max_probe slots is refused (false) and joined in a
 // later pass; lookups use the same bound, so a refused key is never half-found.
 // Every lane inserts its own tuple: with the sums' native 32-bit atomics this
 // beats combining a warp's equal keys first, at every skew measured.
@@ -1052,7 +1142,7 @@ __device__ __forceinline__ bool ct_insert(const CountTable &t, uint32_t key, uin
         return true;
     }
     uint32_t s = ct_home(key, C);
-    for (uint32_t probe = 0; probe < kMaxProbe; probe++) {
+    for (uint32_t probe = 0; probe < t.max_probe; probe++) {
         uint32_t k = *(volatile uint32_t *)&t.keys[s];
         if (k == kEmptyKey) {
             const uint32_t prev = atomicCAS(&t.keys[s], kEmptyKey, key);
@@ -1072,7 +1162,7 @@ __device__ __forceinline__ int ct_lookup(const CountTable &t, uint32_t key) {
     const uint32_t C = t.C;
     if (key == kEmptyKey) return t.cnt[C] ? (int)C : -1;
     uint32_t s = ct_home(key, C);
-    for (uint32_t probe = 0; probe < kMaxProbe; probe++) {
+    for (uint32_t probe = 0; probe < t.max_probe; probe++) {
         const uint32_t k = t.keys[s];
         if (k == key) return (int)s;
         if (k == kEmptyKey) return -1;
@@ -1083,74 +1173,226 @@ __device__ __forceinline__ int ct_lookup(const CountTable &t, uint32_t key) {
 
 constexpr int kJoinPer = 8;   // elements per thread per tile (independent loads in flight)
 
-__device__ __forceinline__ void join_count_bucket(const JoinItem &ji, uint64_t *__restrict__ partL,
-                                                  const uint64_t *__restrict__ partR, WinAcc *__restrict__ acc,
-                                                  uint32_t cap) {
+// Probe tuples per join piece: at most kJoinChunk (a piece of a long run then
+// ends within some 20 us of the others), at least kJoinChunkMin, or
+// kJoinChunkEnum when pairs are enumerated.
+constexpr uint32_t kJoinChunk = 65536;
+constexpr uint32_t kJoinChunkMin = 2048, kJoinChunkEnum = 16384;
+
+// A run of tuples: (val << 32 | key) words of a partitioned array, or (kRaw)
+// the key and val of 16-byte tuples.
+template <bool kRaw>
+__device__ __forceinline__ uint64_t run_load(const void *p, uint32_t i) {
+    if (kRaw) {
+        const uint2 v = __ldg(static_cast<const uint2 *>(p) + 2 * (size_t)i);
+        return ((uint64_t)v.y << 32) | v.x;
+    }
+    return static_cast<const uint64_t *>(p)[i];
+}
+
+// Where an item's runs lie and which side builds.
+struct JoinRuns {
+    void *b;         // build run (a partitioned one may be compacted in place)
+    const void *p;   // probe piece
+    uint32_t bside;  // side of the build tuples: 0 left (fr), 1 right (gs); the probes have the other's hash
+};
+__device__ __forceinline__ JoinRuns join_runs(const JoinItem &ji, const sjbg_tuple *__restrict__ L,
+                                              const sjbg_tuple *__restrict__ R, const WinPlan *__restrict__ wins,
+                                              uint64_t *partL, uint64_t *partR) {
+    JoinRuns r;
+    const bool swap = (ji.flags & kItemSwap) != 0;
+    r.bside = swap ? 1u : 0u;
+    if (ji.flags & kItemRaw) {
+        const sjbg_tuple *l = L + wins[ji.w].left_off, *t = R + wins[ji.w].right_off;
+        r.b = const_cast<sjbg_tuple *>((swap ? t : l) + ji.sB);   // never written: every key of a raw window fits
+        r.p = (swap ? l : t) + ji.sP;
+    } else {
+        r.b = (swap ? partR : partL) + ji.sB;
+        r.p = (swap ? partL : partR) + ji.sP;
+    }
+    return r;
+}
+
+// Key filter of a hash-table bucket: about 32 bits per build tuple (at most
+// 2^kFilterBits), one set per build key.  Most probes of mostly distinct keys
+// match nothing; walking the table for them is what a bucket's time went on
+// (every lane of a warp waits for the longest walk).  The filter answers a
+// miss with one shared load, and the survivors are gathered per warp and
+// looked up 32 at a time.  Measured on 1,024 windows whose sides have
+// independent sizes, log-uniform in [2^10, 2^20], keys in [0, 4 max(W)): the
+// bucket joins took 4.17 ms without the filter and with a failed direct-table
+// build in most buckets, 1.78 ms with it and the range known beforehand
+// (pieces of up to 65,536 probes rather than 16,384 among it).
+constexpr uint32_t kFilterBits = 17;
+constexpr uint32_t kQueueSlots = 64;   // per warp: fewer than 32 waiting, and up to 32 more of one step
+
+__device__ __forceinline__ uint32_t filter_hash(uint32_t key) { return key * 0x9E3779B1u; }
+
+// The bucket's table in shared memory (cap slots, filter, survivor queues).
+static inline size_t count_table_bytes(uint32_t cap) {
+    return sizeof(unsigned long long) * (kJoinThreads / 32) * kQueueSlots +
+           (sizeof(unsigned long long) + 2 * sizeof(uint32_t)) * ((size_t)cap + 1) + (1u << kFilterBits) / 8;
+}
+
+// Larger buckets (a radix window's hot keys) keep the hash table when they need
+// a second direct pass, which re-reads the bucket; and every longer build run
+// does, as the direct table's reset re-reads it.
+constexpr uint32_t kDirectMaxRun = 16384;
+
+struct KeyRange {
+    uint32_t lo, hi;
+};
+
+// Loads the first tile of a build run (kJoinPer tuples per thread) and returns
+// the run's smallest and largest keys to every thread (those of its first
+// tile, when the run is too long for a direct table anyway); ends with a barrier.
+template <bool kRaw>
+__device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer]) {
+    __shared__ uint32_t min_s, max_s;
+    if (threadIdx.x == 0) {
+        min_s = 0xFFFFFFFFu;
+        max_s = 0;
+    }
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+    for (int k = 0; k < kJoinPer; k++) {
+        const uint32_t i = k * kJoinThreads + threadIdx.x;
+        e[k] = i < ji.nB ? run_load<kRaw>(jr.b, i) : 0ull;
+    }
+    SJBG_BARRIER();
+#pragma unroll
+    for (int k = 0; k < kJoinPer; k++) {
+        if (k * kJoinThreads + threadIdx.x < ji.nB) {
+            lo = min(lo, (uint32_t)e[k]);
+            hi = max(hi, (uint32_t)e[k]);
+        }
+    }
+    if (ji.nB <= kDirectMaxRun) {
+        for (uint32_t i = kJoinPer * kJoinThreads + threadIdx.x; i < ji.nB; i += kJoinThreads) {
+            const uint32_t key = (uint32_t)run_load<kRaw>(jr.b, i);
+            lo = min(lo, key);
+            hi = max(hi, key);
+        }
+    }
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    if (lane_id() == 0) {
+        atomicMin(&min_s, lo);
+        atomicMax(&max_s, hi);
+    }
+    SJBG_BARRIER();
+    return KeyRange{min_s, max_s};
+}
+
+// e: the build run's first tile (build_head), when loaded.  kFilter: probes go
+// through the key filter.  A learned bucket's go straight to the table: its
+// light keys cover its range, most probes match, and the filter only adds to
+// them (z = 1.5, 8 x 2^24: 53.6 us without, 67.0 us with).
+template <bool kRaw, bool kFilter>
+__device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
+                                                  bool loaded, WinAcc *__restrict__ acc, uint32_t cap) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ uint32_t novf;
-    const uint32_t nR = ji.nR, nS = ji.nS;
-    if (nR == 0 || nS == 0) return;
-    uint64_t *Rb = partL + ji.sR;
-    const uint64_t *Sb = partR + ji.sS;
-    // the table holds at most nR distinct keys: 2 slots per left tuple (at
+    const uint32_t nB = ji.nB, nP = ji.nP;
+    const uint32_t bside = jr.bside, pside = bside ^ 1u;
+    // the table holds at most nB distinct keys: 2 slots per build tuple (at
     // least 64, at most the launch's capacity of 1.3 per target tuple, which
     // lets two CTAs share an SM), so buckets under the target probe at load
     // <= 1/2: with mostly distinct keys a miss then walks ~3 slots, not ~10
-    const uint32_t C = min(cap, max(64u, (nR * 2u + 31u) & ~31u));
+    const uint32_t C = min(cap, max(64u, (nB * 2u + 31u) & ~31u));
+    const uint32_t fbits = min(kFilterBits, 37u - (uint32_t)__clz(nB));   // 32 to 64 bits per build tuple
+    const uint32_t fshift = 32u - fbits;
     CountTable t;
-    t.sumf = reinterpret_cast<unsigned long long *>(smem_raw);
+    unsigned long long *queue = reinterpret_cast<unsigned long long *>(smem_raw) + warp_id() * kQueueSlots;
+    t.sumf = reinterpret_cast<unsigned long long *>(smem_raw) + (kJoinThreads / 32) * kQueueSlots;
     t.keys = reinterpret_cast<uint32_t *>(t.sumf + C + 1);
     t.cnt = t.keys + C + 1;
+    uint32_t *filter = t.cnt + C + 1;
     t.C = C;
-    const uint32_t tile = kJoinPer * blockDim.x;
+    t.max_probe = nB < C ? C : kMaxProbe;
+    // an oversized build run is a hot key's: its probes match, so they skip the filter
+    const bool filtered = kFilter && nB < cap;
+    constexpr uint32_t tile = kJoinPer * kJoinThreads;
 
     unsigned long long count = 0, prod = 0;
-    uint32_t n = nR;
+    uint32_t n = nB;
     for (;;) {
-        for (uint32_t i = threadIdx.x; i <= C; i += blockDim.x) {
+        for (uint32_t i = threadIdx.x; i <= C; i += kJoinThreads) {
             t.keys[i] = kEmptyKey;
             t.cnt[i] = 0;
             t.sumf[i] = 0;
         }
+        if (kFilter)
+            for (uint32_t i = threadIdx.x; i < (1u << fbits) / 32; i += kJoinThreads) filter[i] = 0;
         if (threadIdx.x == 0) novf = 0;
         SJBG_BARRIER();
         // build: kJoinPer independent loads per thread, then insert them
         for (uint32_t base = 0; base < n; base += tile) {
-            uint64_t e[kJoinPer];
+            if (!loaded) {
 #pragma unroll
-            for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t i = base + k * blockDim.x + threadIdx.x;
-                e[k] = i < n ? Rb[i] : 0ull;
+                for (int k = 0; k < kJoinPer; k++) {
+                    const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+                    e[k] = i < n ? run_load<kRaw>(jr.b, i) : 0ull;
+                }
+                SJBG_BARRIER();   // every read of this tile precedes any overflow write
             }
-            SJBG_BARRIER();   // every read of this tile precedes any overflow write
+            loaded = false;
 #pragma unroll
             for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t i = base + k * blockDim.x + threadIdx.x;
+                const uint32_t i = base + k * kJoinThreads + threadIdx.x;
                 const bool valid = i < n;
-                const bool ok = !valid || ct_insert(t, (uint32_t)e[k], 1u, sjbg_fr((uint32_t)(e[k] >> 32)));
-                if (valid && !ok) Rb[atomicAdd(&novf, 1u)] = e[k];
+                if (valid) {
+                    const uint32_t key = (uint32_t)e[k], f = filter_hash(key) >> fshift;
+                    if (ct_insert(t, key, 1u, sjbg_fside((uint32_t)(e[k] >> 32), bside))) {
+                        if (filtered) atomicOr(&filter[f >> 5], 1u << (f & 31u));
+                    } else if (!kRaw) {   // (a piece's table, and a raw window's, takes every key)
+                        static_cast<uint64_t *>(jr.b)[atomicAdd(&novf, 1u)] = e[k];
+                    }
+                }
             }
         }
         SJBG_BARRIER();
         // probe: the same independent-load tiling, no barriers needed
-        for (uint32_t base = 0; base < nS; base += tile) {
-            uint64_t e[kJoinPer];
+        uint32_t waiting = 0;   // the warp's survivors in its queue (uniform over the warp)
+        auto look = [&](bool valid, unsigned long long x) {
+            const int s = valid ? ct_lookup(t, (uint32_t)x) : -1;
+            if (s >= 0) {
+                count += t.cnt[s];
+                prod += t.sumf[s] * sjbg_fside((uint32_t)(x >> 32), pside);
+            }
+        };
+        // (the filter's steps keep more in registers: four loads in flight, not eight)
+        constexpr int kPer = kFilter ? 4 : kJoinPer;
+        for (uint32_t base = 0; base < nP; base += kPer * kJoinThreads) {
+            uint64_t q[kPer];
 #pragma unroll
-            for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t j = base + k * blockDim.x + threadIdx.x;
-                e[k] = j < nS ? Sb[j] : ~0ull;
+            for (int k = 0; k < kPer; k++) {
+                const uint32_t j = base + k * kJoinThreads + threadIdx.x;
+                q[k] = j < nP ? run_load<kRaw>(jr.p, j) : 0ull;
             }
 #pragma unroll
-            for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t j = base + k * blockDim.x + threadIdx.x;
-                if (j < nS) {
-                    const int s = ct_lookup(t, (uint32_t)e[k]);
-                    if (s >= 0) {
-                        count += t.cnt[s];
-                        prod += t.sumf[s] * sjbg_gs((uint32_t)(e[k] >> 32));
-                    }
+            for (int k = 0; k < kPer; k++) {
+                const uint32_t j = base + k * kJoinThreads + threadIdx.x;
+                if (!kFilter) {
+                    look(j < nP, q[k]);
+                    continue;
+                }
+                const uint32_t f = filter_hash((uint32_t)q[k]) >> fshift;
+                const bool in = j < nP && (!filtered || ((filter[f >> 5] >> (f & 31u)) & 1u));
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
+                if (in) queue[waiting + __popc(m & ((1u << lane_id()) - 1u))] = q[k];
+                waiting += __popc(m);
+                if (waiting >= 32u) {
+                    __syncwarp();
+                    waiting -= 32u;
+                    look(true, queue[waiting + lane_id()]);
+                    __syncwarp();   // read before the slots are reused
                 }
             }
+        }
+        if (kFilter) {
+            __syncwarp();
+            look(lane_id() < waiting, queue[lane_id()]);
         }
         SJBG_BARRIER();
         n = novf;
@@ -1160,117 +1402,189 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, uint64_t *
     flush_acc(&acc[ji.w], count, 0, prod);
 }
 
-// ---- direct-addressed bucket join (radix windows)
+// A pair of pieces of a bucket whose build run is longer than its table (a hot
+// key's tuples, or those of many keys).  Other CTAs read the same runs, so
+// nothing is compacted: when a key finds no slot, the pieces are joined again
+// in twice as many passes, each over the keys of one residue of a mixed key,
+// until every pass fits.  A warp adds the tuples of its first lane's key at
+// once when they are many: same-address shared atomics take the lanes in turn.
+__device__ __noinline__ void join_count_hot(const uint64_t *b, uint32_t nB, const uint64_t *p, uint32_t nP,
+                                            uint32_t bside, WinAcc *acc, uint32_t C) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ uint32_t refused;
+    CountTable t;
+    t.sumf = reinterpret_cast<unsigned long long *>(smem_raw);
+    t.keys = reinterpret_cast<uint32_t *>(t.sumf + C + 1);
+    t.cnt = t.keys + C + 1;
+    t.C = C;
+    t.max_probe = kMaxProbe;
+    auto residue = [](uint32_t key, uint32_t passes) {   // of a bijection of the key
+        uint32_t x = key * 0x85EBCA6Bu;
+        x ^= x >> 16;
+        return x & (passes - 1);
+    };
+    unsigned long long count = 0, prod = 0;
+    bool done = false;
+    for (uint32_t passes = 1; !done && passes < (1u << 31); passes <<= 1) {
+        count = prod = 0;
+        done = true;
+        for (uint32_t s = 0; s < passes && done; s++) {
+            for (uint32_t i = threadIdx.x; i <= C; i += kJoinThreads) {
+                t.keys[i] = kEmptyKey;
+                t.cnt[i] = 0;
+                t.sumf[i] = 0;
+            }
+            if (threadIdx.x == 0) refused = 0;
+            SJBG_BARRIER();
+            for (uint32_t base = 0; base < nB; base += 4 * kJoinThreads) {
+                uint64_t e[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+                    e[k] = i < nB ? b[i] : 0ull;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t key = (uint32_t)e[k];
+                    bool in = base + k * kJoinThreads + threadIdx.x < nB && residue(key, passes) == s;
+                    unsigned long long f = sjbg_fside((uint32_t)(e[k] >> 32), bside);
+                    uint32_t c = 1;
+                    const uint32_t key0 = __shfl_sync(0xFFFFFFFFu, key, 0);   // (every lane: not inside the &&)
+                    const bool same = in && key == key0;
+                    const unsigned grp = __ballot_sync(0xFFFFFFFFu, same);
+                    if (__popc(grp) >= 8) {   // the first lane's group as one
+                        const unsigned long long sum = warp_sum_u64(same ? f : 0ull);
+                        if (same) {
+                            in = (int)lane_id() == __ffs(grp) - 1;
+                            f = sum;
+                            c = __popc(grp);
+                        }
+                    }
+                    if (in && !ct_insert(t, key, c, f)) refused = 1;
+                }
+            }
+            SJBG_BARRIER();
+            done = refused == 0;
+            if (done) {
+                for (uint32_t base = 0; base < nP; base += 4 * kJoinThreads) {
+                    uint64_t e[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+                        e[k] = i < nP ? p[i] : 0ull;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const uint32_t key = (uint32_t)e[k];
+                        if (base + k * kJoinThreads + threadIdx.x >= nP || residue(key, passes) != s) continue;
+                        const int x = ct_lookup(t, key);
+                        if (x >= 0) {
+                            count += t.cnt[x];
+                            prod += t.sumf[x] * sjbg_fside((uint32_t)(e[k] >> 32), bside ^ 1u);
+                        }
+                    }
+                }
+            }
+            SJBG_BARRIER();   // the table and `refused` are read before they are reset
+        }
+    }
+    flush_acc(acc, count, 0, prod);
+}
+
+// ---- direct-addressed bucket join
 // In a radix window every key of bucket b has key & (2^lg - 1) == b, so key >> lg
-// tells the bucket's keys apart.  When those indices span few values the
-// build side is a direct table {count, sum of fr} indexed by key >> lg: an
-// insert is three shared atomics and a probe two loads, with no key compares
-// or probe loop (the hash table spends about 120 thread instructions per tuple
-// there, and is issue- and shared-memory-bound).  A pass covers kDirectMax
-// indices; a bucket whose indices need more than kDirectPasses passes is left
-// to the hash table, decided after the first build pass and before anything is
-// counted.  Measured on 1,024 uneven windows (keys in [0, 4W), about 4,096
-// left tuples per bucket, two passes): the bucket joins take 2.02 ms, against
-// 2.91 ms with hash tables.
+// tells the bucket's keys apart (lg = 0 in a window that is not partitioned).
+// When the build run's indices key >> lg span few values the build side is a
+// direct table {count, hash sum} indexed from the smallest one: an insert is
+// three shared atomics and a probe two loads, with no key compares or probe
+// loop (the hash table spends about 120 thread instructions per tuple there,
+// and is issue- and shared-memory-bound).  A pass covers kDirectMax indices; a
+// bucket whose indices need more than kDirectPasses passes goes through the
+// hash table: the build run's smallest and largest keys, found while its first
+// tile is loaded, decide.  (Learned buckets, which are key ranges, gained
+// nothing: their probes match, and the range costs a barrier to find.)  Measured on 1,024 uneven windows (keys in [0, 4W),
+// about 4,096 left tuples per bucket, two passes): the bucket joins take
+// 2.02 ms, against 2.91 ms with hash tables.
 constexpr uint32_t kDirectMax = 8192;
 constexpr uint32_t kDirectPasses = 2;
-// Larger buckets (a radix window's hot keys) keep the hash table: every extra
-// pass and the table reset re-read the bucket, which one CTA would do serially.
-constexpr uint32_t kDirectMaxRun = 16384;
-// A left run of at most kDirectSave tuples keeps each tuple's table index (16
+// A build run of at most kDirectSave tuples keeps each tuple's table index (16
 // bits, 0xFFFF outside the pass's range) in shared memory during the build, so
 // the table is reset from there instead of from a second read of the run.
 constexpr uint32_t kDirectSave = 4096;
 constexpr size_t kDirectBytes =
     (sizeof(unsigned long long) + sizeof(uint32_t)) * kDirectMax + sizeof(uint16_t) * kDirectSave;
 
+// Passes of a bucket whose build run has keys in kr, or 0: the hash table.
+__device__ __forceinline__ uint32_t direct_passes(const JoinItem &ji, KeyRange kr) {
+    if (ji.nB > kDirectMaxRun) return 0;
+    const uint32_t passes = ((kr.hi >> ji.lg) - (kr.lo >> ji.lg)) / kDirectMax + 1;
+    if (passes > kDirectPasses || (passes > 1 && ji.nB + ji.nP > kDirectMaxRun)) return 0;
+    return passes;
+}
+
 // `clean`: the leading table entries known to be zero (CTA-uniform); a direct
-// bucket leaves the table zero again, a hash-table bucket does not.  Returns
-// false when the bucket's key range is too wide (the table is left zero).
-__device__ __forceinline__ bool join_count_direct(const JoinItem &ji, const uint64_t *__restrict__ partL,
-                                                  const uint64_t *__restrict__ partR, WinAcc *__restrict__ acc,
+// bucket leaves the table zero again, a hash-table bucket does not.  e: the
+// build run's first tile (build_head); first: its smallest index.
+template <bool kRaw>
+__device__ __forceinline__ void join_count_direct(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
+                                                  uint32_t first, uint32_t passes, WinAcc *__restrict__ acc,
                                                   uint32_t &clean) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    __shared__ uint32_t maxidx_s;
-    const uint32_t nR = ji.nR, nS = ji.nS, lg = ji.lg;
-    if (nR == 0 || nS == 0) return true;
+    const uint32_t nB = ji.nB, nP = ji.nP, lg = ji.lg;
+    const uint32_t bside = jr.bside, pside = bside ^ 1u;
     unsigned long long *dsum = reinterpret_cast<unsigned long long *>(smem_raw);
     uint32_t *dcnt = reinterpret_cast<uint32_t *>(dsum + kDirectMax);
     uint16_t *dsave = reinterpret_cast<uint16_t *>(dcnt + kDirectMax);   // kDirectSave indices
-    const bool save = nR <= kDirectSave;
-    const uint64_t *Rb = partL + ji.sR;
-    const uint64_t *Sb = partR + ji.sS;
-    for (uint32_t i = clean + threadIdx.x; i < kDirectMax; i += blockDim.x) {
+    const bool save = nB <= kDirectSave;
+    for (uint32_t i = clean + threadIdx.x; i < kDirectMax; i += kJoinThreads) {
         dsum[i] = 0;
         dcnt[i] = 0;
     }
+    if (clean != kDirectMax) SJBG_BARRIER();
     clean = kDirectMax;
-    if (threadIdx.x == 0) maxidx_s = 0;
-    SJBG_BARRIER();
-    const uint32_t tile = kJoinPer * blockDim.x;
+    constexpr uint32_t tile = kJoinPer * kJoinThreads;
     unsigned long long count = 0, prod = 0;
-    uint32_t passes = 1;
     for (uint32_t p = 0; p < passes; p++) {
-        const uint32_t lo = p * kDirectMax;
-        uint32_t tmax = 0;
-        // build: the left keys whose index falls in [lo, lo + kDirectMax)
-        for (uint32_t base = 0; base < nR; base += tile) {
-            uint64_t e[kJoinPer];
+        const uint32_t lo = first + p * kDirectMax;
+        // build: the build keys whose index falls in [lo, lo + kDirectMax)
+        for (uint32_t base = 0; base < nB; base += tile) {
+            if (p || base) {
 #pragma unroll
-            for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t i = base + k * blockDim.x + threadIdx.x;
-                e[k] = i < nR ? Rb[i] : 0ull;
+                for (int k = 0; k < kJoinPer; k++) {
+                    const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+                    e[k] = i < nB ? run_load<kRaw>(jr.b, i) : 0ull;
+                }
             }
 #pragma unroll
             for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t i = base + k * blockDim.x + threadIdx.x;
-                if (i < nR) {
-                    const uint32_t idx = (uint32_t)e[k] >> lg;
-                    tmax = max(tmax, idx);
-                    const uint32_t d = idx - lo;   // wraps for indices below the range
+                const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+                if (i < nB) {
+                    const uint32_t d = ((uint32_t)e[k] >> lg) - lo;   // wraps for indices below the range
                     if (save) dsave[i] = d < kDirectMax ? (uint16_t)d : (uint16_t)0xFFFFu;
                     if (d < kDirectMax) {
                         atomicAdd(&dcnt[d], 1u);
-                        ct_add_sum(&dsum[d], sjbg_fr((uint32_t)(e[k] >> 32)));
+                        ct_add_sum(&dsum[d], sjbg_fside((uint32_t)(e[k] >> 32), bside));
                     }
                 }
             }
-        }
-        if (p == 0) {
-            const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, tmax);
-            if (lane_id() == 0) atomicMax(&maxidx_s, m);
         }
         SJBG_BARRIER();
-        if (p == 0) {
-            passes = maxidx_s / kDirectMax + 1;
-            if (passes > kDirectPasses) {   // too wide: undo the first pass, the hash table takes the bucket
-                for (uint32_t i = threadIdx.x; i < nR; i += blockDim.x) {
-                    const uint32_t d = (uint32_t)Rb[i] >> lg;
-                    if (d < kDirectMax) {
-                        dcnt[d] = 0;
-                        dsum[d] = 0;
-                    }
-                }
-                SJBG_BARRIER();
-                return false;
-            }
-        }
-        // probe: the right keys in the range
-        for (uint32_t base = 0; base < nS; base += tile) {
-            uint64_t e[kJoinPer];
+        // probe: the probe keys in the range
+        for (uint32_t base = 0; base < nP; base += tile) {
+            uint64_t q[kJoinPer];
 #pragma unroll
             for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t j = base + k * blockDim.x + threadIdx.x;
-                e[k] = j < nS ? Sb[j] : 0ull;
+                const uint32_t j = base + k * kJoinThreads + threadIdx.x;
+                q[k] = j < nP ? run_load<kRaw>(jr.p, j) : 0ull;
             }
 #pragma unroll
             for (int k = 0; k < kJoinPer; k++) {
-                const uint32_t d = ((uint32_t)e[k] >> lg) - lo;
-                if (base + k * blockDim.x + threadIdx.x < nS && d < kDirectMax) {
+                const uint32_t d = ((uint32_t)q[k] >> lg) - lo;
+                if (base + k * kJoinThreads + threadIdx.x < nP && d < kDirectMax) {
                     const uint32_t c = dcnt[d];
                     if (c) {
                         count += c;
-                        prod += dsum[d] * sjbg_gs((uint32_t)(e[k] >> 32));
+                        prod += dsum[d] * sjbg_fside((uint32_t)(q[k] >> 32), pside);
                     }
                 }
             }
@@ -1278,8 +1592,8 @@ __device__ __forceinline__ bool join_count_direct(const JoinItem &ji, const uint
         SJBG_BARRIER();
         // leave the table zero: the range's build entries (their saved indices,
         // or for a longer run the run again, from L2)
-        for (uint32_t i = threadIdx.x; i < nR; i += blockDim.x) {
-            const uint32_t d = save ? (uint32_t)dsave[i] : ((uint32_t)Rb[i] >> lg) - lo;
+        for (uint32_t i = threadIdx.x; i < nB; i += kJoinThreads) {
+            const uint32_t d = save ? (uint32_t)dsave[i] : ((uint32_t)run_load<kRaw>(jr.b, i) >> lg) - lo;
             if (d < kDirectMax) {
                 dcnt[d] = 0;
                 dsum[d] = 0;
@@ -1288,24 +1602,21 @@ __device__ __forceinline__ bool join_count_direct(const JoinItem &ji, const uint
         SJBG_BARRIER();
     }
     flush_acc(&acc[ji.w], count, 0, prod);
-    return true;
 }
 
 constexpr uint32_t kEnumChunk = 4096;  // left tuples per chained chunk
 constexpr uint32_t kNil = 0xFFFFFFFFu;
 
-__device__ __forceinline__ void join_enum_bucket(uint32_t b, const uint64_t *__restrict__ partL,
-                                                 const uint64_t *__restrict__ partR,
-                                                 const uint32_t *__restrict__ start, const uint32_t *__restrict__ cnt,
-                                                 uint32_t B, const uint32_t *__restrict__ bucket_win,
-                                                 WinAcc *__restrict__ acc, const WinPlan *__restrict__ wins,
-                                                 sjbg_pair *__restrict__ pairs, uint32_t table_bits) {
+__device__ __forceinline__ void join_enum_bucket(const JoinItem &ji, const uint64_t *__restrict__ partL,
+                                                 const uint64_t *__restrict__ partR, WinAcc *__restrict__ acc,
+                                                 const WinPlan *__restrict__ wins, sjbg_pair *__restrict__ pairs,
+                                                 uint32_t table_bits) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    const uint32_t nR = cnt[b], nS = cnt[B + b];
+    const uint32_t nR = ji.nB, nS = ji.nP;   // (enumerating joins build from the left)
     if (nR == 0 || nS == 0) return;
-    const uint64_t *Rb = partL + start[b];
-    const uint64_t *Sb = partR + start[B + b];
-    const uint32_t w = bucket_win[b];
+    const uint64_t *Rb = partL + ji.sB;
+    const uint64_t *Sb = partR + ji.sP;
+    const uint32_t w = ji.w;
     const uint32_t Cmax = 1u << table_bits;
     uint32_t *keys = reinterpret_cast<uint32_t *>(smem_raw);   // Cmax + 1
     uint32_t *head = keys + Cmax + 1;                          // Cmax + 1
@@ -1401,8 +1712,8 @@ __device__ __forceinline__ void join_enum_bucket(uint32_t b, const uint64_t *__r
     flush_acc(&acc[w], count, xr, prod);
 }
 
-// Bucket joins over the join list (items, length *jn; or, without a list,
-// buckets 0 .. B-1, hash tables only): one CTA per item (queue == nullptr) or
+// Bucket joins over the join list (items, length *jn; or, without a list, the
+// one window's buckets 0 .. B-1, whole): CTAs that stride over the items (queue == nullptr) or
 // persistent CTAs that take items from a device work queue (an atomic counter)
 // until it runs dry.  Buckets of radix windows are joined through direct
 // tables when their key indices allow it.
@@ -1412,27 +1723,61 @@ __device__ __forceinline__ void join_enum_bucket(uint32_t b, const uint64_t *__r
 // into L2, and item k+2's record is on its way (an asynchronous copy into
 // shared memory, from the index claimed during item k-1).  So no step of a
 // bucket waits on the queue, the list or the first loads of its runs.
-__global__ void __launch_bounds__(kJoinThreads)
-bucket_join_count_kernel(uint64_t *__restrict__ partL, const uint64_t *__restrict__ partR,
-                         const uint32_t *__restrict__ start, const uint32_t *__restrict__ cnt, uint32_t B,
-                         const uint32_t *__restrict__ bucket_win, WinAcc *__restrict__ acc, uint32_t cap,
+// kModels: the call has learned buckets (and no raw windows).
+template <bool kModels>
+__global__ void __launch_bounds__(kJoinThreads, 2)
+bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
+                         const WinPlan *__restrict__ wins, uint64_t *__restrict__ partL,
+                         uint64_t *__restrict__ partR, const uint32_t *__restrict__ start,
+                         const uint32_t *__restrict__ cnt, uint32_t B, WinAcc *__restrict__ acc, uint32_t cap,
                          uint32_t *queue, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn) {
     const uint32_t nitems = items ? *jn : B;
     uint32_t clean = 0;
-    auto join = [&](const JoinItem &ji) {
-        if (ji.direct && ji.nR + ji.nS <= kDirectMaxRun && join_count_direct(ji, partL, partR, acc, clean)) return;
-        join_count_bucket(ji, partL, partR, acc, cap);
+    auto join_as = [&](const JoinItem &ji, const JoinRuns &jr, auto raw_t) {
+        constexpr bool kRaw = decltype(raw_t)::value;
+        uint64_t e[kJoinPer];
+        if (kModels && (ji.flags & kItemModel)) {
+            join_count_bucket<kRaw, false>(ji, jr, e, false, acc, cap);
+        } else {
+            const KeyRange kr = build_head<kRaw>(ji, jr, e);
+            if (const uint32_t passes = direct_passes(ji, kr)) {
+                join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, acc, clean);
+                return;
+            }
+            join_count_bucket<kRaw, true>(ji, jr, e, true, acc, cap);
+        }
         clean = 0;
     };
+    auto join = [&](const JoinItem &ji) {
+        if (ji.nB == 0 || ji.nP == 0) return;
+        const JoinRuns jr = join_runs(ji, L, R, wins, partL, partR);
+        if (ji.flags & kItemHot) {
+            join_count_hot(static_cast<const uint64_t *>(jr.b), ji.nB, static_cast<const uint64_t *>(jr.p), ji.nP,
+                           jr.bside, &acc[ji.w], cap);
+            clean = 0;
+            return;
+        }
+        if constexpr (!kModels) {
+            if (ji.flags & kItemRaw) {
+                join_as(ji, jr, std::true_type{});
+                return;
+            }
+        }
+        join_as(ji, jr, std::false_type{});
+    };
     if (!queue || !items) {
-        if (blockIdx.x >= nitems) return;
+        for (uint32_t i = blockIdx.x; items && i < nitems; i += gridDim.x) {
+            SJBG_BARRIER();   // the previous item's shared-memory readers are done
+            join(items[i]);
+        }
+        if (items || blockIdx.x >= nitems) return;
         JoinItem ji;
-        if (items) {
-            ji = items[blockIdx.x];
-        } else {
-            const uint32_t i = blockIdx.x;
-            ji.b = i; ji.nR = cnt[i]; ji.nS = cnt[B + i]; ji.sR = start[i]; ji.sS = start[B + i];
-            ji.w = bucket_win[i]; ji.lg = 0; ji.direct = 0;
+        {
+            const uint32_t i = blockIdx.x, nL = cnt[i], nR = cnt[B + i];
+            const bool swap = nR < nL;
+            ji.nB = swap ? nR : nL; ji.nP = swap ? nL : nR;
+            ji.sB = swap ? start[B + i] : start[i]; ji.sP = swap ? start[i] : start[B + i];
+            ji.w = 0; ji.lg = wins[0].log2_buckets; ji.flags = swap ? kItemSwap : 0u; ji.pad = 0;
         }
         join(ji);
         return;
@@ -1441,12 +1786,13 @@ bucket_join_count_kernel(uint64_t *__restrict__ partL, const uint64_t *__restric
     __shared__ uint32_t cur_s, valid_s;   // slot of item k; bit q: slot (cur + q) % 3 holds an item
     uint32_t claim = 0;                   // thread 0: index claimed for item k+2
     if (threadIdx.x == 0) {
-        const uint32_t i0 = atomicAdd(queue, 1u), i1 = atomicAdd(queue, 1u);
+        // the first two items are the CTA's by position; the queue hands out the rest
+        const uint32_t i0 = blockIdx.x, i1 = gridDim.x + blockIdx.x;
+        claim = 2 * gridDim.x + atomicAdd(queue, 1u);
         if (i0 < nitems) slot_s[0] = items[i0];
         if (i1 < nitems) slot_s[1] = items[i1];
         cur_s = 0;
         valid_s = (i0 < nitems ? 1u : 0u) | (i1 < nitems ? 2u : 0u);
-        claim = atomicAdd(queue, 1u);
     }
     SJBG_BARRIER();
     while (valid_s & 1u) {
@@ -1456,9 +1802,11 @@ bucket_join_count_kernel(uint64_t *__restrict__ partL, const uint64_t *__restric
         uint32_t claim_next = 0;
         if (threadIdx.x == 0) {
             if (v & 2u) {   // item k+1: its runs into L2 while item k is joined
-                const JoinItem &nx = slot_s[c1];
-                l2_prefetch_bulk(partL + nx.sR, sizeof(uint64_t) * nx.nR);
-                l2_prefetch_bulk(partR + nx.sS, sizeof(uint64_t) * nx.nS);
+                const JoinItem nx = slot_s[c1];
+                const JoinRuns nr = join_runs(nx, L, R, wins, partL, partR);
+                const size_t word = (nx.flags & kItemRaw) ? sizeof(sjbg_tuple) : sizeof(uint64_t);
+                l2_prefetch_bulk(nr.b, word * nx.nB);
+                l2_prefetch_bulk(nr.p, word * nx.nP);
             }
             if (claim < nitems) {   // item k+2's record: shared memory, without blocking
                 const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&slot_s[c2]);
@@ -1469,7 +1817,7 @@ bucket_join_count_kernel(uint64_t *__restrict__ partL, const uint64_t *__restric
                              "l"(reinterpret_cast<const uint8_t *>(src) + 16)
                              : "memory");
             }
-            claim_next = atomicAdd(queue, 1u);   // read after this item's join
+            claim_next = 2 * gridDim.x + atomicAdd(queue, 1u);   // read after this item's join
         }
         join(ji);
         if (threadIdx.x == 0) {
@@ -1482,29 +1830,12 @@ bucket_join_count_kernel(uint64_t *__restrict__ partL, const uint64_t *__restric
     }
 }
 
+// One CTA per join item (the grid covers the longest possible list).
 __global__ void __launch_bounds__(kJoinThreads)
 bucket_join_enum_kernel(const uint64_t *__restrict__ partL, const uint64_t *__restrict__ partR,
-                        const uint32_t *__restrict__ start, const uint32_t *__restrict__ cnt, uint32_t B,
-                        const uint32_t *__restrict__ bucket_win, WinAcc *__restrict__ acc,
-                        const WinPlan *__restrict__ wins, sjbg_pair *__restrict__ pairs, uint32_t table_bits,
-                        uint32_t *queue, const JoinItem *__restrict__ jitems, const uint32_t *__restrict__ jn) {
-    const uint32_t items = jitems ? *jn : B;
-    if (!queue) {
-        if (blockIdx.x < items)
-            join_enum_bucket(jitems ? jitems[blockIdx.x].b : blockIdx.x, partL, partR, start, cnt, B, bucket_win,
-                             acc, wins, pairs, table_bits);
-        return;
-    }
-    __shared__ uint32_t item_s;
-    for (;;) {
-        SJBG_BARRIER();
-        if (threadIdx.x == 0) item_s = atomicAdd(queue, 1u);
-        SJBG_BARRIER();
-        const uint32_t it = item_s;
-        if (it >= items) break;
-        join_enum_bucket(jitems ? jitems[it].b : it, partL, partR, start, cnt, B, bucket_win, acc, wins, pairs,
-                         table_bits);
-    }
+                        WinAcc *__restrict__ acc, const WinPlan *__restrict__ wins, sjbg_pair *__restrict__ pairs,
+                        uint32_t table_bits, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn) {
+    if (blockIdx.x < *jn) join_enum_bucket(items[blockIdx.x], partL, partR, acc, wins, pairs, table_bits);
 }
 
 // ------------------------------------------------------------------ host driver
@@ -1539,8 +1870,11 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     }
     const bool learned = part == SJBG_PART_LEARNED;
     if (part_used) *part_used = learned ? SJBG_PART_LEARNED : SJBG_PART_RADIX;
-    // left tuples per bucket: 2048 when chains are built, else the tuned target
+    // build tuples per bucket: 2048 when chains are built, else the tuned target
     const uint64_t target = enumerate ? 2048 : h->tune.bucket_target;
+    // slots of a count table (a target whose table would not fit is joined in passes)
+    const uint32_t cap = (uint32_t)std::min<size_t>(
+        count_table_cap((uint32_t)target), (h->max_smem_optin - count_table_bytes(0) - 1024) / 16);
 
     // ---- plan
     std::vector<WinPlan> plan(n);
@@ -1548,28 +1882,35 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     std::vector<uint32_t> pbL(n + 1), pbR(n + 1);   // window bases in the partitioned arrays
     uint64_t B = 0, totL = 0, totR = 0;
     uint32_t maxP = 1;
-    bool any_two = false, any_one = false;
+    bool any_two = false, any_one = false, any_raw = false;
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &wh = wins[w];
         WinPlan &p = plan[w];
         p.left_off = wh.left_off; p.n_left = wh.n_left; p.right_off = wh.right_off; p.n_right = wh.n_right;
         p.pairs_off = wh.pairs_off; p.pairs_cap = dPairs ? wh.pairs_cap : 0;
+        // a counting join builds from the smaller side of a bucket, so the fan-out
+        // follows the window's smaller side
+        const uint64_t build = enumerate ? wh.n_left : std::min(wh.n_left, wh.n_right);
         uint32_t lg;
         if (learned) lg = learned_log2_buckets(h, wh.n_left);
         else if (h->cfg.radix_bits) lg = h->cfg.radix_bits;
-        else lg = ceil_log2((wh.n_left + target - 1) / target);
+        else lg = ceil_log2((build + target - 1) / target);
         lg = std::min(lg, kMaxBucketsLog2);
         if (wh.n_left == 0 || wh.n_right == 0) lg = 0;
+        // (a handle that names radix partitioning gets it for every window)
+        p.raw = h->cfg.partitioner == SJBG_PART_AUTO && !enumerate && lg == 0 && build < cap ? 1u : 0u;
         p.log2_buckets = lg;
         p.bucket_base = (uint32_t)B;
         p.model = 0xFFFFFFFFu;
         p.two_level = lg >= kTwoLevelMinLog2 ? 1u : 0u;
         any_two |= p.two_level != 0;
-        any_one |= p.two_level == 0;
+        any_one |= p.two_level == 0 && !p.raw;
+        any_raw |= p.raw != 0;
         B += 1ull << lg;
         maxP = std::max(maxP, 1u << lg);
-        tileL[w + 1] = tileL[w] + (uint32_t)((wh.n_left + kTile - 1) / kTile);
-        tileR[w + 1] = tileR[w] + (uint32_t)((wh.n_right + kTile - 1) / kTile);
+        // (no tile of an unpartitioned window is counted or scattered)
+        tileL[w + 1] = tileL[w] + (p.raw ? 0u : (uint32_t)((wh.n_left + kTile - 1) / kTile));
+        tileR[w + 1] = tileR[w] + (p.raw ? 0u : (uint32_t)((wh.n_right + kTile - 1) / kTile));
         // fine-pass CTAs: coarse partitions x groups of kGroupTiles tiles
         const uint32_t nc = 1u << coarse_bits(lg);
         itL[w + 1] = itL[w] + nc * ((tileL[w + 1] - tileL[w] + kGroupTiles - 1) / kGroupTiles);
@@ -1581,11 +1922,17 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     }
     if (B > 0xFFFFFFFFull / 4 || totL >= 0xFFFFFFFFull || totR >= 0xFFFFFFFFull)
         return fail(h, SJBG_E_CAPACITY, "hash join batch exceeds 2^32 tuples per side");
-    // counting CTAs per window side: shares of about T / (resident CTAs) tiles
-    // (at least kHistTiles), so that one wave holds the call when its window
-    // sides are large and the set-up of each CTA is paid over many tiles.
+    // counting CTAs per window side: shares of about T / (resident CTAs) tiles,
+    // so that one wave holds the call when its window sides are large and the
+    // set-up of each CTA is paid over many tiles.  A share has at least
+    // kHistTiles tiles with a model (whose copy and heavy-key sums each CTA sets
+    // up), and for radix windows at least as many as make flushing the P
+    // counters cheap (2, or P / 256): a call of few tiles otherwise leaves most
+    // SMs idle (one window of 2^20 tuples per side, 490 tiles: 32 CTAs of 16
+    // tiles took 17.5 us).
     // When many sides are smaller than a share (uneven batches), shares of an
     // eighth of that keep the CTAs small enough to balance the SMs.
+    uint32_t join_chunk;
     {
         const size_t histSmem = sizeof(uint32_t) * ((maxP + 1) / 2 * 2) + sizeof(uint64_t) * kTile;
         allow_big_smem(part_hist_kernel, histSmem);
@@ -1595,24 +1942,30 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             return fail(h, SJBG_E_CUDA, "counting pass occupancy");
         const uint64_t slots = (uint64_t)std::max(per_sm, 1) * (uint64_t)std::max(h->num_sms, 1);
         const uint64_t T = (uint64_t)tileL[n] + tileR[n];
-        uint64_t share = std::max<uint64_t>(kHistTiles, (T + slots - 1) / slots);
+        const uint64_t least = learned ? kHistTiles : std::max<uint64_t>(2, maxP / 256);
+        uint64_t share = std::max<uint64_t>(least, (T + slots - 1) / slots);
         uint64_t ctas = 0;
         for (uint32_t w = 0; w < n; w++)
             ctas += (tileL[w + 1] - tileL[w] + share - 1) / share + (tileR[w + 1] - tileR[w] + share - 1) / share;
-        if (ctas > slots + slots / 8) share = std::max<uint64_t>(kHistTiles, T / (8 * slots));
+        if (ctas > slots + slots / 8) share = std::max<uint64_t>(least, T / (8 * slots));
         for (uint32_t w = 0; w < n; w++) {
             hgL[w + 1] = hgL[w] + (uint32_t)((tileL[w + 1] - tileL[w] + share - 1) / share);
             hgR[w + 1] = hgR[w] + (uint32_t)((tileR[w + 1] - tileR[w] + share - 1) / share);
         }
+        // probe tuples per join piece: small enough to spread a call over the SMs, at most kJoinChunk
+        // (chains cost more to build: with pieces of 4,000 probes the enumerating
+        // join of 500,009 and 2,000,003 tuples took 78 us, against 66)
+        join_chunk = (uint32_t)std::min<uint64_t>(
+            kJoinChunk, std::max<uint64_t>(enumerate ? kJoinChunkEnum : kJoinChunkMin,
+                                           (totL + totR) / (4 * (uint64_t)std::max(h->num_sms, 1))));
     }
-    std::vector<uint32_t> bwin(B);
-    for (uint32_t w = 0; w < n; w++)
-        for (uint32_t k = 0; k < (1u << plan[w].log2_buckets); k++) bwin[plan[w].bucket_base + k] = w;
+    const uint64_t max_items = join_items_bound(B, totL + totR, join_chunk, enumerate ? 0x0FFFFFFFu : cap);
+    if (max_items > 0x7FFFFFFFull) return fail(h, SJBG_E_CAPACITY, "hash join batch has too many join items");
 
-    // ---- upload plan, tile prefixes, bucket->window map and (learned) the
+    // ---- upload plan, tile prefixes and (learned) the
     // sampling plan in one copy
-    const size_t planB = sizeof(WinPlan) * n, tileB = sizeof(uint32_t) * (n + 1), bwB = sizeof(uint32_t) * B;
-    const size_t lsOff = (planB + 8 * tileB + bwB + 15) & ~(size_t)15;
+    const size_t planB = sizeof(WinPlan) * n, tileB = sizeof(uint32_t) * (n + 1);
+    const size_t lsOff = (planB + 8 * tileB + 15) & ~(size_t)15;
     const size_t upB = lsOff + (learned ? learned_stage_bytes(n) : 0);
     uint8_t *hst = static_cast<uint8_t *>(pinned_get(h, 0, upB));
     uint8_t *dev = static_cast<uint8_t *>(ws_get(h, WS_WIN_PLAN, upB));
@@ -1626,7 +1979,6 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     std::memcpy(hst + planB + 5 * tileB, itR.data(), tileB);
     std::memcpy(hst + planB + 6 * tileB, pbL.data(), tileB);
     std::memcpy(hst + planB + 7 * tileB, pbR.data(), tileB);
-    std::memcpy(hst + planB + 8 * tileB, bwin.data(), bwB);
     LearnedStage lst{};
     if (learned) lst = learned_stage(h, plan.data(), n, hst + lsOff);
     // the bucket counters are zeroed by the same launch as the upload
@@ -1642,7 +1994,6 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     const uint32_t *dItR = reinterpret_cast<const uint32_t *>(dev + planB + 5 * tileB);
     const uint32_t *dPbL = reinterpret_cast<const uint32_t *>(dev + planB + 6 * tileB);
     const uint32_t *dPbR = reinterpret_cast<const uint32_t *>(dev + planB + 7 * tileB);
-    const uint32_t *dBwin = reinterpret_cast<const uint32_t *>(dev + planB + 8 * tileB);
 
     uint32_t *dStart = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_START, sizeof(uint32_t) * 2 * B));
     uint32_t *dCur = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_CURSOR, sizeof(uint32_t) * 2 * B));
@@ -1668,16 +2019,22 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     // per window side its compacted light tuples, then the join list's length
     uint32_t *dCcnt = static_cast<uint32_t *>(ws_get(h, WS_COMPACT_CNT, sizeof(uint32_t) * (2 * n + 1)));
     uint32_t *dJn = dCcnt + 2 * n;
-    // the passes' work prefixes (6 arrays of n + 1), then (16-byte aligned) the join list (B items)
+    // the passes' work prefixes (6 arrays of n + 1), then (16-byte aligned) the join list
     const size_t workWords = (6 * (size_t)(n + 1) + 3) & ~(size_t)3;
     uint32_t *dWork = static_cast<uint32_t *>(
-        ws_get(h, WS_TILE_PREFIX, sizeof(uint32_t) * workWords + sizeof(JoinItem) * (size_t)std::max<uint64_t>(B, 1)));
+        ws_get(h, WS_TILE_PREFIX, sizeof(uint32_t) * workWords + sizeof(JoinItem) * (size_t)max_items));
     JoinItem *dJlist = dWork ? reinterpret_cast<JoinItem *>(dWork + workWords) : nullptr;
     if (!dComp || !dRows || !dCcnt || !dWork) return fail(h, SJBG_E_NOMEM, "partition staging buffers");
     SJBG_CK(h, cudaMemsetAsync(dCcnt, 0, sizeof(uint32_t) * (2 * n + 1), h->stream));
     uint64_t *dCompR = dComp + (uint64_t)kTile * tileL[n];
 
     const uint32_t tiles = tileL[n] + tileR[n];
+    auto scan = [&]() {
+        return launch(h, "part_scan", part_scan_win_kernel, dim3(n), dim3(1024), 0, (const WinPlan *)dPlan, dPbL, dPbR,
+                      (const uint32_t *)dCnt, dStart, dCur, (uint32_t)B, dModels, dJlist, dJn, join_chunk,
+                      enumerate ? 0x0FFFFFFFu : cap, !enumerate);
+    };
+    if (!tiles && any_raw) SJBG_CK(h, scan());
     if (tiles) {
         const size_t histSmem = sizeof(uint32_t) * ((maxP + 1) / 2 * 2) + sizeof(uint64_t) * kTile;
         SJBG_CK(h, launch(h, "part_hist", part_hist_kernel, dim3(hgL[n] + hgR[n]), dim3(kPartThreads), histSmem, dL,
@@ -1697,8 +2054,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
                               (const uint32_t *)dWork, dCnt, (uint32_t)B, dModels, (const uint64_t *)dComp,
                               (const uint64_t *)dCompR, (const uint32_t *)dCcnt));
         }
-        SJBG_CK(h, launch(h, "part_scan", part_scan_win_kernel, dim3(n), dim3(1024), 0, (const WinPlan *)dPlan, dPbL,
-                          dPbR, (const uint32_t *)dCnt, dStart, dCur, (uint32_t)B, dModels, dJlist, dJn));
+        SJBG_CK(h, scan());
         // single-level windows, and compacted windows (their packed light tuples):
         // a local counting sort per tile
         if (any_one || (learned && !enumerate)) {
@@ -1722,35 +2078,31 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
                               (const uint32_t *)dRows));
         }
     }
-    // persistent CTAs draining a work queue of buckets, or one CTA per bucket
+    // persistent CTAs draining a work queue of join items, or about one CTA per item
     uint32_t *queue = nullptr;
-    dim3 jgrid((uint32_t)B);
-    // (chain-building joins keep one CTA per bucket)
-    if (!enumerate && h->tune.persistent_join && B > (uint64_t)h->num_sms) {
-        queue = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_WIN, 64));
-        if (!queue) return fail(h, SJBG_E_NOMEM, "work queue");
-        SJBG_CK(h, cudaMemsetAsync(queue, 0, 4, h->stream));
-        jgrid = dim3((uint32_t)std::min<uint64_t>(B, (uint64_t)h->num_sms));
-    }
-    if (enumerate) {
+    dim3 jgrid((uint32_t)std::min<uint64_t>(max_items, B + (totL + totR) / join_chunk));
+    if (enumerate) {   // (chain-building joins: one CTA per item)
         const uint32_t bits = 13;   // 8192 slots for chunks of 4096
         const size_t smem = sizeof(uint32_t) * (2 * ((1u << bits) + 1) + 2 * kEnumChunk);
         allow_big_smem(bucket_join_enum_kernel, smem);
         SJBG_CK(h, launch(h, "bucket_join_enum", bucket_join_enum_kernel, jgrid, dim3(kJoinThreads), smem,
-                          dPL, dPR, dStart, dCnt, (uint32_t)B, dBwin, acc, dPlan, dPairs, bits, queue,
+                          (const uint64_t *)dPL, (const uint64_t *)dPR, acc, (const WinPlan *)dPlan, dPairs, bits,
                           (const JoinItem *)dJlist, (const uint32_t *)dJn));
     } else {
-        const uint32_t cap = count_table_cap((uint32_t)target);
-        const size_t smem =
-            std::max((sizeof(unsigned long long) + 2 * sizeof(uint32_t)) * (cap + 1) + 16, kDirectBytes);
-        allow_big_smem(bucket_join_count_kernel, smem);
-        if (queue) {   // as many persistent CTAs as fit on an SM at this table size (at most 2 by registers)
+        const size_t smem = std::max(count_table_bytes(cap), kDirectBytes);
+        auto join = learned ? bucket_join_count_kernel<true> : bucket_join_count_kernel<false>;
+        allow_big_smem(join, smem);
+        if (h->tune.persistent_join && max_items > (uint64_t)h->num_sms) {
+            queue = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_WIN, 64));
+            if (!queue) return fail(h, SJBG_E_NOMEM, "work queue");
+            SJBG_CK(h, cudaMemsetAsync(queue, 0, 4, h->stream));
+            // as many persistent CTAs as fit on an SM at this table size (at most 2 by registers)
             const uint32_t per_sm = std::max<uint32_t>(1, (uint32_t)((228u << 10) / (smem + 1024)));
-            jgrid = dim3((uint32_t)std::min<uint64_t>(B, (uint64_t)h->num_sms * std::min<uint32_t>(per_sm, 2u)));
+            jgrid = dim3((uint32_t)std::min<uint64_t>(max_items, (uint64_t)h->num_sms * std::min<uint32_t>(per_sm, 2u)));
         }
-        SJBG_CK(h, launch(h, "bucket_join_count", bucket_join_count_kernel, jgrid, dim3(kJoinThreads), smem,
-                          dPL, dPR, dStart, dCnt, (uint32_t)B, dBwin, acc, cap, queue, (const JoinItem *)dJlist,
-                          (const uint32_t *)dJn));
+        SJBG_CK(h, launch(h, "bucket_join_count", join, jgrid, dim3(kJoinThreads), smem, dL, dR,
+                          (const WinPlan *)dPlan, dPL, dPR, (const uint32_t *)dStart, (const uint32_t *)dCnt,
+                          (uint32_t)B, acc, cap, queue, (const JoinItem *)dJlist, (const uint32_t *)dJn));
     }
     return SJBG_OK;
 }
@@ -1768,11 +2120,11 @@ struct RawScratch {
 };
 
 // Byte offsets of the scratch buffers from a 256-byte aligned base: the
-// RawScratch record, the bucket arrays (bucket_win P words, counts, starts and
-// cursors 2P words each) and the partitioned sides (8 bytes per tuple).  The
+// RawScratch record, the bucket arrays (counts, starts and cursors, 2P words
+// each) and the partitioned sides (8 bytes per tuple).  The
 // size check of the entry point and the carving below both use it.
 struct RawLayout {
-    size_t rs, bwin, part_left, part_right, end;
+    size_t rs, cnt, part_left, part_right, end;
 };
 
 static size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -1780,8 +2132,8 @@ static size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 static RawLayout raw_layout(uint64_t nL, uint64_t nR, uint32_t P) {
     RawLayout l;
     l.rs = 0;
-    l.bwin = round256(sizeof(RawScratch));
-    l.part_left = l.bwin + round256(sizeof(uint32_t) * 7 * (size_t)P);
+    l.cnt = round256(sizeof(RawScratch));
+    l.part_left = l.cnt + round256(sizeof(uint32_t) * 6 * (size_t)P);
     l.part_right = l.part_left + sizeof(uint64_t) * std::max<uint64_t>(nL, 1);
     l.end = l.part_right + sizeof(uint64_t) * std::max<uint64_t>(nR, 1);
     return l;
@@ -1794,13 +2146,13 @@ static uint32_t raw_log2_buckets(uint64_t nL, uint64_t nR) {
     return (nL == 0 || nR == 0) ? 0 : lg;
 }
 
-__global__ void raw_setup_kernel(RawScratch *rs, uint32_t *bucket_win, uint32_t *cnt, uint32_t P, uint64_t nL,
-                                 uint64_t nR, uint32_t lg, uint32_t tL, uint32_t tR) {
+__global__ void raw_setup_kernel(RawScratch *rs, uint32_t *cnt, uint32_t P, uint64_t nL, uint64_t nR, uint32_t lg,
+                                 uint32_t tL, uint32_t tR) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         WinPlan &p = rs->plan;
         p.left_off = 0; p.n_left = nL; p.right_off = 0; p.n_right = nR;
         p.pairs_off = 0; p.pairs_cap = 0;
-        p.bucket_base = 0; p.log2_buckets = lg; p.model = 0xFFFFFFFFu; p.two_level = 0;
+        p.bucket_base = 0; p.log2_buckets = lg; p.model = 0xFFFFFFFFu; p.two_level = 0; p.raw = 0;
         rs->tile[0] = 0; rs->tile[1] = tL;
         rs->tile[2] = 0; rs->tile[3] = tR;
         rs->tile[4] = 0; rs->tile[5] = (tL + kHistTiles - 1) / kHistTiles;
@@ -1808,10 +2160,7 @@ __global__ void raw_setup_kernel(RawScratch *rs, uint32_t *bucket_win, uint32_t 
         rs->acc[0] = WinAcc{0, 0, 0, 0, 0};
         rs->acc[1] = WinAcc{0, 0, 0, 0, 0};
     }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * P; i += gridDim.x * blockDim.x) {
-        cnt[i] = 0;
-        if (i < P) bucket_win[i] = 0;
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * P; i += gridDim.x * blockDim.x) cnt[i] = 0;
 }
 
 // The window's result, with the device status word turned into a status code
@@ -1851,8 +2200,7 @@ int hj_count_window_raw(const sjbg_tuple *dL, uint64_t nL, const sjbg_tuple *dR,
     if (base + lay.end > sc + sc_bytes)
         return fail(nullptr, SJBG_E_CAPACITY, "sjbg_lazy_hj_noalloc: the window does not fit the fixed scratch");
     RawScratch *rs = reinterpret_cast<RawScratch *>(base + lay.rs);
-    uint32_t *bwin = reinterpret_cast<uint32_t *>(base + lay.bwin);
-    uint32_t *cnt = bwin + P;
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(base + lay.cnt);
     uint32_t *start = cnt + 2 * P;
     uint32_t *cur = start + 2 * P;
     uint64_t *pL = reinterpret_cast<uint64_t *>(base + lay.part_left);
@@ -1863,7 +2211,7 @@ int hj_count_window_raw(const sjbg_tuple *dL, uint64_t nL, const sjbg_tuple *dR,
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? SJBG_OK : cuda_fail(nullptr, e, what);
     };
-    raw_setup_kernel<<<4, 256, 0, st>>>(rs, bwin, cnt, P, nL, nR, lg, tL, tR);
+    raw_setup_kernel<<<4, 256, 0, st>>>(rs, cnt, P, nL, nR, lg, tL, tR);
     if (int rc = launched("sjbg_lazy_hj_noalloc: raw_setup_kernel")) return rc;
     const uint32_t *tl = rs->tile;
     if (tL && tR) {
@@ -1883,10 +2231,10 @@ int hj_count_window_raw(const sjbg_tuple *dL, uint64_t nL, const sjbg_tuple *dR,
                                                                           nullptr);
         if (int rc = launched("sjbg_lazy_hj_noalloc: part_scatter_kernel")) return rc;
         const uint32_t cap = count_table_cap(4096);
-        const size_t smem = (sizeof(unsigned long long) + 2 * sizeof(uint32_t)) * (cap + 1) + 16;
-        allow_big_smem(bucket_join_count_kernel, smem);
-        bucket_join_count_kernel<<<P, kJoinThreads, smem, st>>>(pL, pR, start, cnt, P, bwin, rs->acc, cap, nullptr,
-                                                                nullptr, nullptr);
+        const size_t smem = std::max(count_table_bytes(cap), kDirectBytes);
+        allow_big_smem(bucket_join_count_kernel<false>, smem);
+        bucket_join_count_kernel<false><<<P, kJoinThreads, smem, st>>>(dL, dR, &rs->plan, pL, pR, start, cnt, P, rs->acc,
+                                                                cap, nullptr, nullptr, nullptr);
         if (int rc = launched("sjbg_lazy_hj_noalloc: bucket_join_count_kernel")) return rc;
     }
     raw_finish_kernel<<<1, 32, 0, st>>>(rs, dOut);
