@@ -46,18 +46,27 @@ EagerState::~EagerState() {
 template <bool kEnum, bool kPairs>
 __global__ void __launch_bounds__(256)
 eager_hj_kernel(const sjbg_tuple *__restrict__ batch, uint32_t n, uint32_t base, int side, ETab own, ETab oth,
-                const sjbg_tuple *__restrict__ oth_tuples, uint32_t oth_n, WinAcc *acc, unsigned long long *bcount,
-                sjbg_pair *__restrict__ pairs, uint64_t pcap) {
+                sjbg_tuple *__restrict__ store, const sjbg_tuple *__restrict__ oth_tuples, uint32_t oth_n, WinAcc *acc,
+                BatchCount bc, sjbg_pair *__restrict__ pairs, uint64_t pcap) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
     uint32_t key = 0, val = 0;
     if (valid) {
-        const uint2 t = *reinterpret_cast<const uint2 *>(batch + i);
-        key = t.x;
-        val = t.y;
+        if (kEnum || kPairs) {   // the chains index the side's tuple store
+            const uint4 t = *reinterpret_cast<const uint4 *>(batch + i);
+            *reinterpret_cast<uint4 *>(store + base + i) = t;
+            key = t.x;
+            val = t.y;
+        } else {
+            const uint2 t = *reinterpret_cast<const uint2 *>(batch + i);
+            key = t.x;
+            val = t.y;
+        }
     }
-    eager_hj_step<kEnum, kPairs>(valid, key, val, base + i, side, own, oth, oth_tuples, oth_n, acc, bcount, pairs,
-                                 pcap);
+    unsigned long long count = 0, xr = 0, prod = 0;
+    eager_hj_step<kEnum, kPairs>(valid, key, val, base + i, side, own, oth, oth_tuples, oth_n, acc, pairs, pcap, count,
+                                 xr, prod);
+    publish_batch(bc, acc, count, xr, prod);
 }
 
 // ---------------------------------------------------------------- sort-merge join
@@ -100,7 +109,7 @@ template <bool kEnum, bool kPairs>
 __global__ void __launch_bounds__(256)
 eager_smj_probe_kernel(const uint32_t *__restrict__ bkeys, const uint32_t *__restrict__ bvals, uint32_t n, int side,
                        const uint32_t *__restrict__ okeys, const uint32_t *__restrict__ ovals,
-                       const unsigned long long *__restrict__ oF, uint32_t on, WinAcc *acc, unsigned long long *bcount,
+                       const unsigned long long *__restrict__ oF, uint32_t on, WinAcc *acc, BatchCount bc,
                        sjbg_pair *__restrict__ pairs, uint64_t pcap) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t lo = 0, hi = 0, val = 0;
@@ -126,7 +135,7 @@ eager_smj_probe_kernel(const uint32_t *__restrict__ bkeys, const uint32_t *__res
         for (uint32_t a = lo; a < hi; a++, b++)
             if (b < pcap) pairs[b] = side == 0 ? sjbg_pair{val, ovals[a]} : sjbg_pair{ovals[a], val};
     }
-    flush_batch(acc, bcount, count, xr, prod);
+    publish_batch(bc, acc, count, xr, prod);
 }
 
 // Merge the sorted run A (na) with the sorted batch B (nb) into out: equal
@@ -270,6 +279,7 @@ static int eager_clear(sjbg_handle *h);
 int eager_init_and_clear(sjbg_handle *h) {
     int rc = eager_init(h);
     if (rc) return rc;
+    SJBG_CK(h, cudaMemsetAsync(h->eager->batch_count, 0, 64, h->stream));   // then zero between batches
     rc = eager_clear(h);
     if (rc) return rc;
     SJBG_CK(h, cudaStreamSynchronize(h->stream));
@@ -299,9 +309,37 @@ static int eager_clear(sjbg_handle *h) {
     return SJBG_OK;
 }
 
-// Enqueue one batch (no synchronisation); its matches are added to *count_slot.
+// The address at which kernels may read a caller's batch in place, or null: a
+// 16-byte aligned device batch, or a host batch in pinned memory or, where the
+// device reads pageable host memory coherently, in any.  (The call waits for
+// its kernels, so the batch stays unchanged while they read it.)
+static const sjbg_tuple *batch_in_place(sjbg_handle *h, const sjbg_tuple *batch, bool from_host) {
+    if (reinterpret_cast<uintptr_t>(batch) & 15u) return nullptr;
+    if (!from_host) return batch;
+    EagerState &st = *h->eager;
+    if (st.host_direct < 0) {
+        int pageable = 0;
+        if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, h->device) != cudaSuccess) {
+            cudaGetLastError();
+            pageable = 0;
+        }
+        st.host_direct = pageable;
+    }
+    if (st.host_direct) return batch;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, batch) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
+        return static_cast<const sjbg_tuple *>(at.devicePointer);
+    cudaGetLastError();
+    return nullptr;
+}
+
+// Enqueue one batch (no synchronisation); its matches go to *host_count (mapped
+// pinned memory, zeroed by the caller).  The hash and sort-merge joins read the
+// batch where it lies, and their last CTA writes the count, so a batch is the
+// join's launches and nothing else: with a memset, a copy in and a copy out
+// around the one kernel of the hash join, a batch of 4,096 took 30 us.
 static int eager_enqueue(sjbg_handle *h, const sjbg_tuple *batch, uint64_t n, int side, bool from_host,
-                         unsigned long long *count_slot) {
+                         unsigned long long *host_count) {
     EagerState &st = *h->eager;
     EagerSide &S = st.side[side];
     EagerSide &O = st.side[1 - side];
@@ -310,8 +348,14 @@ static int eager_enqueue(sjbg_handle *h, const sjbg_tuple *batch, uint64_t n, in
     if (h->cfg.algorithm == SJBG_ALG_SMJ && n > kEagerMaxSortBatch)
         return fail(h, SJBG_E_UNSUPPORTED, "eager sort-merge batches are limited to 8192 tuples");
     sjbg_tuple *dst = S.tuples + S.n;
-    SJBG_CK(h, cudaMemcpyAsync(dst, batch, sizeof(sjbg_tuple) * n,
-                               from_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, h->stream));
+    const sjbg_tuple *src = h->cfg.algorithm == SJBG_ALG_NLJ ? nullptr : batch_in_place(h, batch, from_host);
+    if (!src) {
+        SJBG_CK(h, cudaMemcpyAsync(dst, batch, sizeof(sjbg_tuple) * n,
+                                   from_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, h->stream));
+        src = dst;
+    }
+    const BatchCount bc{st.batch_count, host_count,
+                        (double)n * (double)O.n >= (double)(1ull << kCountBits) || (n + 255) / 256 >= (1u << 16) - 1};
     const bool en = eager_enumerates(h);
     sjbg_pair *pairs = st.pairs;
     const uint32_t blocks = (uint32_t)((n + 255) / 256);
@@ -321,8 +365,11 @@ static int eager_enqueue(sjbg_handle *h, const sjbg_tuple *batch, uint64_t n, in
             const sjbg_tuple *L = side == 0 ? dst : Ls.tuples;
             const sjbg_tuple *R = side == 0 ? Rs.tuples : dst;
             const uint64_t nl = side == 0 ? n : Ls.n, nr = side == 0 ? Rs.n : n;
-            int rc = nlj_pair_launch(h, L, nl, R, nr, st.acc, count_slot, pairs, st.pairs_cap, en);
+            // (compared from the stores; the count is copied out and its slot zeroed again)
+            int rc = nlj_pair_launch(h, L, nl, R, nr, st.acc, st.batch_count, pairs, st.pairs_cap, en);
             if (rc) return rc;
+            SJBG_CK(h, cudaMemcpyAsync(host_count, st.batch_count, 8, cudaMemcpyDeviceToHost, h->stream));
+            SJBG_CK(h, cudaMemsetAsync(st.batch_count, 0, 8, h->stream));
             break;
         }
         case SJBG_ALG_HJ: {
@@ -330,19 +377,16 @@ static int eager_enqueue(sjbg_handle *h, const sjbg_tuple *batch, uint64_t n, in
             const ETab oth{O.tkeys, O.tcnt, O.thead, O.next, O.tsum, st.table_bits};
             if (pairs)
                 SJBG_CK(h, launch(h, "eager_hj_pairs", eager_hj_kernel<true, true>, dim3(blocks), dim3(256), 0,
-                                  (const sjbg_tuple *)dst, (uint32_t)n, (uint32_t)S.n, side, own, oth,
-                                  (const sjbg_tuple *)O.tuples, (uint32_t)O.n, st.acc, count_slot, pairs,
-                                  st.pairs_cap));
+                                  src, (uint32_t)n, (uint32_t)S.n, side, own, oth, S.tuples,
+                                  (const sjbg_tuple *)O.tuples, (uint32_t)O.n, st.acc, bc, pairs, st.pairs_cap));
             else if (en)
                 SJBG_CK(h, launch(h, "eager_hj_xor", eager_hj_kernel<true, false>, dim3(blocks), dim3(256), 0,
-                                  (const sjbg_tuple *)dst, (uint32_t)n, (uint32_t)S.n, side, own, oth,
-                                  (const sjbg_tuple *)O.tuples, (uint32_t)O.n, st.acc, count_slot, pairs,
-                                  st.pairs_cap));
+                                  src, (uint32_t)n, (uint32_t)S.n, side, own, oth, S.tuples,
+                                  (const sjbg_tuple *)O.tuples, (uint32_t)O.n, st.acc, bc, pairs, st.pairs_cap));
             else
                 SJBG_CK(h, launch(h, "eager_hj_count", eager_hj_kernel<false, false>, dim3(blocks), dim3(256), 0,
-                                  (const sjbg_tuple *)dst, (uint32_t)n, (uint32_t)S.n, side, own, oth,
-                                  (const sjbg_tuple *)O.tuples, (uint32_t)O.n, st.acc, count_slot, pairs,
-                                  st.pairs_cap));
+                                  src, (uint32_t)n, (uint32_t)S.n, side, own, oth, S.tuples,
+                                  (const sjbg_tuple *)O.tuples, (uint32_t)O.n, st.acc, bc, pairs, st.pairs_cap));
             break;
         }
         case SJBG_ALG_SMJ: {
@@ -351,25 +395,22 @@ static int eager_enqueue(sjbg_handle *h, const sjbg_tuple *batch, uint64_t n, in
             while (P < n) P <<= 1;
             allow_big_smem(eager_sort_batch_kernel, sizeof(unsigned long long) * kEagerMaxSortBatch);
             SJBG_CK(h, launch(h, "eager_sort_batch", eager_sort_batch_kernel, dim3(1), dim3(1024),
-                              sizeof(unsigned long long) * P, (const sjbg_tuple *)dst, (uint32_t)n, bk, bv));
+                              sizeof(unsigned long long) * P, src, (uint32_t)n, bk, bv));
             if (pairs)
                 SJBG_CK(h, launch(h, "eager_smj_probe_pairs", eager_smj_probe_kernel<true, true>, dim3(blocks),
                                   dim3(256), 0, (const uint32_t *)bk, (const uint32_t *)bv, (uint32_t)n, side,
                                   (const uint32_t *)O.skeys, (const uint32_t *)O.svals,
-                                  (const unsigned long long *)O.F, (uint32_t)O.n, st.acc, count_slot, pairs,
-                                  st.pairs_cap));
+                                  (const unsigned long long *)O.F, (uint32_t)O.n, st.acc, bc, pairs, st.pairs_cap));
             else if (en)
                 SJBG_CK(h, launch(h, "eager_smj_probe_xor", eager_smj_probe_kernel<true, false>, dim3(blocks),
                                   dim3(256), 0, (const uint32_t *)bk, (const uint32_t *)bv, (uint32_t)n, side,
                                   (const uint32_t *)O.skeys, (const uint32_t *)O.svals,
-                                  (const unsigned long long *)O.F, (uint32_t)O.n, st.acc, count_slot, pairs,
-                                  st.pairs_cap));
+                                  (const unsigned long long *)O.F, (uint32_t)O.n, st.acc, bc, pairs, st.pairs_cap));
             else
                 SJBG_CK(h, launch(h, "eager_smj_probe_count", eager_smj_probe_kernel<false, false>, dim3(blocks),
                                   dim3(256), 0, (const uint32_t *)bk, (const uint32_t *)bv, (uint32_t)n, side,
                                   (const uint32_t *)O.skeys, (const uint32_t *)O.svals,
-                                  (const unsigned long long *)O.F, (uint32_t)O.n, st.acc, count_slot, pairs,
-                                  st.pairs_cap));
+                                  (const unsigned long long *)O.F, (uint32_t)O.n, st.acc, bc, pairs, st.pairs_cap));
             const uint32_t nt = (uint32_t)(S.n + n);
             SJBG_CK(h, launch(h, "eager_merge", eager_merge_kernel, dim3((nt + 255) / 256), dim3(256), 0,
                               (const uint32_t *)S.skeys, (const uint32_t *)S.svals, (uint32_t)S.n,
@@ -434,13 +475,11 @@ int sjbg_eager_execute(sjbg_handle *h, const sjbg_tuple *batch, uint64_t n, int 
     if (rc) return rc;
     if ((n && !batch) || (mem != SJBG_MEM_HOST && mem != SJBG_MEM_DEVICE)) return fail(h, SJBG_E_INVALID, "bad batch");
     if (persistent(h)) return pk_execute(h, batch, n, is_left ? 0 : 1, mem == SJBG_MEM_HOST, match_count);
-    EagerState &st = *h->eager;
-    SJBG_CK(h, cudaMemsetAsync(st.batch_count, 0, 8, h->stream));
-    rc = eager_enqueue(h, batch, n, is_left ? 0 : 1, mem == SJBG_MEM_HOST, st.batch_count);
-    if (rc) return rc;
     unsigned long long *hc = static_cast<unsigned long long *>(pinned_get(h, 5, 64));
     if (!hc) return fail(h, SJBG_E_NOMEM, "count staging");
-    SJBG_CK(h, cudaMemcpyAsync(hc, st.batch_count, 8, cudaMemcpyDeviceToHost, h->stream));
+    hc[0] = 0;
+    rc = eager_enqueue(h, batch, n, is_left ? 0 : 1, mem == SJBG_MEM_HOST, hc);
+    if (rc) return rc;
     SJBG_CK(h, cudaStreamSynchronize(h->stream));
     profile_collect(h);
     if (match_count) *match_count = hc[0];

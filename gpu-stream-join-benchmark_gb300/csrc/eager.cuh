@@ -32,7 +32,8 @@ struct EagerState {
     uint64_t cap = 0;          // tuples per side
     uint32_t table_bits = 0;
     WinAcc *acc = nullptr;     // current window totals (device)
-    unsigned long long *batch_count = nullptr;   // device slot for the last batch's matches
+    unsigned long long *batch_count = nullptr;   // matches and finished CTAs of the batch in flight (zero between batches)
+    int host_direct = -1;      // whether kernels read pageable host memory in place (-1: not asked yet)
     sjbg_pair *pairs = nullptr;   // current window's pairs (device), pairs_cap entries
     uint64_t pairs_cap = 0;
     uint32_t *sort_tmp = nullptr;  // sorted incoming batch: keys then vals (2 * kEagerMaxSortBatch)

@@ -363,9 +363,10 @@ __device__ void pk_hj_batch(const PkArgs &a, const PkWork &w) {
             key = t.x;
             val = t.y;
         }
+        unsigned long long count = 0, xr = 0, prod = 0;
         eager_hj_step<kEnum, kPairs>(valid, key, val, w.base + i, side, a.tab[side], a.tab[side ^ 1],
-                                     a.tuples[side ^ 1], w.oth_n, a.acc, &a.dev->sync.tcount, a.pairs,
-                                     a.pairs_cap);
+                                     a.tuples[side ^ 1], w.oth_n, a.acc, a.pairs, a.pairs_cap, count, xr, prod);
+        flush_batch(a.acc, &a.dev->sync.tcount, count, xr, prod);
     }
 }
 
