@@ -576,19 +576,38 @@ int sjbg_eager_run(sjbg_handle *h, const sjbg_tuple *left, const sjbg_tuple *rig
         dl = sl;
         dr = sr;
     }
-    unsigned long long *dCounts = static_cast<unsigned long long *>(ws_get(h, WS_AUX0, 8 * std::max<uint64_t>(2 * n_batches, 1)));
-    WinAcc *dWin = static_cast<WinAcc *>(ws_get(h, WS_AUX1, sizeof(WinAcc) * (2 * n_batches + 3)));
-    if (!dCounts || !dWin) return fail(h, SJBG_E_NOMEM, "eager run buffers");
-    rc = eager_clear(h);
-    if (rc) return rc;
+    // batch counts, then the window totals and the status word, in one buffer:
+    // zeroed at once, and copied out at once into pinned memory (two copies to
+    // pageable memory and a memset per array cost 40 us of a 200 us call)
+    const size_t cntB = (8 * 2 * n_batches + 15) & ~(size_t)15, winB = sizeof(WinAcc) * (2 * n_batches + 3);
+    uint8_t *dOut = static_cast<uint8_t *>(ws_get(h, WS_AUX0, cntB + winB));
+    if (!dOut) return fail(h, SJBG_E_NOMEM, "eager run buffers");
+    unsigned long long *dCounts = reinterpret_cast<unsigned long long *>(dOut);
+    WinAcc *dWin = reinterpret_cast<WinAcc *>(dOut + cntB);
+    // (a window no batch has reached is clear; a persistent kernel's batches are not counted here)
+    if (persistent(h) || h->eager->side[0].n || h->eager->side[1].n) {
+        rc = eager_clear(h);
+        if (rc) return rc;
+    }
     uint32_t windows = 0;
-    rc = eager_run_batched(h, dl, dr, n_batches, eager_enumerates(h), dCounts, dWin, &windows);
-    if (rc) return rc;
-    std::vector<WinAcc> hw(windows + 1);
-    if (batch_counts && n_batches)
-        SJBG_CK(h, cudaMemcpyAsync(batch_counts, dCounts, 8 * 2 * n_batches, cudaMemcpyDeviceToHost, h->stream));
-    SJBG_CK(h, cudaMemcpyAsync(hw.data(), dWin, sizeof(WinAcc) * (windows + 1), cudaMemcpyDeviceToHost, h->stream));
-    SJBG_CK(h, cudaStreamSynchronize(h->stream));
+    const WinAcc *hw = nullptr;
+    // by buckets first, then, if the key groups were too large, by sorting (as
+    // every later stream of a handle that has met such a one)
+    for (bool grouped = !h->eager->few_keys;; grouped = false) {
+        rc = eager_run_batched(h, dl, dr, n_batches, eager_enumerates(h), grouped, dCounts, dWin, &windows);
+        if (rc) return rc;
+        const size_t outB = cntB + sizeof(WinAcc) * (windows + 1);
+        uint8_t *hOut = static_cast<uint8_t *>(pinned_get(h, 3, outB));
+        if (!hOut) return fail(h, SJBG_E_NOMEM, "result staging");
+        if (int rc_out = stage_copy(h, hOut, dOut, outB)) return rc_out;
+        SJBG_CK(h, cudaStreamSynchronize(h->stream));
+        hw = reinterpret_cast<const WinAcc *>(hOut + cntB);
+        if (!(hw[windows].info & kErrRegroup)) {
+            if (batch_counts && n_batches) std::memcpy(batch_counts, hOut, 8 * 2 * n_batches);
+            break;
+        }
+        h->eager->few_keys = true;
+    }
     profile_collect(h);
     if (int se = device_status_error(h, hw[windows].info)) return se;
     for (uint32_t w = 0; w < windows && w < n_windows_out; w++) fill_eager_result(h, hw[w], &out[w]);

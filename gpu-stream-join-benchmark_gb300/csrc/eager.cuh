@@ -33,6 +33,7 @@ struct EagerState {
     uint32_t table_bits = 0;
     WinAcc *acc = nullptr;     // current window totals (device)
     unsigned long long *batch_count = nullptr;   // matches and finished CTAs of the batch in flight (zero between batches)
+    bool few_keys = false;     // a recorded stream had too few distinct keys to go by buckets (eager_run.cu)
     int host_direct = -1;      // whether kernels read pageable host memory in place (-1: not asked yet)
     sjbg_pair *pairs = nullptr;   // current window's pairs (device), pairs_cap entries
     uint64_t pairs_cap = 0;
@@ -59,7 +60,7 @@ uint32_t nlj_left_tile();   // left tuples per nested-loop CTA
 // A whole recorded eager stream (eager_run.cu): batch counts into dCounts
 // (2 * n_batches), window totals into dWin (then the status word).
 int eager_run_batched(sjbg_handle *h, const sjbg_tuple *dl, const sjbg_tuple *dr, uint64_t n_batches, bool enumerate,
-                      unsigned long long *dCounts, WinAcc *dWin, uint32_t *n_windows);
+                      bool grouped, unsigned long long *dCounts, WinAcc *dWin, uint32_t *n_windows);
 
 int eager_init(sjbg_handle *h);
 int eager_init_and_clear(sjbg_handle *h);

@@ -32,6 +32,7 @@
 
 #include "eager.cuh"
 #include "sort.cuh"
+#include "tiles.cuh"
 
 namespace sjbg {
 
@@ -414,6 +415,210 @@ eattr_kernel(const SortView *__restrict__ view, const SortSeg *__restrict__ segs
     }
 }
 
+// ---------------------------------------------------------------- bucket-based batch counts
+// The counting form of a recorded stream, when its key groups are small: every
+// batch is cut into tiles of one arrival tag each, sorted by bucket of a
+// multiplicative hash of the key (tiles.cuh), and a CTA per bucket takes the
+// bucket's left words out of all tiles of a window into lists by key in shared
+// memory, then lets every right word, as it is read, walk its key's list: a
+// left tuple with a smaller tag counts for the right tuple's batch, another for
+// its own, and all of them for the window's checksum.  One pass over the tuples
+// and one over their words, where the sort reads and writes them three or four
+// times and the attribution twice more (windows of 2^20, batches of 4,096,
+// 6.3 M tuples: 485 us by sorting).  A bucket of more than kGroupCap left
+// tuples, or lists longer than kGroupSteps allows (few distinct keys), sets
+// kErrRegroup and the host runs the sort instead.
+constexpr uint32_t kGroupCap = 2048;     // left tuples of a bucket
+constexpr uint32_t kGroupSlots = 2048;   // list heads
+constexpr uint32_t kGroupTilesMax = 1040, kGroupTagsMax = 1040;   // per window
+constexpr uint32_t kGroupSteps = 1024;   // list steps per thread and bucket
+constexpr uint32_t kGroupMaxLog2 = 11;
+constexpr int kGroupThreads = 512;
+
+// One window of the stream; a tile is part `j % tpb` of arrival slot `j / tpb`.
+struct EGroupWin {
+    uint32_t first_tag, tags, tile0, pad_;   // arrival tag of the first batch, batches, first tile of the call
+};
+
+__device__ __forceinline__ uint32_t group_bucket(uint32_t key, uint32_t lg) {
+    return lg ? (key * 0x9E3779B1u) >> (32u - lg) : 0u;
+}
+__device__ __forceinline__ uint32_t group_slot(uint32_t key) {   // independent of the bucket's bits
+    return (key * 0x85EBCA6Bu) >> 21;
+}
+static_assert(kGroupSlots == 1u << 11, "group_slot takes 11 bits");
+
+__global__ void __launch_bounds__(kSortedThreads, 3)
+egroup_sort_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
+                   const EGroupWin *__restrict__ wins, uint32_t nw, uint32_t B, uint32_t ts, uint32_t tpb, uint32_t lg,
+                   uint64_t *__restrict__ words, uint32_t wstride, uint16_t *__restrict__ rows) {
+    uint32_t lo = 0, hi = nw;   // largest w with tile0 <= tile
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (wins[mid].tile0 <= blockIdx.x) lo = mid; else hi = mid;
+    }
+    const uint32_t j = blockIdx.x - wins[lo].tile0;
+    const uint32_t tag = wins[lo].first_tag + j / tpb, part = j % tpb;
+    const sjbg_tuple *src = ((tag & 1u) ? R : L) + (uint64_t)(tag >> 1) * B + part * ts;
+    sort_tile(src, min(ts, B - part * ts), lg, words + (uint64_t)blockIdx.x * wstride,
+              rows + (uint64_t)blockIdx.x * sorted_row(lg), [lg](uint32_t key) { return group_bucket(key, lg); });
+}
+
+struct EGroupSmem {
+    unsigned long long f[kGroupCap];     // fr of the left tuple
+    uint32_t key[kGroupCap];
+    uint32_t link[kGroupCap];            // arrival slot in the window (tag - first_tag) << 16 | next of the list + 1 (0: none)
+    uint32_t head[kGroupSlots];          // list head + 1, 0: none
+    uint32_t tagc[kGroupTagsMax];        // matches per arrival slot
+    // the window's tiles, the left side's first: the bucket's run in the tile,
+    // the bucket's words before it, the tile's arrival position
+    uint16_t off[kGroupTilesMax], pre[kGroupTilesMax], tile[kGroupTilesMax];
+    uint16_t owner[2 * kGroupCap];       // of the bucket's i-th word, the entry above
+    uint32_t warp_tot[32];
+    uint32_t n_left, stop;
+};
+static_assert(kGroupCap < 1u << 16 && kGroupTagsMax < 1u << 16, "16-bit links");
+
+// Persistent CTAs over equal shares of the call's buckets (nw * 2^lg, window by
+// window), so that a window's batch counters are added to the global ones a
+// few times per CTA, not once per bucket.  A run is a few words, so the words
+// of a bucket are numbered across its runs and every lane has one: with a group
+// of lanes per run the kernel took 119 us, a third of its lanes working.
+__global__ void __launch_bounds__(kGroupThreads, 3)
+egroup_count_kernel(const uint64_t *__restrict__ words, uint32_t wstride, const uint16_t *__restrict__ rows,
+                    const EGroupWin *__restrict__ wins, uint32_t nw, uint32_t tpb, uint32_t lg,
+                    unsigned long long *__restrict__ counts, WinAcc *__restrict__ acc, uint32_t *__restrict__ status) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    EGroupSmem &sm = *reinterpret_cast<EGroupSmem *>(smem_raw);
+    const uint32_t nb = nw << lg;
+    const uint32_t g0 = (uint32_t)((uint64_t)nb * blockIdx.x / gridDim.x);
+    const uint32_t g1 = (uint32_t)((uint64_t)nb * (blockIdx.x + 1) / gridDim.x);
+    uint32_t cur = 0xFFFFFFFFu;   // window of the counters in tagc
+    unsigned long long count = 0, prod = 0;
+    auto flush = [&](uint32_t w) {   // ends with a barrier
+        SJBG_BARRIER();
+        for (uint32_t i = threadIdx.x; i < wins[w].tags; i += kGroupThreads)
+            if (sm.tagc[i]) atomicAdd(&counts[wins[w].first_tag + i], (unsigned long long)sm.tagc[i]);
+        flush_acc(&acc[w], count, 0ull, prod);
+        count = prod = 0;
+        SJBG_BARRIER();
+    };
+    for (uint32_t g = g0; g < g1; g++) {
+        const uint32_t w = g >> lg, b = g & ((1u << lg) - 1u);
+        if (w != cur) {
+            if (cur != 0xFFFFFFFFu) flush(cur);
+            for (uint32_t i = threadIdx.x; i < kGroupTagsMax; i += kGroupThreads) sm.tagc[i] = 0;
+            cur = w;
+        }
+        const EGroupWin gw = wins[w];
+        const uint32_t T = gw.tags * tpb, lslot = gw.first_tag & 1u;   // the left side's first slot
+        const uint32_t TL = gw.tags > lslot ? (gw.tags - lslot + 1) / 2 * tpb : 0u;   // its tiles
+        const uint16_t *rw = rows + (uint64_t)gw.tile0 * sorted_row(lg) + b;
+        if (threadIdx.x == 0) sm.stop = *(volatile uint32_t *)status & kErrRegroup;
+        // thread t's entries [t * per, t * per + per)
+        constexpr uint32_t kPerMax = (kGroupTilesMax + kGroupThreads - 1) / kGroupThreads;
+        const uint32_t per = (T + kGroupThreads - 1) / kGroupThreads, x0 = threadIdx.x * per;
+        uint32_t len[kPerMax], sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPerMax; q++) {
+            const uint32_t x = x0 + q;
+            len[q] = 0;
+            if (q < per && x < T) {
+                const bool right = x >= TL;
+                const uint32_t y = right ? x - TL : x, z = tpb == 1 ? y : y / tpb;
+                const uint32_t slot = (right ? lslot ^ 1u : lslot) + 2 * z;
+                const uint32_t t = tpb == 1 ? slot : slot * tpb + (y - z * tpb);
+                const uint16_t *r = rw + (uint64_t)t * sorted_row(lg);
+                const uint32_t o = __ldg(r);
+                len[q] = __ldg(r + 1) - o;
+                sm.off[x] = (uint16_t)o;
+                sm.tile[x] = (uint16_t)t;
+            }
+            sum += len[q];
+        }
+        uint32_t tot;
+        uint32_t run = warp_excl_scan(sum, &tot);
+        if (lane_id() == 31) sm.warp_tot[warp_id()] = tot;
+        for (uint32_t i = threadIdx.x; i < kGroupSlots; i += kGroupThreads) sm.head[i] = 0;
+        SJBG_BARRIER();
+        const uint32_t v = lane_id() < kGroupThreads / 32 ? sm.warp_tot[lane_id()] : 0u;
+        const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, v);
+        run += __reduce_add_sync(0xFFFFFFFFu, lane_id() < warp_id() ? v : 0u);
+        if (sm.stop || n > 2 * kGroupCap) {   // (n and stop are the same for the whole CTA)
+            if (threadIdx.x == 0) atomicOr(status, kErrRegroup);
+            return;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kPerMax; q++) {
+            const uint32_t x = x0 + q;
+            if (q < per && x < T) {
+                sm.pre[x] = (uint16_t)run;
+                if (x == TL) sm.n_left = run;
+                for (uint32_t m = 0; m < len[q]; m++) sm.owner[run + m] = (uint16_t)x;
+            }
+            run += len[q];
+        }
+        if (TL == T && threadIdx.x == 0) sm.n_left = n;
+        SJBG_BARRIER();
+        const uint32_t nl = sm.n_left;
+        if (nl > kGroupCap) {   // (the same for the whole CTA)
+            if (threadIdx.x == 0) atomicOr(status, kErrRegroup);
+            return;
+        }
+        // words [i0, i1) of the bucket, four of a thread in flight
+        auto each = [&](uint32_t i0, uint32_t i1, auto use) {
+            for (uint32_t i = i0 + threadIdx.x; i < i1; i += 4 * kGroupThreads) {
+                uint64_t e[4];
+                uint32_t t[4];
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++) {
+                    const uint32_t k = i + q * kGroupThreads;
+                    if (k < i1) {
+                        const uint32_t x = sm.owner[k];
+                        t[q] = sm.tile[x];
+                        e[q] = __ldg(words + (uint64_t)(gw.tile0 + t[q]) * wstride + (sm.off[x] + (k - sm.pre[x])));
+                    }
+                }
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++)
+                    if (i + q * kGroupThreads < i1) use(e[q], tpb == 1 ? t[q] : t[q] / tpb, i + q * kGroupThreads);
+            }
+        };
+        each(0u, nl, [&](uint64_t e, uint32_t slot, uint32_t i) {
+            const uint32_t key = (uint32_t)e;
+            sm.key[i] = key;
+            sm.f[i] = sjbg_fr((uint32_t)(e >> 32));
+            sm.link[i] = (slot << 16) | atomicExch(&sm.head[group_slot(key)], i + 1u);
+        });
+        SJBG_BARRIER();
+        uint32_t steps = 0;
+        each(nl, n, [&](uint64_t e, uint32_t slot, uint32_t) {
+            const uint32_t key = (uint32_t)e;
+            uint32_t c = 0, later = 0;
+            unsigned long long f = 0;
+            for (uint32_t j = sm.head[group_slot(key)]; j != 0 && steps < kGroupSteps; steps++) {
+                const uint32_t x = sm.link[j - 1];
+                if (sm.key[j - 1] == key) {
+                    f += sm.f[j - 1];
+                    if ((x >> 16) < slot) {
+                        c++;
+                    } else {
+                        later++;
+                        atomicAdd(&sm.tagc[x >> 16], 1u);
+                    }
+                }
+                j = x & 0xFFFFu;
+            }
+            if (c) atomicAdd(&sm.tagc[slot], c);
+            count += c + later;
+            if (f) prod += f * sjbg_gs((uint32_t)(e >> 32));
+        });
+        if (steps >= kGroupSteps) atomicOr(status, kErrRegroup);
+        SJBG_BARRIER();   // the lists are read before the next bucket's
+    }
+    if (cur != 0xFFFFFFFFu) flush(cur);
+}
+
 struct ERunWin {
     uint64_t l0, l1, r0, r1;   // batch ranges [l0, l1) and [r0, r1)
 };
@@ -444,22 +649,80 @@ static std::vector<ERunWin> erun_windows(uint64_t n_batches, uint64_t B, uint64_
     return wins;
 }
 
+// Batch counts and window totals by buckets; *done false when the stream's
+// shape does not suit: batches under 1,024 tuples (rows would outweigh the
+// tiles), more tiles or batches in a window than a CTA's arrays hold, or
+// windows whose buckets would be more than 2^kGroupMaxLog2.
+static int eager_run_grouped(sjbg_handle *h, const sjbg_tuple *dl, const sjbg_tuple *dr,
+                             const std::vector<ERunWin> &ew, unsigned long long *dCounts, size_t zeroB, WinAcc *dWin,
+                             bool *done) {
+    const uint64_t B = h->cfg.batch_size;
+    const uint32_t nw = (uint32_t)ew.size();
+    if (B < 1024) return SJBG_OK;
+    const uint64_t tpb = (B + kSortedTile - 1) / kSortedTile, ts = (B + tpb - 1) / tpb;
+    uint64_t most = 0, tiles = 0;
+    for (const ERunWin &x : ew) most = std::max(most, (x.l1 - x.l0) + (x.r1 - x.r0));
+    if (most > kGroupTagsMax || most * tpb > kGroupTilesMax) return SJBG_OK;
+    // at most kGroupCap / 2 left tuples per bucket on average: room for uneven buckets
+    uint32_t lg = 0;
+    while (((uint64_t)kGroupCap << lg) < most * B) lg++;
+    if (lg > kGroupMaxLog2 || ((uint64_t)nw << lg) > 0x7FFFFFFFull) return SJBG_OK;
+    std::vector<EGroupWin> gw(nw);
+    for (uint32_t w = 0; w < nw; w++) {
+        const ERunWin &x = ew[w];
+        // a window opens with left batch l0 (r0 == l0) or with right batch r0 (l0 == r0 + 1)
+        gw[w] = EGroupWin{x.l0 <= x.r0 ? (uint32_t)(2 * x.l0) : (uint32_t)(2 * x.r0 + 1),
+                          (uint32_t)((x.l1 - x.l0) + (x.r1 - x.r0)), (uint32_t)tiles, 0};
+        tiles += gw[w].tags * tpb;
+    }
+    const uint32_t wstride = (uint32_t)((ts + 1) & ~1ull);   // tiles start on 16 bytes
+    const size_t upB = sizeof(EGroupWin) * nw;
+    uint8_t *hst = static_cast<uint8_t *>(pinned_get(h, 2, upB));
+    uint8_t *dev = static_cast<uint8_t *>(ws_get(h, WS_EAGER_META, upB + 16));
+    uint64_t *words = static_cast<uint64_t *>(ws_get(h, WS_EAGER_K0, sizeof(uint64_t) * wstride * tiles));
+    uint16_t *rows = static_cast<uint16_t *>(ws_get(h, WS_EAGER_V0, sizeof(uint16_t) * sorted_row(lg) * tiles));
+    if (!hst || !dev || !words || !rows) return fail(h, SJBG_E_NOMEM, "eager run buffers");
+    std::memcpy(hst, gw.data(), upB);
+    if (int rc = stage_copy_zero(h, dev, hst, upB, dCounts, zeroB)) return rc;
+    const EGroupWin *dW = reinterpret_cast<const EGroupWin *>(dev);
+    const size_t s1 = sorted_tile_bytes(lg), s2 = sizeof(EGroupSmem);
+    allow_big_smem(egroup_sort_kernel, s1);
+    SJBG_CK(h, launch(h, "erun_tile_sort", egroup_sort_kernel, dim3((uint32_t)tiles), dim3(kSortedThreads), s1, dl, dr,
+                      dW, nw, (uint32_t)B, (uint32_t)ts, (uint32_t)tpb, lg, words, wstride, rows));
+    allow_big_smem(egroup_count_kernel, s2);
+    const uint32_t grid = std::min<uint32_t>(nw << lg, 3u * (uint32_t)std::max(h->num_sms, 1));
+    SJBG_CK(h, launch(h, "erun_group_count", egroup_count_kernel, dim3(grid), dim3(kGroupThreads), s2,
+                      (const uint64_t *)words, wstride, (const uint16_t *)rows, dW, nw, (uint32_t)tpb, lg, dCounts,
+                      dWin, reinterpret_cast<uint32_t *>(&dWin[nw].info)));
+    *done = true;
+    return SJBG_OK;
+}
+
 int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                   sjbg_pair *dPairs, WinAcc *acc, bool enumerate, uint32_t *part_used);
 
-// Whole recorded stream; dCounts (2 * n_batches) and dWin (one entry per
-// window, then the status word) are device arrays zeroed here.  Returns the
-// number of windows in *n_windows.
+// Whole recorded stream; dCounts (2 * n_batches) and, after it in the same
+// buffer, dWin (one entry per window, then the status word) are device arrays
+// zeroed here.  Returns the
+// number of windows in *n_windows.  grouped: the counting joins may go by
+// buckets; the status word then may hold kErrRegroup, and the call is made
+// again without.
 int eager_run_batched(sjbg_handle *h, const sjbg_tuple *dl, const sjbg_tuple *dr, uint64_t n_batches, bool enumerate,
-                      unsigned long long *dCounts, WinAcc *dWin, uint32_t *n_windows) {
+                      bool grouped, unsigned long long *dCounts, WinAcc *dWin, uint32_t *n_windows) {
     const uint64_t B = h->cfg.batch_size, W = h->cfg.window_size;
     const std::vector<ERunWin> ew = erun_windows(n_batches, B, W);
     const uint32_t nw = (uint32_t)ew.size();
     *n_windows = nw;
-    SJBG_CK(h, cudaMemsetAsync(dCounts, 0, 8 * std::max<uint64_t>(2 * n_batches, 1), h->stream));
-    SJBG_CK(h, cudaMemsetAsync(dWin, 0, sizeof(WinAcc) * (nw + 1), h->stream));
+    const size_t zeroB = reinterpret_cast<uint8_t *>(dWin + nw + 1) - reinterpret_cast<uint8_t *>(dCounts);
+    if (nw && B * n_batches >= 0x7FFFFFFFull)
+        return fail(h, SJBG_E_CAPACITY, "eager streams are limited to 2^31 tuples");
+    if (nw && grouped && !enumerate && h->cfg.algorithm != SJBG_ALG_NLJ) {
+        bool done = false;
+        if (int rc = eager_run_grouped(h, dl, dr, ew, dCounts, zeroB, dWin, &done)) return rc;
+        if (done) return SJBG_OK;
+    }
+    SJBG_CK(h, cudaMemsetAsync(dCounts, 0, zeroB, h->stream));
     if (nw == 0) return SJBG_OK;
-    if (B * n_batches >= 0x7FFFFFFFull) return fail(h, SJBG_E_CAPACITY, "eager streams are limited to 2^31 tuples");
 
     if (h->cfg.algorithm == SJBG_ALG_NLJ) {
         const uint32_t lt = nlj_left_tile();
