@@ -223,6 +223,12 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
                            sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used) {
     const bool pairs = dPairs != nullptr;
     const bool enumerate = pairs || (h->cfg.flags & SJBG_F_XOR);
+    if (h->cfg.algorithm == SJBG_ALG_HJ && !enumerate) {
+        bool done = false;
+        *part_used = SJBG_PART_NONE;
+        if (int rc = hj_raw_batch(h, dL, dR, wins, n, hAcc, &done)) return rc;
+        if (done) return SJBG_OK;
+    }
     // acc[n].info is the call's device status word (kErr* bits)
     WinAcc *acc = static_cast<WinAcc *>(ws_get(h, WS_WIN_ACC, sizeof(WinAcc) * (n + 1)));
     if (!acc) return fail(h, SJBG_E_NOMEM, "window accumulators");

@@ -1178,6 +1178,7 @@ constexpr int kJoinPer = 8;   // elements per thread per tile (independent loads
 // kJoinChunkEnum when pairs are enumerated.
 constexpr uint32_t kJoinChunk = 65536;
 constexpr uint32_t kJoinChunkMin = 2048, kJoinChunkEnum = 16384;
+constexpr uint32_t kRawPiece = 1024;   // least build and probe tuples of a raw-only call's items
 
 // A run of tuples: (val << 32 | key) words of a partitioned array, or (kRaw)
 // the key and val of 16-byte tuples.
@@ -1290,7 +1291,8 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
 // them (z = 1.5, 8 x 2^24: 53.6 us without, 67.0 us with).
 template <bool kRaw, bool kFilter>
 __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
-                                                  bool loaded, WinAcc *__restrict__ acc, uint32_t cap) {
+                                                  bool loaded, uint32_t cap, unsigned long long &count,
+                                                  unsigned long long &prod) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ uint32_t novf;
     const uint32_t nB = ji.nB, nP = ji.nP;
@@ -1314,7 +1316,6 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
     const bool filtered = kFilter && nB < cap;
     constexpr uint32_t tile = kJoinPer * kJoinThreads;
 
-    unsigned long long count = 0, prod = 0;
     uint32_t n = nB;
     for (;;) {
         for (uint32_t i = threadIdx.x; i <= C; i += kJoinThreads) {
@@ -1399,7 +1400,6 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
         SJBG_BARRIER();
         if (n == 0) break;
     }
-    flush_acc(&acc[ji.w], count, 0, prod);
 }
 
 // A pair of pieces of a bucket whose build run is longer than its table (a hot
@@ -1524,11 +1524,12 @@ __device__ __forceinline__ uint32_t direct_passes(const JoinItem &ji, KeyRange k
 
 // `clean`: the leading table entries known to be zero (CTA-uniform); a direct
 // bucket leaves the table zero again, a hash-table bucket does not.  e: the
-// build run's first tile (build_head); first: its smallest index.
+// build run's first tile (build_head); first: its smallest index.  The matches
+// are added to count and prod, as in join_count_bucket.
 template <bool kRaw>
 __device__ __forceinline__ void join_count_direct(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
-                                                  uint32_t first, uint32_t passes, WinAcc *__restrict__ acc,
-                                                  uint32_t &clean) {
+                                                  uint32_t first, uint32_t passes, uint32_t &clean,
+                                                  unsigned long long &count, unsigned long long &prod) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     const uint32_t nB = ji.nB, nP = ji.nP, lg = ji.lg;
     const uint32_t bside = jr.bside, pside = bside ^ 1u;
@@ -1543,7 +1544,6 @@ __device__ __forceinline__ void join_count_direct(const JoinItem &ji, const Join
     if (clean != kDirectMax) SJBG_BARRIER();
     clean = kDirectMax;
     constexpr uint32_t tile = kJoinPer * kJoinThreads;
-    unsigned long long count = 0, prod = 0;
     for (uint32_t p = 0; p < passes; p++) {
         const uint32_t lo = first + p * kDirectMax;
         // build: the build keys whose index falls in [lo, lo + kDirectMax)
@@ -1601,7 +1601,6 @@ __device__ __forceinline__ void join_count_direct(const JoinItem &ji, const Join
         }
         SJBG_BARRIER();
     }
-    flush_acc(&acc[ji.w], count, 0, prod);
 }
 
 constexpr uint32_t kEnumChunk = 4096;  // left tuples per chained chunk
@@ -1712,6 +1711,24 @@ __device__ __forceinline__ void join_enum_bucket(const JoinItem &ji, const uint6
     flush_acc(&acc[w], count, xr, prod);
 }
 
+// One item's matches; `clean` as in join_count_direct.
+template <bool kRaw, bool kModels>
+__device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr, uint32_t cap, uint32_t &clean,
+                                          unsigned long long &count, unsigned long long &prod) {
+    uint64_t e[kJoinPer];
+    if (kModels && (ji.flags & kItemModel)) {
+        join_count_bucket<kRaw, false>(ji, jr, e, false, cap, count, prod);
+    } else {
+        const KeyRange kr = build_head<kRaw>(ji, jr, e);
+        if (const uint32_t passes = direct_passes(ji, kr)) {
+            join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, clean, count, prod);
+            return;
+        }
+        join_count_bucket<kRaw, true>(ji, jr, e, true, cap, count, prod);
+    }
+    clean = 0;
+}
+
 // Bucket joins over the join list (items, length *jn; or, without a list, the
 // one window's buckets 0 .. B-1, whole): CTAs that stride over the items (queue == nullptr) or
 // persistent CTAs that take items from a device work queue (an atomic counter)
@@ -1733,21 +1750,6 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
                          uint32_t *queue, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn) {
     const uint32_t nitems = items ? *jn : B;
     uint32_t clean = 0;
-    auto join_as = [&](const JoinItem &ji, const JoinRuns &jr, auto raw_t) {
-        constexpr bool kRaw = decltype(raw_t)::value;
-        uint64_t e[kJoinPer];
-        if (kModels && (ji.flags & kItemModel)) {
-            join_count_bucket<kRaw, false>(ji, jr, e, false, acc, cap);
-        } else {
-            const KeyRange kr = build_head<kRaw>(ji, jr, e);
-            if (const uint32_t passes = direct_passes(ji, kr)) {
-                join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, acc, clean);
-                return;
-            }
-            join_count_bucket<kRaw, true>(ji, jr, e, true, acc, cap);
-        }
-        clean = 0;
-    };
     auto join = [&](const JoinItem &ji) {
         if (ji.nB == 0 || ji.nP == 0) return;
         const JoinRuns jr = join_runs(ji, L, R, wins, partL, partR);
@@ -1757,13 +1759,16 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
             clean = 0;
             return;
         }
+        unsigned long long count = 0, prod = 0;
         if constexpr (!kModels) {
             if (ji.flags & kItemRaw) {
-                join_as(ji, jr, std::true_type{});
+                join_item<true, kModels>(ji, jr, cap, clean, count, prod);
+                flush_acc(&acc[ji.w], count, 0, prod);
                 return;
             }
         }
-        join_as(ji, jr, std::false_type{});
+        join_item<false, kModels>(ji, jr, cap, clean, count, prod);
+        flush_acc(&acc[ji.w], count, 0, prod);
     };
     if (!queue || !items) {
         for (uint32_t i = blockIdx.x; items && i < nitems; i += gridDim.x) {
@@ -1830,6 +1835,89 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
     }
 }
 
+// ---- calls of unpartitioned windows only
+// Small windows are all launches: the general path's upload, clears, scan,
+// join and result copy took 28 us on the device for one window of 4,096 tuples
+// per side, of which the tuples are well under one.  Here the host lists the
+// items, the one kernel gets them by value (or reads them in pinned memory),
+// and its last CTA writes the results to pinned memory, leaving its
+// accumulators zero for the next call.
+struct RawItem {
+    uint64_t b, p;   // first build and probe tuple, in their sides' arrays
+    uint32_t nB, nP, w, flags;
+};
+constexpr uint32_t kRawByValue = 64;
+struct RawItems {
+    RawItem v[kRawByValue];
+};
+constexpr uint32_t kRawWindows = 1024;   // accumulators kept
+
+// Matches of the windows of raw-only calls, and the CTAs that are done.
+struct RawAcc {
+    unsigned long long count[kRawWindows], prod[kRawWindows];
+    uint32_t done;
+};
+
+__global__ void __launch_bounds__(kJoinThreads, 2)
+raw_join_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
+                const __grid_constant__ RawItems items, const RawItem *__restrict__ list, uint32_t n, uint32_t cap,
+                RawAcc *__restrict__ acc, WinAcc *__restrict__ out) {
+    __shared__ unsigned long long part[2][kJoinThreads / 32];
+    __shared__ uint32_t last_s;
+    const RawItem it = list ? list[blockIdx.x] : items.v[blockIdx.x];
+    const bool swap = (it.flags & kItemSwap) != 0;
+    JoinItem ji;
+    ji.nB = it.nB; ji.nP = it.nP; ji.sB = 0; ji.sP = 0;
+    ji.w = it.w; ji.lg = 0; ji.flags = it.flags; ji.pad = 0;
+    JoinRuns jr;
+    jr.b = const_cast<sjbg_tuple *>((swap ? R : L) + it.b);   // (never written)
+    jr.p = (swap ? L : R) + it.p;
+    jr.bside = swap ? 1u : 0u;
+    uint32_t clean = 0;
+    unsigned long long count = 0, prod = 0;
+    if (it.nB && it.nP) join_item<true, false>(ji, jr, cap, clean, count, prod);
+    count = warp_sum_u64(count);
+    prod = warp_sum_u64(prod);
+    if (lane_id() == 0) {
+        part[0][warp_id()] = count;
+        part[1][warp_id()] = prod;
+    }
+    SJBG_BARRIER();
+    if (threadIdx.x == 0) {
+        for (uint32_t q = 1; q < kJoinThreads / 32; q++) {
+            count += part[0][q];
+            prod += part[1][q];
+        }
+        if (gridDim.x == 1) {
+            last_s = 2;
+        } else {
+            if (count) atomicAdd(&acc->count[it.w], count);
+            if (prod) atomicAdd(&acc->prod[it.w], prod);
+            __threadfence();
+            last_s = atomicAdd(&acc->done, 1u) == gridDim.x - 1 ? 1u : 0u;
+            __threadfence();
+        }
+    }
+    SJBG_BARRIER();
+    if (last_s == 0) return;
+    for (uint32_t w = threadIdx.x; w <= n; w += kJoinThreads) {   // out[n]: the call's status word
+        WinAcc r{0, 0, 0, 0, 0};
+        if (last_s == 2) {
+            if (w == it.w) {   // (thread it.w holds no sum: thread 0's are in part)
+                for (uint32_t q = 0; q < kJoinThreads / 32; q++) {
+                    r.count += part[0][q];
+                    r.prod += part[1][q];
+                }
+            }
+        } else if (w < n) {
+            r.count = atomicExch(&acc->count[w], 0ull);
+            r.prod = atomicExch(&acc->prod[w], 0ull);
+        }
+        out[w] = r;
+    }
+    if (last_s == 1 && threadIdx.x == 0) acc->done = 0;
+}
+
 // One CTA per join item (the grid covers the longest possible list).
 __global__ void __launch_bounds__(kJoinThreads)
 bucket_join_enum_kernel(const uint64_t *__restrict__ partL, const uint64_t *__restrict__ partR,
@@ -1860,6 +1948,78 @@ uint32_t choose_partitioner(const sjbg_handle *h, const WinHost *wins, uint32_t 
     return (mx <= (1u << 18) && tot <= (1u << 21)) ? SJBG_PART_NONE : SJBG_PART_RADIX;
 }
 
+// Slots of a count table for buckets of the target size (a target whose table
+// would not fit is joined in passes).
+static uint32_t join_cap(const sjbg_handle *h, uint64_t target) {
+    return (uint32_t)std::min<size_t>(count_table_cap((uint32_t)target),
+                                      (h->max_smem_optin - count_table_bytes(0) - 1024) / 16);
+}
+
+int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                 WinAcc *hAcc, bool *done) {
+    *done = false;
+    if (h->cfg.partitioner != SJBG_PART_AUTO || (h->tune.partitioner && h->tune.partitioner != SJBG_PART_NONE) ||
+        n == 0 || n > kRawWindows)
+        return SJBG_OK;
+    const uint32_t cap = join_cap(h, h->tune.bucket_target);
+    uint64_t tuples = 0;
+    for (uint32_t w = 0; w < n; w++) {
+        if (std::min(wins[w].n_left, wins[w].n_right) >= cap ||
+            std::max(wins[w].n_left, wins[w].n_right) > 0xFFFFFFFFull)
+            return SJBG_OK;
+        tuples += wins[w].n_left + wins[w].n_right;
+    }
+    // pieces of both sides: any cut of the build run will do (the sums are over
+    // pairs of tuples), so a call of few windows is spread over the SMs in
+    // pieces of about kRawPiece tuples, and a larger one in pieces that cost
+    // the SMs about equal shares
+    const uint64_t share = tuples / (4 * (uint64_t)std::max(h->num_sms, 1));
+    const uint32_t piece = (uint32_t)std::min<uint64_t>(cap - 1, std::max<uint64_t>(kRawPiece, share));
+    const uint32_t chunk = (uint32_t)std::min<uint64_t>(kJoinChunk, std::max<uint64_t>(kRawPiece, share));
+    std::vector<RawItem> list;
+    for (uint32_t w = 0; w < n; w++) {
+        const WinHost &x = wins[w];
+        if (!x.n_left || !x.n_right) continue;
+        const bool swap = x.n_right < x.n_left;
+        const uint32_t nB = (uint32_t)(swap ? x.n_right : x.n_left), nP = (uint32_t)(swap ? x.n_left : x.n_right);
+        const uint64_t b0 = swap ? x.right_off : x.left_off, p0 = swap ? x.left_off : x.right_off;
+        const uint32_t kb = std::max(1u, (nB + piece / 2) / piece), per = std::max(chunk, nB / kb);
+        const uint32_t kp = std::max<uint32_t>(1, (uint32_t)(((uint64_t)nP + per / 2) / per));
+        for (uint32_t i = 0; i < kb; i++)
+            for (uint32_t j = 0; j < kp; j++) {
+                const uint32_t b = (uint32_t)((uint64_t)nB * i / kb), p = (uint32_t)((uint64_t)nP * j / kp);
+                list.push_back(RawItem{b0 + b, p0 + p, (uint32_t)((uint64_t)nB * (i + 1) / kb) - b,
+                                       (uint32_t)((uint64_t)nP * (j + 1) / kp) - p, w,
+                                       kItemRaw | (swap ? (uint32_t)kItemSwap : 0u)});
+            }
+    }
+    if (list.empty()) {   // nothing can match
+        std::memset(hAcc, 0, sizeof(WinAcc) * (n + 1));
+        *done = true;
+        return SJBG_OK;
+    }
+    const bool fresh = h->ws[WS_RAW_ACC].p == nullptr;
+    RawAcc *acc = static_cast<RawAcc *>(ws_get(h, WS_RAW_ACC, sizeof(RawAcc)));
+    if (!acc) return fail(h, SJBG_E_NOMEM, "window accumulators");
+    if (fresh) SJBG_CK(h, cudaMemsetAsync(acc, 0, sizeof(RawAcc), h->stream));
+    RawItems items;
+    const RawItem *dList = nullptr;
+    if (list.size() <= kRawByValue) {
+        std::copy(list.begin(), list.end(), items.v);
+    } else {
+        RawItem *hst = static_cast<RawItem *>(pinned_get(h, 0, sizeof(RawItem) * list.size()));
+        if (!hst) return fail(h, SJBG_E_NOMEM, "plan buffers");
+        std::copy(list.begin(), list.end(), hst);
+        dList = hst;
+    }
+    const size_t smem = std::max(count_table_bytes(cap), kDirectBytes);
+    allow_big_smem(raw_join_kernel, smem);
+    SJBG_CK(h, launch(h, "raw_join", raw_join_kernel, dim3((uint32_t)list.size()), dim3(kJoinThreads), smem, dL, dR,
+                      items, dList, n, cap, acc, hAcc));
+    *done = true;
+    return SJBG_OK;
+}
+
 int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                   sjbg_pair *dPairs, WinAcc *acc, bool enumerate, uint32_t *part_used) {
     if (n == 0) return SJBG_OK;
@@ -1872,9 +2032,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     if (part_used) *part_used = learned ? SJBG_PART_LEARNED : SJBG_PART_RADIX;
     // build tuples per bucket: 2048 when chains are built, else the tuned target
     const uint64_t target = enumerate ? 2048 : h->tune.bucket_target;
-    // slots of a count table (a target whose table would not fit is joined in passes)
-    const uint32_t cap = (uint32_t)std::min<size_t>(
-        count_table_cap((uint32_t)target), (h->max_smem_optin - count_table_bytes(0) - 1024) / 16);
+    const uint32_t cap = join_cap(h, target);
 
     // ---- plan
     std::vector<WinPlan> plan(n);

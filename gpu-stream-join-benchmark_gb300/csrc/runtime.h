@@ -27,6 +27,7 @@ enum WsSlot : int {
     WS_COMPACT, WS_COMPACT_CNT,      // light tuples written by the counting pass
     WS_COARSE_ROWS,                  // per tile: coarse-partition offsets of its light tuples
     WS_EAGER_META, WS_EAGER_K0, WS_EAGER_K1, WS_EAGER_V0, WS_EAGER_V1, WS_EAGER_TILES,   // recorded eager streams
+    WS_RAW_ACC,                      // accumulators of raw-only hash joins (zero between calls)
     WS_COUNT
 };
 
@@ -170,6 +171,11 @@ struct WinHost {
 // acc[n].info, and leave the stream unsynchronised.
 int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                   sjbg_pair *dPairs, WinAcc *acc, bool enumerate, uint32_t *part_used);
+// Hash join of a call whose windows all stay unpartitioned in shared memory
+// (automatic choice, counting): one launch, results straight into hAcc (n + 1
+// entries, pinned).  *done false: not such a call.
+int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                 WinAcc *hAcc, bool *done);
 uint32_t choose_partitioner(const sjbg_handle *h, const WinHost *wins, uint32_t n);
 int hj_global_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                     sjbg_pair *dPairs, WinAcc *acc, bool enumerate);

@@ -53,3 +53,30 @@ def test_windows_of_different_sides(lib, oracle, kind, flags, part, bits):
         assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
         if flags == "xor":
             assert g["xor"] == w["xor"], d
+
+
+RAW = [(1, 1), (0, 5), (5, 0), (1535, 1537), (4096, 4096), (5343, 5343), (3, 100_000), (100_000, 3), (700, 40_000)]
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("kind", ["dense", "wide", "hot"])
+@pytest.mark.parametrize("windows", [RAW[:1], RAW[1:2], RAW[3:4], RAW[4:5], RAW, RAW * 30, RAW * 120])
+def test_calls_of_small_windows_only(lib, oracle, windows, kind, graph):
+    """One launch for the call: one item, items passed by value, items in a list,
+    more windows than it takes; repeated calls (accumulators left zero)."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(len(windows))
+    lefts, rights, descs, lo, ro = [], [], [], 0, 0
+    for nl, nr in windows:
+        lefts.append(keys_of(kind, nl, rng))
+        rights.append(keys_of(kind, nr, rng))
+        descs.append((lo, nl, ro, nr, 0, 0))
+        lo, ro = lo + nl, ro + nr
+    left, right = make_tuples(np.concatenate(lefts)), make_tuples(np.concatenate(rights))
+    want, _ = oracle.join_windows(left, right, descs, enumerate_pairs=False)
+    dl, dr = torch.from_numpy(left.view(np.uint8)).cuda(), torch.from_numpy(right.view(np.uint8)).cuda()
+    with lib.Joiner(lib.ALG_HJ, lib.LAZY, flags=lib.F_GRAPH if graph else 0, max_tuples_per_window=1 << 17) as j:
+        for _ in range(3):
+            got = j.lazy_execute_batch(dl, dr, descs, mem=lib.MEM_DEVICE)
+            for d, g, w in zip(descs, got, want):
+                assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
