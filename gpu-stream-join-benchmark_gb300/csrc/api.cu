@@ -245,6 +245,16 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
     return stage_copy(h, hAcc, acc, sizeof(WinAcc) * (n + 1));
 }
 
+int run_lazy_watched(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                     sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used) {
+    for (;;) {
+        if (int rc = run_lazy_device(h, dL, dR, wins, n, dPairs, hAcc, part_used)) return rc;
+        SJBG_CK(h, cudaStreamSynchronize(h->stream));
+        if (!(hAcc[n].info & kErrRegroup) || h->smj_full_sort) return SJBG_OK;
+        h->smj_full_sort = true;   // (from now on, on this handle)
+    }
+}
+
 int device_status_error(sjbg_handle *h, unsigned long long bits) {
     if (!bits) return SJBG_OK;
     if (bits & kErrTimeout) return fail(h, SJBG_E_TIMEOUT, "a bounded device-side wait gave up");
@@ -278,11 +288,12 @@ static void fill_result(const sjbg_handle *h, const WinAcc &a, const WinHost &w,
 // Batched lazy call on device inputs through a cached CUDA graph: the first
 // call with a given signature runs normally (sizing every workspace), then is
 // captured with private pinned staging buffers; later identical calls replay it.
+constexpr size_t kGraphKeySort = 11;   // smj_full_sort's place in a graph's key
 static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                       sjbg_pair *dPairs, bool enumerate, sjbg_window_result *out) {
     std::vector<uint64_t> key = {h->cfg.algorithm, h->cfg.partitioner, h->tune.partitioner, h->cfg.flags, h->cfg.result_mode,
                                  (uint64_t)(uintptr_t)dL, (uint64_t)(uintptr_t)dR, (uint64_t)(uintptr_t)dPairs, n,
-                                 h->tune.bucket_target, (uint64_t)h->tune.persistent_join,
+                                 h->tune.bucket_target, (uint64_t)h->tune.persistent_join, (uint64_t)h->smj_full_sort,
                                  (uint64_t)(uintptr_t)h->stream};
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &x = wins[w];
@@ -305,11 +316,12 @@ static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR
         hAcc = static_cast<WinAcc *>(pinned_get(h, 3, sizeof(WinAcc) * (n + 1)));
         if (!hAcc) return fail(h, SJBG_E_NOMEM, "result staging");
         SJBG_CK(h, cudaEventRecord(e0, h->stream));
-        int rc = run_lazy_device(h, dL, dR, wins, n, dPairs, hAcc, &part_used);   // warm-up: sizes every buffer
+        int rc = run_lazy_watched(h, dL, dR, wins, n, dPairs, hAcc, &part_used);   // warm-up: sizes every buffer
         if (rc) return rc;
         SJBG_CK(h, cudaEventRecord(e1, h->stream));
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
         profile_collect(h);
+        key[kGraphKeySort] = (uint64_t)h->smj_full_sort;   // (it may have been met just now)
         auto e = std::make_unique<sjbg_handle::GraphEntry>();
         e->key = key;
         e->part_used = part_used;
@@ -361,6 +373,10 @@ static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR
     cudaEventElapsedTime(&ms, e0, e1);
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
+    if ((hAcc[n].info & kErrRegroup) && !h->smj_full_sort) {   // a replay met keys that do not fit: the other graph
+        h->smj_full_sort = true;
+        return lazy_graph(h, dL, dR, wins, n, dPairs, enumerate, out);
+    }
     if (int se = device_status_error(h, hAcc[n].info)) return se;
     for (uint32_t w = 0; w < n; w++) fill_result(h, hAcc[w], wins[w], enumerate, dPairs != nullptr, part_used, ms, &out[w]);
     return SJBG_OK;
@@ -435,15 +451,14 @@ static int lazy_host_pipelined(sjbg_handle *h, const sjbg_tuple *L, const sjbg_t
         }
         SJBG_CK(h, cudaStreamWaitEvent(h->stream, landed[g], 0));
         uint32_t pu = SJBG_PART_NONE;
-        int rc = run_lazy_device(h, sL, sR, wins + w0, m, dP, hAcc, &pu);
+        // (waited for: the staging buffers (pinned plan uploads, accumulators) are reused by the next group)
+        int rc = run_lazy_watched(h, sL, sR, wins + w0, m, dP, hAcc, &pu);
         if (rc) {
             cudaStreamSynchronize(h->copy_stream);
             release();
             return rc;
         }
         if (g == 0) part_used = pu;
-        // the staging buffers (pinned plan uploads, accumulators) are reused by the next group
-        SJBG_CK(h, cudaStreamSynchronize(h->stream));
         if (int se = device_status_error(h, hAcc[m].info)) {
             cudaStreamSynchronize(h->copy_stream);
             release();
@@ -521,9 +536,8 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
         WinAcc *hp = static_cast<WinAcc *>(pinned_get(h, 4, sizeof(WinAcc) * (n + 1)));
         if (!hp) return fail(h, SJBG_E_NOMEM, "count staging");
         uint32_t pu;
-        int rc = run_lazy_device(h, dL, dR, wins, n, nullptr, hp, &pu);
+        int rc = run_lazy_watched(h, dL, dR, wins, n, nullptr, hp, &pu);
         if (rc) return rc;
-        SJBG_CK(h, cudaStreamSynchronize(h->stream));
         if (int se = device_status_error(h, hp[n].info)) return se;
         for (uint32_t w = 0; w < n; w++)
             if (hp[w].count > wins[w].pairs_cap)
@@ -552,6 +566,10 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
     profile_collect(h);
+    if ((hAcc[n].info & kErrRegroup) && !h->smj_full_sort) {   // (a counting sort-merge join: no pairs were written)
+        h->smj_full_sort = true;
+        return lazy_common(h, L, R, mem, wins, n, pairs, out);
+    }
     if (int se = device_status_error(h, hAcc[n].info)) return se;
     for (uint32_t w = 0; w < n; w++) fill_result(h, hAcc[w], wins[w], enumerate, want, part_used, ms, &out[w]);
     return SJBG_OK;

@@ -27,7 +27,7 @@ enum : uint32_t {
     kErrTimeout = 1u << 1,     // a bounded wait gave up
     kErrBadWindow = 1u << 2,   // a window descriptor is inconsistent
     kErrQueue = 1u << 3,       // work queue overflow
-    kErrRegroup = 1u << 4,     // recorded eager stream: key groups too large to go by buckets (the host sorts instead)
+    kErrRegroup = 1u << 4,     // key groups or ranges too large for shared memory: the host makes the call again with the full sort
 };
 
 // Per-window accumulators kept in device memory.

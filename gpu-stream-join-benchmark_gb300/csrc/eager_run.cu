@@ -450,18 +450,28 @@ static_assert(kGroupSlots == 1u << 11, "group_slot takes 11 bits");
 
 __global__ void __launch_bounds__(kSortedThreads, 3)
 egroup_sort_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
-                   const EGroupWin *__restrict__ wins, uint32_t nw, uint32_t B, uint32_t ts, uint32_t tpb, uint32_t lg,
-                   uint64_t *__restrict__ words, uint32_t wstride, uint16_t *__restrict__ rows) {
-    uint32_t lo = 0, hi = nw;   // largest w with tile0 <= tile
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (wins[mid].tile0 <= blockIdx.x) lo = mid; else hi = mid;
-    }
-    const uint32_t j = blockIdx.x - wins[lo].tile0;
-    const uint32_t tag = wins[lo].first_tag + j / tpb, part = j % tpb;
-    const sjbg_tuple *src = ((tag & 1u) ? R : L) + (uint64_t)(tag >> 1) * B + part * ts;
-    sort_tile(src, min(ts, B - part * ts), lg, words + (uint64_t)blockIdx.x * wstride,
-              rows + (uint64_t)blockIdx.x * sorted_row(lg), [lg](uint32_t key) { return group_bucket(key, lg); });
+                   const EGroupWin *__restrict__ wins, uint32_t nw, uint32_t tiles, uint32_t B, uint32_t ts,
+                   uint32_t tpb, uint32_t lg, uint64_t *__restrict__ words, uint32_t wstride,
+                   uint16_t *__restrict__ rows) {
+    struct Bucket {
+        uint32_t lg;
+        __device__ uint32_t operator()(uint32_t key) const { return group_bucket(key, lg); }
+    };
+    sort_tiles(tiles, [&](uint32_t tile, SortedTile &t) {
+        uint32_t lo = 0, hi = nw;   // largest w with tile0 <= tile
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (__ldg(&wins[mid].tile0) <= tile) lo = mid; else hi = mid;
+        }
+        const uint32_t j = tile - wins[lo].tile0;
+        const uint32_t tag = wins[lo].first_tag + j / tpb, part = j % tpb;
+        t.src = ((tag & 1u) ? R : L) + (uint64_t)(tag >> 1) * B + part * ts;
+        t.n = min(ts, B - part * ts);
+        t.P = 1u << lg;
+        t.words = words + (uint64_t)tile * wstride;
+        t.row = rows + (uint64_t)tile * sorted_row(1u << lg);
+        return Bucket{lg};
+    });
 }
 
 struct EGroupSmem {
@@ -513,7 +523,7 @@ egroup_count_kernel(const uint64_t *__restrict__ words, uint32_t wstride, const 
         const EGroupWin gw = wins[w];
         const uint32_t T = gw.tags * tpb, lslot = gw.first_tag & 1u;   // the left side's first slot
         const uint32_t TL = gw.tags > lslot ? (gw.tags - lslot + 1) / 2 * tpb : 0u;   // its tiles
-        const uint16_t *rw = rows + (uint64_t)gw.tile0 * sorted_row(lg) + b;
+        const uint16_t *rw = rows + (uint64_t)gw.tile0 * sorted_row(1u << lg) + b;
         if (threadIdx.x == 0) sm.stop = *(volatile uint32_t *)status & kErrRegroup;
         // thread t's entries [t * per, t * per + per)
         constexpr uint32_t kPerMax = (kGroupTilesMax + kGroupThreads - 1) / kGroupThreads;
@@ -528,7 +538,7 @@ egroup_count_kernel(const uint64_t *__restrict__ words, uint32_t wstride, const 
                 const uint32_t y = right ? x - TL : x, z = tpb == 1 ? y : y / tpb;
                 const uint32_t slot = (right ? lslot ^ 1u : lslot) + 2 * z;
                 const uint32_t t = tpb == 1 ? slot : slot * tpb + (y - z * tpb);
-                const uint16_t *r = rw + (uint64_t)t * sorted_row(lg);
+                const uint16_t *r = rw + (uint64_t)t * sorted_row(1u << lg);
                 const uint32_t o = __ldg(r);
                 len[q] = __ldg(r + 1) - o;
                 sm.off[x] = (uint16_t)o;
@@ -680,15 +690,16 @@ static int eager_run_grouped(sjbg_handle *h, const sjbg_tuple *dl, const sjbg_tu
     uint8_t *hst = static_cast<uint8_t *>(pinned_get(h, 2, upB));
     uint8_t *dev = static_cast<uint8_t *>(ws_get(h, WS_EAGER_META, upB + 16));
     uint64_t *words = static_cast<uint64_t *>(ws_get(h, WS_EAGER_K0, sizeof(uint64_t) * wstride * tiles));
-    uint16_t *rows = static_cast<uint16_t *>(ws_get(h, WS_EAGER_V0, sizeof(uint16_t) * sorted_row(lg) * tiles));
+    uint16_t *rows = static_cast<uint16_t *>(ws_get(h, WS_EAGER_V0, sizeof(uint16_t) * sorted_row(1u << lg) * tiles));
     if (!hst || !dev || !words || !rows) return fail(h, SJBG_E_NOMEM, "eager run buffers");
     std::memcpy(hst, gw.data(), upB);
     if (int rc = stage_copy_zero(h, dev, hst, upB, dCounts, zeroB)) return rc;
     const EGroupWin *dW = reinterpret_cast<const EGroupWin *>(dev);
-    const size_t s1 = sorted_tile_bytes(lg), s2 = sizeof(EGroupSmem);
+    const size_t s1 = sorted_tile_bytes(1u << lg), s2 = sizeof(EGroupSmem);
     allow_big_smem(egroup_sort_kernel, s1);
-    SJBG_CK(h, launch(h, "erun_tile_sort", egroup_sort_kernel, dim3((uint32_t)tiles), dim3(kSortedThreads), s1, dl, dr,
-                      dW, nw, (uint32_t)B, (uint32_t)ts, (uint32_t)tpb, lg, words, wstride, rows));
+    SJBG_CK(h, launch(h, "erun_tile_sort", egroup_sort_kernel,
+                      dim3(std::min<uint32_t>((uint32_t)tiles, 3u * (uint32_t)std::max(h->num_sms, 1))),
+                      dim3(kSortedThreads), s1, dl, dr, dW, nw, (uint32_t)tiles, (uint32_t)B, (uint32_t)ts, (uint32_t)tpb, lg, words, wstride, rows));
     allow_big_smem(egroup_count_kernel, s2);
     const uint32_t grid = std::min<uint32_t>(nw << lg, 3u * (uint32_t)std::max(h->num_sms, 1));
     SJBG_CK(h, launch(h, "erun_group_count", egroup_count_kernel, dim3(grid), dim3(kGroupThreads), s2,

@@ -128,8 +128,10 @@ static int ring_launch(sjbg_handle *h, RingState &st, RingSlot &s) {
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], s.pinned[i]);
     WinHost wh{0, st.W, 0, st.W, 0, 0};
     WinAcc *hacc = static_cast<WinAcc *>(pinned_get(h, 3, 2 * sizeof(WinAcc)));   // window + status word
+    h->unwatched = true;
     int rc = hacc ? run_lazy_device(h, st.buf[0] + off, st.buf[1] + off, &wh, 1, nullptr, hacc, &s.part_used)
                   : fail(h, SJBG_E_NOMEM, "window staging");
+    h->unwatched = false;
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], s.pinned[i]);
     if (rc) return rc;
     SJBG_CK(h, cudaEventRecord(s.done, h->stream));

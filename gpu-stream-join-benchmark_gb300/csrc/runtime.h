@@ -67,6 +67,8 @@ struct sjbg_handle {
     std::vector<double> kms;
     uint64_t launches = 0;
     bool capturing = false;
+    bool smj_full_sort = false;   // sort-merge: windows whose key ranges did not fit were met (smj_range.cu)
+    bool unwatched = false;       // the call being enqueued is not waited for: it must not need a second try
 
     // tunables (the autotuner picks them per workload shape)
     struct Tune {
@@ -184,6 +186,12 @@ int nlj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, c
 int smj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                    sjbg_pair *dPairs, WinAcc *acc, bool enumerate);
 
+// Sort-merge join by key ranges (smj_range.cu): whether the windows' sizes suit
+// it, and the call, whose status word holds kErrRegroup when a range did not fit.
+bool smj_range_fits(const WinHost *wins, uint32_t n);
+int smj_range_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                    WinAcc *acc);
+
 int generate_device(sjbg_handle *h, sjbg_tuple *out, uint64_t first, uint64_t n, uint64_t seed, uint64_t domain,
                     const uint64_t *table, uint64_t perm_seed);
 
@@ -196,6 +204,10 @@ int autotune_lazy(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
 // then the call's device status word in hAcc[n].info (kErr* bits).
 int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                     sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used);
+// run_lazy_device, waited for, and made again with the full sort when a
+// sort-merge join's key ranges did not fit.
+int run_lazy_watched(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                     sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used);
 // SJBG_OK, or the error a device status word reports (recorded on the handle).
 int device_status_error(sjbg_handle *h, unsigned long long bits);
 

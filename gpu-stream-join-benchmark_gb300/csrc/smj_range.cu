@@ -1,0 +1,566 @@
+// smj_range.cu - lazy sort-merge join by key ranges, counting (sm_103a).
+//
+// The counting form of the sort-merge join (smj.cu) when the windows' keys
+// spread evenly enough: a most-significant-first sort that ends in shared
+// memory.  The matching rule is the lazy CPU_SMJ's
+// (src/sjb/windowing/lazy/executor/CPU/CPU_SMJ.cpp:23-139).
+//   1. range_sample   per window: smallest and largest of a key sample -> a
+//                     linear map of keys to P ranges (keys outside the
+//                     sample's span fall into the end ranges: the map is
+//                     monotone whatever the sample saw);
+//   2. range_tiles    every tile of both sides sorted by range and written
+//                     whole with its offsets (tiles.cuh);
+//   3. range_join     persistent CTAs over the ranges: the left words of the
+//                     range come into shared memory, distributed over its
+//                     kRangeSubs equal subranges (a word or so each), and
+//                     every right word meets the left words of its subrange.
+//                     A range with a crowded subrange is sorted by the key
+//                     bits in which its words differ, and its right words
+//                     find their key groups by binary search: count += hi -
+//                     lo, prod += gs * (F[hi] - F[lo]), F the prefix sums of fr.
+// The tuples are read once, their words written and read once; the full radix
+// sort reads and writes them three or four times, and the merge once more
+// (128 windows of 2^10 to 2^20 tuples per side, keys in [0, 4 max(W)), 22.5 M
+// tuples: 1.64 ms).  A range that does not fit (hot or clustered keys) sets
+// kErrRegroup, and the host makes the call again with the full sort.
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "sort.cuh"
+#include "tiles.cuh"
+
+namespace sjbg {
+
+constexpr int kRangeThreads = 512;
+constexpr int kRangeWarps = kRangeThreads / 32;
+constexpr uint32_t kRangeCap = 4096;            // left words of a range (shared memory)
+constexpr uint32_t kRangeWords = 8192;          // words of both sides
+constexpr uint32_t kRangeTarget = 3328;         // words of the larger side per range: uneven ranges still fit
+constexpr uint32_t kRangesMax = 1024;           // more ranges: runs of under 4 words per tile
+constexpr uint32_t kRangeTilesMax = 1536;       // tiles of both sides of a window
+constexpr uint32_t kRangeDigit = 7;             // bits per shared-memory sorting pass
+constexpr uint32_t kRangeDigits = 1u << kRangeDigit;
+constexpr uint32_t kRangeSample = 8192;         // sampled keys per side
+constexpr uint32_t kRangeSubs = 2048;           // subranges of a range
+constexpr uint32_t kRangeCrowd = 16;            // most left words of a subrange that its right words are shown
+
+struct RangeWin {
+    uint64_t off[2], n[2];   // left, right
+    uint32_t tile[2];        // first tile of the side
+    uint32_t tiles[2];
+    uint32_t bucket0, P;     // first range of the call, ranges
+};
+
+// The window's map of keys to ranges.
+struct RangeMap {
+    uint32_t lo, span, mult, P;   // span 0: every key in its own range, from lo
+};
+
+__device__ __forceinline__ uint32_t range_of(const RangeMap &m, uint32_t key) {
+    const uint32_t d = key > m.lo ? key - m.lo : 0u, last = m.P - 1u;
+    if (m.span == 0u) return min(d, last);
+    return d >= m.span ? last : min(last, __umulhi(d, m.mult));
+}
+
+// Keys sampled from a side of n tuples: one in 256, at least 1,024, at most kRangeSample.
+__device__ __forceinline__ uint64_t range_samples(uint64_t n) {
+    return min(n, max((uint64_t)1024, min(n / 256, (uint64_t)kRangeSample)));
+}
+
+__global__ void __launch_bounds__(1024)
+range_sample_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
+                    const RangeWin *__restrict__ wins, RangeMap *__restrict__ maps) {
+    __shared__ uint32_t lo_s, hi_s;
+    const RangeWin w = wins[blockIdx.x];
+    if (threadIdx.x == 0) {
+        lo_s = 0xFFFFFFFFu;
+        hi_s = 0;
+    }
+    SJBG_BARRIER();
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+    for (uint32_t side = 0; side < 2; side++) {
+        const sjbg_tuple *src = (side ? R : L) + w.off[side];
+        const uint64_t n = w.n[side], m = range_samples(n);
+        uint32_t k[kRangeSample / 1024];
+#pragma unroll
+        for (uint32_t q = 0; q < kRangeSample / 1024; q++) {
+            const uint64_t i = threadIdx.x + q * 1024;
+            k[q] = i < m ? __ldg(&src[n == m ? i : i * n / m].key) : 0u;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kRangeSample / 1024; q++) {
+            if (threadIdx.x + q * 1024 < m) {
+                lo = min(lo, k[q]);
+                hi = max(hi, k[q]);
+            }
+        }
+    }
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    if (lane_id() == 0) {
+        atomicMin(&lo_s, lo);
+        atomicMax(&hi_s, hi);
+    }
+    SJBG_BARRIER();
+    if (threadIdx.x == 0) {
+        RangeMap m;
+        m.P = w.P;
+        m.lo = 0;
+        uint64_t span = 1;
+        if (lo_s <= hi_s) {
+            // the keys go a little beyond the sample's: by about span / sample at each end
+            const uint64_t sampled = max(max(range_samples(w.n[0]), range_samples(w.n[1])), (uint64_t)64);
+            const uint32_t more = (uint32_t)(((uint64_t)hi_s - lo_s) / sampled);
+            m.lo = lo_s > more ? lo_s - more : 0u;
+            span = (uint64_t)(hi_s < 0xFFFFFFFFu - more ? hi_s + more : 0xFFFFFFFFu) - m.lo + 1;
+        }
+        if (span <= w.P) {
+            m.span = m.mult = 0;
+        } else {
+            m.span = (uint32_t)(span > 0xFFFFFFFFull ? 0xFFFFFFFFull : span);
+            m.mult = (uint32_t)(((uint64_t)w.P << 32) / span);   // P < span: below 2^32
+        }
+        maps[blockIdx.x] = m;
+    }
+}
+
+struct RangeOf {
+    RangeMap m;
+    __device__ uint32_t operator()(uint32_t key) const { return range_of(m, key); }
+};
+
+__global__ void __launch_bounds__(kSortedThreads, 3)
+range_tiles_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
+                   const RangeWin *__restrict__ wins, uint32_t nwin, uint32_t tiles, const RangeMap *__restrict__ maps,
+                   uint32_t P, uint64_t *__restrict__ words, uint16_t *__restrict__ rows) {
+    sort_tiles(tiles, [&](uint32_t tile, SortedTile &t) {
+        uint32_t lo = 0, hi = nwin;   // largest w with tile[0] <= tile (a window's left tiles, then its right ones)
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (__ldg(&wins[mid].tile[0]) <= tile) lo = mid; else hi = mid;
+        }
+        const RangeWin &w = wins[lo];
+        const uint32_t right = tile >= w.tile[1] ? 1u : 0u;
+        const uint64_t start = (uint64_t)(tile - w.tile[right]) * kSortedTile, left = w.n[right] - start;
+        const RangeOf f{maps[lo]};
+        t.src = (right ? R : L) + w.off[right] + start;
+        t.n = (uint32_t)(left < kSortedTile ? left : kSortedTile);
+        t.P = f.m.P;
+        t.words = words + (uint64_t)tile * kSortedTile;
+        t.row = rows + (uint64_t)tile * sorted_row(P);   // (as long as the call's largest fan-out needs)
+        return f;
+    });
+}
+
+struct RangeSmem {
+    union {
+        uint64_t word[kRangeCap];                   // left words by subrange
+        uint32_t buf[2][2][kRangeCap];              // sorting: keys and vals, before and after a pass; then F in the free pair
+    };
+    union {
+        uint32_t sub[kRangeSubs + 1];               // first left word of each subrange, and their number
+        uint32_t wcnt[kRangeWarps][kRangeDigits + 1];   // sorting: per-warp digit counters (+ 1: no word)
+    };
+    uint32_t loc[kRangeDigits + 1];                 // first word of each digit of the last pass, and n
+    uint16_t off[kRangeTilesMax], pre[kRangeTilesMax];   // per tile (left side's first): the run, the words before it
+    uint16_t owner[kRangeWords];                    // tile of the range's i-th word
+    uint32_t warp_tot[32];
+    unsigned long long wsum[32];
+    uint32_t lo, hi, n_left, next, stop;
+};
+
+// One stable pass over the n left words in shared memory, on kRangeDigit bits
+// of key - lo from `shift`.  Warp-private counters; a lane's digit peers come
+// from one ballot per bit.
+__device__ __forceinline__ void range_pass(RangeSmem &sm, uint32_t from, uint32_t n, uint32_t lo, uint32_t shift) {
+    constexpr uint32_t kItems = kRangeCap / kRangeThreads;
+    const uint32_t w = warp_id(), lane = lane_id();
+    const uint32_t *keys = sm.buf[from][0], *vals = sm.buf[from][1];
+    uint32_t *ko = sm.buf[from ^ 1][0], *vo = sm.buf[from ^ 1][1];
+    for (uint32_t i = threadIdx.x; i < kRangeWarps * (kRangeDigits + 1); i += kRangeThreads) (&sm.wcnt[0][0])[i] = 0;
+    SJBG_BARRIER();
+    // warp w's positions [w * per, w * per + per), in order; per covers n evenly
+    const uint32_t rounds = (n + kRangeThreads - 1) / kRangeThreads, first = w * rounds * 32;
+    uint32_t rank[kItems], dig[kItems];
+    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; k++) {
+        if (k >= rounds) break;   // (the same for the whole CTA)
+        const uint32_t pos = first + k * 32 + lane;
+        const uint32_t d = pos < n ? ((keys[pos] - lo) >> shift) & (kRangeDigits - 1) : kRangeDigits;
+        unsigned peers = 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t b = 0; b <= kRangeDigit; b++) {
+            const bool bit = (d >> b) & 1u;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, bit);
+            peers &= bit ? m : ~m;
+        }
+        const uint32_t cur = sm.wcnt[w][d];
+        __syncwarp();
+        rank[k] = cur + __popc(peers & lt);
+        dig[k] = d;
+        if (lane == (uint32_t)(__ffs(peers) - 1)) sm.wcnt[w][d] = cur + __popc(peers);
+        __syncwarp();
+    }
+    SJBG_BARRIER();
+    // per digit: exclusive over the warps, four threads per digit and four warps
+    // per thread; then the digits' totals, by one warp
+    {
+        static_assert(kRangeThreads == 4 * kRangeDigits && kRangeWarps == 16, "four threads per digit");
+        const uint32_t digit = threadIdx.x >> 2, q0 = (threadIdx.x & 3u) * 4;
+        uint32_t c[4], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            c[q] = sm.wcnt[q0 + q][digit];
+            sum += c[q];
+        }
+        uint32_t run = sum;
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, run, o, 4);
+            if ((threadIdx.x & 3u) >= (uint32_t)o) run += y;
+        }
+        if ((threadIdx.x & 3u) == 3u) sm.loc[digit] = run;
+        run -= sum;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            sm.wcnt[q0 + q][digit] = run;
+            run += c[q];
+        }
+    }
+    SJBG_BARRIER();
+    if (w == 0) {
+        constexpr uint32_t kPer = kRangeDigits / 32;
+        uint32_t a[kPer], sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; q++) {
+            a[q] = sm.loc[lane * kPer + q];
+            sum += a[q];
+        }
+        uint32_t tot;
+        uint32_t run = warp_excl_scan(sum, &tot);
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; q++) {
+            sm.loc[lane * kPer + q] = run;
+            run += a[q];
+        }
+        if (lane == 31) sm.loc[kRangeDigits] = run;
+    }
+    SJBG_BARRIER();
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; k++) {
+        const uint32_t pos = first + k * 32 + lane;
+        if (k < rounds && pos < n) {
+            const uint32_t p = sm.loc[dig[k]] + sm.wcnt[w][dig[k]] + rank[k];
+            ko[p] = keys[pos];
+            vo[p] = vals[pos];
+        }
+    }
+    SJBG_BARRIER();
+}
+
+// Exclusive prefix sums of fr over the range's n sorted words; returns their
+// total to every thread; ends with a barrier.
+__device__ __forceinline__ unsigned long long range_prefix(RangeSmem &sm, const uint32_t *vals, uint32_t n,
+                                                           unsigned long long *F) {
+    const uint32_t lane = lane_id(), wid = warp_id();
+    const uint32_t rounds = (n + kRangeThreads - 1) / kRangeThreads, c0 = wid * rounds * 32;
+    unsigned long long wtot = 0;
+    for (uint32_t k = 0; k < rounds; k++) {
+        const uint32_t i = c0 + k * 32 + lane;
+        const unsigned long long f = i < n ? sjbg_fr(vals[i]) : 0ull;
+        unsigned long long x = f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (i < n) F[i] = wtot + x - f;   // within the warp's words
+        wtot += __shfl_sync(0xFFFFFFFFu, x, 31);
+    }
+    if (lane == 0) sm.wsum[wid] = wtot;
+    SJBG_BARRIER();
+    const unsigned long long s = lane < kRangeWarps ? sm.wsum[lane] : 0ull;
+    const unsigned long long base = warp_sum_u64(lane < wid ? s : 0ull), all = warp_sum_u64(s);
+    for (uint32_t k = 0; k < rounds; k++) {   // each warp its own words
+        const uint32_t i = c0 + k * 32 + lane;
+        if (i < n) F[i] += base;
+    }
+    SJBG_BARRIER();
+    return all;
+}
+
+__global__ void __launch_bounds__(kRangeThreads, 2)
+range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict__ rows,
+                  const RangeWin *__restrict__ wins, uint32_t nwin, uint32_t nb, uint32_t P,
+                  uint32_t *__restrict__ queue, WinAcc *__restrict__ acc, uint32_t *__restrict__ status) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    RangeSmem &sm = *reinterpret_cast<RangeSmem *>(smem_raw);
+    const uint32_t lane = lane_id(), wid = warp_id();
+    uint32_t g = blockIdx.x;   // the first range by position, the others from the queue
+    while (g < nb) {
+        uint32_t claim = 0;
+        if (threadIdx.x == 0) {
+            claim = gridDim.x + atomicAdd(queue, 1u);   // stored once this range is done
+            sm.stop = *(volatile uint32_t *)status & kErrRegroup;
+            sm.lo = 0xFFFFFFFFu;
+            sm.hi = 0;
+        }
+        uint32_t wlo = 0, whi = nwin;   // the range's window
+        while (whi - wlo > 1) {
+            const uint32_t mid = (wlo + whi) >> 1;
+            if (__ldg(&wins[mid].bucket0) <= g) wlo = mid; else whi = mid;
+        }
+        const RangeWin &w = wins[wlo];
+        const uint32_t TL = w.tiles[0], T = TL + w.tiles[1], tile0 = w.tile[0];   // (its right tiles follow its left ones)
+        const uint16_t *rw = rows + (uint64_t)tile0 * sorted_row(P) + (g - w.bucket0);
+        constexpr uint32_t kPerMax = kRangeTilesMax / kRangeThreads;
+        const uint32_t per = (T + kRangeThreads - 1) / kRangeThreads, x0 = threadIdx.x * per;
+        uint32_t len[kPerMax], sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPerMax; q++) {
+            const uint32_t x = x0 + q;
+            len[q] = 0;
+            if (q < per && x < T) {
+                const uint16_t *r = rw + (uint64_t)x * sorted_row(P);
+                const uint32_t o = __ldg(r);
+                len[q] = __ldg(r + 1) - o;
+                sm.off[x] = (uint16_t)o;
+            }
+            sum += len[q];
+        }
+        uint32_t tot;
+        uint32_t run = warp_excl_scan(sum, &tot);
+        if (lane == 31) sm.warp_tot[wid] = tot;
+        SJBG_BARRIER();
+        const uint32_t v = lane < kRangeWarps ? sm.warp_tot[lane] : 0u;
+        const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, v);
+        run += __reduce_add_sync(0xFFFFFFFFu, lane < wid ? v : 0u);
+        if (sm.stop || n > kRangeWords) {   // (the same for the whole CTA)
+            if (threadIdx.x == 0) atomicOr(status, kErrRegroup);
+            return;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kPerMax; q++) {
+            const uint32_t x = x0 + q;
+            if (q < per && x < T) {
+                sm.pre[x] = (uint16_t)run;
+                if (x == TL) sm.n_left = run;
+                for (uint32_t m = 0; m < len[q]; m++) sm.owner[run + m] = (uint16_t)x;
+            }
+            run += len[q];
+        }
+        if (TL == T && threadIdx.x == 0) sm.n_left = n;
+        SJBG_BARRIER();
+        const uint32_t nl = sm.n_left;
+        if (nl > kRangeCap) {   // (the same for the whole CTA)
+            if (threadIdx.x == 0) atomicOr(status, kErrRegroup);
+            return;
+        }
+        auto word = [&](uint32_t i) {
+            const uint32_t x = sm.owner[i];
+            return __ldg(words + (uint64_t)(tile0 + x) * kSortedTile + (sm.off[x] + (i - sm.pre[x])));
+        };
+        if (nl != 0 && nl != n) {
+            // the left words, and the span of their keys
+            constexpr uint32_t kItems = kRangeCap / kRangeThreads;
+            uint64_t e[kItems];
+            uint32_t klo = 0xFFFFFFFFu, khi = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kItems; k++) {
+                const uint32_t i = threadIdx.x + k * kRangeThreads;
+                e[k] = i < nl ? word(i) : 0ull;
+            }
+            for (uint32_t i = threadIdx.x; i <= kRangeSubs; i += kRangeThreads) sm.sub[i] = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kItems; k++) {
+                if (threadIdx.x + k * kRangeThreads < nl) {
+                    klo = min(klo, (uint32_t)e[k]);
+                    khi = max(khi, (uint32_t)e[k]);
+                }
+            }
+            klo = __reduce_min_sync(0xFFFFFFFFu, klo);
+            khi = __reduce_max_sync(0xFFFFFFFFu, khi);
+            if (lane == 0) {
+                atomicMin(&sm.lo, klo);
+                atomicMax(&sm.hi, khi);
+            }
+            SJBG_BARRIER();
+            const uint32_t lo = sm.lo, hi = sm.hi;
+            // the subrange of a key in [lo, hi] (the same rounding for every holder of the key)
+            const float scale = (float)kRangeSubs / ((float)(hi - lo) + 1.0f);
+            auto sub_of = [&](uint32_t key) { return min(kRangeSubs - 1, (uint32_t)((float)(key - lo) * scale)); };
+            uint32_t rank[kItems];
+#pragma unroll
+            for (uint32_t k = 0; k < kItems; k++)
+                if (threadIdx.x + k * kRangeThreads < nl) rank[k] = atomicAdd(&sm.sub[sub_of((uint32_t)e[k])], 1u);
+            SJBG_BARRIER();
+            bool crowded = false;
+            {
+                constexpr uint32_t kPer = kRangeSubs / kRangeThreads;
+                uint32_t c[kPer], csum = 0;
+#pragma unroll
+                for (uint32_t q = 0; q < kPer; q++) {
+                    c[q] = sm.sub[threadIdx.x * kPer + q];
+                    csum += c[q];
+                    crowded |= c[q] > kRangeCrowd;
+                }
+                uint32_t ctot;
+                uint32_t crun = warp_excl_scan(csum, &ctot);
+                if (lane == 31) sm.warp_tot[wid] = ctot;
+                crowded = __syncthreads_or(crowded);
+                crun += __reduce_add_sync(0xFFFFFFFFu, lane < wid ? sm.warp_tot[lane] : 0u);
+#pragma unroll
+                for (uint32_t q = 0; q < kPer; q++) {
+                    sm.sub[threadIdx.x * kPer + q] = crun;
+                    crun += c[q];
+                }
+                if (threadIdx.x == kRangeThreads - 1) sm.sub[kRangeSubs] = crun;
+            }
+            unsigned long long count = 0, prod = 0;
+            if (!crowded) {
+                SJBG_BARRIER();
+#pragma unroll
+                for (uint32_t k = 0; k < kItems; k++)
+                    if (threadIdx.x + k * kRangeThreads < nl) sm.word[sm.sub[sub_of((uint32_t)e[k])] + rank[k]] = e[k];
+                SJBG_BARRIER();
+                for (uint32_t i = nl + threadIdx.x; i < n; i += 4 * kRangeThreads) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; q++) e[q] = i + q * kRangeThreads < n ? word(i + q * kRangeThreads) : 0ull;
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; q++) {
+                        const uint32_t key = (uint32_t)e[q];
+                        if (i + q * kRangeThreads >= n || key < lo || key > hi) continue;
+                        const uint32_t b = sub_of(key), end = sm.sub[b + 1];
+                        uint32_t c = 0;
+                        unsigned long long f = 0;
+                        for (uint32_t j = sm.sub[b]; j < end; j++) {
+                            const uint64_t x = sm.word[j];
+                            if ((uint32_t)x == key) {
+                                c++;
+                                f += sjbg_fr((uint32_t)(x >> 32));
+                            }
+                        }
+                        if (c) {
+                            count += c;
+                            prod += f * sjbg_gs((uint32_t)(e[q] >> 32));
+                        }
+                    }
+                }
+            } else {
+#pragma unroll
+                for (uint32_t k = 0; k < kItems; k++) {
+                    const uint32_t i = threadIdx.x + k * kRangeThreads;
+                    if (i < nl) {
+                        sm.buf[0][0][i] = (uint32_t)e[k];
+                        sm.buf[0][1][i] = (uint32_t)(e[k] >> 32);
+                    }
+                }
+                SJBG_BARRIER();   // (sub is read by now: its space holds the sort's counters)
+                const uint32_t bits = 32u - (uint32_t)__clz(hi - lo);   // (0: one key)
+                uint32_t at = 0;   // the buffer pair that holds the words
+                for (uint32_t shift = 0; shift < bits; shift += kRangeDigit, at ^= 1u) range_pass(sm, at, nl, lo, shift);
+                const uint32_t *keys = sm.buf[at][0], *vals = sm.buf[at][1];
+                unsigned long long *F = reinterpret_cast<unsigned long long *>(&sm.buf[at ^ 1][0][0]);
+                const unsigned long long all = range_prefix(sm, vals, nl, F);   // ends with a barrier
+                // right words: the words of the key's top digit, then its group among them
+                const uint32_t shift = bits ? (bits - 1) / kRangeDigit * kRangeDigit : 0u;   // of the last pass
+                for (uint32_t i = nl + threadIdx.x; i < n; i += kRangeThreads) {
+                    const uint64_t x = word(i);
+                    const uint32_t key = (uint32_t)x;
+                    if (key < lo || key > hi) continue;
+                    uint32_t l = 0, r = nl;
+                    if (bits) {
+                        const uint32_t digit = (key - lo) >> shift;
+                        l = sm.loc[digit];
+                        r = sm.loc[digit + 1];
+                    }
+                    const uint32_t end = r;
+                    while (l < r) {
+                        const uint32_t mid = (l + r) >> 1;
+                        if (keys[mid] < key) l = mid + 1; else r = mid;
+                    }
+                    if (l >= end || keys[l] != key) continue;
+                    uint32_t h = l + 1;
+                    r = end;
+                    while (h < r) {
+                        const uint32_t mid = (h + r) >> 1;
+                        if (keys[mid] <= key) h = mid + 1; else r = mid;
+                    }
+                    count += h - l;
+                    prod += ((h < nl ? F[h] : all) - F[l]) * sjbg_gs((uint32_t)(x >> 32));
+                }
+            }
+            flush_acc(&acc[wlo], count, 0ull, prod);
+        }
+        if (threadIdx.x == 0) sm.next = claim;
+        SJBG_BARRIER();
+        g = sm.next;
+        SJBG_BARRIER();   // read before the next claim is stored
+    }
+}
+
+bool smj_range_fits(const WinHost *wins, uint32_t n) {
+    for (uint32_t w = 0; w < n; w++) {
+        const uint64_t most = std::max(wins[w].n_left, wins[w].n_right);
+        if (most > (uint64_t)kRangeTarget * kRangesMax) return false;
+        if ((wins[w].n_left + kSortedTile - 1) / kSortedTile + (wins[w].n_right + kSortedTile - 1) / kSortedTile >
+            kRangeTilesMax)
+            return false;
+    }
+    return true;
+}
+
+int smj_range_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                    WinAcc *acc) {
+    std::vector<RangeWin> rw(n);
+    uint64_t tiles = 0, nb = 0;
+    uint32_t pmax = 1;
+    for (uint32_t w = 0; w < n; w++) {
+        RangeWin &r = rw[w];
+        std::memset(&r, 0, sizeof(r));
+        r.off[0] = wins[w].left_off; r.n[0] = wins[w].n_left;
+        r.off[1] = wins[w].right_off; r.n[1] = wins[w].n_right;
+        const bool empty = r.n[0] == 0 || r.n[1] == 0;   // (nothing of such a window is read)
+        r.P = (uint32_t)((std::max(r.n[0], r.n[1]) + kRangeTarget - 1) / kRangeTarget);
+        for (int s = 0; s < 2; s++) {
+            r.tile[s] = (uint32_t)tiles;
+            r.tiles[s] = empty ? 0u : (uint32_t)((r.n[s] + kSortedTile - 1) / kSortedTile);
+            tiles += r.tiles[s];
+        }
+        r.bucket0 = (uint32_t)nb;
+        nb += empty ? 0u : r.P;
+        pmax = std::max(pmax, r.P);
+    }
+    if (tiles > 0x7FFFFFFFull || nb > 0x7FFFFFFFull)
+        return fail(h, SJBG_E_CAPACITY, "sort-merge batch has too many tiles");
+    if (nb == 0) return SJBG_OK;
+    const size_t upB = sizeof(RangeWin) * n;
+    uint8_t *hst = static_cast<uint8_t *>(pinned_get(h, 0, upB));
+    uint8_t *dev = static_cast<uint8_t *>(ws_get(h, WS_WIN_PLAN, upB));
+    uint64_t *words = static_cast<uint64_t *>(ws_get(h, WS_SORT_K0, sizeof(uint64_t) * kSortedTile * tiles));
+    uint16_t *rows = static_cast<uint16_t *>(ws_get(h, WS_SORT_HIST, sizeof(uint16_t) * sorted_row(pmax) * tiles));
+    RangeMap *maps = static_cast<RangeMap *>(ws_get(h, WS_SORT_MAP, sizeof(RangeMap) * n));
+    uint32_t *queue = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_WIN, 64));
+    if (!hst || !dev || !words || !rows || !maps || !queue) return fail(h, SJBG_E_NOMEM, "sort-merge buffers");
+    std::memcpy(hst, rw.data(), upB);
+    if (int rc = stage_copy_zero(h, dev, hst, upB, queue, 64)) return rc;
+    const RangeWin *dW = reinterpret_cast<const RangeWin *>(dev);
+    SJBG_CK(h, launch(h, "range_sample", range_sample_kernel, dim3(n), dim3(1024), 0, dL, dR, dW, maps));
+    const size_t s1 = sorted_tile_bytes(pmax), s2 = sizeof(RangeSmem);
+    allow_big_smem(range_tiles_kernel, s1);
+    SJBG_CK(h, launch(h, "range_tiles", range_tiles_kernel,
+                      dim3((uint32_t)std::min<uint64_t>(tiles, 3u * (uint64_t)std::max(h->num_sms, 1))),
+                      dim3(kSortedThreads), s1, dL, dR, dW, n, (uint32_t)tiles, (const RangeMap *)maps, pmax, words,
+                      rows));
+    allow_big_smem(range_join_kernel, s2);
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(nb, 2u * (uint64_t)std::max(h->num_sms, 1));
+    SJBG_CK(h, launch(h, "range_join", range_join_kernel, dim3(grid), dim3(kRangeThreads), s2, (const uint64_t *)words,
+                      (const uint16_t *)rows, dW, n, (uint32_t)nb, pmax, queue, acc,
+                      reinterpret_cast<uint32_t *>(&acc[n].info)));
+    return SJBG_OK;
+}
+
+}  // namespace sjbg

@@ -6,8 +6,8 @@
 // a row of its buckets' offsets.  Nothing is counted beforehand and no global
 // position is reserved: one read of the tuples, one coalesced write of half
 // their bytes, no atomic outside shared memory.  A bucket is then the runs
-// row[b] .. row[b + 1] of all tiles, in tile order; with 2^lg buckets a run
-// has about kSortedTile / 2^lg words.
+// row[b] .. row[b + 1] of all tiles, in tile order; with P buckets a run has
+// about kSortedTile / P words.
 #pragma once
 
 #include "runtime.h"
@@ -18,12 +18,12 @@ constexpr uint32_t kSortedTile = 4096;
 constexpr int kSortedThreads = 512;
 constexpr int kSortedPer = kSortedTile / kSortedThreads;
 
-// Row length in 16-bit words: offsets of 2^lg buckets and the end, 16-byte rows.
-__host__ __device__ __forceinline__ uint32_t sorted_row(uint32_t lg) { return (1u << lg) + 8u; }
+// Row length in 16-bit words: offsets of P buckets and the end.
+__host__ __device__ __forceinline__ uint32_t sorted_row(uint32_t P) { return (P + 8u) & ~7u; }
 
 // Shared memory of sort_tile.
-static inline size_t sorted_tile_bytes(uint32_t lg) {
-    return sizeof(uint64_t) * kSortedTile + sizeof(uint32_t) * (size_t)(1u << lg);
+static inline size_t sorted_tile_bytes(uint32_t P) {
+    return sizeof(uint64_t) * kSortedTile + sizeof(uint32_t) * (size_t)P;
 }
 
 // Block-wide exclusive scan of P shared counters in place.
@@ -51,42 +51,74 @@ __device__ __forceinline__ void tile_scan(uint32_t *a, uint32_t P, uint32_t *war
     SJBG_BARRIER();
 }
 
-// Sorts the n <= kSortedTile tuples at src by bucket_of(key) in [0, 2^lg) into
-// words[0 .. n) (16-byte aligned) and writes their row.  All kSortedThreads
-// threads call it.
-template <typename BucketOf>
-__device__ __forceinline__ void sort_tile(const sjbg_tuple *__restrict__ src, uint32_t n, uint32_t lg,
-                                          uint64_t *__restrict__ words, uint16_t *__restrict__ row,
-                                          BucketOf bucket_of) {
+// Where a tile's tuples lie and its sorted words and row go.
+struct SortedTile {
+    const sjbg_tuple *src;
+    uint64_t *words;   // 16-byte aligned
+    uint16_t *row;
+    uint32_t n, P;     // n <= kSortedTile tuples, P buckets
+};
+
+// Sorts tiles blockIdx.x, blockIdx.x + gridDim.x, ... of `count`: tile_of(i, t)
+// fills t and returns the tile's map of keys to buckets [0, P).  All
+// kSortedThreads threads call it.  A tile's tuples are loaded while the one
+// before it is written out (its registers are free by then), and are on their
+// way into L2 before that.
+template <typename TileOf>
+__device__ __forceinline__ void sort_tiles(uint32_t count, TileOf tile_of) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ uint32_t warp_tot[32];
     uint64_t *stage = reinterpret_cast<uint64_t *>(smem_raw);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(stage + kSortedTile);
-    const uint32_t P = 1u << lg;
+    uint32_t it = blockIdx.x;
+    if (it >= count) return;
     uint2 v[kSortedPer];
+    auto load = [&](const SortedTile &t) {
 #pragma unroll
-    for (int k = 0; k < kSortedPer; k++) {
-        const uint32_t i = threadIdx.x + k * kSortedThreads;
-        v[k] = i < n ? __ldg(reinterpret_cast<const uint2 *>(src + i)) : make_uint2(0u, 0u);
+        for (int k = 0; k < kSortedPer; k++) {
+            const uint32_t i = threadIdx.x + k * kSortedThreads;
+            v[k] = i < t.n ? __ldg(reinterpret_cast<const uint2 *>(t.src + i)) : make_uint2(0u, 0u);
+        }
+    };
+    SortedTile t;
+    auto bucket_of = tile_of(it, t);
+    load(t);
+    for (;;) {
+        for (uint32_t i = threadIdx.x; i < t.P; i += kSortedThreads) cnt[i] = 0;
+        SJBG_BARRIER();
+        uint32_t br[kSortedPer];   // bucket << 16 | rank in the tile's bucket
+#pragma unroll
+        for (int k = 0; k < kSortedPer; k++)
+            if (threadIdx.x + k * kSortedThreads < t.n) {
+                const uint32_t b = bucket_of(v[k].x);
+                br[k] = (b << 16) | atomicAdd(&cnt[b], 1u);
+            }
+        const uint32_t nit = it + gridDim.x;
+        const bool more = nit < count;
+        SortedTile nt = t;
+        auto nbucket_of = bucket_of;
+        if (more) {
+            nbucket_of = tile_of(nit, nt);
+            if (threadIdx.x == 0) l2_prefetch_bulk(nt.src, sizeof(sjbg_tuple) * nt.n);
+        }
+        SJBG_BARRIER();
+        tile_scan(cnt, t.P, warp_tot);
+#pragma unroll
+        for (int k = 0; k < kSortedPer; k++)
+            if (threadIdx.x + k * kSortedThreads < t.n)
+                stage[cnt[br[k] >> 16] + (br[k] & 0xFFFFu)] = ((uint64_t)v[k].y << 32) | v[k].x;
+        for (uint32_t i = threadIdx.x; i < t.P; i += kSortedThreads) t.row[i] = (uint16_t)cnt[i];
+        if (threadIdx.x == 0) t.row[t.P] = (uint16_t)t.n;
+        if (more) load(nt);
+        SJBG_BARRIER();
+        const uint4 *s4 = reinterpret_cast<const uint4 *>(stage);
+        for (uint32_t i = threadIdx.x; i < t.n / 2; i += kSortedThreads) reinterpret_cast<uint4 *>(t.words)[i] = s4[i];
+        if ((t.n & 1u) && threadIdx.x == 0) t.words[t.n - 1] = stage[t.n - 1];
+        if (!more) return;
+        it = nit;
+        t = nt;
+        bucket_of = nbucket_of;
     }
-    for (uint32_t i = threadIdx.x; i < P; i += kSortedThreads) cnt[i] = 0;
-    SJBG_BARRIER();
-    uint32_t rank[kSortedPer];
-#pragma unroll
-    for (int k = 0; k < kSortedPer; k++)
-        if (threadIdx.x + k * kSortedThreads < n) rank[k] = atomicAdd(&cnt[bucket_of(v[k].x)], 1u);
-    SJBG_BARRIER();
-    tile_scan(cnt, P, warp_tot);
-#pragma unroll
-    for (int k = 0; k < kSortedPer; k++)
-        if (threadIdx.x + k * kSortedThreads < n)
-            stage[cnt[bucket_of(v[k].x)] + rank[k]] = ((uint64_t)v[k].y << 32) | v[k].x;
-    for (uint32_t i = threadIdx.x; i < P; i += kSortedThreads) row[i] = (uint16_t)cnt[i];
-    if (threadIdx.x == 0) row[P] = (uint16_t)n;
-    SJBG_BARRIER();
-    const uint4 *s4 = reinterpret_cast<const uint4 *>(stage);
-    for (uint32_t i = threadIdx.x; i < n / 2; i += kSortedThreads) reinterpret_cast<uint4 *>(words)[i] = s4[i];
-    if ((n & 1u) && threadIdx.x == 0) words[n - 1] = stage[n - 1];
 }
 
 }  // namespace sjbg
