@@ -229,6 +229,10 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
         if (int rc = hj_raw_batch(h, dL, dR, wins, n, hAcc, &done)) return rc;
         if (done) return SJBG_OK;
     }
+    if (n && !enumerate && h->cfg.algorithm != SJBG_ALG_NLJ && range_join_pays(h, wins, n)) {
+        *part_used = h->cfg.algorithm == SJBG_ALG_HJ ? SJBG_PART_RADIX : SJBG_PART_NONE;
+        return range_join_batch(h, dL, dR, wins, n, hAcc, h->cfg.algorithm == SJBG_ALG_HJ);
+    }
     // acc[n].info is the call's device status word (kErr* bits)
     WinAcc *acc = static_cast<WinAcc *>(ws_get(h, WS_WIN_ACC, sizeof(WinAcc) * (n + 1)));
     if (!acc) return fail(h, SJBG_E_NOMEM, "window accumulators");
@@ -250,8 +254,8 @@ int run_lazy_watched(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
     for (;;) {
         if (int rc = run_lazy_device(h, dL, dR, wins, n, dPairs, hAcc, part_used)) return rc;
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
-        if (!(hAcc[n].info & kErrRegroup) || h->smj_full_sort) return SJBG_OK;
-        h->smj_full_sort = true;   // (from now on, on this handle)
+        if (!(hAcc[n].info & kErrRegroup) || h->regrouped) return SJBG_OK;
+        h->regrouped = true;   // (from now on, on this handle)
     }
 }
 
@@ -288,12 +292,12 @@ static void fill_result(const sjbg_handle *h, const WinAcc &a, const WinHost &w,
 // Batched lazy call on device inputs through a cached CUDA graph: the first
 // call with a given signature runs normally (sizing every workspace), then is
 // captured with private pinned staging buffers; later identical calls replay it.
-constexpr size_t kGraphKeySort = 11;   // smj_full_sort's place in a graph's key
+constexpr size_t kGraphKeyRegrouped = 11;   // regrouped's place in a graph's key
 static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                       sjbg_pair *dPairs, bool enumerate, sjbg_window_result *out) {
     std::vector<uint64_t> key = {h->cfg.algorithm, h->cfg.partitioner, h->tune.partitioner, h->cfg.flags, h->cfg.result_mode,
                                  (uint64_t)(uintptr_t)dL, (uint64_t)(uintptr_t)dR, (uint64_t)(uintptr_t)dPairs, n,
-                                 h->tune.bucket_target, (uint64_t)h->tune.persistent_join, (uint64_t)h->smj_full_sort,
+                                 h->tune.bucket_target, (uint64_t)h->tune.persistent_join, (uint64_t)h->regrouped,
                                  (uint64_t)(uintptr_t)h->stream};
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &x = wins[w];
@@ -321,7 +325,7 @@ static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR
         SJBG_CK(h, cudaEventRecord(e1, h->stream));
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
         profile_collect(h);
-        key[kGraphKeySort] = (uint64_t)h->smj_full_sort;   // (it may have been met just now)
+        key[kGraphKeyRegrouped] = (uint64_t)h->regrouped;   // (it may have been met just now)
         auto e = std::make_unique<sjbg_handle::GraphEntry>();
         e->key = key;
         e->part_used = part_used;
@@ -373,8 +377,8 @@ static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR
     cudaEventElapsedTime(&ms, e0, e1);
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
-    if ((hAcc[n].info & kErrRegroup) && !h->smj_full_sort) {   // a replay met keys that do not fit: the other graph
-        h->smj_full_sort = true;
+    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // a replay met keys that do not fit: the general path's graph
+        h->regrouped = true;
         return lazy_graph(h, dL, dR, wins, n, dPairs, enumerate, out);
     }
     if (int se = device_status_error(h, hAcc[n].info)) return se;
@@ -566,8 +570,8 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
     profile_collect(h);
-    if ((hAcc[n].info & kErrRegroup) && !h->smj_full_sort) {   // (a counting sort-merge join: no pairs were written)
-        h->smj_full_sort = true;
+    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (a counting join: no pairs were written)
+        h->regrouped = true;
         return lazy_common(h, L, R, mem, wins, n, pairs, out);
     }
     if (int se = device_status_error(h, hAcc[n].info)) return se;

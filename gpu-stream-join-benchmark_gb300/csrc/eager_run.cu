@@ -441,11 +441,9 @@ struct EGroupWin {
 };
 
 __device__ __forceinline__ uint32_t group_bucket(uint32_t key, uint32_t lg) {
-    return lg ? (key * 0x9E3779B1u) >> (32u - lg) : 0u;
+    return lg ? bucket_hash(key) >> (32u - lg) : 0u;
 }
-__device__ __forceinline__ uint32_t group_slot(uint32_t key) {   // independent of the bucket's bits
-    return (key * 0x85EBCA6Bu) >> 21;
-}
+__device__ __forceinline__ uint32_t group_slot(uint32_t key) { return place_hash(key) >> 21; }
 static_assert(kGroupSlots == 1u << 11, "group_slot takes 11 bits");
 
 __global__ void __launch_bounds__(kSortedThreads, 3)

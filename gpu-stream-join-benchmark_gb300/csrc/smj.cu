@@ -6,8 +6,8 @@
 // is the lazy CPU_SMJ's (src/sjb/windowing/lazy/executor/CPU/CPU_SMJ.cpp:23-139):
 // both sides sorted by key, then every key group's cartesian product.
 //
-// Counting joins of windows whose keys spread evenly go by key ranges instead
-// (smj_range.cu).  Steps for a batch of windows (left sides are segments [0, n), right sides
+// Counting joins that are waited for go by key ranges instead when the windows'
+// sizes and keys suit them (range_join.cu).  Steps for a batch of windows (left sides are segments [0, n), right sides
 // [n, 2n) of one segmented sort):
 //   1. sort_extract + radix_sort_segments (sort.cu): stable LSD sort of
 //      (key, val) for every window side;
@@ -184,10 +184,6 @@ int smj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, c
         lens[n + w] = wins[w].n_right;
         srcs[n + w] = wins[w].right_off;
     }
-    // counting joins go by key ranges (smj_range.cu), unless the handle has met
-    // windows whose ranges did not fit, or nobody waits for the call's status
-    if (!enumerate && !h->smj_full_sort && !h->unwatched && smj_range_fits(wins, n))
-        return smj_range_batch(h, dL, dR, wins, n, acc);
     SortPlan plan = sort_plan(lens.data(), srcs.data(), 2 * n);
     std::vector<MergeWin> mw(n);
     uint32_t cuts = 0, tiles = 0;

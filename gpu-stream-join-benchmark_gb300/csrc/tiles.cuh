@@ -26,6 +26,16 @@ static inline size_t sorted_tile_bytes(uint32_t P) {
     return sizeof(uint64_t) * kSortedTile + sizeof(uint32_t) * (size_t)P;
 }
 
+// Multiplicative hash that picks a key's bucket (from its top bits), and the
+// bits that spread a bucket's keys.  The second is not another multiple of the
+// key: for dense keys the pairs of two multiples form a lattice, and one
+// bucket's keys then crowd on a few places of the second.
+__device__ __forceinline__ uint32_t bucket_hash(uint32_t key) { return key * 0x9E3779B1u; }
+__device__ __forceinline__ uint32_t place_hash(uint32_t key) {
+    const uint32_t h = bucket_hash(key);
+    return (h ^ (h >> 13)) * 0x85EBCA6Bu;
+}
+
 // Block-wide exclusive scan of P shared counters in place.
 __device__ __forceinline__ void tile_scan(uint32_t *a, uint32_t P, uint32_t *warp_tot) {
     const uint32_t per = (P + blockDim.x - 1) / blockDim.x;

@@ -80,3 +80,34 @@ def test_calls_of_small_windows_only(lib, oracle, windows, kind, graph):
             got = j.lazy_execute_batch(dl, dr, descs, mem=lib.MEM_DEVICE)
             for d, g, w in zip(descs, got, want):
                 assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
+
+
+MIDDLE = [(40_000, 30_001), (4096, 4097), (3328, 6657), (1, 70_000), (0, 9000), (100_000, 100), (65_536, 65_537)]
+
+
+@pytest.mark.parametrize("where", ["device", "host", "graph"])
+@pytest.mark.parametrize("kind", ["dense", "wide", "hot", "thick"])
+def test_calls_of_the_middle_sizes(lib, oracle, kind, where):
+    """Hash ranges finished in shared memory; keys whose ranges do not fit (hot, or
+    each key a thousand times) send the call to the general path."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(8)
+    lefts, rights, descs, lo, ro = [], [], [], 0, 0
+    for nl, nr in MIDDLE:
+        make = (lambda n: rng.integers(0, 90, n, dtype=np.uint32)) if kind == "thick" else \
+            (lambda n: keys_of(kind, n, rng))
+        lefts.append(make(nl))
+        rights.append(make(nr))
+        descs.append((lo, nl, ro, nr, 0, 0))
+        lo, ro = lo + nl, ro + nr
+    left, right = make_tuples(np.concatenate(lefts)), make_tuples(np.concatenate(rights))
+    want, _ = oracle.join_windows(left, right, descs, enumerate_pairs=False)
+    mem = lib.MEM_HOST if where == "host" else lib.MEM_DEVICE
+    if where != "host":
+        left, right = torch.from_numpy(left.view(np.uint8)).cuda(), torch.from_numpy(right.view(np.uint8)).cuda()
+    with lib.Joiner(lib.ALG_HJ, lib.LAZY, flags=lib.F_GRAPH if where == "graph" else 0,
+                    max_tuples_per_window=1 << 17) as j:
+        for _ in range(3):
+            got = j.lazy_execute_batch(left, right, descs, mem=mem)
+            for d, g, w in zip(descs, got, want):
+                assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
