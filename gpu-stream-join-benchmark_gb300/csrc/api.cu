@@ -229,9 +229,9 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
         if (int rc = hj_raw_batch(h, dL, dR, wins, n, hAcc, &done)) return rc;
         if (done) return SJBG_OK;
     }
-    if (n && !enumerate && h->cfg.algorithm != SJBG_ALG_NLJ && range_join_pays(h, wins, n)) {
+    if (n && h->cfg.algorithm != SJBG_ALG_NLJ && range_join_pays(h, wins, n)) {
         *part_used = h->cfg.algorithm == SJBG_ALG_HJ ? SJBG_PART_RADIX : SJBG_PART_NONE;
-        return range_join_batch(h, dL, dR, wins, n, hAcc, h->cfg.algorithm == SJBG_ALG_HJ);
+        return range_join_batch(h, dL, dR, wins, n, dPairs, hAcc, enumerate, h->cfg.algorithm == SJBG_ALG_HJ);
     }
     // acc[n].info is the call's device status word (kErr* bits)
     WinAcc *acc = static_cast<WinAcc *>(ws_get(h, WS_WIN_ACC, sizeof(WinAcc) * (n + 1)));
@@ -555,6 +555,10 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     if (mem == SJBG_MEM_HOST && want) {
         // copy back each window's written pairs
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
+        if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (the general path, before anything is copied back)
+            h->regrouped = true;
+            if (int rc2 = run_lazy_watched(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc2;
+        }
         if (int se = device_status_error(h, hAcc[n].info)) return se;
         for (uint32_t w = 0; w < n; w++) {
             const uint64_t np = std::min<uint64_t>(hAcc[w].npairs, wins[w].pairs_cap);
@@ -570,7 +574,7 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
     profile_collect(h);
-    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (a counting join: no pairs were written)
+    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (pairs written so far are written over)
         h->regrouped = true;
         return lazy_common(h, L, R, mem, wins, n, pairs, out);
     }

@@ -39,6 +39,7 @@
 
 #include "learned.cuh"
 #include "runtime.h"
+#include "tiles.cuh"
 
 namespace sjbg {
 
@@ -1178,7 +1179,9 @@ constexpr int kJoinPer = 8;   // elements per thread per tile (independent loads
 // kJoinChunkEnum when pairs are enumerated.
 constexpr uint32_t kJoinChunk = 65536;
 constexpr uint32_t kJoinChunkMin = 2048, kJoinChunkEnum = 16384;
-constexpr uint32_t kRawPiece = 1024;   // least build and probe tuples of a raw-only call's items
+// Build and probe tuples of a raw-only call's items: at least kRawPiece; square
+// pieces of up to kRawPieceMost, when they make one wave of CTAs.
+constexpr uint32_t kRawPiece = 1024, kRawPieceMost = 4096;
 
 // A run of tuples: (val << 32 | key) words of a partitioned array, or (kRaw)
 // the key and val of 16-byte tuples.
@@ -1214,25 +1217,120 @@ __device__ __forceinline__ JoinRuns join_runs(const JoinItem &ji, const sjbg_tup
     return r;
 }
 
-// Key filter of a hash-table bucket: about 32 bits per build tuple (at most
-// 2^kFilterBits), one set per build key.  Most probes of mostly distinct keys
-// match nothing; walking the table for them is what a bucket's time went on
-// (every lane of a warp waits for the longest walk).  The filter answers a
-// miss with one shared load, and the survivors are gathered per warp and
-// looked up 32 at a time.  Measured on 1,024 windows whose sides have
-// independent sizes, log-uniform in [2^10, 2^20], keys in [0, 4 max(W)): the
-// bucket joins took 4.17 ms without the filter and with a failed direct-table
-// build in most buckets, 1.78 ms with it and the range known beforehand
-// (pieces of up to 65,536 probes rather than 16,384 among it).
-constexpr uint32_t kFilterBits = 17;
-constexpr uint32_t kQueueSlots = 64;   // per warp: fewer than 32 waiting, and up to 32 more of one step
-
-__device__ __forceinline__ uint32_t filter_hash(uint32_t key) { return key * 0x9E3779B1u; }
-
-// The bucket's table in shared memory (cap slots, filter, survivor queues).
+// The bucket's count table in shared memory (cap slots).
 static inline size_t count_table_bytes(uint32_t cap) {
-    return sizeof(unsigned long long) * (kJoinThreads / 32) * kQueueSlots +
-           (sizeof(unsigned long long) + 2 * sizeof(uint32_t)) * ((size_t)cap + 1) + (1u << kFilterBits) / 8;
+    return (sizeof(unsigned long long) + 2 * sizeof(uint32_t)) * ((size_t)cap + 1);
+}
+
+// ---- bucket join by places
+// The build run is distributed over `places` short lists (about two tuples
+// each) by a hash of the key: one pass counts the places, a scan gives their
+// starts, a second pass writes the (key, val) words; a probe then compares the
+// words of its key's place.  Two shared atomics per build tuple and two or
+// three shared loads per probe, and nothing that grows with the table's load:
+// the open-addressing table it replaced for these buckets (16-byte slots, a
+// compare-and-swap and three atomics per build tuple, load up to 0.77) left a
+// warp's lanes waiting for the longest walk, 9 of 32 active, even with a key
+// filter in front.  A window of 65,536 tuples per side in 256 pieces of 4,096
+// by 4,096: 82 us with the table, 24 us by places.
+constexpr uint32_t kPlaceCap = 8192;      // build tuples
+constexpr uint32_t kPlacesMax = 4096;
+// Crowded places (hot or repeated keys) leave the bucket to a direct or hash
+// table, which aggregate: one of more than kPlaceMost tuples, or more than one
+// thread in ten with one of more than kPlaceMany.
+constexpr uint32_t kPlaceMany = 16, kPlaceMost = 128;
+constexpr size_t kPlaceBytes = sizeof(uint64_t) * kPlaceCap + sizeof(uint32_t) * (kPlacesMax + 1);
+
+// Adds the matches to count and prod; false, with nothing added and e still the
+// build run's first tile (build_head), when the run (nB <= kPlaceCap) is crowded.
+template <bool kRaw>
+__device__ __forceinline__ bool join_count_places(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
+                                                  unsigned long long &count, unsigned long long &prod) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ uint32_t warp_tot[kJoinThreads / 32];
+    __shared__ uint32_t most_s;
+    uint64_t *word = reinterpret_cast<uint64_t *>(smem_raw);
+    uint32_t *at = reinterpret_cast<uint32_t *>(word + kPlaceCap);   // at[p]: first word of place p; at[0] = 0
+    const uint32_t nB = ji.nB, nP = ji.nP, bside = jr.bside, pside = bside ^ 1u;
+    const uint32_t bits = min(12u, max(9u, 31u - (uint32_t)__clz(nB))), places = 1u << bits, shift = 32u - bits;
+    static_assert(kPlacesMax == 1u << 12 && kJoinThreads == 1 << 9, "places per thread");
+    auto load = [&](uint32_t base) {
+#pragma unroll
+        for (int k = 0; k < kJoinPer; k++) {
+            const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+            e[k] = i < nB ? run_load<kRaw>(jr.b, i) : 0ull;
+        }
+    };
+    constexpr uint32_t tile = kJoinPer * kJoinThreads;
+    for (uint32_t i = threadIdx.x; i <= places; i += kJoinThreads) at[i] = 0;
+    if (threadIdx.x == 0) most_s = 0;
+    SJBG_BARRIER();
+    for (uint32_t base = 0; base < nB; base += tile) {
+        if (base) load(base);
+#pragma unroll
+        for (int k = 0; k < kJoinPer; k++)
+            if (base + k * kJoinThreads + threadIdx.x < nB) atomicAdd(&at[1 + (place_hash((uint32_t)e[k]) >> shift)], 1u);
+    }
+    SJBG_BARRIER();
+    const uint32_t per = places / kJoinThreads, p0 = 1 + threadIdx.x * per;   // 1 to 8 places
+    uint32_t sum = 0, largest = 0;
+    for (uint32_t q = 0; q < per; q++) {
+        const uint32_t c = at[p0 + q];
+        sum += c;
+        largest = max(largest, c);
+    }
+    uint32_t tot;
+    uint32_t run = warp_excl_scan(sum, &tot);
+    if (lane_id() == 31) warp_tot[warp_id()] = tot;
+    if (largest > kPlaceMost) most_s = 1;
+    const bool crowded = __syncthreads_count(largest > kPlaceMany) > kJoinThreads / 10 || most_s;
+    if (crowded) {
+        if (nB > tile) load(0);
+        SJBG_BARRIER();   // the places are read before the next table's entries
+        return false;
+    }
+    run += __reduce_add_sync(0xFFFFFFFFu, lane_id() < warp_id() ? warp_tot[lane_id() & (kJoinThreads / 32 - 1)] : 0u);
+    for (uint32_t q = 0; q < per; q++) {
+        const uint32_t c = at[p0 + q];
+        at[p0 + q] = run;   // the place's next free word, in the end the next place's first
+        run += c;
+    }
+    SJBG_BARRIER();
+    for (uint32_t base = 0; base < nB; base += tile) {
+        if (nB > tile) load(base);
+#pragma unroll
+        for (int k = 0; k < kJoinPer; k++)
+            if (base + k * kJoinThreads + threadIdx.x < nB)
+                word[atomicAdd(&at[1 + (place_hash((uint32_t)e[k]) >> shift)], 1u)] = e[k];
+    }
+    SJBG_BARRIER();
+    for (uint32_t base = 0; base < nP; base += tile) {
+#pragma unroll
+        for (int k = 0; k < kJoinPer; k++) {
+            const uint32_t j = base + k * kJoinThreads + threadIdx.x;
+            e[k] = j < nP ? run_load<kRaw>(jr.p, j) : 0ull;
+        }
+#pragma unroll
+        for (int k = 0; k < kJoinPer; k++) {
+            if (base + k * kJoinThreads + threadIdx.x >= nP) continue;
+            const uint32_t key = (uint32_t)e[k], p = place_hash(key) >> shift, end = at[p + 1];
+            uint32_t c = 0;
+            unsigned long long f = 0;
+            for (uint32_t j = at[p]; j < end; j++) {
+                const uint64_t x = word[j];
+                if ((uint32_t)x == key) {
+                    c++;
+                    f += sjbg_fside((uint32_t)(x >> 32), bside);
+                }
+            }
+            if (c) {
+                count += c;
+                prod += f * sjbg_fside((uint32_t)(e[k] >> 32), pside);
+            }
+        }
+    }
+    SJBG_BARRIER();   // the words are read before the next item's
+    return true;
 }
 
 // Larger buckets (a radix window's hot keys) keep the hash table when they need
@@ -1285,11 +1383,8 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
     return KeyRange{min_s, max_s};
 }
 
-// e: the build run's first tile (build_head), when loaded.  kFilter: probes go
-// through the key filter.  A learned bucket's go straight to the table: its
-// light keys cover its range, most probes match, and the filter only adds to
-// them (z = 1.5, 8 x 2^24: 53.6 us without, 67.0 us with).
-template <bool kRaw, bool kFilter>
+// e: the build run's first tile (build_head), when loaded.
+template <bool kRaw>
 __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
                                                   bool loaded, uint32_t cap, unsigned long long &count,
                                                   unsigned long long &prod) {
@@ -1302,18 +1397,12 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
     // lets two CTAs share an SM), so buckets under the target probe at load
     // <= 1/2: with mostly distinct keys a miss then walks ~3 slots, not ~10
     const uint32_t C = min(cap, max(64u, (nB * 2u + 31u) & ~31u));
-    const uint32_t fbits = min(kFilterBits, 37u - (uint32_t)__clz(nB));   // 32 to 64 bits per build tuple
-    const uint32_t fshift = 32u - fbits;
     CountTable t;
-    unsigned long long *queue = reinterpret_cast<unsigned long long *>(smem_raw) + warp_id() * kQueueSlots;
-    t.sumf = reinterpret_cast<unsigned long long *>(smem_raw) + (kJoinThreads / 32) * kQueueSlots;
+    t.sumf = reinterpret_cast<unsigned long long *>(smem_raw);
     t.keys = reinterpret_cast<uint32_t *>(t.sumf + C + 1);
     t.cnt = t.keys + C + 1;
-    uint32_t *filter = t.cnt + C + 1;
     t.C = C;
     t.max_probe = nB < C ? C : kMaxProbe;
-    // an oversized build run is a hot key's: its probes match, so they skip the filter
-    const bool filtered = kFilter && nB < cap;
     constexpr uint32_t tile = kJoinPer * kJoinThreads;
 
     uint32_t n = nB;
@@ -1323,8 +1412,6 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
             t.cnt[i] = 0;
             t.sumf[i] = 0;
         }
-        if (kFilter)
-            for (uint32_t i = threadIdx.x; i < (1u << fbits) / 32; i += kJoinThreads) filter[i] = 0;
         if (threadIdx.x == 0) novf = 0;
         SJBG_BARRIER();
         // build: kJoinPer independent loads per thread, then insert them
@@ -1342,58 +1429,30 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
             for (int k = 0; k < kJoinPer; k++) {
                 const uint32_t i = base + k * kJoinThreads + threadIdx.x;
                 const bool valid = i < n;
-                if (valid) {
-                    const uint32_t key = (uint32_t)e[k], f = filter_hash(key) >> fshift;
-                    if (ct_insert(t, key, 1u, sjbg_fside((uint32_t)(e[k] >> 32), bside))) {
-                        if (filtered) atomicOr(&filter[f >> 5], 1u << (f & 31u));
-                    } else if (!kRaw) {   // (a piece's table, and a raw window's, takes every key)
-                        static_cast<uint64_t *>(jr.b)[atomicAdd(&novf, 1u)] = e[k];
-                    }
-                }
+                const bool ok = !valid || ct_insert(t, (uint32_t)e[k], 1u, sjbg_fside((uint32_t)(e[k] >> 32), bside));
+                // (a piece's table, and a raw window's, takes every key: nothing is written back)
+                if (!kRaw && valid && !ok) static_cast<uint64_t *>(jr.b)[atomicAdd(&novf, 1u)] = e[k];
             }
         }
         SJBG_BARRIER();
         // probe: the same independent-load tiling, no barriers needed
-        uint32_t waiting = 0;   // the warp's survivors in its queue (uniform over the warp)
-        auto look = [&](bool valid, unsigned long long x) {
-            const int s = valid ? ct_lookup(t, (uint32_t)x) : -1;
-            if (s >= 0) {
-                count += t.cnt[s];
-                prod += t.sumf[s] * sjbg_fside((uint32_t)(x >> 32), pside);
-            }
-        };
-        // (the filter's steps keep more in registers: four loads in flight, not eight)
-        constexpr int kPer = kFilter ? 4 : kJoinPer;
-        for (uint32_t base = 0; base < nP; base += kPer * kJoinThreads) {
-            uint64_t q[kPer];
+        for (uint32_t base = 0; base < nP; base += tile) {
 #pragma unroll
-            for (int k = 0; k < kPer; k++) {
+            for (int k = 0; k < kJoinPer; k++) {
                 const uint32_t j = base + k * kJoinThreads + threadIdx.x;
-                q[k] = j < nP ? run_load<kRaw>(jr.p, j) : 0ull;
+                e[k] = j < nP ? run_load<kRaw>(jr.p, j) : ~0ull;
             }
 #pragma unroll
-            for (int k = 0; k < kPer; k++) {
+            for (int k = 0; k < kJoinPer; k++) {
                 const uint32_t j = base + k * kJoinThreads + threadIdx.x;
-                if (!kFilter) {
-                    look(j < nP, q[k]);
-                    continue;
-                }
-                const uint32_t f = filter_hash((uint32_t)q[k]) >> fshift;
-                const bool in = j < nP && (!filtered || ((filter[f >> 5] >> (f & 31u)) & 1u));
-                const unsigned m = __ballot_sync(0xFFFFFFFFu, in);
-                if (in) queue[waiting + __popc(m & ((1u << lane_id()) - 1u))] = q[k];
-                waiting += __popc(m);
-                if (waiting >= 32u) {
-                    __syncwarp();
-                    waiting -= 32u;
-                    look(true, queue[waiting + lane_id()]);
-                    __syncwarp();   // read before the slots are reused
+                if (j < nP) {
+                    const int s = ct_lookup(t, (uint32_t)e[k]);
+                    if (s >= 0) {
+                        count += t.cnt[s];
+                        prod += t.sumf[s] * sjbg_fside((uint32_t)(e[k] >> 32), pside);
+                    }
                 }
             }
-        }
-        if (kFilter) {
-            __syncwarp();
-            look(lane_id() < waiting, queue[lane_id()]);
         }
         SJBG_BARRIER();
         n = novf;
@@ -1716,17 +1775,22 @@ template <bool kRaw, bool kModels>
 __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr, uint32_t cap, uint32_t &clean,
                                           unsigned long long &count, unsigned long long &prod) {
     uint64_t e[kJoinPer];
+    // a learned bucket's light keys are a range (no direct table) and repeat, up
+    // to the heavy cut: the hash table, which aggregates them (z = 1.5, 8 x 2^24:
+    // 54 us, by places 130)
     if (kModels && (ji.flags & kItemModel)) {
-        join_count_bucket<kRaw, false>(ji, jr, e, false, cap, count, prod);
-    } else {
-        const KeyRange kr = build_head<kRaw>(ji, jr, e);
-        if (const uint32_t passes = direct_passes(ji, kr)) {
-            join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, clean, count, prod);
-            return;
-        }
-        join_count_bucket<kRaw, true>(ji, jr, e, true, cap, count, prod);
+        join_count_bucket<kRaw>(ji, jr, e, false, cap, count, prod);
+        clean = 0;
+        return;
+    }
+    const KeyRange kr = build_head<kRaw>(ji, jr, e);
+    if (const uint32_t passes = direct_passes(ji, kr)) {
+        join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, clean, count, prod);
+        return;
     }
     clean = 0;
+    if (ji.nB <= kPlaceCap && join_count_places<kRaw>(ji, jr, e, count, prod)) return;
+    join_count_bucket<kRaw>(ji, jr, e, true, cap, count, prod);
 }
 
 // Bucket joins over the join list (items, length *jn; or, without a list, the
@@ -1841,7 +1905,10 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
 // per side, of which the tuples are well under one.  Here the host lists the
 // items, the one kernel gets them by value (or reads them in pinned memory),
 // and its last CTA writes the results to pinned memory, leaving its
-// accumulators zero for the next call.
+// accumulators zero for the next call.  Windows beyond one table are cut on
+// both sides while the pieces make one wave of CTAs: the work grows with their
+// product, but one window of 65,536 tuples per side is done in 24 us on the
+// device, where partitioning it first takes 28 and an HBM table 30.
 struct RawItem {
     uint64_t b, p;   // first build and probe tuple, in their sides' arrays
     uint32_t nB, nP, w, flags;
@@ -1962,20 +2029,32 @@ int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, con
         n == 0 || n > kRawWindows)
         return SJBG_OK;
     const uint32_t cap = join_cap(h, h->tune.bucket_target);
+    const uint64_t slots = 2 * (uint64_t)std::max(h->num_sms, 1);   // resident CTAs
     uint64_t tuples = 0;
+    bool small = true;   // every build side fits one table
     for (uint32_t w = 0; w < n; w++) {
-        if (std::min(wins[w].n_left, wins[w].n_right) >= cap ||
-            std::max(wins[w].n_left, wins[w].n_right) > 0xFFFFFFFFull)
-            return SJBG_OK;
-        tuples += wins[w].n_left + wins[w].n_right;
+        const uint64_t nB = std::min(wins[w].n_left, wins[w].n_right), nP = std::max(wins[w].n_left, wins[w].n_right);
+        if (nP > 0xFFFFFFFFull) return SJBG_OK;
+        small &= nB < cap;
+        tuples += nB + nP;
     }
-    // pieces of both sides: any cut of the build run will do (the sums are over
-    // pairs of tuples), so a call of few windows is spread over the SMs in
-    // pieces of about kRawPiece tuples, and a larger one in pieces that cost
-    // the SMs about equal shares
-    const uint64_t share = tuples / (4 * (uint64_t)std::max(h->num_sms, 1));
-    const uint32_t piece = (uint32_t)std::min<uint64_t>(cap - 1, std::max<uint64_t>(kRawPiece, share));
-    const uint32_t chunk = (uint32_t)std::min<uint64_t>(kJoinChunk, std::max<uint64_t>(kRawPiece, share));
+    // Any cut of the two runs will do (the sums are over pairs of tuples).  The
+    // smallest square pieces that make one wave of CTAs; windows that need more
+    // are taken when every build side fits a table, in pieces that cost the SMs
+    // about equal shares.
+    uint32_t piece = 0, chunk = 0;
+    for (uint32_t s = kRawPiece; s <= kRawPieceMost && s < cap && piece == 0; s += kRawPiece / 2) {
+        uint64_t items = 0;
+        for (uint32_t w = 0; w < n && items <= slots; w++)
+            items += ((wins[w].n_left + s - 1) / s) * ((wins[w].n_right + s - 1) / s);
+        if (items <= slots) piece = chunk = s;
+    }
+    if (piece == 0) {
+        if (!small) return SJBG_OK;
+        const uint64_t share = tuples / (2 * slots);
+        piece = (uint32_t)std::min<uint64_t>(cap - 1, std::max<uint64_t>(kRawPiece, share));
+        chunk = (uint32_t)std::min<uint64_t>(kJoinChunk, std::max<uint64_t>(kRawPiece, share));
+    }
     std::vector<RawItem> list;
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &x = wins[w];
@@ -1983,8 +2062,8 @@ int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, con
         const bool swap = x.n_right < x.n_left;
         const uint32_t nB = (uint32_t)(swap ? x.n_right : x.n_left), nP = (uint32_t)(swap ? x.n_left : x.n_right);
         const uint64_t b0 = swap ? x.right_off : x.left_off, p0 = swap ? x.left_off : x.right_off;
-        const uint32_t kb = std::max(1u, (nB + piece / 2) / piece), per = std::max(chunk, nB / kb);
-        const uint32_t kp = std::max<uint32_t>(1, (uint32_t)(((uint64_t)nP + per / 2) / per));
+        const uint32_t kb = (nB + piece - 1) / piece, per = std::max(chunk, nB / kb);
+        const uint32_t kp = (uint32_t)(((uint64_t)nP + per - 1) / per);
         for (uint32_t i = 0; i < kb; i++)
             for (uint32_t j = 0; j < kp; j++) {
                 const uint32_t b = (uint32_t)((uint64_t)nB * i / kb), p = (uint32_t)((uint64_t)nP * j / kp);
@@ -2012,7 +2091,7 @@ int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, con
         std::copy(list.begin(), list.end(), hst);
         dList = hst;
     }
-    const size_t smem = std::max(count_table_bytes(cap), kDirectBytes);
+    const size_t smem = std::max({count_table_bytes(cap), kDirectBytes, kPlaceBytes});
     allow_big_smem(raw_join_kernel, smem);
     SJBG_CK(h, launch(h, "raw_join", raw_join_kernel, dim3((uint32_t)list.size()), dim3(kJoinThreads), smem, dL, dR,
                       items, dList, n, cap, acc, hAcc));
@@ -2247,7 +2326,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
                           (const uint64_t *)dPL, (const uint64_t *)dPR, acc, (const WinPlan *)dPlan, dPairs, bits,
                           (const JoinItem *)dJlist, (const uint32_t *)dJn));
     } else {
-        const size_t smem = std::max(count_table_bytes(cap), kDirectBytes);
+        const size_t smem = std::max({count_table_bytes(cap), kDirectBytes, kPlaceBytes});
         auto join = learned ? bucket_join_count_kernel<true> : bucket_join_count_kernel<false>;
         allow_big_smem(join, smem);
         if (h->tune.persistent_join && max_items > (uint64_t)h->num_sms) {
@@ -2389,7 +2468,7 @@ int hj_count_window_raw(const sjbg_tuple *dL, uint64_t nL, const sjbg_tuple *dR,
                                                                           nullptr);
         if (int rc = launched("sjbg_lazy_hj_noalloc: part_scatter_kernel")) return rc;
         const uint32_t cap = count_table_cap(4096);
-        const size_t smem = std::max(count_table_bytes(cap), kDirectBytes);
+        const size_t smem = std::max({count_table_bytes(cap), kDirectBytes, kPlaceBytes});
         allow_big_smem(bucket_join_count_kernel<false>, smem);
         bucket_join_count_kernel<false><<<P, kJoinThreads, smem, st>>>(dL, dR, &rs->plan, pL, pR, start, cnt, P, rs->acc,
                                                                 cap, nullptr, nullptr, nullptr);

@@ -42,7 +42,7 @@ constexpr int kRangeThreads = 512;
 constexpr int kRangeWarps = kRangeThreads / 32;
 constexpr uint32_t kRangeCap = 4096;            // left words of a range (shared memory)
 constexpr uint32_t kRangeWords = 8192;          // words of both sides
-constexpr uint32_t kRangeTarget = 3328;         // words of the larger side per range: uneven ranges still fit
+constexpr uint32_t kRangeTarget = 3328;         // left words per range, and half the words of both: uneven ranges still fit
 constexpr uint32_t kRangeTargetMost = 3456;     // the same, when it saves a second wave of CTAs
 constexpr uint32_t kRangesMax = 1024;           // more ranges: runs of under 4 words per tile
 constexpr uint32_t kRangeTilesMax = 1536;       // tiles of both sides of a window
@@ -62,6 +62,7 @@ struct RangeWin {
     uint32_t tile[2];        // first tile of the side
     uint32_t tiles[2];
     uint32_t bucket0, P;     // first range of the call, ranges
+    uint64_t pairs_off, pairs_cap;
 };
 
 // The window's map of keys to ranges.
@@ -186,7 +187,7 @@ struct RangeSmem {
     uint16_t off[kRangeTilesMax], pre[kRangeTilesMax];   // per tile (left side's first): the run, the words before it
     uint16_t owner[kRangeWords];                    // tile of the range's i-th word
     uint32_t warp_tot[32];
-    unsigned long long wsum[32];
+    unsigned long long wsum[32], base;
     uint32_t lo, hi, crowd, n_left, next, stop;
 };
 
@@ -311,11 +312,13 @@ __device__ __forceinline__ unsigned long long range_prefix(RangeSmem &sm, const 
     return all;
 }
 
-template <bool kHash>
+// kEnum: every pair is visited for the xor checksum, kPairs: and written.
+template <bool kHash, bool kEnum, bool kPairs>
 __global__ void __launch_bounds__(kRangeThreads, 2)
 range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict__ rows,
                   const RangeWin *__restrict__ wins, uint32_t nwin, uint32_t nb, uint32_t P,
-                  uint32_t *__restrict__ queue, WinAcc *__restrict__ acc, WinAcc *__restrict__ out) {
+                  uint32_t *__restrict__ queue, WinAcc *__restrict__ acc, WinAcc *__restrict__ out,
+                  sjbg_pair *__restrict__ pairs) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     RangeSmem &sm = *reinterpret_cast<RangeSmem *>(smem_raw);
     const uint32_t lane = lane_id(), wid = warp_id();
@@ -446,33 +449,88 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                 }
                 if (threadIdx.x == kRangeThreads - 1) sm.sub[kRangeSubs] = crun;
             }
-            unsigned long long count = 0, prod = 0;
+            unsigned long long count = 0, prod = 0, xr = 0;
+            // the right words one by one: matches(x, use) calls use(val) for the
+            // left words with x's key
+            auto enumerate = [&](auto matches) {
+                for (uint32_t i = nl + threadIdx.x; i < n; i += kRangeThreads) {
+                    const uint64_t x = word(i);
+                    const uint32_t rv = (uint32_t)(x >> 32);
+                    unsigned long long f = 0;
+                    matches(x, [&](uint32_t lv) {
+                        count++;
+                        f += sjbg_fr(lv);
+                        xr ^= sjbg_pair_hash(lv, rv);
+                    });
+                    prod += f * sjbg_gs(rv);
+                }
+                if constexpr (kPairs) {
+                    // one reservation for the range's pairs; each warp writes its own in turn
+                    uint32_t wt = (uint32_t)warp_sum_u64(count);
+                    if (lane == 0) sm.warp_tot[wid] = wt;
+                    SJBG_BARRIER();
+                    const uint32_t c = lane < kRangeWarps ? sm.warp_tot[lane] : 0u;
+                    const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, c);
+                    if (threadIdx.x == 0 && total)
+                        sm.base = atomicAdd(&acc[wlo].npairs, (unsigned long long)total);
+                    SJBG_BARRIER();
+                    unsigned long long at = sm.base + __reduce_add_sync(0xFFFFFFFFu, lane < wid ? c : 0u);
+                    sjbg_pair *out_pairs = pairs + w.pairs_off;
+                    for (uint32_t i0 = nl; total && i0 < n; i0 += kRangeThreads) {   // (whole warps step)
+                        const uint32_t i = i0 + threadIdx.x;
+                        const uint64_t x = i < n ? word(i) : 0ull;
+                        uint32_t mine = 0;
+                        if (i < n) matches(x, [&](uint32_t) { mine++; });
+                        uint32_t tot;
+                        unsigned long long pos = at + warp_excl_scan(mine, &tot);
+                        if (mine)
+                            matches(x, [&](uint32_t lv) {
+                                if (pos < w.pairs_cap) out_pairs[pos] = sjbg_pair{lv, (uint32_t)(x >> 32)};
+                                pos++;
+                            });
+                        at += tot;
+                    }
+                }
+            };
             if (!crowded) {
                 SJBG_BARRIER();
 #pragma unroll
                 for (uint32_t k = 0; k < kItems; k++)
                     if (threadIdx.x + k * kRangeThreads < nl) sm.word[sm.sub[sub_of((uint32_t)e[k])] + rank[k]] = e[k];
                 SJBG_BARRIER();
-                for (uint32_t i = nl + threadIdx.x; i < n; i += 4 * kRangeThreads) {
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; q++) e[q] = i + q * kRangeThreads < n ? word(i + q * kRangeThreads) : 0ull;
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; q++) {
-                        const uint32_t key = (uint32_t)e[q];
-                        if (i + q * kRangeThreads >= n || key < lo || key > hi) continue;
+                if constexpr (kEnum) {
+                    enumerate([&](uint64_t x, auto use) {
+                        const uint32_t key = (uint32_t)x;
+                        if (key < lo || key > hi) return;
                         const uint32_t b = sub_of(key), end = sm.sub[b + 1];
-                        uint32_t c = 0;
-                        unsigned long long f = 0;
                         for (uint32_t j = sm.sub[b]; j < end; j++) {
-                            const uint64_t x = sm.word[j];
-                            if ((uint32_t)x == key) {
-                                c++;
-                                f += sjbg_fr((uint32_t)(x >> 32));
-                            }
+                            const uint64_t y = sm.word[j];
+                            if ((uint32_t)y == key) use((uint32_t)(y >> 32));
                         }
-                        if (c) {
-                            count += c;
-                            prod += f * sjbg_gs((uint32_t)(e[q] >> 32));
+                    });
+                } else {
+                    for (uint32_t i = nl + threadIdx.x; i < n; i += 4 * kRangeThreads) {
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++)
+                            e[q] = i + q * kRangeThreads < n ? word(i + q * kRangeThreads) : 0ull;
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++) {
+                            const uint32_t key = (uint32_t)e[q];
+                            if (i + q * kRangeThreads >= n || key < lo || key > hi) continue;
+                            const uint32_t b = sub_of(key), end = sm.sub[b + 1];
+                            uint32_t c = 0;
+                            unsigned long long f = 0;
+                            for (uint32_t j = sm.sub[b]; j < end; j++) {
+                                const uint64_t x = sm.word[j];
+                                if ((uint32_t)x == key) {
+                                    c++;
+                                    f += sjbg_fr((uint32_t)(x >> 32));
+                                }
+                            }
+                            if (c) {
+                                count += c;
+                                prod += f * sjbg_gs((uint32_t)(e[q] >> 32));
+                            }
                         }
                     }
                 }
@@ -490,15 +548,12 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                 uint32_t at = 0;   // the buffer pair that holds the words
                 for (uint32_t shift = 0; shift < bits; shift += kRangeDigit, at ^= 1u) range_pass(sm, at, nl, lo, shift);
                 const uint32_t *keys = sm.buf[at][0], *vals = sm.buf[at][1];
-                unsigned long long *F = reinterpret_cast<unsigned long long *>(&sm.buf[at ^ 1][0][0]);
-                const unsigned long long all = range_prefix(sm, vals, nl, F);   // ends with a barrier
-                // right words: the words of the key's top digit, then its group among them
+                // the key's group [l, h) among the words of its top digit
                 const uint32_t shift = bits ? (bits - 1) / kRangeDigit * kRangeDigit : 0u;   // of the last pass
-                for (uint32_t i = nl + threadIdx.x; i < n; i += kRangeThreads) {
-                    const uint64_t x = word(i);
-                    const uint32_t key = (uint32_t)x;
-                    if (key < lo || key > hi) continue;
-                    uint32_t l = 0, r = nl;
+                auto group = [&](uint32_t key, uint32_t &l, uint32_t &h) {
+                    l = h = 0;
+                    if (key < lo || key > hi) return false;
+                    uint32_t r = nl;
                     if (bits) {
                         const uint32_t digit = (key - lo) >> shift;
                         l = sm.loc[digit];
@@ -509,18 +564,34 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                         const uint32_t mid = (l + r) >> 1;
                         if (keys[mid] < key) l = mid + 1; else r = mid;
                     }
-                    if (l >= end || keys[l] != key) continue;
-                    uint32_t h = l + 1;
+                    if (l >= end || keys[l] != key) return false;
+                    h = l + 1;
                     r = end;
                     while (h < r) {
                         const uint32_t mid = (h + r) >> 1;
                         if (keys[mid] <= key) h = mid + 1; else r = mid;
                     }
-                    count += h - l;
-                    prod += ((h < nl ? F[h] : all) - F[l]) * sjbg_gs((uint32_t)(x >> 32));
+                    return true;
+                };
+                if constexpr (kEnum) {
+                    enumerate([&](uint64_t x, auto use) {
+                        uint32_t l, h;
+                        if (group((uint32_t)x, l, h))
+                            for (; l < h; l++) use(vals[l]);
+                    });
+                } else {
+                    unsigned long long *F = reinterpret_cast<unsigned long long *>(&sm.buf[at ^ 1][0][0]);
+                    const unsigned long long all = range_prefix(sm, vals, nl, F);   // ends with a barrier
+                    for (uint32_t i = nl + threadIdx.x; i < n; i += kRangeThreads) {
+                        const uint64_t x = word(i);
+                        uint32_t l, h;
+                        if (!group((uint32_t)x, l, h)) continue;
+                        count += h - l;
+                        prod += ((h < nl ? F[h] : all) - F[l]) * sjbg_gs((uint32_t)(x >> 32));
+                    }
                 }
             }
-            flush_acc(&acc[wlo], count, 0ull, prod);
+            flush_acc(&acc[wlo], count, xr, prod);
         }
         if (threadIdx.x == 0) sm.next = claim;
         SJBG_BARRIER();
@@ -551,7 +622,7 @@ static bool range_join_fits(const WinHost *wins, uint32_t n) {
 }
 
 int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
-                     WinAcc *hAcc, bool hash) {
+                     sjbg_pair *dPairs, WinAcc *hAcc, bool enumerate, bool hash) {
     std::vector<RangeWin> rw(n);
     const uint32_t slots = 2u * (uint32_t)std::max(h->num_sms, 1);   // resident CTAs of the join
     uint64_t tiles, nb;
@@ -564,8 +635,12 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
             std::memset(&r, 0, sizeof(r));
             r.off[0] = wins[w].left_off; r.n[0] = wins[w].n_left;
             r.off[1] = wins[w].right_off; r.n[1] = wins[w].n_right;
+            r.pairs_off = wins[w].pairs_off;
+            r.pairs_cap = dPairs ? wins[w].pairs_cap : 0;
             const bool empty = r.n[0] == 0 || r.n[1] == 0;   // (nothing of such a window is read)
-            r.P = (uint32_t)((std::max(r.n[0], r.n[1]) + target - 1) / target);
+            // by the left side, which a range holds whole, and by the words of both
+            r.P = (uint32_t)std::max<uint64_t>({(r.n[0] + target - 1) / target,
+                                                (r.n[0] + r.n[1] + 2 * target - 1) / (2 * target), 1});
             for (int s = 0; s < 2; s++) {
                 r.tile[s] = (uint32_t)tiles;
                 r.tiles[s] = empty ? 0u : (uint32_t)((r.n[s] + kSortedTile - 1) / kSortedTile);
@@ -609,11 +684,13 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
                       dim3((uint32_t)std::min<uint64_t>(tiles, 3u * (uint64_t)std::max(h->num_sms, 1))),
                       dim3(kSortedThreads), s1, dL, dR, dW, n, (uint32_t)tiles, (const RangeMap *)maps, pmax, words,
                       rows));
-    auto join_kernel = hash ? range_join_kernel<true> : range_join_kernel<false>;
+    auto join_kernel = dPairs      ? (hash ? range_join_kernel<true, true, true> : range_join_kernel<false, true, true>)
+                       : enumerate ? (hash ? range_join_kernel<true, true, false> : range_join_kernel<false, true, false>)
+                                   : (hash ? range_join_kernel<true, false, false> : range_join_kernel<false, false, false>);
     allow_big_smem(join_kernel, s2);
     const uint32_t grid = (uint32_t)std::min<uint64_t>(nb, slots);
     SJBG_CK(h, launch(h, "range_join", join_kernel, dim3(grid), dim3(kRangeThreads), s2, (const uint64_t *)words,
-                      (const uint16_t *)rows, dW, n, (uint32_t)nb, pmax, queue, acc, hAcc));
+                      (const uint16_t *)rows, dW, n, (uint32_t)nb, pmax, queue, acc, hAcc, dPairs));
     return SJBG_OK;
 }
 

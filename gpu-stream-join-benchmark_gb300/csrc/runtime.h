@@ -67,7 +67,7 @@ struct sjbg_handle {
     std::vector<double> kms;
     uint64_t launches = 0;
     bool capturing = false;
-    bool regrouped = false;       // a counting join's ranges did not fit: the handle's joins take the general path (range_join.cu)
+    bool regrouped = false;       // a join's ranges did not fit: the handle's joins take the general path (range_join.cu)
     bool unwatched = false;       // the call being enqueued is not waited for: it must not need a second try
 
     // tunables (the autotuner picks them per workload shape)
@@ -186,13 +186,13 @@ int nlj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, c
 int smj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                    sjbg_pair *dPairs, WinAcc *acc, bool enumerate);
 
-// Counting joins by key ranges (sort-merge) or hash ranges (hash join),
+// Joins by key ranges (sort-merge) or hash ranges (hash join),
 // range_join.cu: whether they suit the handle and the windows' sizes, and the
 // call, which leaves n + 1 entries in hAcc (pinned); the last one, the status
 // word, holds kErrRegroup when a range did not fit.
 bool range_join_pays(const sjbg_handle *h, const WinHost *wins, uint32_t n);
 int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
-                     WinAcc *hAcc, bool hash);
+                     sjbg_pair *dPairs, WinAcc *hAcc, bool enumerate, bool hash);
 
 int generate_device(sjbg_handle *h, sjbg_tuple *out, uint64_t first, uint64_t n, uint64_t seed, uint64_t domain,
                     const uint64_t *table, uint64_t perm_seed);

@@ -60,7 +60,8 @@ RAW = [(1, 1), (0, 5), (5, 0), (1535, 1537), (4096, 4096), (5343, 5343), (3, 100
 
 @pytest.mark.parametrize("graph", [False, True])
 @pytest.mark.parametrize("kind", ["dense", "wide", "hot"])
-@pytest.mark.parametrize("windows", [RAW[:1], RAW[1:2], RAW[3:4], RAW[4:5], RAW, RAW * 30, RAW * 120])
+@pytest.mark.parametrize("windows", [RAW[:1], RAW[1:2], RAW[3:4], RAW[4:5], RAW, RAW * 30, RAW * 120,
+                                     [(11_727, 11_727)], [(65_536, 65_536)], [(9000, 30_001), (20_000, 6000)]])
 def test_calls_of_small_windows_only(lib, oracle, windows, kind, graph):
     """One launch for the call: one item, items passed by value, items in a list,
     more windows than it takes; repeated calls (accumulators left zero)."""
