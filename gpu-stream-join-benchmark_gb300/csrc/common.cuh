@@ -48,8 +48,10 @@ struct WinPlan {
     uint32_t bucket_base;   // first global bucket id of this window
     uint32_t log2_buckets;  // buckets of this window = 1 << log2_buckets
     uint32_t model;         // learned partitioner model slot, or 0xFFFFFFFF for radix
-    uint16_t two_level;     // hash join: partitioned in two passes (coarse runs, then fine buckets)
-    uint16_t raw;           // hash join: not partitioned, the bucket join reads its tuples
+    uint8_t two_level;      // hash join: partitioned in two passes (coarse runs, then fine buckets)
+    uint8_t raw;            // hash join: not partitioned, the bucket join reads its tuples
+    uint8_t rows;           // hash join, learned: may be joined from sorted tiles once compacted
+    uint8_t pad8_;
 };
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }

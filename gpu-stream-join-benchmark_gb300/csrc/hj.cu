@@ -53,7 +53,10 @@ constexpr uint32_t kMaxBucketsLog2 = 14;
 constexpr uint32_t kCoarseMax = 128;
 constexpr uint32_t kRow = kCoarseMax + 1;   // per tile: exclusive coarse offsets, then its total
 constexpr uint32_t kGroupTiles = 64;        // tiles whose runs of one coarse partition a fine CTA gathers
-constexpr uint32_t kFineChunk = 2048;       // tuples a fine CTA sorts at a time
+// Tuples a fine CTA sorts at a time.  An item of a window that is half light
+// has 2,048 tuples on average and an all-light one 4,096, so chunks hold a
+// quarter more: at 2,048 every second item had a chunk of a few tuples.
+constexpr uint32_t kFineChunk = 2560;
 constexpr int kFineThreads = 256;
 
 __host__ __device__ __forceinline__ uint32_t coarse_bits(uint32_t lg) { return (lg + 1) / 2; }
@@ -87,6 +90,29 @@ struct Classifier {
 // The window's model in global memory, or null for radix partitioning.
 __device__ __forceinline__ const LearnedModel *model_of(const WinPlan &wp, const LearnedModel *models) {
     return (wp.model != 0xFFFFFFFFu && !models[wp.model].fallback) ? &models[wp.model] : nullptr;
+}
+
+// ---- compacted windows joined from sorted tiles
+// The light tuples of a compacted learned window are few, so they need not be
+// counted, scanned and scattered: each tile of the compact array is sorted by
+// bucket in place (part_light_kernel) and the join takes a bucket's runs out of
+// all tiles (rows_join).  z = 1.5, 8 x 2^24 (6.4 M light tuples): counting,
+// scan, scatter and join took 160 us, sorting and join 109.  (Sorting every
+// tile of the other windows while they are counted, with rows of 512 to 2,048
+// buckets, lost: runs of one to four tuples, 2 x 5 M at z = 1.0 668 us against
+// 541, 1 M 232 against 218.)
+constexpr uint32_t kRowsTilesMax = 2560;      // compact tiles of a window's two sides in a bucket's row list
+constexpr uint32_t kRowsMaxLog2 = 9;          // more buckets: runs of a few tuples per tile
+
+// Whether window w takes this form.  ccnt: the compacted light tuples per
+// window side, once the counting pass is done.
+__device__ __forceinline__ bool rows_form(const WinPlan &wp, uint32_t w, const LearnedModel *models,
+                                          const uint32_t *ccnt) {
+    if (!wp.rows || wp.model == 0xFFFFFFFFu) return false;
+    const LearnedModel &m = models[wp.model];
+    if (m.fallback || !m.n_heavy || !m.compact || m.log2_buckets > kRowsMaxLog2) return false;
+    const uint32_t tiles = (ccnt[2 * w] + kTile - 1) / kTile + (ccnt[2 * w + 1] + kTile - 1) / kTile;
+    return tiles <= kRowsTilesMax;
 }
 
 // All threads of the CTA; ends with a barrier when the window has a model.
@@ -231,7 +257,7 @@ part_hist_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict_
                         const uint32_t old = atomicAdd(&hsum_lo[a], flo);
                         atomicAdd(&hsum_hi[a], add_carry((uint32_t)(f >> 32), old, flo));
                     } else if (valid) {
-                        // light keys: compacted windows count them in part_hist_light
+                        // light keys: compacted windows count or sort them in part_light
                         if constexpr (kCompact) {
                             lightmask |= 1u << k;
                         } else {
@@ -354,22 +380,22 @@ part_hist_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict_
     }
 }
 
-// Bucket counts of the compacted light tuples of compacted learned windows
-// (part_hist only wrote them out).  Persistent CTAs stride over the tiles of
-// all window sides; tiles past a side's compacted count are skipped.
-// Per window side, the tiles (or fine items) that each later pass has work
-// for, as exclusive prefixes over the windows, written once the counting pass
-// is done: kind 0 part_hist_light (the compacted windows' light tiles), kind 1
-// part_scatter (those, plus every tile of a single-level window that was not
-// compacted), kind 2 part_fine (two-level windows that were not compacted).
+// Per window side, the tiles (or fine items, or buckets) that each later pass
+// has work for, as exclusive prefixes over the windows, written once the
+// counting pass is done: kind 0 part_light (the compacted windows' light
+// tiles), kind 1 part_scatter (those, plus every tile of a single-level window
+// that was not compacted), kind 2 part_fine (two-level windows that were not
+// compacted), kind 3 part_light too (the light tiles of compacted windows joined
+// from sorted tiles, which the others leave out), kind 4 rows_join (buckets of
+// windows joined from sorted tiles; left array only).
 // Array 2 * kind + side (left 0, right 1) of n + 1 entries.  One warp per array.
-enum : uint32_t { kWorkLight = 0, kWorkScatter = 1, kWorkFine = 2 };
+enum : uint32_t { kWorkLight = 0, kWorkScatter = 1, kWorkFine = 2, kWorkSort = 3, kWorkRows = 4, kWorkArrays = 9 };
 __global__ void part_work_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_t *__restrict__ tileL,
                                  const uint32_t *__restrict__ tileR, const uint32_t *__restrict__ itemL,
                                  const uint32_t *__restrict__ itemR, const LearnedModel *__restrict__ models,
                                  const uint32_t *__restrict__ ccnt, uint32_t *__restrict__ work) {
     const uint32_t a = warp_id();
-    if (a >= 6) return;   // whole warp
+    if (a >= kWorkArrays) return;   // whole warp
     const uint32_t kind = a >> 1, right = a & 1u;
     const uint32_t *tp = right ? tileR : tileL, *ip = right ? itemR : itemL;
     uint32_t *out = work + a * (nwin + 1);
@@ -382,7 +408,11 @@ __global__ void part_work_kernel(const WinPlan *__restrict__ wins, uint32_t nwin
             const LearnedModel *gm = model_of(wp, models);
             const bool compact = gm && gm->n_heavy && gm->compact;
             const uint32_t light = (ccnt[2 * w + right] + kTile - 1) / kTile;
-            if (kind == kWorkLight) c = compact ? light : 0u;
+            const bool form = rows_form(wp, w, models, ccnt);
+            if (kind == kWorkRows) c = form ? 1u << gm->log2_buckets : 0u;
+            else if (kind == kWorkSort) c = form ? light : 0u;
+            else if (form) c = 0;
+            else if (kind == kWorkLight) c = compact ? light : 0u;
             else if (kind == kWorkScatter) c = compact ? light : (wp.two_level ? 0u : tp[w + 1] - tp[w]);
             else c = (wp.two_level && !compact) ? ip[w + 1] - ip[w] : 0u;
         }
@@ -410,37 +440,66 @@ __device__ __forceinline__ WorkItem work_item(const uint32_t *pl, const uint32_t
     return it;
 }
 
-__global__ void __launch_bounds__(kPartThreads)
-part_hist_light_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_t *__restrict__ tileL,
-                       const uint32_t *__restrict__ tileR, const uint32_t *__restrict__ work,
-                       uint32_t *__restrict__ cnt, uint32_t B, const LearnedModel *__restrict__ models,
-                       const uint64_t *__restrict__ compL, const uint64_t *__restrict__ compR,
-                       const uint32_t *__restrict__ ccnt) {
-    extern __shared__ uint32_t hist[];
+// The compacted light tuples of compacted learned windows (part_hist only wrote
+// them out).  Work kind 0: bucket counts, for the scatter.  Work kind 3: a tile
+// of a window joined from sorted tiles is sorted by bucket (in place: it is in
+// registers before it is written) and gets its row.  Persistent CTAs over both.
+__global__ void __launch_bounds__(kPartThreads, 2)
+part_light_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_t *__restrict__ tileL,
+                  const uint32_t *__restrict__ tileR, const uint32_t *__restrict__ work, uint32_t *__restrict__ counts,
+                  uint32_t B, const LearnedModel *__restrict__ models, uint64_t *__restrict__ compL,
+                  uint64_t *__restrict__ compR, const uint32_t *__restrict__ ccnt, uint16_t *__restrict__ rows16,
+                  uint32_t rstride) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ LearnedCore core;
-    const uint32_t *pl = work + 2 * kWorkLight * (nwin + 1), *pr = pl + (nwin + 1);
-    const uint32_t items = pl[nwin] + pr[nwin];
+    __shared__ uint32_t warp_tot[32];
+    uint64_t *stage = reinterpret_cast<uint64_t *>(smem_raw);
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(stage + kTile);
+    const uint32_t *cl = work + 2 * kWorkLight * (nwin + 1), *cr = cl + (nwin + 1);
+    const uint32_t *pl = work + 2 * kWorkSort * (nwin + 1), *pr = pl + (nwin + 1);
+    const uint32_t counted = cl[nwin] + cr[nwin], items = counted + pl[nwin] + pr[nwin];
+    uint32_t cur = 0xFFFFFFFFu;   // window of the model in core
     for (uint32_t bt = blockIdx.x; bt < items; bt += gridDim.x) {
-        const WorkItem it = work_item(pl, pr, nwin, bt);
-        const bool right = it.right;
-        const uint32_t w = it.w;
-        const uint32_t *tp = right ? tileR : tileL;
-        const WinPlan wp = wins[w];
-        const LearnedModel *gm = model_of(wp, models);   // a compacted window's model
-        const uint64_t nside = ccnt[2 * w + (right ? 1 : 0)];
-        const uint64_t start = (uint64_t)it.local * kTile;
-        const uint32_t n = (uint32_t)(nside - start < (uint64_t)kTile ? nside - start : (uint64_t)kTile);
-        SJBG_BARRIER();   // the previous tile's readers of hist and core are done
-        const Classifier cls = make_classifier(wp, gm, core);   // ends with a barrier
+        const bool sort = bt >= counted;
+        const WorkItem it = sort ? work_item(pl, pr, nwin, bt - counted) : work_item(cl, cr, nwin, bt);
+        const uint32_t side_tile = (it.right ? tileR : tileL)[it.w] + it.local;
+        uint64_t *words = (it.right ? compR : compL) + (uint64_t)side_tile * kTile;
+        const uint32_t left = ccnt[2 * it.w + (it.right ? 1 : 0)] - it.local * kTile, n = min((uint32_t)kTile, left);
+        uint64_t e[kTile / kPartThreads];
+#pragma unroll
+        for (int k = 0; k < kTile / kPartThreads; k++) {
+            const uint32_t i = threadIdx.x + k * kPartThreads;
+            e[k] = i < n ? words[i] : 0ull;
+        }
+        SJBG_BARRIER();   // the previous tile's readers of the stage, its counters and its model are done
+        if (it.w != cur) copy_to_smem(&core, &models[wins[it.w].model], sizeof(LearnedCore));   // ends with a barrier
+        cur = it.w;
         const uint32_t P = 1u << core.log2_buckets;
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) hist[i] = 0;
+        for (uint32_t i = threadIdx.x; i < P; i += kPartThreads) cnt[i] = 0;
         SJBG_BARRIER();
-        const uint64_t *src = (right ? compR : compL) + (uint64_t)tp[w] * kTile + start;
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&hist[cls.bucket((uint32_t)__ldg(src + i))], 1u);
+        uint32_t br[kTile / kPartThreads];   // bucket << 16 | rank
+#pragma unroll
+        for (int k = 0; k < kTile / kPartThreads; k++)
+            if (threadIdx.x + k * kPartThreads < n) {
+                const uint32_t b = learned_bucket(core, (uint32_t)e[k]);
+                br[k] = (b << 16) | atomicAdd(&cnt[b], 1u);
+            }
         SJBG_BARRIER();
-        uint32_t *dst = cnt + (right ? B : 0) + wp.bucket_base;
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x)
-            if (hist[i]) atomicAdd(&dst[i], hist[i]);
+        if (!sort) {
+            uint32_t *dst = counts + (it.right ? B : 0) + wins[it.w].bucket_base;
+            for (uint32_t i = threadIdx.x; i < P; i += kPartThreads)
+                if (cnt[i]) atomicAdd(&dst[i], cnt[i]);
+            continue;
+        }
+        tile_scan(cnt, P, warp_tot);
+#pragma unroll
+        for (int k = 0; k < kTile / kPartThreads; k++)
+            if (threadIdx.x + k * kPartThreads < n) stage[cnt[br[k] >> 16] + (br[k] & 0xFFFFu)] = e[k];
+        uint16_t *row = rows16 + ((uint64_t)(it.right ? tileL[nwin] : 0) + side_tile) * rstride;
+        for (uint32_t i = threadIdx.x; i < P; i += kPartThreads) row[i] = (uint16_t)cnt[i];
+        if (threadIdx.x == 0) row[P] = (uint16_t)n;
+        SJBG_BARRIER();
+        for (uint32_t i = threadIdx.x; i < n; i += kPartThreads) words[i] = stage[i];
     }
 }
 
@@ -598,7 +657,8 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
                      const uint32_t *__restrict__ baseR, const uint32_t *__restrict__ cnt,
                      uint32_t *__restrict__ start, uint32_t *__restrict__ cursor, uint32_t B,
                      const LearnedModel *__restrict__ models, JoinItem *__restrict__ items,
-                     uint32_t *__restrict__ jn, uint32_t chunk, uint32_t cap, bool either) {
+                     uint32_t *__restrict__ jn, uint32_t chunk, uint32_t cap, bool either,
+                     const uint32_t *__restrict__ ccnt) {
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry_s;
     const uint32_t w = blockIdx.x;
@@ -619,6 +679,7 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
         }
         return;
     }
+    if (models && rows_form(wp, w, models, ccnt)) return;   // (whole CTA: nothing of it is in the join list)
     const uint32_t P = 1u << wp.log2_buckets, b0 = wp.bucket_base;
     constexpr uint32_t kItems = 4;
     const uint32_t tchunk = blockDim.x * kItems;
@@ -1046,6 +1107,9 @@ __device__ __forceinline__ void fine_item(const WorkItem it, const WinPlan *__re
                 }
             }
             SJBG_BARRIER();
+            // the reservations go out now and are stored after the staging, which hides their latency
+            uint32_t reserved = 0;
+            if (threadIdx.x < nfine && fcnt[threadIdx.x]) reserved = atomicAdd(&gcur[threadIdx.x], fcnt[threadIdx.x]);
             if (warp_id() == 0) {
                 uint32_t a[kCoarseMax / 32], sum = 0;
 #pragma unroll
@@ -1059,10 +1123,7 @@ __device__ __forceinline__ void fine_item(const WorkItem it, const WinPlan *__re
 #pragma unroll
                 for (int q = 0; q < (int)(kCoarseMax / 32); q++) {
                     const uint32_t f = lane_id() * (kCoarseMax / 32) + q;
-                    if (f < nfine) {
-                        floc[f] = run;
-                        fbase[f] = a[q] ? atomicAdd(&gcur[f], a[q]) : 0u;
-                    }
+                    if (f < nfine) floc[f] = run;
                     run += a[q];
                 }
             }
@@ -1075,6 +1136,7 @@ __device__ __forceinline__ void fine_item(const WorkItem it, const WinPlan *__re
                     sf[pos] = (uint8_t)(fr[k] >> 16);
                 }
             }
+            if (threadIdx.x < nfine) fbase[threadIdx.x] = reserved;
             SJBG_BARRIER();
             for (uint32_t pos = threadIdx.x; pos < m; pos += blockDim.x) {
                 const uint32_t f = sf[pos];
@@ -1111,7 +1173,7 @@ struct CountTable {
     uint32_t *cnt;               // C + 1
     unsigned long long *sumf;    // C + 1
     uint32_t C;                  // slots (any size: the hash is scaled, not masked)
-    uint32_t max_probe;          // kMaxProbe, or C when the build run is shorter than the table (every key fits)
+    uint32_t max_probe;          // kMaxProbe, or C where every key of a shorter build run has to fit (its pieces share it)
 };
 
 // Home slot of a key in a table of C slots: a 32-bit multiplicative hash scaled to [0, C).
@@ -1344,21 +1406,28 @@ struct KeyRange {
 
 // Loads the first tile of a build run (kJoinPer tuples per thread) and returns
 // the run's smallest and largest keys to every thread (those of its first
-// tile, when the run is too long for a direct table anyway); ends with a barrier.
+// tile, when the run is too long for a direct table anyway); ends with a
+// barrier, its only one after the CTA's first call (turn 0): the calls take the
+// two result slots in turn and leave the other one reset.
 template <bool kRaw>
-__device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer]) {
-    __shared__ uint32_t min_s, max_s;
-    if (threadIdx.x == 0) {
-        min_s = 0xFFFFFFFFu;
-        max_s = 0;
+__device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
+                                               uint32_t &turn) {
+    __shared__ uint32_t min_s[2], max_s[2];
+    if (turn == 0) {
+        if (threadIdx.x == 0) {
+            min_s[0] = min_s[1] = 0xFFFFFFFFu;
+            max_s[0] = max_s[1] = 0;
+        }
+        SJBG_BARRIER();
     }
+    const uint32_t slot = turn & 1u;
+    turn = slot + 1;
     uint32_t lo = 0xFFFFFFFFu, hi = 0;
 #pragma unroll
     for (int k = 0; k < kJoinPer; k++) {
         const uint32_t i = k * kJoinThreads + threadIdx.x;
         e[k] = i < ji.nB ? run_load<kRaw>(jr.b, i) : 0ull;
     }
-    SJBG_BARRIER();
 #pragma unroll
     for (int k = 0; k < kJoinPer; k++) {
         if (k * kJoinThreads + threadIdx.x < ji.nB) {
@@ -1376,11 +1445,15 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
     lo = __reduce_min_sync(0xFFFFFFFFu, lo);
     hi = __reduce_max_sync(0xFFFFFFFFu, hi);
     if (lane_id() == 0) {
-        atomicMin(&min_s, lo);
-        atomicMax(&max_s, hi);
+        atomicMin(&min_s[slot], lo);
+        atomicMax(&max_s[slot], hi);
     }
     SJBG_BARRIER();
-    return KeyRange{min_s, max_s};
+    if (threadIdx.x == 0) {
+        min_s[slot ^ 1u] = 0xFFFFFFFFu;
+        max_s[slot ^ 1u] = 0;
+    }
+    return KeyRange{min_s[slot], max_s[slot]};
 }
 
 // e: the build run's first tile (build_head), when loaded.
@@ -1432,6 +1505,7 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
                 const bool ok = !valid || ct_insert(t, (uint32_t)e[k], 1u, sjbg_fside((uint32_t)(e[k] >> 32), bside));
                 // (a piece's table, and a raw window's, takes every key: nothing is written back)
                 if (!kRaw && valid && !ok) static_cast<uint64_t *>(jr.b)[atomicAdd(&novf, 1u)] = e[k];
+                __syncwarp();
             }
         }
         SJBG_BARRIER();
@@ -1452,6 +1526,7 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
                         prod += t.sumf[s] * sjbg_fside((uint32_t)(e[k] >> 32), pside);
                     }
                 }
+                __syncwarp();
             }
         }
         SJBG_BARRIER();
@@ -1770,10 +1845,11 @@ __device__ __forceinline__ void join_enum_bucket(const JoinItem &ji, const uint6
     flush_acc(&acc[w], count, xr, prod);
 }
 
-// One item's matches; `clean` as in join_count_direct.
+// One item's matches; `clean` as in join_count_direct, `turn` as in build_head
+// (0 at the CTA's first item).
 template <bool kRaw, bool kModels>
 __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr, uint32_t cap, uint32_t &clean,
-                                          unsigned long long &count, unsigned long long &prod) {
+                                          uint32_t &turn, unsigned long long &count, unsigned long long &prod) {
     uint64_t e[kJoinPer];
     // a learned bucket's light keys are a range (no direct table) and repeat, up
     // to the heavy cut: the hash table, which aggregates them (z = 1.5, 8 x 2^24:
@@ -1783,7 +1859,7 @@ __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr
         clean = 0;
         return;
     }
-    const KeyRange kr = build_head<kRaw>(ji, jr, e);
+    const KeyRange kr = build_head<kRaw>(ji, jr, e, turn);
     if (const uint32_t passes = direct_passes(ji, kr)) {
         join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, clean, count, prod);
         return;
@@ -1791,6 +1867,187 @@ __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr
     clean = 0;
     if (ji.nB <= kPlaceCap && join_count_places<kRaw>(ji, jr, e, count, prod)) return;
     join_count_bucket<kRaw>(ji, jr, e, true, cap, count, prod);
+}
+
+// ---- joins from sorted tiles
+// Buckets of windows joined from sorted tiles: a bucket is the runs of all
+// tiles of the window, the left side's tiles first.  Their words are numbered
+// across the runs (owner: the tile of each of kRowsOwner words at a time), so
+// that every lane has one; the smaller side's words build a count table, the
+// others probe it.  Words whose keys the table cannot take are written back over
+// the first words of their side (this CTA's alone) and joined in a further pass.  Part of the
+// bucket join's launch: persistent CTAs over work kind 4.
+constexpr uint32_t kRowsOwner = 4096;
+constexpr uint32_t kRowsRun = 64;   // a longer run: the owners are written by warps, not by threads
+struct RowsLists {
+    uint32_t pre[kRowsTilesMax + 1];    // words of the bucket in the tiles before
+    uint16_t off[kRowsTilesMax];        // its run in the tile
+    uint16_t owner[kRowsOwner];
+};
+static inline size_t rows_join_bytes(uint32_t cap) { return ((count_table_bytes(cap) + 15) & ~(size_t)15) + sizeof(RowsLists); }
+
+struct RowsJoin {
+    uint32_t nwin, rstride;
+    const uint32_t *tileL, *tileR, *work, *ccnt;
+    uint64_t *compL, *compR;
+    const uint16_t *rows16;
+    uint32_t *queue;   // null: no window of the call may take the form
+};
+
+__device__ __forceinline__ void rows_join(const RowsJoin &rj, const WinPlan *__restrict__ wins, WinAcc *__restrict__ acc,
+                                          uint32_t cap) {
+    const uint32_t nwin = rj.nwin, rstride = rj.rstride;
+    const uint32_t *__restrict__ tileL = rj.tileL, *__restrict__ tileR = rj.tileR, *__restrict__ ccnt = rj.ccnt;
+    uint64_t *compL = rj.compL, *compR = rj.compR;
+    const uint16_t *__restrict__ rows16 = rj.rows16;
+    uint32_t *queue = rj.queue;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ uint32_t warp_tot[32];
+    __shared__ uint32_t next_s, novf_s, n_left_s;
+    RowsLists &ls = *reinterpret_cast<RowsLists *>(smem_raw + ((sizeof(unsigned long long) + 2 * sizeof(uint32_t)) *
+                                                                   ((size_t)cap + 1) + 15 & ~(size_t)15));
+    const uint32_t *pw = rj.work + 2 * kWorkRows * (nwin + 1);
+    const uint32_t items = pw[nwin];
+    uint32_t g = blockIdx.x;
+    while (g < items) {
+        uint32_t claim = 0;
+        if (threadIdx.x == 0) claim = gridDim.x + atomicAdd(queue, 1u);
+        const uint32_t w = find_window(pw, nwin, g), b = g - pw[w];
+        const uint32_t TL = (ccnt[2 * w] + kTile - 1) / kTile, T = TL + (ccnt[2 * w + 1] + kTile - 1) / kTile;
+        uint64_t *wl = compL + (uint64_t)tileL[w] * kTile, *wr = compR + (uint64_t)tileR[w] * kTile;
+        const uint16_t *rl = rows16 + (uint64_t)tileL[w] * rstride + b;
+        const uint16_t *rr = rows16 + ((uint64_t)tileL[nwin] + tileR[w]) * rstride + b;
+        // thread t's tiles [t * per, t * per + per)
+        constexpr uint32_t kPerMax = kRowsTilesMax / kJoinThreads;
+        const uint32_t per = (T + kJoinThreads - 1) / kJoinThreads, x0 = threadIdx.x * per;
+        uint32_t sum = 0;
+        bool lengthy = false;
+        uint32_t len[kPerMax];
+#pragma unroll
+        for (uint32_t q = 0; q < kPerMax; q++) {
+            const uint32_t x = x0 + q;
+            len[q] = 0;
+            if (q < per && x < T) {
+                const uint16_t *r = x < TL ? rl + (uint64_t)x * rstride : rr + (uint64_t)(x - TL) * rstride;
+                const uint32_t o = __ldg(r);
+                len[q] = __ldg(r + 1) - o;
+                ls.off[x] = (uint16_t)o;
+            }
+            sum += len[q];
+            lengthy |= len[q] > kRowsRun;
+        }
+        lengthy = __any_sync(0xFFFFFFFFu, lengthy);
+        uint32_t tot;
+        uint32_t run = warp_excl_scan(sum, &tot);
+        if (lane_id() == 31) warp_tot[warp_id()] = tot | (lengthy ? 1u << 31 : 0u);   // (at most kRowsTilesMax * kTile)
+        SJBG_BARRIER();
+        uint32_t v = lane_id() < kJoinThreads / 32 ? warp_tot[lane_id()] : 0u;
+        lengthy = __any_sync(0xFFFFFFFFu, v >> 31);
+        v &= 0x7FFFFFFFu;
+        const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, v);
+        run += __reduce_add_sync(0xFFFFFFFFu, lane_id() < warp_id() ? v : 0u);
+#pragma unroll
+        for (uint32_t q = 0; q < kPerMax; q++) {
+            const uint32_t x = x0 + q;
+            if (q < per && x < T) {
+                ls.pre[x] = run;
+                if (x == TL) n_left_s = run;
+            }
+            run += len[q];
+        }
+        if (TL == T && threadIdx.x == 0) n_left_s = n;
+        if (threadIdx.x == 0) ls.pre[T] = n;
+        SJBG_BARRIER();
+        const uint32_t nl = n_left_s;
+        auto tile_of = [&](uint32_t x) { return x < TL ? wl + (uint64_t)x * kTile : wr + (uint64_t)(x - TL) * kTile; };
+        // words [i0, i1) of the bucket, kRowsOwner at a time; use(word) by every lane
+        // that has one (build: once all lanes have loaded theirs)
+        auto each = [&](uint32_t i0, uint32_t i1, auto build, auto use) {
+            for (uint32_t c0 = i0; c0 < i1; c0 += kRowsOwner) {
+                const uint32_t c1 = min(i1, c0 + kRowsOwner);
+                if (lengthy) {   // a warp per run
+                    for (uint32_t x = warp_id(); x < T; x += kJoinThreads / 32) {
+                        const uint32_t a = max(ls.pre[x], c0), z = min(ls.pre[x + 1], c1);
+                        for (uint32_t i = a + lane_id(); i < z; i += 32) ls.owner[i - c0] = (uint16_t)x;
+                    }
+                } else {         // a thread per run
+                    for (uint32_t q = 0; q < per; q++) {
+                        const uint32_t x = x0 + q;
+                        if (x >= T) break;
+                        const uint32_t a = max(ls.pre[x], c0), z = min(ls.pre[x + 1], c1);
+                        for (uint32_t i = a; i < z; i++) ls.owner[i - c0] = (uint16_t)x;
+                    }
+                }
+                SJBG_BARRIER();
+                // (the trip count is uniform per CTA, and every warp reconverges after each use)
+                for (uint32_t i0 = c0; i0 < c1; i0 += 4 * kJoinThreads) {
+                    const uint32_t i = i0 + threadIdx.x;
+                    uint64_t e[4];
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; q++) {
+                        const uint32_t k = i + q * kJoinThreads;
+                        e[q] = 0;
+                        if (k < c1) {
+                            const uint32_t x = ls.owner[k - c0], at = ls.off[x] + (k - ls.pre[x]);
+                            e[q] = build() ? tile_of(x)[at] : __ldg(tile_of(x) + at);
+                        }
+                    }
+                    if constexpr (build()) SJBG_BARRIER();
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; q++) {
+                        if (i + q * kJoinThreads < c1) use(e[q]);
+                        __syncwarp();
+                    }
+                }
+                SJBG_BARRIER();   // (the owners are read before the next ones are written)
+            }
+        };
+        if (nl != 0 && nl != n) {   // (the same for the whole CTA)
+            CountTable t;
+            const uint32_t right = n - nl < nl, nb = right ? n - nl : nl;   // built from the smaller side
+            const uint32_t b0 = right ? nl : 0u, p0 = nl - b0, p1 = right ? nl : n;
+            t.C = min(cap, max(64u, (nb * 2u + 31u) & ~31u));
+            t.max_probe = kMaxProbe;   // (crowded homes are cheaper to join in a further pass)
+            t.sumf = reinterpret_cast<unsigned long long *>(smem_raw);
+            t.keys = reinterpret_cast<uint32_t *>(t.sumf + t.C + 1);
+            t.cnt = t.keys + t.C + 1;
+            unsigned long long count = 0, prod = 0;
+            for (uint32_t rem = nb; rem;) {
+                for (uint32_t i = threadIdx.x; i <= t.C; i += kJoinThreads) {
+                    t.keys[i] = kEmptyKey;
+                    t.cnt[i] = 0;
+                    t.sumf[i] = 0;
+                }
+                if (threadIdx.x == 0) novf_s = 0;
+                SJBG_BARRIER();
+                each(b0, b0 + rem, std::true_type{}, [&](uint64_t e) {
+                    if (ct_insert(t, (uint32_t)e, 1u, sjbg_fside((uint32_t)(e >> 32), right))) return;
+                    const uint32_t k = b0 + atomicAdd(&novf_s, 1u);   // (no further than the words read so far)
+                    uint32_t x0 = right ? TL : 0u, x1 = right ? T : TL;   // the last tile with its first word at or before k
+                    while (x1 - x0 > 1) {
+                        const uint32_t xm = (x0 + x1) / 2;
+                        if (ls.pre[xm] <= k) x0 = xm;
+                        else x1 = xm;
+                    }
+                    tile_of(x0)[ls.off[x0] + (k - ls.pre[x0])] = e;
+                });   // ends with a barrier
+                each(p0, p1, std::false_type{}, [&](uint64_t e) {
+                    const int s = ct_lookup(t, (uint32_t)e);
+                    if (s >= 0) {
+                        count += t.cnt[s];
+                        prod += t.sumf[s] * sjbg_fside((uint32_t)(e >> 32), right ^ 1u);
+                    }
+                });   // ends with a barrier
+                rem = novf_s;
+                SJBG_BARRIER();   // read before it is reset
+            }
+            flush_acc(&acc[w], count, 0, prod);
+        }
+        if (threadIdx.x == 0) next_s = claim;
+        SJBG_BARRIER();
+        g = next_s;
+        SJBG_BARRIER();   // read before the next claim is stored
+    }
 }
 
 // Bucket joins over the join list (items, length *jn; or, without a list, the
@@ -1811,9 +2068,11 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
                          const WinPlan *__restrict__ wins, uint64_t *__restrict__ partL,
                          uint64_t *__restrict__ partR, const uint32_t *__restrict__ start,
                          const uint32_t *__restrict__ cnt, uint32_t B, WinAcc *__restrict__ acc, uint32_t cap,
-                         uint32_t *queue, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn) {
+                         uint32_t *queue, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn,
+                         const RowsJoin rj) {
+    if (kModels && rj.queue) rows_join(rj, wins, acc, cap);   // ends with a barrier
     const uint32_t nitems = items ? *jn : B;
-    uint32_t clean = 0;
+    uint32_t clean = 0, turn = 0;
     auto join = [&](const JoinItem &ji) {
         if (ji.nB == 0 || ji.nP == 0) return;
         const JoinRuns jr = join_runs(ji, L, R, wins, partL, partR);
@@ -1826,12 +2085,12 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
         unsigned long long count = 0, prod = 0;
         if constexpr (!kModels) {
             if (ji.flags & kItemRaw) {
-                join_item<true, kModels>(ji, jr, cap, clean, count, prod);
+                join_item<true, kModels>(ji, jr, cap, clean, turn, count, prod);
                 flush_acc(&acc[ji.w], count, 0, prod);
                 return;
             }
         }
-        join_item<false, kModels>(ji, jr, cap, clean, count, prod);
+        join_item<false, kModels>(ji, jr, cap, clean, turn, count, prod);
         flush_acc(&acc[ji.w], count, 0, prod);
     };
     if (!queue || !items) {
@@ -1940,9 +2199,9 @@ raw_join_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__
     jr.b = const_cast<sjbg_tuple *>((swap ? R : L) + it.b);   // (never written)
     jr.p = (swap ? L : R) + it.p;
     jr.bside = swap ? 1u : 0u;
-    uint32_t clean = 0;
+    uint32_t clean = 0, turn = 0;
     unsigned long long count = 0, prod = 0;
-    if (it.nB && it.nP) join_item<true, false>(ji, jr, cap, clean, count, prod);
+    if (it.nB && it.nP) join_item<true, false>(ji, jr, cap, clean, turn, count, prod);
     count = warp_sum_u64(count);
     prod = warp_sum_u64(prod);
     if (lane_id() == 0) {
@@ -2118,7 +2377,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     std::vector<uint32_t> tileL(n + 1), tileR(n + 1), hgL(n + 1), hgR(n + 1), itL(n + 1), itR(n + 1);
     std::vector<uint32_t> pbL(n + 1), pbR(n + 1);   // window bases in the partitioned arrays
     uint64_t B = 0, totL = 0, totR = 0;
-    uint32_t maxP = 1;
+    uint32_t maxP = 1, rows_lg = 0;   // rows_lg: log2 of the most buckets of a window joined from sorted tiles
     bool any_two = false, any_one = false, any_raw = false;
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &wh = wins[w];
@@ -2148,6 +2407,8 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
         // (no tile of an unpartitioned window is counted or scattered)
         tileL[w + 1] = tileL[w] + (p.raw ? 0u : (uint32_t)((wh.n_left + kTile - 1) / kTile));
         tileR[w + 1] = tileR[w] + (p.raw ? 0u : (uint32_t)((wh.n_right + kTile - 1) / kTile));
+        p.rows = learned && !enumerate && lg > 0 ? 1u : 0u;
+        if (p.rows) rows_lg = std::max(rows_lg, std::min(lg, kRowsMaxLog2));
         // fine-pass CTAs: coarse partitions x groups of kGroupTiles tiles
         const uint32_t nc = 1u << coarse_bits(lg);
         itL[w + 1] = itL[w] + nc * ((tileL[w + 1] - tileL[w] + kGroupTiles - 1) / kGroupTiles);
@@ -2256,11 +2517,18 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     // per window side its compacted light tuples, then the join list's length
     uint32_t *dCcnt = static_cast<uint32_t *>(ws_get(h, WS_COMPACT_CNT, sizeof(uint32_t) * (2 * n + 1)));
     uint32_t *dJn = dCcnt + 2 * n;
-    // the passes' work prefixes (6 arrays of n + 1), then (16-byte aligned) the join list
-    const size_t workWords = (6 * (size_t)(n + 1) + 3) & ~(size_t)3;
+    // the passes' work prefixes (kWorkArrays of n + 1), then (16-byte aligned) the join list
+    const size_t workWords = (kWorkArrays * (size_t)(n + 1) + 3) & ~(size_t)3;
     uint32_t *dWork = static_cast<uint32_t *>(
         ws_get(h, WS_TILE_PREFIX, sizeof(uint32_t) * workWords + sizeof(JoinItem) * (size_t)max_items));
     JoinItem *dJlist = dWork ? reinterpret_cast<JoinItem *>(dWork + workWords) : nullptr;
+    // sorted tiles' rows
+    const uint32_t rstride = sorted_row(1u << rows_lg);
+    uint16_t *dRows16 = nullptr;
+    if (rows_lg) {
+        dRows16 = static_cast<uint16_t *>(ws_get(h, WS_ROWS16, sizeof(uint16_t) * rstride * std::max<uint64_t>(tiles64, 1)));
+        if (!dRows16) return fail(h, SJBG_E_NOMEM, "partition staging buffers");
+    }
     if (!dComp || !dRows || !dCcnt || !dWork) return fail(h, SJBG_E_NOMEM, "partition staging buffers");
     SJBG_CK(h, cudaMemsetAsync(dCcnt, 0, sizeof(uint32_t) * (2 * n + 1), h->stream));
     uint64_t *dCompR = dComp + (uint64_t)kTile * tileL[n];
@@ -2269,7 +2537,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     auto scan = [&]() {
         return launch(h, "part_scan", part_scan_win_kernel, dim3(n), dim3(1024), 0, (const WinPlan *)dPlan, dPbL, dPbR,
                       (const uint32_t *)dCnt, dStart, dCur, (uint32_t)B, dModels, dJlist, dJn, join_chunk,
-                      enumerate ? 0x0FFFFFFFu : cap, !enumerate);
+                      enumerate ? 0x0FFFFFFFu : cap, !enumerate, (const uint32_t *)dCcnt);
     };
     if (!tiles && any_raw) SJBG_CK(h, scan());
     if (tiles) {
@@ -2281,15 +2549,15 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             SJBG_CK(h, launch(h, "heavy_finish", heavy_finish_kernel, dim3(n), dim3(256), 0, (const WinPlan *)dPlan, n,
                               dModels, (const HeavyAcc *)dHeavy, acc));
         // the tiles each later pass has work for (compacted windows: their light tiles only)
-        SJBG_CK(h, launch(h, "part_work", part_work_kernel, dim3(1), dim3(192), 0, (const WinPlan *)dPlan, n, dTileL,
+        SJBG_CK(h, launch(h, "part_work", part_work_kernel, dim3(1), dim3(32 * kWorkArrays), 0, (const WinPlan *)dPlan, n, dTileL,
                           dTileR, dItL, dItR, dModels, (const uint32_t *)dCcnt, dWork));
         if (learned && !enumerate) {   // compacted windows exist only with heavy keys
-            allow_big_smem(part_hist_light_kernel, sizeof(uint32_t) * maxP);
-            const uint32_t lgrid = std::min<uint32_t>(tiles, 4u * (uint32_t)h->num_sms);
-            SJBG_CK(h, launch(h, "part_hist_light", part_hist_light_kernel, dim3(lgrid), dim3(kPartThreads),
-                              sizeof(uint32_t) * maxP, (const WinPlan *)dPlan, n, dTileL, dTileR,
-                              (const uint32_t *)dWork, dCnt, (uint32_t)B, dModels, (const uint64_t *)dComp,
-                              (const uint64_t *)dCompR, (const uint32_t *)dCcnt));
+            const size_t lightSmem = kTile * sizeof(uint64_t) + sizeof(uint32_t) * maxP;
+            allow_big_smem(part_light_kernel, lightSmem);
+            SJBG_CK(h, launch(h, "part_light", part_light_kernel, dim3(std::min<uint32_t>(tiles, 2u * (uint32_t)h->num_sms)),
+                              dim3(kPartThreads), lightSmem, (const WinPlan *)dPlan, n, dTileL, dTileR,
+                              (const uint32_t *)dWork, dCnt, (uint32_t)B, dModels, dComp, dCompR, (const uint32_t *)dCcnt,
+                              dRows16, rstride));
         }
         SJBG_CK(h, scan());
         // single-level windows, and compacted windows (their packed light tuples):
@@ -2326,20 +2594,26 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
                           (const uint64_t *)dPL, (const uint64_t *)dPR, acc, (const WinPlan *)dPlan, dPairs, bits,
                           (const JoinItem *)dJlist, (const uint32_t *)dJn));
     } else {
-        const size_t smem = std::max({count_table_bytes(cap), kDirectBytes, kPlaceBytes});
+        const size_t smem = std::max({count_table_bytes(cap), kDirectBytes, kPlaceBytes, rows_lg ? rows_join_bytes(cap) : 0});
+        RowsJoin rj{};
+        // the queues: join items, then (16 bytes on) the buckets joined from sorted tiles
+        uint32_t *queues = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_WIN, 64));
+        if (!queues) return fail(h, SJBG_E_NOMEM, "work queue");
+        SJBG_CK(h, cudaMemsetAsync(queues, 0, 32, h->stream));
+        if (rows_lg && tiles)
+            rj = RowsJoin{n, rstride, dTileL, dTileR, (const uint32_t *)dWork, (const uint32_t *)dCcnt,
+                          dComp, dCompR, (const uint16_t *)dRows16, queues + 4};
         auto join = learned ? bucket_join_count_kernel<true> : bucket_join_count_kernel<false>;
         allow_big_smem(join, smem);
         if (h->tune.persistent_join && max_items > (uint64_t)h->num_sms) {
-            queue = static_cast<uint32_t *>(ws_get(h, WS_BUCKET_WIN, 64));
-            if (!queue) return fail(h, SJBG_E_NOMEM, "work queue");
-            SJBG_CK(h, cudaMemsetAsync(queue, 0, 4, h->stream));
+            queue = queues;
             // as many persistent CTAs as fit on an SM at this table size (at most 2 by registers)
             const uint32_t per_sm = std::max<uint32_t>(1, (uint32_t)((228u << 10) / (smem + 1024)));
             jgrid = dim3((uint32_t)std::min<uint64_t>(max_items, (uint64_t)h->num_sms * std::min<uint32_t>(per_sm, 2u)));
         }
         SJBG_CK(h, launch(h, "bucket_join_count", join, jgrid, dim3(kJoinThreads), smem, dL, dR,
                           (const WinPlan *)dPlan, dPL, dPR, (const uint32_t *)dStart, (const uint32_t *)dCnt,
-                          (uint32_t)B, acc, cap, queue, (const JoinItem *)dJlist, (const uint32_t *)dJn));
+                          (uint32_t)B, acc, cap, queue, (const JoinItem *)dJlist, (const uint32_t *)dJn, rj));
     }
     return SJBG_OK;
 }
@@ -2389,7 +2663,7 @@ __global__ void raw_setup_kernel(RawScratch *rs, uint32_t *cnt, uint32_t P, uint
         WinPlan &p = rs->plan;
         p.left_off = 0; p.n_left = nL; p.right_off = 0; p.n_right = nR;
         p.pairs_off = 0; p.pairs_cap = 0;
-        p.bucket_base = 0; p.log2_buckets = lg; p.model = 0xFFFFFFFFu; p.two_level = 0; p.raw = 0;
+        p.bucket_base = 0; p.log2_buckets = lg; p.model = 0xFFFFFFFFu; p.two_level = 0; p.raw = 0; p.rows = 0;
         rs->tile[0] = 0; rs->tile[1] = tL;
         rs->tile[2] = 0; rs->tile[3] = tR;
         rs->tile[4] = 0; rs->tile[5] = (tL + kHistTiles - 1) / kHistTiles;
@@ -2471,7 +2745,7 @@ int hj_count_window_raw(const sjbg_tuple *dL, uint64_t nL, const sjbg_tuple *dR,
         const size_t smem = std::max({count_table_bytes(cap), kDirectBytes, kPlaceBytes});
         allow_big_smem(bucket_join_count_kernel<false>, smem);
         bucket_join_count_kernel<false><<<P, kJoinThreads, smem, st>>>(dL, dR, &rs->plan, pL, pR, start, cnt, P, rs->acc,
-                                                                cap, nullptr, nullptr, nullptr);
+                                                                cap, nullptr, nullptr, nullptr, RowsJoin{});
         if (int rc = launched("sjbg_lazy_hj_noalloc: bucket_join_count_kernel")) return rc;
     }
     raw_finish_kernel<<<1, 32, 0, st>>>(rs, dOut);

@@ -27,6 +27,7 @@ enum WsSlot : int {
     WS_COMPACT, WS_COMPACT_CNT,      // light tuples written by the counting pass
     WS_COARSE_ROWS,                  // per tile: coarse-partition offsets of its light tuples
     WS_EAGER_META, WS_EAGER_K0, WS_EAGER_K1, WS_EAGER_V0, WS_EAGER_V1, WS_EAGER_TILES,   // recorded eager streams
+    WS_ROWS16,                       // rows of sorted tiles (learned windows)
     WS_RAW_ACC,                      // accumulators of raw-only hash joins (zero between calls)
     WS_COUNT
 };
