@@ -241,6 +241,14 @@ part_hist_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict_
             // the tuples of a tile, compiled apart for full tiles (no bounds test)
             auto count_tuples = [&](auto full_t) {
             constexpr bool kFull = decltype(full_t)::value;
+            auto lookup = [&](int k) {
+                return kFull || threadIdx.x + k * kPartThreads < n ? heavy_find(hs, v[k].x) : kHeavyBucket;
+            };
+            // the next tuple's lookup is under way while one is summed, and the count
+            // is added while the low word's old value returns (2 x 2^24: z = 1.0
+            // 1,175 -> 1,123 us; four lookups, then four sums: z = 1.5 406 -> 431)
+            uint32_t next_hid = kHeavyBucket;
+            if constexpr (kHeavy) next_hid = lookup(0);
 #pragma unroll
             for (int k = 0; k < kPer; k++) {
                 const uint32_t i = threadIdx.x + k * kPartThreads;
@@ -248,13 +256,14 @@ part_hist_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict_
                 const uint32_t key = v[k].x, val = v[k].y;
                 pk[k] = 0xFFFFFFFFu;
                 if constexpr (kHeavy) {
-                    const uint32_t hid = valid ? heavy_find(hs, key) : kHeavyBucket;
+                    const uint32_t hid = next_hid;
+                    if (k + 1 < kPer) next_hid = lookup(k + 1);
                     if (hid != kHeavyBucket) {
                         const unsigned long long f = sjbg_fside(val, right ? 1u : 0u);   // one mix, either side
                         const uint32_t a = hid < kHotHeavy ? kMaxHeavy + 32u * hid + lane_id() : hid;
-                        atomicAdd(&hcnt[a], 1u);
                         const uint32_t flo = (uint32_t)f;
                         const uint32_t old = atomicAdd(&hsum_lo[a], flo);
+                        atomicAdd(&hcnt[a], 1u);
                         atomicAdd(&hsum_hi[a], add_carry((uint32_t)(f >> 32), old, flo));
                     } else if (valid) {
                         // light keys: compacted windows count or sort them in part_light
