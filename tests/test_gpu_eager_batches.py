@@ -22,6 +22,8 @@ def place(torch, t, kind):
         return raw.cuda(), "MEM_DEVICE"
     buf = torch.zeros(raw.numel() + 16, dtype=torch.uint8, device="cuda" if kind == "device+8" else "cpu")
     buf[8:8 + raw.numel()] = raw.to(buf.device)
+    if kind == "device+8":
+        torch.cuda.synchronize()   # the copy above is on another stream than the handle's
     return buf[8:8 + raw.numel()], "MEM_DEVICE" if kind == "device+8" else "MEM_HOST"
 
 
