@@ -964,27 +964,44 @@ part_scatter_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restri
                     const uint64_t *__restrict__ compR, const uint32_t *__restrict__ ccnt) {
     // persistent CTAs over the tiles listed by the work prefixes workL / workR
     // (a compacted window's light tiles; a single-level window's tiles), each
-    // tile's loads issued while the previous tile is written out
-    const uint32_t items = workL[nwin] + workR[nwin];
-    uint32_t bt = blockIdx.x;
-    if (bt >= items) return;
+    // tile's loads issued while the previous tile is written out.  Without models
+    // a CTA takes a run of neighbours: the prefixes are searched once per window
+    // side instead of once per tile (ten loads, one after the other, with 1,024
+    // windows: 1,347 -> 1,215 us).  With models tiles cost what their light
+    // tuples cost, and every gridDim.x-th spreads them better (3 x 2,000,000 at
+    // z = 1.0: 113 us, by runs 119).
+    const uint64_t items = workL[nwin] + workR[nwin];
+    uint32_t bt = kRadixOnly ? (uint32_t)(blockIdx.x * items / gridDim.x) : blockIdx.x;
+    const uint32_t bt_end = kRadixOnly ? (uint32_t)((blockIdx.x + 1) * items / gridDim.x) : (uint32_t)items;
+    const uint32_t step = kRadixOnly ? 1u : gridDim.x;
+    if (bt >= bt_end) return;
     WorkItem it = work_item(workL, workR, nwin, bt);
+    auto last_of = [&](const WorkItem &x) {   // the last tile of x's window side
+        const uint32_t *p = x.right ? workR : workL;
+        return p[x.w + 1] - p[x.w] - 1;
+    };
+    uint32_t last = kRadixOnly ? last_of(it) : 0u;
     TileIn in = tile_input(it, L, R, wins, tileL, tileR, models, compL, compR, ccnt);
     uint64_t e[kScatterPer];
     tile_load(in, e);
-    for (; bt < items; bt += gridDim.x) {
+    for (; bt < bt_end; bt += step) {
         SJBG_BARRIER();   // the previous tile's shared-memory readers are done
-        const uint32_t nb = bt + gridDim.x;
+        const uint32_t nb = bt + step;
         WorkItem nit = it;
         TileIn nin = in;
-        if (nb < items) {
-            nit = work_item(workL, workR, nwin, nb);
+        if (nb < bt_end) {
+            if (kRadixOnly && it.local < last) {
+                nit.local++;
+            } else {
+                nit = work_item(workL, workR, nwin, nb);
+                if (kRadixOnly) last = last_of(nit);
+            }
             nin = tile_input(nit, L, R, wins, tileL, tileR, models, compL, compR, ccnt);
         }
         if (kRadixOnly || (!in.packed && !model_of(wins[it.w], models)))
-            scatter_tile_radix(it, in, e, nb < items ? &nin : nullptr, wins, cursor, B, outL, outR);
+            scatter_tile_radix(it, in, e, nb < bt_end ? &nin : nullptr, wins, cursor, B, outL, outR);
         else
-            scatter_tile(it, in, e, nb < items ? &nin : nullptr, wins, cursor, B, outL, outR, models);
+            scatter_tile(it, in, e, nb < bt_end ? &nin : nullptr, wins, cursor, B, outL, outR, models);
         it = nit;
         in = nin;
     }
@@ -1375,28 +1392,49 @@ __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const Join
                 word[atomicAdd(&at[1 + (place_hash((uint32_t)e[k]) >> shift)], 1u)] = e[k];
     }
     SJBG_BARRIER();
-    for (uint32_t base = 0; base < nP; base += tile) {
+    // kProbe probes of a thread at a time, step by step for all of them: the
+    // bounds of their places, the first two words of each, and what is left of
+    // longer ones.  The hash of a matching word is taken after the compares, once
+    // per probe instead of once per compare that matches in some lane.  (1,024
+    // windows of 2^10 to 2^20: 1,681 -> 1,470 us, one probe at a time before;
+    // with the hash table out of line as well, 1,406.)
+    constexpr int kProbe = 4;
+    for (uint32_t base = 0; base < nP; base += kProbe * kJoinThreads) {
+        uint64_t pr[kProbe], x0[kProbe], x1[kProbe];
+        uint32_t j[kProbe], end[kProbe];
 #pragma unroll
-        for (int k = 0; k < kJoinPer; k++) {
-            const uint32_t j = base + k * kJoinThreads + threadIdx.x;
-            e[k] = j < nP ? run_load<kRaw>(jr.p, j) : 0ull;
+        for (int k = 0; k < kProbe; k++) {
+            const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+            pr[k] = i < nP ? run_load<kRaw>(jr.p, i) : 0ull;
         }
 #pragma unroll
-        for (int k = 0; k < kJoinPer; k++) {
-            if (base + k * kJoinThreads + threadIdx.x >= nP) continue;
-            const uint32_t key = (uint32_t)e[k], p = place_hash(key) >> shift, end = at[p + 1];
-            uint32_t c = 0;
+        for (int k = 0; k < kProbe; k++) {
+            const uint32_t q = place_hash((uint32_t)pr[k]) >> shift;
+            j[k] = at[q];
+            end[k] = base + k * kJoinThreads + threadIdx.x < nP ? at[q + 1] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kProbe; k++) {
+            x0[k] = j[k] < end[k] ? word[j[k]] : 0ull;
+            x1[k] = j[k] + 1 < end[k] ? word[j[k] + 1] : 0ull;
+        }
+#pragma unroll
+        for (int k = 0; k < kProbe; k++) {
+            const uint32_t key = (uint32_t)pr[k];
+            uint32_t c = 0, m = 0;
             unsigned long long f = 0;
-            for (uint32_t j = at[p]; j < end; j++) {
-                const uint64_t x = word[j];
-                if ((uint32_t)x == key) {
-                    c++;
-                    f += sjbg_fside((uint32_t)(x >> 32), bside);
+            auto compare = [&](uint64_t x, bool in) {
+                if (in && (uint32_t)x == key) {
+                    if (c++) f += sjbg_fside((uint32_t)(x >> 32), bside);
+                    else m = (uint32_t)(x >> 32);
                 }
-            }
+            };
+            compare(x0[k], j[k] < end[k]);
+            compare(x1[k], j[k] + 1 < end[k]);
+            for (uint32_t i = j[k] + 2; i < end[k]; i++) compare(word[i], true);
             if (c) {
                 count += c;
-                prod += f * sjbg_fside((uint32_t)(e[k] >> 32), pside);
+                prod += (f + sjbg_fside(m, bside)) * sjbg_fside((uint32_t)(pr[k] >> 32), pside);
             }
         }
     }
@@ -1854,6 +1892,15 @@ __device__ __forceinline__ void join_enum_bucket(const JoinItem &ji, const uint6
     flush_acc(&acc[w], count, xr, prod);
 }
 
+// The hash table for what neither a direct table nor the places take: out of
+// line, so that the code of the usual items stays short.
+template <bool kRaw>
+__device__ __noinline__ void join_count_rest(const JoinItem &ji, const JoinRuns &jr, uint32_t cap,
+                                             unsigned long long &count, unsigned long long &prod) {
+    uint64_t e[kJoinPer];
+    join_count_bucket<kRaw>(ji, jr, e, false, cap, count, prod);
+}
+
 // One item's matches; `clean` as in join_count_direct, `turn` as in build_head
 // (0 at the CTA's first item).
 template <bool kRaw, bool kModels>
@@ -1875,7 +1922,7 @@ __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr
     }
     clean = 0;
     if (ji.nB <= kPlaceCap && join_count_places<kRaw>(ji, jr, e, count, prod)) return;
-    join_count_bucket<kRaw>(ji, jr, e, true, cap, count, prod);
+    join_count_rest<kRaw>(ji, jr, cap, count, prod);
 }
 
 // ---- joins from sorted tiles
@@ -2576,7 +2623,9 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             // without a learned partitioner every window is radix-partitioned
             auto scatter = learned ? part_scatter_kernel<false> : part_scatter_kernel<true>;
             allow_big_smem(scatter, scatterSmem);
-            const uint32_t sgrid = std::min<uint32_t>(tiles, 3u * 4u * (uint32_t)h->num_sms);
+            // (radix runs of neighbours: 1,024 windows 3,415 us with 3 CTAs per SM, 3,380
+            // with 6, 3,350 with 12, 3,324 with 24)
+            const uint32_t sgrid = std::min<uint32_t>(tiles, 3u * (learned ? 4u : 8u) * (uint32_t)h->num_sms);
             const uint32_t *wS = dWork + 2 * kWorkScatter * (n + 1);
             SJBG_CK(h, launch(h, "part_scatter", scatter, dim3(sgrid), dim3(kPartThreads), scatterSmem,
                               dL, dR, dPlan, n, dTileL, dTileR, wS, wS + (n + 1), dCur, (uint32_t)B, dPL, dPR,
