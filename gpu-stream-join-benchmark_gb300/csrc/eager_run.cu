@@ -17,15 +17,22 @@
 // compared by one grid of register-blocked CTAs (nlj.cu's block routine); a
 // block pair adds its matches to the later batch's count and its checksums to
 // the window.
-// Hash and sort-merge joins: the batch counts come from one stable sort per
-// window: the window's keys in arrival order are sorted (sort.cu) with each
-// tuple's arrival position as payload, so each key group lists its tuples in
-// arrival order and a tuple's count is the number of other-side tuples before
-// it in its group, which a segmented scan over the sorted window gives.
-// Sort-merge without pair enumeration takes the window totals from the same
-// pass (count = the sum of those counts, prod = the same pairs weighted by
-// fr * gs); otherwise they come from the lazy join of the windows (hj.cu /
-// smj.cu).
+// Hash and sort-merge joins, counting handles: every tile of the window's
+// tuples is sorted by a bucket of the key's hash, and one CTA per bucket lists
+// the left words of each key in arrival order and counts, for every word, the
+// other side's earlier ones (egroup_*; the batch counts and the window totals
+// in one pass).  A bucket that does not fit (few distinct keys) sets
+// kErrRegroup: the call is made again by the sort below, which the handle then
+// keeps to.  2^20 tuples per window, 768 batches of 4,096: 478 us by the sort,
+// 167 by buckets.
+// By the sort (also pair enumeration and xor): the window's keys in arrival
+// order are sorted (sort.cu) with each tuple's arrival position as payload, so
+// each key group lists its tuples in arrival order and a tuple's count is the
+// number of other-side tuples before it in its group, which a segmented scan
+// over the sorted window gives.  Sort-merge without pair enumeration takes the
+// window totals from the same pass (count = the sum of those counts, prod =
+// the same pairs weighted by fr * gs); otherwise they come from the lazy join
+// of the windows (hj.cu / smj.cu).
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -11,20 +11,26 @@
 //                    -> one atomicAdd per non-empty bucket into the global counts.
 //   2. part_scan     per window, exclusive scan of its counts on both sides ->
 //                    bucket starts; buckets with tuples on both sides form the
-//                    join list (item records), the only buckets step 4 visits.
+//                    join list: the smaller run builds, a long probe run is cut
+//                    in pieces, and both runs of a bucket far longer than its
+//                    table are.  A window whose smaller side is one bucket is
+//                    not partitioned: its pieces read the tuples themselves.
 //   3. part_scatter  per tile: local counting sort by bucket in shared memory,
 //                    one atomicAdd per bucket to reserve a range, then the tile
 //                    is written as contiguous per-bucket runs of (key,val) words
 //                    (windows of many buckets: a coarse pass inside part_hist,
-//                    then part_fine).
+//                    then part_fine).  A learned window's compacted light tuples
+//                    are only sorted by bucket inside their tiles (part_light),
+//                    and the join takes a bucket's runs out of all tiles.
 //   4. bucket_join   per join item (persistent CTAs, one item ahead): a radix
-//                    window's bucket through a direct table indexed by
-//                    key >> radix bits when its indices allow it, else an
-//                    open-addressing table in shared memory from the left run,
-//                    probed with the right run.
-//        count mode: table slot = {key, count, sum fr(val)}, updated with
+//                    bucket through a direct table indexed by key >> radix bits
+//                    when its indices allow it, else by places (short lists by
+//                    a hash of the key), else through an open-addressing table,
+//                    as learned buckets; built from the build run, probed with
+//                    the other.
+//        count mode: table slot = {key, count, hash sum}, updated with
 //                    32-bit shared atomics (the sum as two words with carry);
-//                    keys that do not fit go back into the left run (compacted
+//                    keys that do not fit go back into the build run (compacted
 //                    in place) and are joined in a further pass, so any bucket,
 //                    however skewed, finishes.
 //        enum mode:  table slot = {key, chain head}, chains over a staged chunk
@@ -32,6 +38,8 @@
 //                    and, when asked, written with one atomic per warp.
 // The bucket of a key is its low radix bits (plain radix partitioning) or the
 // learned partitioner's prediction (learned.cu).
+// Counting calls of small windows only take one launch (hj_raw_batch), and
+// those of the middle of the size range go by hash ranges (range_join.cu).
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -1691,9 +1699,10 @@ __device__ __noinline__ void join_count_hot(const uint64_t *b, uint32_t nB, cons
 // bucket whose indices need more than kDirectPasses passes goes through the
 // hash table: the build run's smallest and largest keys, found while its first
 // tile is loaded, decide.  (Learned buckets, which are key ranges, gained
-// nothing: their probes match, and the range costs a barrier to find.)  Measured on 1,024 uneven windows (keys in [0, 4W),
-// about 4,096 left tuples per bucket, two passes): the bucket joins take
-// 2.02 ms, against 2.91 ms with hash tables.
+// nothing: their probes match, and the range costs a barrier to find.)
+// Measured on 1,024 uneven windows (keys in [0, 4W), about 4,096 left tuples
+// per bucket, two passes): the bucket joins take 2.02 ms, against 2.91 ms with
+// hash tables.
 constexpr uint32_t kDirectMax = 8192;
 constexpr uint32_t kDirectPasses = 2;
 // A build run of at most kDirectSave tuples keeps each tuple's table index (16
@@ -1901,12 +1910,17 @@ __device__ __forceinline__ void join_enum_bucket(const JoinItem &ji, const uint6
 }
 
 // The hash table for what neither a direct table nor the places take: out of
-// line, so that the code of the usual items stays short.
+// line, so that the code of the usual items stays short (and by value, so that
+// nothing of theirs lives in local memory).
+struct JoinSums {
+    unsigned long long count, prod;
+};
 template <bool kRaw>
-__device__ __noinline__ void join_count_rest(const JoinItem &ji, const JoinRuns &jr, uint32_t cap,
-                                             unsigned long long &count, unsigned long long &prod) {
+__device__ __noinline__ JoinSums join_count_rest(const JoinItem ji, const JoinRuns jr, uint32_t cap) {
     uint64_t e[kJoinPer];
-    join_count_bucket<kRaw>(ji, jr, e, false, cap, count, prod);
+    JoinSums r{0, 0};
+    join_count_bucket<kRaw>(ji, jr, e, false, cap, r.count, r.prod);
+    return r;
 }
 
 // One item's matches; `clean` as in join_count_direct, `turn` as in build_head
@@ -1930,7 +1944,9 @@ __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr
     }
     clean = 0;
     if (ji.nB <= kPlaceCap && join_count_places<kRaw>(ji, jr, e, count, prod)) return;
-    join_count_rest<kRaw>(ji, jr, cap, count, prod);
+    const JoinSums r = join_count_rest<kRaw>(ji, jr, cap);
+    count += r.count;
+    prod += r.prod;
 }
 
 // ---- joins from sorted tiles

@@ -21,7 +21,7 @@
 // The tuples are read once, their words written and read once; the full radix
 // sort reads and writes them three or four times, and the merge once more
 // (128 windows of 2^10 to 2^20 tuples per side, keys in [0, 4 max(W)), 22.5 M
-// tuples: 1.64 ms, and 0.60 by ranges).  A range that does not fit (hot or
+// tuples: 1.64 ms, and 0.55 by ranges).  A range that does not fit (hot or
 // clustered keys) sets kErrRegroup, and the host makes the call again with the
 // full sort.
 //

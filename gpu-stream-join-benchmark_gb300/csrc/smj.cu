@@ -6,9 +6,9 @@
 // is the lazy CPU_SMJ's (src/sjb/windowing/lazy/executor/CPU/CPU_SMJ.cpp:23-139):
 // both sides sorted by key, then every key group's cartesian product.
 //
-// Counting joins that are waited for go by key ranges instead when the windows'
-// sizes and keys suit them (range_join.cu).  Steps for a batch of windows (left sides are segments [0, n), right sides
-// [n, 2n) of one segmented sort):
+// Joins that are waited for go by key ranges instead when the windows' sizes
+// and keys suit them (range_join.cu).  Steps for a batch of windows (left sides
+// are segments [0, n), right sides [n, 2n) of one segmented sort):
 //   1. sort_extract + radix_sort_segments (sort.cu): stable LSD sort of
 //      (key, val) for every window side;
 //   2. segmented_fr_prefix: F[i] = sum of fr(val) over the first i sorted left
