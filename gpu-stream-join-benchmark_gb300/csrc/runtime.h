@@ -19,12 +19,12 @@ namespace sjbg {
 enum WsSlot : int {
     WS_IN_LEFT, WS_IN_RIGHT,         // staging copies of host inputs
     WS_PART_LEFT, WS_PART_RIGHT,     // partitioned (key,val) arrays
-    WS_BUCKET_CNT, WS_BUCKET_START, WS_BUCKET_CURSOR, WS_BUCKET_WIN,
+    WS_BUCKET_CNT, WS_BUCKET_START, WS_BUCKET_CURSOR,
     WS_WIN_PLAN, WS_TILE_PREFIX, WS_WIN_ACC, WS_PAIRS, WS_STATUS,
-    WS_MODEL, WS_SAMPLE, WS_SAMPLE_KEYS, WS_HEAVY, WS_AUX0, WS_AUX1, WS_AUX2, WS_AUX3,
+    WS_MODEL, WS_SAMPLE, WS_SAMPLE_KEYS, WS_AUX0, WS_AUX1, WS_AUX2, WS_AUX3,
     WS_SORT_K0, WS_SORT_K1, WS_SORT_V0, WS_SORT_V1, WS_SORT_HIST, WS_SORT_MAP, WS_SORT_VIEW,
     WS_GEN_TABLE,
-    WS_COMPACT, WS_COMPACT_CNT,      // light tuples written by the counting pass
+    WS_COMPACT,                      // light tuples written by the counting pass
     WS_COARSE_ROWS,                  // per tile: coarse-partition offsets of its light tuples
     WS_EAGER_META, WS_EAGER_K0, WS_EAGER_K1, WS_EAGER_V0, WS_EAGER_V1, WS_EAGER_TILES,   // recorded eager streams
     WS_ROWS16,                       // rows of sorted tiles (learned windows)
@@ -150,6 +150,29 @@ cudaError_t launch(sjbg_handle *h, const char *name, void (*kernel)(KArgs...), d
         h->pending.push_back({kernel_id(h, name), a, b});
     }
     return e;
+}
+
+// The same for a kernel that follows another one of this library on the
+// stream and begins with kernel_chain(): its launch overlaps the end of the
+// kernel before (a profiled call keeps the two apart).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_next(sjbg_handle *h, const char *name, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                        size_t smem, Args &&...args) {
+    if ((h->cfg.flags & SJBG_F_PROFILE) && !h->capturing)
+        return launch(h, name, kernel, grid, block, smem, std::forward<Args>(args)...);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    h->launches++;
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 // Raise a kernel's dynamic shared-memory limit on the current device to at
