@@ -512,7 +512,7 @@ bool PowerSampler::start() {
     n = 0;
     thread = new std::thread([this, nv, dev] {
         FILE *fp = std::fopen(path.c_str(), "a");
-        while (run) {
+        do {   // (a run that ends before this thread starts is sampled once)
             unsigned mw = 0;
             if (fp && nv->power(dev, &mw) == 0) {
                 const long long ms = std::chrono::duration_cast<std::chrono::milliseconds>(
@@ -522,7 +522,7 @@ bool PowerSampler::start() {
                 n++;
             }
             std::this_thread::sleep_for(std::chrono::milliseconds(period_ms));
-        }
+        } while (run);
         if (fp) std::fclose(fp);
         nv->shutdown();
         dlclose(nv->lib);
