@@ -1246,19 +1246,27 @@ __device__ __forceinline__ bool ct_insert(const CountTable &t, uint32_t key, uin
         return true;
     }
     uint32_t s = ct_home(key, C);
-    for (uint32_t probe = 0; probe < t.max_probe; probe++) {
+    auto step = [&]() {   // the key is in slot s now
         uint32_t k = *(volatile uint32_t *)&t.keys[s];
         if (k == kEmptyKey) {
             const uint32_t prev = atomicCAS(&t.keys[s], kEmptyKey, key);
             k = prev == kEmptyKey ? key : prev;
         }
-        if (k == key) {
-            atomicAdd(&t.cnt[s], c);
-            ct_add_sum(&t.sumf[s], f);
-            return true;
+        if (k != key) {
+            s = s + 1 == C ? 0 : s + 1;
+            return false;
         }
-        s = s + 1 == C ? 0 : s + 1;
-    }
+        atomicAdd(&t.cnt[s], c);
+        ct_add_sum(&t.sumf[s], f);
+        return true;
+    };
+    // (a constant bound, unrolled, and the rest apart: with the bound in a register
+    // the joins of 2 x 2^24 tuples at 2^10 buckets took 4.9 ms instead of 3.5)
+    for (uint32_t probe = 0; probe < kMaxProbe; probe++)
+        if (step()) return true;
+#pragma unroll 1
+    for (uint32_t probe = kMaxProbe; probe < t.max_probe; probe++)
+        if (step()) return true;
     return false;
 }
 
@@ -1266,7 +1274,14 @@ __device__ __forceinline__ int ct_lookup(const CountTable &t, uint32_t key) {
     const uint32_t C = t.C;
     if (key == kEmptyKey) return t.cnt[C] ? (int)C : -1;
     uint32_t s = ct_home(key, C);
-    for (uint32_t probe = 0; probe < t.max_probe; probe++) {
+    for (uint32_t probe = 0; probe < kMaxProbe; probe++) {
+        const uint32_t k = t.keys[s];
+        if (k == key) return (int)s;
+        if (k == kEmptyKey) return -1;
+        s = s + 1 == C ? 0 : s + 1;
+    }
+#pragma unroll 1
+    for (uint32_t probe = kMaxProbe; probe < t.max_probe; probe++) {
         const uint32_t k = t.keys[s];
         if (k == key) return (int)s;
         if (k == kEmptyKey) return -1;
@@ -1466,8 +1481,8 @@ __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const Join
 }
 
 // Larger buckets (a radix window's hot keys) keep the hash table when they need
-// a second direct pass, which re-reads the bucket; and every longer build run
-// does, as the direct table's reset re-reads it.
+// a second direct pass, which re-reads the bucket; every build run of more than
+// kPlaceCap tuples does, and its range is not looked for.
 constexpr uint32_t kDirectMaxRun = 16384;
 
 struct KeyRange {
@@ -1475,9 +1490,7 @@ struct KeyRange {
 };
 
 // Loads the first tile of a build run (kJoinPer tuples per thread) and returns
-// the run's smallest and largest keys to every thread (those of its first
-// tile, when the run is too long for a direct table anyway); ends with a
-// barrier, its only one after the CTA's first call (turn 0): the calls take the
+// the run's smallest and largest keys to every thread; ends with a barrier, its only one after the CTA's first call (turn 0): the calls take the
 // two result slots in turn and leave the other one reset.
 template <bool kRaw>
 __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
@@ -1505,12 +1518,10 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
             hi = max(hi, (uint32_t)e[k]);
         }
     }
-    if (ji.nB <= kDirectMaxRun) {
-        for (uint32_t i = kJoinPer * kJoinThreads + threadIdx.x; i < ji.nB; i += kJoinThreads) {
-            const uint32_t key = (uint32_t)run_load<kRaw>(jr.b, i);
-            lo = min(lo, key);
-            hi = max(hi, key);
-        }
+    for (uint32_t i = kJoinPer * kJoinThreads + threadIdx.x; i < ji.nB; i += kJoinThreads) {
+        const uint32_t key = (uint32_t)run_load<kRaw>(jr.b, i);
+        lo = min(lo, key);
+        hi = max(hi, key);
     }
     lo = __reduce_min_sync(0xFFFFFFFFu, lo);
     hi = __reduce_max_sync(0xFFFFFFFFu, hi);
@@ -1721,7 +1732,6 @@ constexpr size_t kDirectBytes =
 
 // Passes of a bucket whose build run has keys in kr, or 0: the hash table.
 __device__ __forceinline__ uint32_t direct_passes(const JoinItem &ji, KeyRange kr) {
-    if (ji.nB > kDirectMaxRun) return 0;
     const uint32_t passes = ((kr.hi >> ji.lg) - (kr.lo >> ji.lg)) / kDirectMax + 1;
     if (passes > kDirectPasses || (passes > 1 && ji.nB + ji.nP > kDirectMaxRun)) return 0;
     return passes;
@@ -1944,10 +1954,12 @@ __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr
         clean = 0;
         return;
     }
-    const KeyRange kr = build_head<kRaw>(ji, jr, e, turn);
-    if (const uint32_t passes = direct_passes(ji, kr)) {
-        join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, clean, count, prod);
-        return;
+    if (ji.nB <= kPlaceCap) {
+        const KeyRange kr = build_head<kRaw>(ji, jr, e, turn);
+        if (const uint32_t passes = direct_passes(ji, kr)) {
+            join_count_direct<kRaw>(ji, jr, e, kr.lo >> ji.lg, passes, clean, count, prod);
+            return;
+        }
     }
     clean = 0;
     if (ji.nB <= kPlaceCap && join_count_places<kRaw>(ji, jr, e, count, prod)) return;
