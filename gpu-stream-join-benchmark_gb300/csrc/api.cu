@@ -122,7 +122,6 @@ void *pinned_get(sjbg_handle *h, int i, size_t bytes) {
 // loads over the host link, no byte tail.
 __global__ void stage_copy_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, size_t bytes,
                                   bool vec) {
-    kernel_chain();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t n16 = vec ? (bytes + 15) / 16 : 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += stride)
@@ -149,7 +148,6 @@ int zero_fill(sjbg_handle *h, void *dst, size_t bytes) {
 // CTA zeroes its share of zdst.
 __global__ void stage_copy_zero_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, size_t bytes,
                                        bool vec, uint4 *__restrict__ zdst, size_t n16) {
-    kernel_chain();
     if (blockIdx.x == 0) {
         if (vec) {
             for (size_t i = threadIdx.x; i < (bytes + 15) / 16; i += blockDim.x)
@@ -179,7 +177,7 @@ int stage_copy(sjbg_handle *h, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return SJBG_OK;
     const bool vec = (((uintptr_t)dst | (uintptr_t)src) & 15u) == 0;
     const uint32_t blocks = (uint32_t)std::min<size_t>(64, (bytes + 4095) / 4096);
-    SJBG_CK(h, launch_next(h, "stage_copy", stage_copy_kernel, dim3(blocks), dim3(256), 0, static_cast<uint8_t *>(dst),
+    SJBG_CK(h, launch(h, "stage_copy", stage_copy_kernel, dim3(blocks), dim3(256), 0, static_cast<uint8_t *>(dst),
                       static_cast<const uint8_t *>(src), bytes, vec));
     return SJBG_OK;
 }

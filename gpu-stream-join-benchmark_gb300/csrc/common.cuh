@@ -94,16 +94,6 @@ __device__ __forceinline__ uint32_t add_carry(uint32_t hi, uint32_t a, uint32_t 
     return r;
 }
 
-// First statement of a kernel that launch_next starts, and of one before it:
-// waits until the kernel before has finished and its writes are visible, then
-// lets the next one's CTAs take the SMs as this one's leave them.  Nothing of
-// another kernel is read or written before it.  (No effect on a kernel launched
-// in the usual way, but for the second part.)
-__device__ __forceinline__ void kernel_chain() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Exclusive warp prefix sum of a 32-bit value.
 __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *total) {
     uint32_t x = v;

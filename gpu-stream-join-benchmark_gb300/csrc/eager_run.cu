@@ -458,7 +458,6 @@ egroup_sort_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restric
                    const EGroupWin *__restrict__ wins, uint32_t nw, uint32_t tiles, uint32_t B, uint32_t ts,
                    uint32_t tpb, uint32_t lg, uint64_t *__restrict__ words, uint32_t wstride,
                    uint16_t *__restrict__ rows) {
-    kernel_chain();
     struct Bucket {
         uint32_t lg;
         __device__ uint32_t operator()(uint32_t key) const { return group_bucket(key, lg); }
@@ -504,7 +503,6 @@ __global__ void __launch_bounds__(kGroupThreads, 3)
 egroup_count_kernel(const uint64_t *__restrict__ words, uint32_t wstride, const uint16_t *__restrict__ rows,
                     const EGroupWin *__restrict__ wins, uint32_t nw, uint32_t tpb, uint32_t lg,
                     unsigned long long *__restrict__ counts, WinAcc *__restrict__ acc, uint32_t *__restrict__ status) {
-    kernel_chain();
     extern __shared__ __align__(16) uint8_t smem_raw[];
     EGroupSmem &sm = *reinterpret_cast<EGroupSmem *>(smem_raw);
     const uint32_t nb = nw << lg;
@@ -704,12 +702,12 @@ static int eager_run_grouped(sjbg_handle *h, const sjbg_tuple *dl, const sjbg_tu
     const EGroupWin *dW = reinterpret_cast<const EGroupWin *>(dev);
     const size_t s1 = sorted_tile_bytes(1u << lg), s2 = sizeof(EGroupSmem);
     allow_big_smem(egroup_sort_kernel, s1);
-    SJBG_CK(h, launch_next(h, "erun_tile_sort", egroup_sort_kernel,
+    SJBG_CK(h, launch(h, "erun_tile_sort", egroup_sort_kernel,
                       dim3(std::min<uint32_t>((uint32_t)tiles, 3u * (uint32_t)std::max(h->num_sms, 1))),
                       dim3(kSortedThreads), s1, dl, dr, dW, nw, (uint32_t)tiles, (uint32_t)B, (uint32_t)ts, (uint32_t)tpb, lg, words, wstride, rows));
     allow_big_smem(egroup_count_kernel, s2);
     const uint32_t grid = std::min<uint32_t>(nw << lg, 3u * (uint32_t)std::max(h->num_sms, 1));
-    SJBG_CK(h, launch_next(h, "erun_group_count", egroup_count_kernel, dim3(grid), dim3(kGroupThreads), s2,
+    SJBG_CK(h, launch(h, "erun_group_count", egroup_count_kernel, dim3(grid), dim3(kGroupThreads), s2,
                       (const uint64_t *)words, wstride, (const uint16_t *)rows, dW, nw, (uint32_t)tpb, lg, dCounts,
                       dWin, reinterpret_cast<uint32_t *>(&dWin[nw].info)));
     *done = true;

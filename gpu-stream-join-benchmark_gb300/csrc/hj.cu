@@ -145,7 +145,6 @@ part_hist_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict_
                  uint32_t *__restrict__ cnt, uint32_t B, const LearnedModel *__restrict__ models,
                  HeavyAcc *__restrict__ hacc, uint64_t *__restrict__ compL, uint64_t *__restrict__ compR,
                  uint32_t *__restrict__ ccnt, uint32_t *__restrict__ rows) {
-    kernel_chain();
     extern __shared__ __align__(16) uint32_t hist[];   // P counters, then (coarse output) the tile stage
     __shared__ HeavySet hs;
     // heavy-key sums as two 32-bit words: native 32-bit shared atomics, with
@@ -412,7 +411,6 @@ __global__ void part_work_kernel(const WinPlan *__restrict__ wins, uint32_t nwin
                                  const uint32_t *__restrict__ tileR, const uint32_t *__restrict__ itemL,
                                  const uint32_t *__restrict__ itemR, const LearnedModel *__restrict__ models,
                                  const uint32_t *__restrict__ ccnt, uint32_t *__restrict__ work) {
-    kernel_chain();
     const uint32_t a = warp_id();
     if (a >= kWorkArrays) return;   // whole warp
     const uint32_t kind = a >> 1, right = a & 1u;
@@ -469,7 +467,6 @@ part_light_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_
                   uint32_t B, const LearnedModel *__restrict__ models, uint64_t *__restrict__ compL,
                   uint64_t *__restrict__ compR, const uint32_t *__restrict__ ccnt, uint16_t *__restrict__ rows16,
                   uint32_t rstride) {
-    kernel_chain();
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ LearnedCore core;
     __shared__ uint32_t warp_tot[32];
@@ -527,7 +524,6 @@ part_light_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_
 __global__ void heavy_finish_kernel(const WinPlan *__restrict__ wins, uint32_t nwin,
                                     const LearnedModel *__restrict__ models, const HeavyAcc *__restrict__ hacc,
                                     WinAcc *__restrict__ acc) {
-    kernel_chain();
     const uint32_t w = blockIdx.x;
     const WinPlan wp = wins[w];
     if (wp.model == 0xFFFFFFFFu) return;
@@ -680,7 +676,6 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
                      const LearnedModel *__restrict__ models, JoinItem *__restrict__ items,
                      uint32_t *__restrict__ jn, uint32_t chunk, uint32_t cap, bool either,
                      const uint32_t *__restrict__ ccnt) {
-    kernel_chain();
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry_s;
     const uint32_t w = blockIdx.x;
@@ -975,7 +970,6 @@ part_scatter_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restri
                     uint32_t *__restrict__ cursor, uint32_t B, uint64_t *__restrict__ outL, uint64_t *__restrict__ outR,
                     const LearnedModel *__restrict__ models, const uint64_t *__restrict__ compL,
                     const uint64_t *__restrict__ compR, const uint32_t *__restrict__ ccnt) {
-    kernel_chain();
     // persistent CTAs over the tiles listed by the work prefixes workL / workR
     // (a compacted window's light tiles; a single-level window's tiles), each
     // tile's loads issued while the previous tile is written out.  Without models
@@ -1193,7 +1187,6 @@ part_fine_kernel(const WinPlan *__restrict__ wins, uint32_t nwin, const uint32_t
                  uint32_t B, uint64_t *__restrict__ outL, uint64_t *__restrict__ outR,
                  const LearnedModel *__restrict__ models, const uint64_t *__restrict__ srcL,
                  const uint64_t *__restrict__ srcR, const uint32_t *__restrict__ rows) {
-    kernel_chain();
     const uint32_t *pl = work + 2 * kWorkFine * (nwin + 1), *pr = pl + (nwin + 1);
     const uint32_t items = pl[nwin] + pr[nwin];
     for (uint32_t bi = blockIdx.x; bi < items; bi += gridDim.x) {
@@ -2169,7 +2162,6 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
                          const uint32_t *__restrict__ cnt, uint32_t B, WinAcc *__restrict__ acc, uint32_t cap,
                          uint32_t *queue, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn,
                          const RowsJoin rj) {
-    kernel_chain();
     if (kModels && rj.queue) rows_join(rj, wins, acc, cap);   // ends with a barrier
     const uint32_t nitems = items ? *jn : B;
     uint32_t clean = 0, turn = 0;
@@ -2349,7 +2341,6 @@ __global__ void __launch_bounds__(kJoinThreads)
 bucket_join_enum_kernel(const uint64_t *__restrict__ partL, const uint64_t *__restrict__ partR,
                         WinAcc *__restrict__ acc, const WinPlan *__restrict__ wins, sjbg_pair *__restrict__ pairs,
                         uint32_t table_bits, const JoinItem *__restrict__ items, const uint32_t *__restrict__ jn) {
-    kernel_chain();
     if (blockIdx.x < *jn) join_enum_bucket(items[blockIdx.x], partL, partR, acc, wins, pairs, table_bits);
 }
 
@@ -2640,26 +2631,26 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
 
     const uint32_t tiles = tileL[n] + tileR[n];
     auto scan = [&]() {
-        return launch_next(h, "part_scan", part_scan_win_kernel, dim3(n), dim3(1024), 0, (const WinPlan *)dPlan, dPbL, dPbR,
+        return launch(h, "part_scan", part_scan_win_kernel, dim3(n), dim3(1024), 0, (const WinPlan *)dPlan, dPbL, dPbR,
                       (const uint32_t *)dCnt, dStart, dCur, (uint32_t)B, dModels, dJlist, dJn, join_chunk,
                       enumerate ? 0x0FFFFFFFu : cap, !enumerate, (const uint32_t *)dCcnt);
     };
     if (!tiles && any_raw) SJBG_CK(h, scan());
     if (tiles) {
         const size_t histSmem = sizeof(uint32_t) * ((maxP + 1) / 2 * 2) + sizeof(uint64_t) * kTile;
-        SJBG_CK(h, launch_next(h, "part_hist", part_hist_kernel, dim3(hgL[n] + hgR[n]), dim3(kPartThreads), histSmem, dL,
+        SJBG_CK(h, launch(h, "part_hist", part_hist_kernel, dim3(hgL[n] + hgR[n]), dim3(kPartThreads), histSmem, dL,
                           dR, dPlan, n, dTileL, dTileR, dHgL, dHgR, dCnt, (uint32_t)B, dModels, dHeavy, dComp, dCompR,
                           dCcnt, dRows));
         if (learned)
-            SJBG_CK(h, launch_next(h, "heavy_finish", heavy_finish_kernel, dim3(n), dim3(256), 0, (const WinPlan *)dPlan, n,
+            SJBG_CK(h, launch(h, "heavy_finish", heavy_finish_kernel, dim3(n), dim3(256), 0, (const WinPlan *)dPlan, n,
                               dModels, (const HeavyAcc *)dHeavy, acc));
         // the tiles each later pass has work for (compacted windows: their light tiles only)
-        SJBG_CK(h, launch_next(h, "part_work", part_work_kernel, dim3(1), dim3(32 * kWorkArrays), 0, (const WinPlan *)dPlan, n, dTileL,
+        SJBG_CK(h, launch(h, "part_work", part_work_kernel, dim3(1), dim3(32 * kWorkArrays), 0, (const WinPlan *)dPlan, n, dTileL,
                           dTileR, dItL, dItR, dModels, (const uint32_t *)dCcnt, dWork));
         if (learned && !enumerate) {   // compacted windows exist only with heavy keys
             const size_t lightSmem = kTile * sizeof(uint64_t) + sizeof(uint32_t) * maxP;
             allow_big_smem(part_light_kernel, lightSmem);
-            SJBG_CK(h, launch_next(h, "part_light", part_light_kernel, dim3(std::min<uint32_t>(tiles, 2u * (uint32_t)h->num_sms)),
+            SJBG_CK(h, launch(h, "part_light", part_light_kernel, dim3(std::min<uint32_t>(tiles, 2u * (uint32_t)h->num_sms)),
                               dim3(kPartThreads), lightSmem, (const WinPlan *)dPlan, n, dTileL, dTileR,
                               (const uint32_t *)dWork, dCnt, (uint32_t)B, dModels, dComp, dCompR, (const uint32_t *)dCcnt,
                               dRows16, rstride));
@@ -2676,7 +2667,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             // with 6, 3,350 with 12, 3,324 with 24)
             const uint32_t sgrid = std::min<uint32_t>(tiles, 3u * (learned ? 4u : 8u) * (uint32_t)h->num_sms);
             const uint32_t *wS = dWork + 2 * kWorkScatter * (n + 1);
-            SJBG_CK(h, launch_next(h, "part_scatter", scatter, dim3(sgrid), dim3(kPartThreads), scatterSmem,
+            SJBG_CK(h, launch(h, "part_scatter", scatter, dim3(sgrid), dim3(kPartThreads), scatterSmem,
                               dL, dR, dPlan, n, dTileL, dTileR, wS, wS + (n + 1), dCur, (uint32_t)B, dPL, dPR,
                               dModels, (const uint64_t *)dComp, (const uint64_t *)dCompR, (const uint32_t *)dCcnt));
         }
@@ -2684,7 +2675,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
         if (any_two && itL[n] + itR[n]) {
             allow_big_smem(part_fine_kernel, kFineSmem);
             const uint32_t fgrid = std::min<uint32_t>(itL[n] + itR[n], 4u * 4u * (uint32_t)h->num_sms);
-            SJBG_CK(h, launch_next(h, "part_fine", part_fine_kernel, dim3(fgrid), dim3(kFineThreads), kFineSmem,
+            SJBG_CK(h, launch(h, "part_fine", part_fine_kernel, dim3(fgrid), dim3(kFineThreads), kFineSmem,
                               (const WinPlan *)dPlan, n, dTileL, dTileR, (const uint32_t *)dWork, dCur, (uint32_t)B,
                               dPL, dPR, dModels, (const uint64_t *)dComp, (const uint64_t *)dCompR,
                               (const uint32_t *)dRows));
@@ -2697,7 +2688,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
         const uint32_t bits = 13;   // 8192 slots for chunks of 4096
         const size_t smem = sizeof(uint32_t) * (2 * ((1u << bits) + 1) + 2 * kEnumChunk);
         allow_big_smem(bucket_join_enum_kernel, smem);
-        SJBG_CK(h, launch_next(h, "bucket_join_enum", bucket_join_enum_kernel, jgrid, dim3(kJoinThreads), smem,
+        SJBG_CK(h, launch(h, "bucket_join_enum", bucket_join_enum_kernel, jgrid, dim3(kJoinThreads), smem,
                           (const uint64_t *)dPL, (const uint64_t *)dPR, acc, (const WinPlan *)dPlan, dPairs, bits,
                           (const JoinItem *)dJlist, (const uint32_t *)dJn));
     } else {
@@ -2714,7 +2705,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             const uint32_t per_sm = std::max<uint32_t>(1, (uint32_t)((228u << 10) / (smem + 1024)));
             jgrid = dim3((uint32_t)std::min<uint64_t>(max_items, (uint64_t)h->num_sms * std::min<uint32_t>(per_sm, 2u)));
         }
-        SJBG_CK(h, launch_next(h, "bucket_join_count", join, jgrid, dim3(kJoinThreads), smem, dL, dR,
+        SJBG_CK(h, launch(h, "bucket_join_count", join, jgrid, dim3(kJoinThreads), smem, dL, dR,
                           (const WinPlan *)dPlan, dPL, dPR, (const uint32_t *)dStart, (const uint32_t *)dCnt,
                           (uint32_t)B, acc, cap, queue, (const JoinItem *)dJlist, (const uint32_t *)dJn, rj));
     }

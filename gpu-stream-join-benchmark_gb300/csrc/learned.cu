@@ -98,7 +98,6 @@ __device__ __forceinline__ uint32_t sample_key(const SampleWin &s, const sjbg_tu
 __global__ void __launch_bounds__(kSampleThreads)
 sample_minmax_kernel(const sjbg_tuple *L, const sjbg_tuple *R, const SampleWin *wins, SampleScratch *scr,
                      uint32_t *keys) {
-    kernel_chain();
     const uint32_t w = blockIdx.y;
     const SampleWin s = wins[w];
     uint32_t *kw = keys + s.key_off;
@@ -212,7 +211,6 @@ __device__ __forceinline__ void count_update(const SampleWin &s, uint32_t *hw, u
 __global__ void __launch_bounds__(kSampleThreads)
 sample_count_kernel(const uint32_t *keys, const SampleWin *wins, SampleScratch *scr, uint32_t *hist,
                     unsigned long long *table, uint32_t *lists) {
-    kernel_chain();
     __shared__ uint32_t skey[kCountSlots], scnt[kCountSlots + 1];
     __shared__ uint16_t used[kCountChunk + 1];   // slots taken by the chunk's distinct keys
     __shared__ uint32_t n_used;
@@ -316,7 +314,6 @@ __device__ __forceinline__ uint32_t candidate_cut(const SampleScratch &sc, uint3
 __global__ void __launch_bounds__(kSampleThreads)
 heavy_candidates_kernel(const SampleWin *wins, const unsigned long long *table, SampleScratch *scr,
                         const uint32_t *lists, unsigned long long *cand) {
-    kernel_chain();
     const uint32_t w = blockIdx.y;
     const SampleWin s = wins[w];
     const unsigned long long *tw = table + s.table_off;
@@ -382,7 +379,6 @@ __device__ __forceinline__ unsigned long long cta_excl_scan2(unsigned long long 
 __global__ void __launch_bounds__(1024)
 learned_fit_kernel(const SampleWin *wins, SampleScratch *scr, uint32_t *hist, unsigned long long *cand,
                    LearnedModel *models, uint32_t leaves, uint32_t max_heavy, float bound) {
-    kernel_chain();
     extern __shared__ uint32_t fit_smem[];         // kBins histogram counters (dynamic)
     __shared__ unsigned long long sc[kCandMax];
     __shared__ float lfit[kMaxLeaves][5];          // per leaf: n, mean x, mean y, slope, largest y
@@ -659,7 +655,6 @@ learned_fit_kernel(const SampleWin *wins, SampleScratch *scr, uint32_t *hist, un
 __global__ void __launch_bounds__(kSampleThreads)
 learned_check_kernel(const uint32_t *keys, const SampleWin *wins, const LearnedModel *models, uint32_t *pred,
                      uint32_t *prad) {
-    kernel_chain();
     __shared__ HeavySet hs;
     __shared__ LearnedCore core;
     const uint32_t w = blockIdx.y;
@@ -692,7 +687,6 @@ learned_check_kernel(const uint32_t *keys, const SampleWin *wins, const LearnedM
 __global__ void __launch_bounds__(1024)
 learned_overflow_kernel(const SampleWin *wins, LearnedModel *models, const uint32_t *pred, const uint32_t *prad,
                         float bound, WinPlan *plan) {
-    kernel_chain();
     __shared__ uint32_t mx_s, sum_s, rmx_s;
     const uint32_t w = blockIdx.x;
     LearnedModel &M = models[w];
@@ -814,7 +808,7 @@ int learned_prepare(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
 
     // one pass of four loads per thread: all of a window's sample in flight at once
     const uint32_t bs = std::max<uint32_t>(1, std::min<uint32_t>(256, (max_m + 1023) / 1024));
-    SJBG_CK(h, launch_next(h, "learned_sample", sample_minmax_kernel, dim3(bs, n), dim3(kSampleThreads), 0, dL, dR, dSw,
+    SJBG_CK(h, launch(h, "learned_sample", sample_minmax_kernel, dim3(bs, n), dim3(kSampleThreads), 0, dL, dR, dSw,
                       dScr, dKeys));
     // one chunk per CTA, unless the CTAs of all windows would take more than
     // one wave: then each CTA takes several chunks in turn (a second wave
@@ -827,18 +821,18 @@ int learned_prepare(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
     const uint32_t wave = (uint32_t)std::max(count_per_sm, 1) * (uint32_t)std::max(h->num_sms, 1);
     const uint32_t bn = std::max<uint32_t>(1, std::min<uint32_t>({256u, (max_m + kCountChunk - 1) / kCountChunk,
                                                                   std::max<uint32_t>(1, wave / std::max<uint32_t>(n, 1))}));
-    SJBG_CK(h, launch_next(h, "learned_count", sample_count_kernel, dim3(bn, n), dim3(kSampleThreads), 0,
+    SJBG_CK(h, launch(h, "learned_count", sample_count_kernel, dim3(bn, n), dim3(kSampleThreads), 0,
                       (const uint32_t *)dKeys, dSw, dScr, dHist, dTab, dLists));
     const uint32_t tx = std::max<uint32_t>(1, std::min<uint32_t>(16, (max_list + 4095) / 4096));
-    SJBG_CK(h, launch_next(h, "learned_heavy", heavy_candidates_kernel, dim3(tx, n), dim3(kSampleThreads), 0, dSw,
+    SJBG_CK(h, launch(h, "learned_heavy", heavy_candidates_kernel, dim3(tx, n), dim3(kSampleThreads), 0, dSw,
                       (const unsigned long long *)dTab, dScr, (const uint32_t *)dLists, dCand));
     allow_big_smem(learned_fit_kernel, sizeof(uint32_t) * kBins);
-    SJBG_CK(h, launch_next(h, "learned_fit", learned_fit_kernel, dim3(n), dim3(1024), sizeof(uint32_t) * kBins, dSw, dScr,
+    SJBG_CK(h, launch(h, "learned_fit", learned_fit_kernel, dim3(n), dim3(1024), sizeof(uint32_t) * kBins, dSw, dScr,
                       dHist, dCand, dM, leaves, allow_heavy ? kMaxHeavy : 0u, bound));
     const uint32_t bc = std::max<uint32_t>(1, std::min<uint32_t>(64, (max_m + 4095) / 4096));
-    SJBG_CK(h, launch_next(h, "learned_check", learned_check_kernel, dim3(bc, n), dim3(kSampleThreads), 0,
+    SJBG_CK(h, launch(h, "learned_check", learned_check_kernel, dim3(bc, n), dim3(kSampleThreads), 0,
                       (const uint32_t *)dKeys, dSw, (const LearnedModel *)dM, dPred, dPrad));
-    SJBG_CK(h, launch_next(h, "learned_overflow", learned_overflow_kernel, dim3(n), dim3(1024), 0, dSw, dM,
+    SJBG_CK(h, launch(h, "learned_overflow", learned_overflow_kernel, dim3(n), dim3(1024), 0, dSw, dM,
                       (const uint32_t *)dPred, (const uint32_t *)dPrad, bound, dPlan));
     *dModels = dM;
     return SJBG_OK;

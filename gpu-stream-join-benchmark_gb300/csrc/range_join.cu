@@ -84,7 +84,6 @@ __device__ __forceinline__ uint64_t range_samples(uint64_t n) {
 __global__ void __launch_bounds__(1024)
 range_sample_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
                     const RangeWin *__restrict__ wins, RangeMap *__restrict__ maps) {
-    kernel_chain();
     __shared__ uint32_t lo_s, hi_s;
     const RangeWin w = wins[blockIdx.x];
     if (threadIdx.x == 0) {
@@ -154,7 +153,6 @@ __global__ void __launch_bounds__(kSortedThreads, 3)
 range_tiles_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
                    const RangeWin *__restrict__ wins, uint32_t nwin, uint32_t tiles, const RangeMap *__restrict__ maps,
                    uint32_t P, uint64_t *__restrict__ words, uint16_t *__restrict__ rows) {
-    kernel_chain();
     sort_tiles(tiles, [&](uint32_t tile, SortedTile &t) {
         uint32_t lo = 0, hi = nwin;   // largest w with tile[0] <= tile (a window's left tiles, then its right ones)
         while (hi - lo > 1) {
@@ -321,7 +319,6 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                   const RangeWin *__restrict__ wins, uint32_t nwin, uint32_t nb, uint32_t P,
                   uint32_t *__restrict__ queue, WinAcc *__restrict__ acc, WinAcc *__restrict__ out,
                   sjbg_pair *__restrict__ pairs) {
-    kernel_chain();
     extern __shared__ __align__(16) uint8_t smem_raw[];
     RangeSmem &sm = *reinterpret_cast<RangeSmem *>(smem_raw);
     const uint32_t lane = lane_id(), wid = warp_id();
@@ -679,11 +676,11 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
     if (int rc = stage_copy_zero(h, dev, hst, upB, dAcc, accB + 16)) return rc;
     const RangeWin *dW = reinterpret_cast<const RangeWin *>(dev);
     if (!hash)
-        SJBG_CK(h, launch_next(h, "range_sample", range_sample_kernel, dim3(n), dim3(1024), 0, dL, dR, dW, maps));
+        SJBG_CK(h, launch(h, "range_sample", range_sample_kernel, dim3(n), dim3(1024), 0, dL, dR, dW, maps));
     const size_t s1 = sorted_tile_bytes(pmax), s2 = sizeof(RangeSmem);
     auto tiles_kernel = hash ? range_tiles_kernel<true> : range_tiles_kernel<false>;
     allow_big_smem(tiles_kernel, s1);
-    SJBG_CK(h, launch_next(h, "range_tiles", tiles_kernel,
+    SJBG_CK(h, launch(h, "range_tiles", tiles_kernel,
                       dim3((uint32_t)std::min<uint64_t>(tiles, 3u * (uint64_t)std::max(h->num_sms, 1))),
                       dim3(kSortedThreads), s1, dL, dR, dW, n, (uint32_t)tiles, (const RangeMap *)maps, pmax, words,
                       rows));
@@ -692,7 +689,7 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
                                    : (hash ? range_join_kernel<true, false, false> : range_join_kernel<false, false, false>);
     allow_big_smem(join_kernel, s2);
     const uint32_t grid = (uint32_t)std::min<uint64_t>(nb, slots);
-    SJBG_CK(h, launch_next(h, "range_join", join_kernel, dim3(grid), dim3(kRangeThreads), s2, (const uint64_t *)words,
+    SJBG_CK(h, launch(h, "range_join", join_kernel, dim3(grid), dim3(kRangeThreads), s2, (const uint64_t *)words,
                       (const uint16_t *)rows, dW, n, (uint32_t)nb, pmax, queue, acc, hAcc, dPairs));
     return SJBG_OK;
 }

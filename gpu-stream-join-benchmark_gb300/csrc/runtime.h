@@ -152,31 +152,6 @@ cudaError_t launch(sjbg_handle *h, const char *name, void (*kernel)(KArgs...), d
     return e;
 }
 
-// The same for a kernel that follows another one of this library on the
-// stream and begins with kernel_chain(): its launch overlaps the end of the
-// kernel before (a profiled call keeps the two apart).  1,048,576 learned tuples
-// per side at z = 1.25, 13 kernels: 184 us on the device with the usual
-// launches, 149 so, 140 without memsets between them.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_next(sjbg_handle *h, const char *name, void (*kernel)(KArgs...), dim3 grid, dim3 block,
-                        size_t smem, Args &&...args) {
-    if ((h->cfg.flags & SJBG_F_PROFILE) && !h->capturing)
-        return launch(h, name, kernel, grid, block, smem, std::forward<Args>(args)...);
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = h->stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-    h->launches++;
-    return e == cudaSuccess ? cudaGetLastError() : e;
-}
-
 // Raise a kernel's dynamic shared-memory limit on the current device to at
 // least `bytes`.  The limit is process-wide state of the kernel, shared by
 // every handle and thread, so it is only ever raised: a call asking for less
