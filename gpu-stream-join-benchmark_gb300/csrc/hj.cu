@@ -2499,9 +2499,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
         // (no tile of an unpartitioned window is counted or scattered)
         tileL[w + 1] = tileL[w] + (p.raw ? 0u : (uint32_t)((wh.n_left + kTile - 1) / kTile));
         tileR[w + 1] = tileR[w] + (p.raw ? 0u : (uint32_t)((wh.n_right + kTile - 1) / kTile));
-        // Off: a window of one call in some thirty counted a pair twice when a key
-        // found no slot within kMaxProbe (8 x 2^24, z = 1.5), cause not known yet.
-        p.rows = 0u;
+        p.rows = learned && !enumerate && lg > 0 ? 1u : 0u;
         if (p.rows) rows_lg = std::max(rows_lg, std::min(lg, kRowsMaxLog2));
         // fine-pass CTAs: coarse partitions x groups of kGroupTiles tiles
         const uint32_t nc = 1u << coarse_bits(lg);
