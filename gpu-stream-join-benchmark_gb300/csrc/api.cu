@@ -21,11 +21,7 @@ sjbg_handle::~sjbg_handle() {
     eager.reset();
     streaming.reset();
     ring.reset();
-    for (auto &g : graphs) {
-        if (g->exec) cudaGraphExecDestroy(g->exec);
-        for (auto &b : g->pinned)
-            if (b.p) cudaFreeHost(b.p);
-    }
+    sjbg::drop_graphs(this);
     for (auto &b : ws)
         if (b.p) cudaFree(b.p);
     for (auto &b : pinned)
@@ -69,12 +65,22 @@ cudaError_t raise_smem_limit(const void *kernel, size_t bytes) {
     return e;
 }
 
+void drop_graphs(sjbg_handle *h) {
+    for (auto &g : h->graphs) {
+        if (g->exec) cudaGraphExecDestroy(g->exec);
+        for (auto &b : g->pinned)
+            if (b.p) cudaFreeHost(b.p);
+    }
+    h->graphs.clear();
+}
+
 void *ws_get(sjbg_handle *h, WsSlot s, size_t bytes) {
     DevBuf &b = h->ws[s];
     bytes = std::max<size_t>(16, (bytes + 15) & ~(size_t)15);   // whole 16-byte words (stage_copy, zero_fill)
     if (b.bytes >= bytes) return b.p;
     if (b.p) {
         cudaStreamSynchronize(h->stream);   // a kernel may still use the old buffer
+        drop_graphs(h);                     // captured calls hold its address: they are captured again
         cudaFree(b.p);
         b.p = nullptr;
         b.bytes = 0;

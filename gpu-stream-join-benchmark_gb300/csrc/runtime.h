@@ -120,7 +120,11 @@ int zero_fill(sjbg_handle *h, void *dst, size_t bytes);
 // clear: one kernel boundary less on the call's critical path).
 int stage_copy_zero(sjbg_handle *h, void *dst, const void *src, size_t bytes, void *zdst, size_t zbytes);
 
-// Device buffer of at least `bytes` in slot s (contents not preserved on growth).
+// Forget the captured calls (SJBG_F_GRAPH): no replay may be in flight.
+void drop_graphs(sjbg_handle *h);
+// Device buffer of at least `bytes` in slot s (contents not preserved on
+// growth, which also drops the captured calls: their kernels hold the address
+// of the buffer that is freed).
 void *ws_get(sjbg_handle *h, WsSlot s, size_t bytes);
 // Pinned host staging buffer i of at least `bytes`.
 void *pinned_get(sjbg_handle *h, int i, size_t bytes);
