@@ -2485,8 +2485,9 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
         else lg = ceil_log2((build + target - 1) / target);
         lg = std::min(lg, kMaxBucketsLog2);
         if (wh.n_left == 0 || wh.n_right == 0) lg = 0;
-        // (a handle that names radix partitioning gets it for every window)
-        p.raw = h->cfg.partitioner == SJBG_PART_AUTO && !enumerate && lg == 0 && build < cap ? 1u : 0u;
+        // (a handle that names radix partitioning gets it for every window; the join
+        // of a learned call, which a tuned automatic handle may make, takes none)
+        p.raw = h->cfg.partitioner == SJBG_PART_AUTO && !learned && !enumerate && lg == 0 && build < cap ? 1u : 0u;
         p.log2_buckets = lg;
         p.bucket_base = (uint32_t)B;
         p.model = 0xFFFFFFFFu;
