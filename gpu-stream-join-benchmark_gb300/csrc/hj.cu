@@ -2470,6 +2470,9 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     std::vector<uint32_t> pbL(n + 1), pbR(n + 1);   // window bases in the partitioned arrays
     uint64_t B = 0, totL = 0, totR = 0;
     uint32_t maxP = 1, rows_lg = 0;   // rows_lg: log2 of the most buckets of a window joined from sorted tiles
+    // a learned window may be joined from sorted tiles; with a table near the shared
+    // memory's size (large bucket targets) there is no room for their lists
+    const bool rows_fit = learned && !enumerate && rows_join_bytes(cap) + 1024 <= h->max_smem_optin;
     bool any_two = false, any_one = false, any_raw = false;
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &wh = wins[w];
@@ -2500,7 +2503,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
         // (no tile of an unpartitioned window is counted or scattered)
         tileL[w + 1] = tileL[w] + (p.raw ? 0u : (uint32_t)((wh.n_left + kTile - 1) / kTile));
         tileR[w + 1] = tileR[w] + (p.raw ? 0u : (uint32_t)((wh.n_right + kTile - 1) / kTile));
-        p.rows = learned && !enumerate && lg > 0 ? 1u : 0u;
+        p.rows = rows_fit && lg > 0 ? 1u : 0u;
         if (p.rows) rows_lg = std::max(rows_lg, std::min(lg, kRowsMaxLog2));
         // fine-pass CTAs: coarse partitions x groups of kGroupTiles tiles
         const uint32_t nc = 1u << coarse_bits(lg);
