@@ -235,7 +235,7 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
         if (int rc = hj_raw_batch(h, dL, dR, wins, n, hAcc, &done)) return rc;
         if (done) return SJBG_OK;
     }
-    if (n && h->cfg.algorithm != SJBG_ALG_NLJ && range_join_pays(h, wins, n)) {
+    if (n && h->cfg.algorithm != SJBG_ALG_NLJ && range_join_pays(h, wins, n, enumerate)) {
         *part_used = h->cfg.algorithm == SJBG_ALG_HJ ? SJBG_PART_RADIX : SJBG_PART_NONE;
         return range_join_batch(h, dL, dR, wins, n, dPairs, hAcc, enumerate, h->cfg.algorithm == SJBG_ALG_HJ);
     }

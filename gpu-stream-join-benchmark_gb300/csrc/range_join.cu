@@ -702,13 +702,24 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
 // [0, 4W): 493 against 396; 64 of 2^17: 256 against 235).
 constexpr uint64_t kHashLeast = 1u << 17, kHashMost = 1u << 25;
 
-bool range_join_pays(const sjbg_handle *h, const WinHost *wins, uint32_t n) {
+// Many tiny windows whose other choice is an HBM table each: every window costs
+// the ranges two tiles of the word array and a turn of a CTA (counting, W keys
+// in [0, 4W): 16,000 windows of 16 tuples per side 1,200 us and 1 GB against
+// 620 us and 21 MB; 512 of 1,000 92 against 80; 512 of 3,000 114 against 128,
+// with keys in [0, W) 118 against 103).  Up to about a wave of CTAs the fixed
+// costs decide, and the ranges' are lower (pairs, 128 of 1,000: 67 against 86).
+constexpr uint64_t kHashMean = 6144;   // tuples of both sides per window
+
+bool range_join_pays(const sjbg_handle *h, const WinHost *wins, uint32_t n, bool enumerate) {
     if (h->regrouped || h->unwatched) return false;
     if (h->cfg.algorithm == SJBG_ALG_HJ) {
         if (h->cfg.partitioner != SJBG_PART_AUTO || h->tune.partitioner) return false;
         uint64_t tuples = 0;
         for (uint32_t w = 0; w < n; w++) tuples += wins[w].n_left + wins[w].n_right;
         if (tuples < kHashLeast || tuples > kHashMost) return false;
+        if (n > (enumerate ? 2u : 1u) * (uint32_t)std::max(h->num_sms, 1) && tuples < kHashMean * n &&
+            choose_partitioner(h, wins, n) == SJBG_PART_NONE)
+            return false;
     }
     return range_join_fits(wins, n);
 }

@@ -195,7 +195,7 @@ int smj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, c
 // range_join.cu: whether they suit the handle and the windows' sizes, and the
 // call, which leaves n + 1 entries in hAcc (pinned); the last one, the status
 // word, holds kErrRegroup when a range did not fit.
-bool range_join_pays(const sjbg_handle *h, const WinHost *wins, uint32_t n);
+bool range_join_pays(const sjbg_handle *h, const WinHost *wins, uint32_t n, bool enumerate);
 int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                      sjbg_pair *dPairs, WinAcc *hAcc, bool enumerate, bool hash);
 
