@@ -1346,20 +1346,29 @@ static inline size_t count_table_bytes(uint32_t cap) {
 // by 4,096: 82 us with the table, 24 us by places.
 constexpr uint32_t kPlaceCap = 8192;      // build tuples
 constexpr uint32_t kPlacesMax = 4096;
-// Crowded places (hot or repeated keys) leave the bucket to a direct or hash
-// table, which aggregate: one of more than kPlaceMost tuples, or more than one
-// thread in ten with one of more than kPlaceMany.
-constexpr uint32_t kPlaceMany = 16, kPlaceMost = 128;
+// Repeated keys leave the bucket to the hash table, which adds them up: by
+// places a probe pays for every match, with a hash of the match's value.  The
+// squares of the places' tuple numbers tell how many build tuples share a
+// tuple's key on average: distinct keys give about nB + nB^2 / places, a key of
+// k tuples k^2.  64 windows of 2^20, keys spread over 32 bits, 1 / 2 / 3 / 4 / 8
+// tuples per key (a tuple then shares its key with 2 / 3 / 4 / 5 / 9): by places
+// 1.93 / 2.12 / 2.28 / 2.42 / 2.90 ms, by the table 2.40 / 2.71 / 2.31 / 2.12 /
+// 1.64, so the line is at 3.5.  A few hot keys among distinct ones hold up
+// their probes' warps before the mean shows them: a place of more than
+// kPlaceMost decides too (1,024 windows of 30,000, z = 0.5: no limit 1.54 ms,
+// 64 1.30, 32 1.16, 20 1.10; 64 of 2^20, z = 0.4: 64 2.47, 32 2.52, 20 2.86; one of
+// 65,536, z = 0.6: 32 48 us, 24 58).
+constexpr uint32_t kPlaceRepeat2 = 7;   // twice the tuples that share a tuple's key
+constexpr uint32_t kPlaceMost = 32;
 constexpr size_t kPlaceBytes = sizeof(uint64_t) * kPlaceCap + sizeof(uint32_t) * (kPlacesMax + 1);
 
 // Adds the matches to count and prod; false, with nothing added and e still the
-// build run's first tile (build_head), when the run (nB <= kPlaceCap) is crowded.
+// build run's first tile (build_head), when the run's keys repeat (nB <= kPlaceCap).
 template <bool kRaw>
 __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
                                                   unsigned long long &count, unsigned long long &prod) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    __shared__ uint32_t warp_tot[kJoinThreads / 32];
-    __shared__ uint32_t most_s;
+    __shared__ uint32_t warp_tot[kJoinThreads / 32], warp_sq[kJoinThreads / 32];
     uint64_t *word = reinterpret_cast<uint64_t *>(smem_raw);
     uint32_t *at = reinterpret_cast<uint32_t *>(word + kPlaceCap);   // at[p]: first word of place p; at[0] = 0
     const uint32_t nB = ji.nB, nP = ji.nP, bside = jr.bside, pside = bside ^ 1u;
@@ -1374,7 +1383,6 @@ __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const Join
     };
     constexpr uint32_t tile = kJoinPer * kJoinThreads;
     for (uint32_t i = threadIdx.x; i <= places; i += kJoinThreads) at[i] = 0;
-    if (threadIdx.x == 0) most_s = 0;
     SJBG_BARRIER();
     for (uint32_t base = 0; base < nB; base += tile) {
         if (base) load(base);
@@ -1384,18 +1392,23 @@ __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const Join
     }
     SJBG_BARRIER();
     const uint32_t per = places / kJoinThreads, p0 = 1 + threadIdx.x * per;   // 1 to 8 places
-    uint32_t sum = 0, largest = 0;
+    uint32_t sum = 0, squares = 0, largest = 0;   // (squares of at most kPlaceCap tuples: 2^26)
     for (uint32_t q = 0; q < per; q++) {
         const uint32_t c = at[p0 + q];
         sum += c;
+        squares += c * c;
         largest = max(largest, c);
     }
     uint32_t tot;
     uint32_t run = warp_excl_scan(sum, &tot);
-    if (lane_id() == 31) warp_tot[warp_id()] = tot;
-    if (largest > kPlaceMost) most_s = 1;
-    const bool crowded = __syncthreads_count(largest > kPlaceMany) > kJoinThreads / 10 || most_s;
-    if (crowded) {
+    squares = __reduce_add_sync(0xFFFFFFFFu, squares);
+    if (lane_id() == 31) {
+        warp_tot[warp_id()] = tot;
+        warp_sq[warp_id()] = squares;
+    }
+    const bool most = __syncthreads_or(largest > kPlaceMost);
+    squares = __reduce_add_sync(0xFFFFFFFFu, lane_id() < kJoinThreads / 32 ? warp_sq[lane_id()] : 0u);
+    if (most || 2 * (squares - (nB * nB >> bits)) > kPlaceRepeat2 * nB) {   // (the same for the whole CTA)
         if (nB > tile) load(0);
         SJBG_BARRIER();   // the places are read before the next table's entries
         return false;
