@@ -94,6 +94,17 @@ __device__ __forceinline__ uint32_t add_carry(uint32_t hi, uint32_t a, uint32_t 
     return r;
 }
 
+// Adds f to a table slot's fr-sum as two 32-bit words (native shared atomics;
+// the low word's carry, seen in its returned old value, goes to the high word).
+// A 64-bit shared atomicAdd is a compare-and-swap loop, which hot keys turn
+// into a long serial chain.
+__device__ __forceinline__ void ct_add_sum(unsigned long long *slot, unsigned long long f) {
+    uint32_t *w2 = reinterpret_cast<uint32_t *>(slot);   // little-endian: low word first
+    const uint32_t flo = (uint32_t)f;
+    const uint32_t old = atomicAdd(&w2[0], flo);
+    atomicAdd(&w2[1], add_carry((uint32_t)(f >> 32), old, flo));
+}
+
 // Exclusive warp prefix sum of a 32-bit value.
 __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *total) {
     uint32_t x = v;

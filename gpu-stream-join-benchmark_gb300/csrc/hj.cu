@@ -1215,17 +1215,6 @@ __device__ __forceinline__ uint32_t ct_home(uint32_t key, uint32_t C) {
     return (uint32_t)(((uint64_t)slot_hash(key, 32) * C) >> 32);
 }
 
-// Adds f to a table slot's fr-sum as two 32-bit words (native shared atomics;
-// the low word's carry, seen in its returned old value, goes to the high word).
-// A 64-bit shared atomicAdd is a compare-and-swap loop, which hot keys turn
-// into a long serial chain.
-__device__ __forceinline__ void ct_add_sum(unsigned long long *slot, unsigned long long f) {
-    uint32_t *w2 = reinterpret_cast<uint32_t *>(slot);   // little-endian: low word first
-    const uint32_t flo = (uint32_t)f;
-    const uint32_t old = atomicAdd(&w2[0], flo);
-    atomicAdd(&w2[1], add_carry((uint32_t)(f >> 32), old, flo));
-}
-
 // Insert `c` tuples of `key` with hash sum `f`.  A key that finds neither itself
 // nor a free slot within max_probe slots is refused (false) and joined in a
 // later pass; lookups use the same bound, so a refused key is never half-found.

@@ -28,7 +28,8 @@
 // Hash joins of calls in the middle of the size range (hj.cu) take the same
 // steps with ranges of a multiplicative hash of the key: no sample, two
 // launches for the partitioning and the join, where counting, scanning and
-// scattering first need five.
+// scattering first need five; a range whose keys
+// repeat adds them up in a table.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -56,6 +57,18 @@ constexpr uint32_t kRangeSubs = 2048;           // subranges of a range
 // the range (13 us; at a limit of 16 for every subrange, one range in 300 of
 // keys with two duplicates each was sorted).
 constexpr uint32_t kRangeCrowd = 16, kRangeCrowdMost = 128;
+// By the hash, words of one subrange are mostly words of one key: when keys
+// repeat, counting joins add up the left words of each key in a table of
+// kRangeSubs slots in the words' space.  The rule is that of the bucket joins'
+// places (hj.cu): more than 3.5 left words that share a word's key on average,
+// by the squares of the subranges' numbers, or a subrange of more than
+// kRangeMost; and few enough keys that the table is not full, by the subranges
+// in use (kRangeUsed of 2,048: some 1,580 keys).  8 windows of 2^20 with 1 / 2 /
+// 4 / 8 / 16 / 64 tuples per key: lists and sort 238 / 253 / 281 / 335 / 449 /
+// 627 us, with the table 240 / 255 / 249 / 230 / 221 / 214; a kRangeMost of 16
+// takes ranges of two tuples per key too (289), 64 measures the same as 32.
+constexpr uint32_t kRangeRepeat2 = 7, kRangeMost = 32, kRangeUsed = 1100;
+constexpr uint32_t kRangeProbe = 64;   // slots of the table looked at for a key
 
 struct RangeWin {
     uint64_t off[2], n[2];   // left, right
@@ -174,10 +187,16 @@ range_tiles_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restric
     });
 }
 
+struct RangeTable {
+    unsigned long long sum[kRangeSubs];   // of fr
+    uint32_t key[kRangeSubs], cnt[kRangeSubs];
+};
+
 struct RangeSmem {
     union {
         uint64_t word[kRangeCap];                   // left words by subrange
         uint32_t buf[2][2][kRangeCap];              // sorting: keys and vals, before and after a pass; then F in the free pair
+        RangeTable tab;                             // repeated keys
     };
     union {
         uint32_t sub[kRangeSubs + 1];               // first left word of each subrange, and their number
@@ -186,10 +205,37 @@ struct RangeSmem {
     uint32_t loc[kRangeDigits + 1];                 // first word of each digit of the last pass, and n
     uint16_t off[kRangeTilesMax], pre[kRangeTilesMax];   // per tile (left side's first): the run, the words before it
     uint16_t owner[kRangeWords];                    // tile of the range's i-th word
-    uint32_t warp_tot[32];
+    uint32_t warp_tot[32], warp_used[32], warp_sq[32];
     unsigned long long wsum[32], base;
-    uint32_t lo, hi, crowd, n_left, next, stop;
+    uint32_t lo, hi, crowd, n_left, next, stop, refused;
 };
+static_assert(sizeof(RangeTable) <= sizeof(uint64_t) * kRangeCap, "the table takes the words' space");
+
+// The slot of the table that holds the key or is the first free one after its
+// home; kRangeSubs: neither among kRangeProbe slots.
+__device__ __forceinline__ uint32_t range_slot(const RangeTable &t, uint32_t key, uint32_t home) {
+    for (uint32_t p = 0; p < kRangeProbe; p++) {
+        const uint32_t s = (home + p) & (kRangeSubs - 1), k = *(volatile const uint32_t *)&t.key[s];
+        if (k == key || k == kEmptyKey) return s;
+    }
+    return kRangeSubs;
+}
+
+// Adds a left word to the table; false: no slot for its key (or the key is the
+// mark of free slots).
+__device__ __forceinline__ bool range_add(RangeTable &t, uint64_t word, uint32_t home) {
+    const uint32_t key = (uint32_t)word;
+    if (key == kEmptyKey) return false;
+    for (;;) {   // (a slot lost to another key is taken for good: at most kRangeProbe times)
+        const uint32_t s = range_slot(t, key, home);
+        if (s == kRangeSubs) return false;
+        const uint32_t was = atomicCAS(&t.key[s], kEmptyKey, key);
+        if (was != kEmptyKey && was != key) continue;
+        atomicAdd(&t.cnt[s], 1u);
+        ct_add_sum(&t.sum[s], sjbg_fr((uint32_t)(word >> 32)));
+        return true;
+    }
+}
 
 // One stable pass over the n left words in shared memory, on kRangeDigit bits
 // of key - lo from `shift`.  Warp-private counters; a lane's digit peers come
@@ -425,22 +471,44 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
             for (uint32_t k = 0; k < kItems; k++)
                 if (threadIdx.x + k * kRangeThreads < nl) rank[k] = atomicAdd(&sm.sub[sub_of((uint32_t)e[k])], 1u);
             SJBG_BARRIER();
-            bool crowded = false, most = false;
+            constexpr bool kTable = kHash && !kEnum;
+            bool crowded = false, most = false, repeats = false;
             {
                 constexpr uint32_t kPer = kRangeSubs / kRangeThreads;
-                uint32_t c[kPer], csum = 0;
+                uint32_t c[kPer], csum = 0, used = 0, squares = 0, largest = 0;   // (squares of at most kRangeCap words: 2^24)
 #pragma unroll
                 for (uint32_t q = 0; q < kPer; q++) {
                     c[q] = sm.sub[threadIdx.x * kPer + q];
                     csum += c[q];
-                    crowded |= c[q] > kRangeCrowd;
-                    most |= c[q] > kRangeCrowdMost;
+                    used += c[q] != 0;
+                    squares += c[q] * c[q];
+                    largest = max(largest, c[q]);
                 }
                 uint32_t ctot;
                 uint32_t crun = warp_excl_scan(csum, &ctot);
-                if (lane == 31) sm.warp_tot[wid] = ctot;
-                if (most) sm.crowd = 1;
-                crowded = __syncthreads_count(crowded) > kRangeThreads / 10 || sm.crowd;
+                if (kTable) {
+                    used = __reduce_add_sync(0xFFFFFFFFu, used);
+                    squares = __reduce_add_sync(0xFFFFFFFFu, squares);
+                }
+                if (lane == 31) {
+                    sm.warp_tot[wid] = ctot;
+                    if (kTable) {
+                        sm.warp_used[wid] = used;
+                        sm.warp_sq[wid] = squares;
+                    }
+                }
+                if (largest > kRangeCrowdMost) sm.crowd = 1;
+                if (kTable) {
+                    if (threadIdx.x == 0) sm.refused = 0;
+                    most = __syncthreads_or(largest > kRangeMost);
+                }
+                crowded = __syncthreads_count(largest > kRangeCrowd) > kRangeThreads / 10 || sm.crowd;
+                if (kTable) {
+                    used = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_used[lane] : 0u);
+                    squares = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_sq[lane] : 0u);
+                    repeats = used <= kRangeUsed &&
+                              (most || 2 * (squares - nl * nl / kRangeSubs) > kRangeRepeat2 * nl);
+                }
                 crun += __reduce_add_sync(0xFFFFFFFFu, lane < wid ? sm.warp_tot[lane] : 0u);
 #pragma unroll
                 for (uint32_t q = 0; q < kPer; q++) {
@@ -492,7 +560,43 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     }
                 }
             };
-            if (!crowded) {
+            bool done = false;   // (the same for the whole CTA)
+            if constexpr (kTable) {
+                if (repeats) {   // a table of the keys' numbers and sums
+                    for (uint32_t i = threadIdx.x; i < kRangeSubs; i += kRangeThreads) {
+                        sm.tab.key[i] = kEmptyKey;
+                        sm.tab.cnt[i] = 0;
+                        sm.tab.sum[i] = 0;
+                    }
+                    SJBG_BARRIER();
+#pragma unroll
+                    for (uint32_t k = 0; k < kItems; k++) {
+                        if (threadIdx.x + k * kRangeThreads < nl && !range_add(sm.tab, e[k], sub_of((uint32_t)e[k])))
+                            sm.refused = 1;
+                        __syncwarp();
+                    }
+                    SJBG_BARRIER();
+                    done = sm.refused == 0;
+                    for (uint32_t i = nl + threadIdx.x; done && i < n; i += 4 * kRangeThreads) {
+                        uint64_t x[4];
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++)
+                            x[q] = i + q * kRangeThreads < n ? word(i + q * kRangeThreads) : 0ull;
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++) {
+                            const uint32_t key = (uint32_t)x[q];
+                            if (i + q * kRangeThreads >= n || key < lo || key > hi) continue;
+                            const uint32_t s = range_slot(sm.tab, key, sub_of(key));
+                            if (s == kRangeSubs || sm.tab.key[s] != key) continue;
+                            count += sm.tab.cnt[s];
+                            prod += sm.tab.sum[s] * sjbg_gs((uint32_t)(x[q] >> 32));
+                        }
+                    }
+                }
+            }
+            if (done) {
+                // (by the table)
+            } else if (!crowded) {
                 SJBG_BARRIER();
 #pragma unroll
                 for (uint32_t k = 0; k < kItems; k++)
