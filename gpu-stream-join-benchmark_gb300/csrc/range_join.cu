@@ -472,6 +472,10 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                 if (threadIdx.x + k * kRangeThreads < nl) rank[k] = atomicAdd(&sm.sub[sub_of((uint32_t)e[k])], 1u);
             SJBG_BARRIER();
             constexpr bool kTable = kHash && !kEnum;
+            // by the hash a subrange's words are mostly one key's: the xor checksum visits all
+            // of them either way (8 windows of 2^20, 16 tuples per key: 670 us, sorted 701;
+            // written, the pairs of a sorted range take 1,013, else 1,069)
+            constexpr bool kVisit = kHash && kEnum && !kPairs;
             bool crowded = false, most = false, repeats = false;
             {
                 constexpr uint32_t kPer = kRangeSubs / kRangeThreads;
@@ -502,7 +506,7 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     if (threadIdx.x == 0) sm.refused = 0;
                     most = __syncthreads_or(largest > kRangeMost);
                 }
-                crowded = __syncthreads_count(largest > kRangeCrowd) > kRangeThreads / 10 || sm.crowd;
+                crowded = __syncthreads_count(largest > (kVisit ? kRangeCrowdMost : kRangeCrowd)) > kRangeThreads / 10 || sm.crowd;
                 if (kTable) {
                     used = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_used[lane] : 0u);
                     squares = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_sq[lane] : 0u);
@@ -518,22 +522,27 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                 if (threadIdx.x == kRangeThreads - 1) sm.sub[kRangeSubs] = crun;
             }
             unsigned long long count = 0, prod = 0, xr = 0;
-            // the right words one by one: matches(x, use) calls use(val) for the
-            // left words with x's key
-            auto enumerate = [&](auto matches) {
+            // the right words one by one: first(x, j, end) gives the left words [j, end)
+            // among which x's partners are, partner(x, j, lv) whether j is one and its val
+            auto enumerate = [&](auto first, auto partner) {
                 for (uint32_t i = nl + threadIdx.x; i < n; i += kRangeThreads) {
                     const uint64_t x = word(i);
                     const uint32_t rv = (uint32_t)(x >> 32);
+                    uint32_t at, end, lv;
                     unsigned long long f = 0;
-                    matches(x, [&](uint32_t lv) {
+                    for (first(x, at, end); at < end; at++) {
+                        if (!partner(x, at, lv)) continue;
                         count++;
                         f += sjbg_fr(lv);
                         xr ^= sjbg_pair_hash(lv, rv);
-                    });
+                    }
                     prod += f * sjbg_gs(rv);
                 }
                 if constexpr (kPairs) {
-                    // one reservation for the range's pairs; each warp writes its own in turn
+                    // one reservation for the range's pairs; each warp writes its own in turn, a
+                    // pair of every lane that has one at a time, so that they lie side by side
+                    // (8 windows of 2^20 with 1 / 4 / 16 tuples per key: 385 / 550 / 1,013 us, a
+                    // lane's one after another 401 / 569 / 1,906)
                     uint32_t wt = (uint32_t)warp_sum_u64(count);
                     if (lane == 0) sm.warp_tot[wid] = wt;
                     SJBG_BARRIER();
@@ -542,21 +551,20 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     if (threadIdx.x == 0 && total)
                         sm.base = atomicAdd(&acc[wlo].npairs, (unsigned long long)total);
                     SJBG_BARRIER();
-                    unsigned long long at = sm.base + __reduce_add_sync(0xFFFFFFFFu, lane < wid ? c : 0u);
+                    unsigned long long pos = sm.base + __reduce_add_sync(0xFFFFFFFFu, lane < wid ? c : 0u);
                     sjbg_pair *out_pairs = pairs + w.pairs_off;
                     for (uint32_t i0 = nl; total && i0 < n; i0 += kRangeThreads) {   // (whole warps step)
                         const uint32_t i = i0 + threadIdx.x;
                         const uint64_t x = i < n ? word(i) : 0ull;
-                        uint32_t mine = 0;
-                        if (i < n) matches(x, [&](uint32_t) { mine++; });
-                        uint32_t tot;
-                        unsigned long long pos = at + warp_excl_scan(mine, &tot);
-                        if (mine)
-                            matches(x, [&](uint32_t lv) {
-                                if (pos < w.pairs_cap) out_pairs[pos] = sjbg_pair{lv, (uint32_t)(x >> 32)};
-                                pos++;
-                            });
-                        at += tot;
+                        uint32_t at = 0, end = 0, lv = 0;
+                        if (i < n) first(x, at, end);
+                        for (; __any_sync(0xFFFFFFFFu, at < end); at++) {
+                            const bool has = at < end && partner(x, at, lv);
+                            const unsigned m = __ballot_sync(0xFFFFFFFFu, has);
+                            const unsigned long long mine = pos + __popc(m & ((1u << lane) - 1u));
+                            if (has && mine < w.pairs_cap) out_pairs[mine] = sjbg_pair{lv, (uint32_t)(x >> 32)};
+                            pos += __popc(m);
+                        }
                     }
                 }
             };
@@ -603,15 +611,20 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     if (threadIdx.x + k * kRangeThreads < nl) sm.word[sm.sub[sub_of((uint32_t)e[k])] + rank[k]] = e[k];
                 SJBG_BARRIER();
                 if constexpr (kEnum) {
-                    enumerate([&](uint64_t x, auto use) {
-                        const uint32_t key = (uint32_t)x;
-                        if (key < lo || key > hi) return;
-                        const uint32_t b = sub_of(key), end = sm.sub[b + 1];
-                        for (uint32_t j = sm.sub[b]; j < end; j++) {
+                    enumerate(
+                        [&](uint64_t x, uint32_t &j, uint32_t &end) {
+                            const uint32_t key = (uint32_t)x;
+                            j = end = 0;
+                            if (key < lo || key > hi) return;
+                            const uint32_t b = sub_of(key);
+                            j = sm.sub[b];
+                            end = sm.sub[b + 1];
+                        },
+                        [&](uint64_t x, uint32_t j, uint32_t &lv) {
                             const uint64_t y = sm.word[j];
-                            if ((uint32_t)y == key) use((uint32_t)(y >> 32));
-                        }
-                    });
+                            lv = (uint32_t)(y >> 32);
+                            return (uint32_t)y == (uint32_t)x;
+                        });
                 } else {
                     for (uint32_t i = nl + threadIdx.x; i < n; i += 4 * kRangeThreads) {
 #pragma unroll
@@ -678,11 +691,11 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     return true;
                 };
                 if constexpr (kEnum) {
-                    enumerate([&](uint64_t x, auto use) {
-                        uint32_t l, h;
-                        if (group((uint32_t)x, l, h))
-                            for (; l < h; l++) use(vals[l]);
-                    });
+                    enumerate([&](uint64_t x, uint32_t &l, uint32_t &h) { if (!group((uint32_t)x, l, h)) l = h = 0; },
+                              [&](uint64_t, uint32_t l, uint32_t &lv) {
+                                  lv = vals[l];
+                                  return true;
+                              });
                 } else {
                     unsigned long long *F = reinterpret_cast<unsigned long long *>(&sm.buf[at ^ 1][0][0]);
                     const unsigned long long all = range_prefix(sm, vals, nl, F);   // ends with a barrier

@@ -4,7 +4,7 @@ and the mark of its free slots among the keys."""
 import numpy as np
 import pytest
 
-from helpers import make_tuples
+from helpers import make_tuples, sorted_pairs
 
 pytestmark = pytest.mark.gpu
 
@@ -39,4 +39,37 @@ def test_repeated_keys_by_ranges(lib, oracle, per, hot, mark):
             got = j.lazy_execute_batch(dl, dr, descs, mem=lib.MEM_DEVICE)
             for d, g, w in zip(descs, got, want):
                 assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
+        assert "range_join" in j.kernel_stats()
+
+
+@pytest.mark.parametrize("per", [1, 3, 12, 25])
+def test_pairs_of_repeated_keys_by_hash_ranges(lib, oracle, per):
+    """Lists and (12 and more tuples per key) sorted ranges; the second window's pairs are cut short."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(43)
+    sizes = [(70_000, 60_001), (9_000, 20_000), (5, 1000)]
+    lefts = [keys_of(per, 0, False, nl, rng) for nl, _ in sizes]
+    rights = [keys_of(per * max(1.0, nr / nl), 0, False, nr, rng) for nl, nr in sizes]
+    spans, lo, ro = [], 0, 0
+    for nl, nr in sizes:
+        spans.append((lo, nl, ro, nr))
+        lo, ro = lo + nl, ro + nr
+    left, right = make_tuples(np.concatenate(lefts)), make_tuples(np.concatenate(rights))
+    want = [oracle.join(left[a:a + b], right[c:c + d], pairs_capacity=1 << 22) for a, b, c, d in spans]
+    caps = [w["count"] for w in want]
+    caps[1] //= 2
+    offs = np.concatenate([[0], np.cumsum(caps)])
+    descs = [s + (int(o), int(c)) for s, o, c in zip(spans, offs, caps)]
+    l, r, p = [torch.from_numpy(x.view(np.uint8)).cuda() for x in (left, right, np.zeros(int(offs[-1]), lib.PAIR_DTYPE))]
+    with lib.Joiner(lib.ALG_HJ, lib.LAZY, lib.RESULT_ATOMIC, flags=lib.F_PROFILE, max_tuples_per_window=1 << 17) as j:
+        for _ in range(2):
+            got = j.lazy_execute_batch(l, r, descs, mem=lib.MEM_DEVICE, pairs=p)
+            out = p.cpu().numpy().view(lib.PAIR_DTYPE)
+            for i, (g, w) in enumerate(zip(got, want)):
+                assert (g["count"], g["xor"], g["prod"], g["n_pairs"]) == (w["count"], w["xor"], w["prod"], caps[i]), i
+                have = sorted_pairs(out[offs[i]:offs[i] + caps[i]])
+                if i != 1:
+                    assert np.array_equal(have, sorted_pairs(w["pairs"])), i
+                else:
+                    assert len(np.unique(have)) == len(have) and np.isin(have, sorted_pairs(w["pairs"])).all()
         assert "range_join" in j.kernel_stats()
