@@ -295,12 +295,14 @@ static void fill_result(const sjbg_handle *h, const WinAcc &a, const WinHost &w,
     (void)h;
 }
 
-// Batched lazy call on device inputs through a cached CUDA graph: the first
-// call with a given signature runs normally (sizing every workspace), then is
-// captured with private pinned staging buffers; later identical calls replay it.
+// One pass of a batched lazy call on device inputs through a cached CUDA graph,
+// enqueued: the first with a given signature runs normally (sizing every
+// workspace) and is then captured with private pinned staging buffers; later
+// identical ones replay it.  done is recorded behind the pass, whose results
+// and status word will be in *out.
 constexpr size_t kGraphKeyRegrouped = 11;   // regrouped's place in a graph's key
-static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
-                      sjbg_pair *dPairs, bool enumerate, sjbg_window_result *out) {
+static int lazy_graph_pass(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                           sjbg_pair *dPairs, cudaEvent_t done, WinAcc **out, uint32_t *part_used) {
     std::vector<uint64_t> key = {h->cfg.algorithm, h->cfg.partitioner, h->tune.partitioner, h->cfg.flags, h->cfg.result_mode,
                                  (uint64_t)(uintptr_t)dL, (uint64_t)(uintptr_t)dR, (uint64_t)(uintptr_t)dPairs, n,
                                  h->tune.bucket_target, (uint64_t)h->tune.persistent_join, (uint64_t)h->regrouped,
@@ -309,84 +311,87 @@ static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR
         const WinHost &x = wins[w];
         key.insert(key.end(), {x.left_off, x.n_left, x.right_off, x.n_right, x.pairs_off, x.pairs_cap});
     }
-    sjbg_handle::GraphEntry *entry = nullptr;
-    for (auto &g : h->graphs)
-        if (g->key == key) entry = g.get();
+    for (auto &g : h->graphs) {
+        if (g->key != key) continue;
+        SJBG_CK(h, cudaGraphLaunch(g->exec, h->stream));
+        SJBG_CK(h, cudaEventRecord(done, h->stream));
+        h->launches += g->kernels;   // the replay runs every captured kernel again
+        *out = static_cast<WinAcc *>(g->pinned[3].p);
+        *part_used = g->part_used;
+        return SJBG_OK;
+    }
+    WinAcc *hAcc = static_cast<WinAcc *>(pinned_get(h, 3, sizeof(WinAcc) * (n + 1)));
+    if (!hAcc) return fail(h, SJBG_E_NOMEM, "result staging");
+    *out = hAcc;
+    if (int rc = run_lazy_watched(h, dL, dR, wins, n, dPairs, hAcc, part_used)) return rc;   // warm-up: sizes every buffer
+    SJBG_CK(h, cudaEventRecord(done, h->stream));
+    SJBG_CK(h, cudaStreamSynchronize(h->stream));
+    profile_collect(h);
+    key[kGraphKeyRegrouped] = (uint64_t)h->regrouped;   // (it may have been met just now)
+    auto e = std::make_unique<sjbg_handle::GraphEntry>();
+    e->key = key;
+    e->part_used = *part_used;
+    for (int i = 0; i < 6; i++) {   // private copies of the staging buffers the capture will reference
+        if (!h->pinned[i].bytes) continue;
+        if (cudaMallocHost(&e->pinned[i].p, h->pinned[i].bytes) != cudaSuccess) {
+            cudaGetLastError();
+            for (auto &b : e->pinned)
+                if (b.p) cudaFreeHost(b.p);
+            return fail(h, SJBG_E_NOMEM, "graph staging");
+        }
+        e->pinned[i].bytes = h->pinned[i].bytes;
+    }
+    for (int i = 0; i < 6; i++) std::swap(h->pinned[i], e->pinned[i]);
+    h->capturing = true;
+    const uint64_t launches_before = h->launches;
+    cudaGraph_t graph = nullptr;
+    cudaError_t ce = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed);
+    uint32_t pu2 = 0;
+    int rc2 = ce == cudaSuccess ? run_lazy_device(h, dL, dR, wins, n, dPairs,
+                                                  static_cast<WinAcc *>(h->pinned[3].p), &pu2)
+                                : SJBG_E_CUDA;
+    cudaError_t ce2 = cudaStreamEndCapture(h->stream, &graph);
+    h->capturing = false;
+    e->kernels = h->launches - launches_before;
+    h->launches = launches_before;   // capture runs nothing
+    for (int i = 0; i < 6; i++) std::swap(h->pinned[i], e->pinned[i]);
+    if (rc2 == SJBG_OK && ce == cudaSuccess && ce2 == cudaSuccess && graph) {
+        if (cudaGraphInstantiate(&e->exec, graph, 0) != cudaSuccess) e->exec = nullptr;
+    }
+    if (graph) cudaGraphDestroy(graph);
+    cudaGetLastError();
+    if (e->exec) {
+        if (h->graphs.size() >= 8) {
+            auto &old = h->graphs.front();
+            cudaGraphExecDestroy(old->exec);
+            for (auto &b : old->pinned)
+                if (b.p) cudaFreeHost(b.p);
+            h->graphs.erase(h->graphs.begin());
+        }
+        h->graphs.push_back(std::move(e));
+    } else {
+        for (auto &b : e->pinned)
+            if (b.p) cudaFreeHost(b.p);
+    }
+    return SJBG_OK;
+}
+
+static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+                      sjbg_pair *dPairs, bool enumerate, sjbg_window_result *out) {
     cudaEvent_t e0 = event_get(h), e1 = event_get(h);
     WinAcc *hAcc = nullptr;
     uint32_t part_used = SJBG_PART_NONE;
-    if (entry) {
-        SJBG_CK(h, cudaEventRecord(e0, h->stream));
-        SJBG_CK(h, cudaGraphLaunch(entry->exec, h->stream));
-        SJBG_CK(h, cudaEventRecord(e1, h->stream));
-        h->launches += entry->kernels;   // the replay runs every captured kernel again
-        hAcc = static_cast<WinAcc *>(entry->pinned[3].p);
-        part_used = entry->part_used;
-    } else {
-        hAcc = static_cast<WinAcc *>(pinned_get(h, 3, sizeof(WinAcc) * (n + 1)));
-        if (!hAcc) return fail(h, SJBG_E_NOMEM, "result staging");
-        SJBG_CK(h, cudaEventRecord(e0, h->stream));
-        int rc = run_lazy_watched(h, dL, dR, wins, n, dPairs, hAcc, &part_used);   // warm-up: sizes every buffer
-        if (rc) return rc;
-        SJBG_CK(h, cudaEventRecord(e1, h->stream));
+    SJBG_CK(h, cudaEventRecord(e0, h->stream));
+    for (;;) {
+        if (int rc = lazy_graph_pass(h, dL, dR, wins, n, dPairs, e1, &hAcc, &part_used)) return rc;
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
-        profile_collect(h);
-        key[kGraphKeyRegrouped] = (uint64_t)h->regrouped;   // (it may have been met just now)
-        auto e = std::make_unique<sjbg_handle::GraphEntry>();
-        e->key = key;
-        e->part_used = part_used;
-        for (int i = 0; i < 6; i++) {   // private copies of the staging buffers the capture will reference
-            if (!h->pinned[i].bytes) continue;
-            if (cudaMallocHost(&e->pinned[i].p, h->pinned[i].bytes) != cudaSuccess) {
-                cudaGetLastError();
-                for (auto &b : e->pinned)
-                    if (b.p) cudaFreeHost(b.p);
-                return fail(h, SJBG_E_NOMEM, "graph staging");
-            }
-            e->pinned[i].bytes = h->pinned[i].bytes;
-        }
-        for (int i = 0; i < 6; i++) std::swap(h->pinned[i], e->pinned[i]);
-        h->capturing = true;
-        const uint64_t launches_before = h->launches;
-        cudaGraph_t graph = nullptr;
-        cudaError_t ce = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed);
-        uint32_t pu2 = 0;
-        int rc2 = ce == cudaSuccess ? run_lazy_device(h, dL, dR, wins, n, dPairs,
-                                                      static_cast<WinAcc *>(h->pinned[3].p), &pu2)
-                                    : SJBG_E_CUDA;
-        cudaError_t ce2 = cudaStreamEndCapture(h->stream, &graph);
-        h->capturing = false;
-        e->kernels = h->launches - launches_before;
-        h->launches = launches_before;   // capture runs nothing
-        for (int i = 0; i < 6; i++) std::swap(h->pinned[i], e->pinned[i]);
-        if (rc2 == SJBG_OK && ce == cudaSuccess && ce2 == cudaSuccess && graph) {
-            if (cudaGraphInstantiate(&e->exec, graph, 0) != cudaSuccess) e->exec = nullptr;
-        }
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
-        if (e->exec) {
-            if (h->graphs.size() >= 8) {
-                auto &old = h->graphs.front();
-                cudaGraphExecDestroy(old->exec);
-                for (auto &b : old->pinned)
-                    if (b.p) cudaFreeHost(b.p);
-                h->graphs.erase(h->graphs.begin());
-            }
-            h->graphs.push_back(std::move(e));
-        } else {
-            for (auto &b : e->pinned)
-                if (b.p) cudaFreeHost(b.p);
-        }
+        if (!(hAcc[n].info & kErrRegroup) || h->regrouped) break;
+        h->regrouped = true;   // a replay met keys that do not fit: the general path's graph
     }
-    SJBG_CK(h, cudaStreamSynchronize(h->stream));
-    float ms = 0.f;
+    float ms = 0.f;   // (of both passes, when it took two)
     cudaEventElapsedTime(&ms, e0, e1);
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
-    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // a replay met keys that do not fit: the general path's graph
-        h->regrouped = true;
-        return lazy_graph(h, dL, dR, wins, n, dPairs, enumerate, out);
-    }
     if (int se = device_status_error(h, hAcc[n].info)) return se;
     for (uint32_t w = 0; w < n; w++) fill_result(h, hAcc[w], wins[w], enumerate, dPairs != nullptr, part_used, ms, &out[w]);
     return SJBG_OK;
@@ -556,34 +561,32 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     WinAcc *hAcc = static_cast<WinAcc *>(pinned_get(h, 3, sizeof(WinAcc) * (n + 1)));
     if (!hAcc) return fail(h, SJBG_E_NOMEM, "result staging");
     uint32_t part_used = SJBG_PART_NONE;
-    int rc = run_lazy_device(h, dL, dR, wins, n, dP, hAcc, &part_used);
-    if (rc) return rc;
     if (mem == SJBG_MEM_HOST && want) {
-        // copy back each window's written pairs
-        SJBG_CK(h, cudaStreamSynchronize(h->stream));
-        if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (the general path, before anything is copied back)
-            h->regrouped = true;
-            if (int rc2 = run_lazy_watched(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc2;
-        }
+        if (int rc = run_lazy_watched(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
         if (int se = device_status_error(h, hAcc[n].info)) return se;
+        // copy back each window's written pairs
         for (uint32_t w = 0; w < n; w++) {
             const uint64_t np = std::min<uint64_t>(hAcc[w].npairs, wins[w].pairs_cap);
             if (np)
                 SJBG_CK(h, cudaMemcpyAsync(pairs + wins[w].pairs_off, dP + wins[w].pairs_off, sizeof(sjbg_pair) * np,
                                            cudaMemcpyDeviceToHost, h->stream));
         }
+    } else {
+        if (int rc = run_lazy_device(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
     }
     SJBG_CK(h, cudaEventRecord(e1, h->stream));
     SJBG_CK(h, cudaStreamSynchronize(h->stream));
-    float ms = 0.f;
+    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (pairs written so far are written over)
+        h->regrouped = true;
+        if (int rc = run_lazy_watched(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
+        SJBG_CK(h, cudaEventRecord(e1, h->stream));
+        SJBG_CK(h, cudaStreamSynchronize(h->stream));
+    }
+    float ms = 0.f;   // (of both passes, when it took two)
     cudaEventElapsedTime(&ms, e0, e1);
     h->event_pool.push_back(e0);
     h->event_pool.push_back(e1);
     profile_collect(h);
-    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (pairs written so far are written over)
-        h->regrouped = true;
-        return lazy_common(h, L, R, mem, wins, n, pairs, out);
-    }
     if (int se = device_status_error(h, hAcc[n].info)) return se;
     for (uint32_t w = 0; w < n; w++) fill_result(h, hAcc[w], wins[w], enumerate, want, part_used, ms, &out[w]);
     return SJBG_OK;

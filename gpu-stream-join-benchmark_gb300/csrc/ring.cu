@@ -37,6 +37,7 @@ struct RingSlot {
     cudaEvent_t done = nullptr;
     DevBuf pinned[6];                    // private staging of this window's join
     uint32_t part_used = 0;
+    bool again = false;                  // its join was made a second time
     int last_side = 0;                   // the side whose copy completed the window last
 };
 
@@ -71,25 +72,19 @@ void RingDeleter::operator()(RingState *p) const { delete p; }
 
 static RingState *rs(sjbg_handle *h) { return h->ring.get(); }
 
-// The window of slot s with its own staging (both sides are in the slot until
-// it is harvested), its join enqueued or waited for.
-static int ring_join(sjbg_handle *h, RingState &st, RingSlot &s, bool wait) {
+// Enqueue the join of the window in slot s (both sides are in the slot until it
+// is harvested), with the window's own staging.
+static int ring_join(sjbg_handle *h, RingState &st, RingSlot &s) {
     const uint64_t off = (s.id % st.depth) * st.W;
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], s.pinned[i]);
     WinHost wh{0, st.W, 0, st.W, 0, 0};
     WinAcc *hacc = static_cast<WinAcc *>(pinned_get(h, 3, 2 * sizeof(WinAcc)));   // window + status word
-    auto join = wait ? run_lazy_watched : run_lazy_device;
-    const int rc = hacc ? join(h, st.buf[0] + off, st.buf[1] + off, &wh, 1, nullptr, hacc, &s.part_used)
+    const int rc = hacc ? run_lazy_device(h, st.buf[0] + off, st.buf[1] + off, &wh, 1, nullptr, hacc, &s.part_used)
                         : fail(h, SJBG_E_NOMEM, "window staging");
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], s.pinned[i]);
-    return rc;
-}
-
-// A window whose join could not finish by ranges (range_join.cu): by the
-// general path, as every later one.
-static int ring_again(sjbg_handle *h, RingState &st, RingSlot &s) {
-    h->regrouped = true;
-    return ring_join(h, st, s, true);
+    if (rc) return rc;
+    SJBG_CK(h, cudaEventRecord(s.done, h->stream));
+    return SJBG_OK;
 }
 
 // Report the finished windows, in window order (wait: block on each).
@@ -102,8 +97,14 @@ static int ring_harvest(sjbg_handle *h, RingState &st, bool wait) {
             cudaGetLastError();
             break;
         }
-        if (static_cast<const WinAcc *>(s.pinned[3].p)[1].info & kErrRegroup)
-            if (int rc = ring_again(h, st, s)) return rc;
+        if (!s.again && (static_cast<const WinAcc *>(s.pinned[3].p)[1].info & kErrRegroup)) {
+            // the join could not finish by ranges (range_join.cu): by the general path,
+            // as every later one, and reported when that is done
+            h->regrouped = true;
+            if (int rc = ring_join(h, st, s)) return rc;
+            s.again = true;
+            continue;
+        }
         const WinAcc *a = static_cast<const WinAcc *>(s.pinned[3].p);
         sjbg_stream_window r;
         std::memset(&r, 0, sizeof(r));
@@ -137,6 +138,7 @@ static int ring_harvest(sjbg_handle *h, RingState &st, bool wait) {
         st.ready.push_back(r);
         st.joined += 2 * st.W;
         s.state = 0;
+        s.again = false;
         s.filled[0] = s.filled[1] = false;
         st.harvested++;
     }
@@ -147,8 +149,7 @@ static int ring_harvest(sjbg_handle *h, RingState &st, bool wait) {
 static int ring_launch(sjbg_handle *h, RingState &st, RingSlot &s) {
     SJBG_CK(h, cudaStreamWaitEvent(h->stream, s.copied[0], 0));
     SJBG_CK(h, cudaStreamWaitEvent(h->stream, s.copied[1], 0));
-    if (int rc = ring_join(h, st, s, false)) return rc;
-    SJBG_CK(h, cudaEventRecord(s.done, h->stream));
+    if (int rc = ring_join(h, st, s)) return rc;
     s.state = 1;
     st.launched++;
     return SJBG_OK;
