@@ -207,7 +207,7 @@ struct RangeSmem {
     uint16_t owner[kRangeWords];                    // tile of the range's i-th word
     uint32_t warp_tot[32], warp_used[32], warp_sq[32];
     unsigned long long wsum[32], base;
-    uint32_t lo, hi, crowd, n_left, next, stop, refused;
+    uint32_t lo, hi, crowd, most, n_left, next, stop, refused;
 };
 static_assert(sizeof(RangeTable) <= sizeof(uint64_t) * kRangeCap, "the table takes the words' space");
 
@@ -376,7 +376,7 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
             claim = gridDim.x + atomicAdd(queue, 1u);   // stored once this range is done
             sm.stop = *(volatile uint32_t *)status & kErrRegroup;
             sm.lo = 0xFFFFFFFFu;
-            sm.hi = sm.crowd = 0;
+            sm.hi = sm.crowd = sm.most = sm.refused = 0;
         }
         uint32_t wlo = 0, whi = nwin;   // the range's window
         while (whi - wlo > 1) {
@@ -476,7 +476,7 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
             // of them either way (8 windows of 2^20, 16 tuples per key: 670 us, sorted 701;
             // written, the pairs of a sorted range take 1,013, else 1,069)
             constexpr bool kVisit = kHash && kEnum && !kPairs;
-            bool crowded = false, most = false, repeats = false;
+            bool crowded = false, repeats = false;
             {
                 constexpr uint32_t kPer = kRangeSubs / kRangeThreads;
                 uint32_t c[kPer], csum = 0, used = 0, squares = 0, largest = 0;   // (squares of at most kRangeCap words: 2^24)
@@ -502,16 +502,13 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     }
                 }
                 if (largest > kRangeCrowdMost) sm.crowd = 1;
-                if (kTable) {
-                    if (threadIdx.x == 0) sm.refused = 0;
-                    most = __syncthreads_or(largest > kRangeMost);
-                }
+                if (kTable && largest > kRangeMost) sm.most = 1;
                 crowded = __syncthreads_count(largest > (kVisit ? kRangeCrowdMost : kRangeCrowd)) > kRangeThreads / 10 || sm.crowd;
                 if (kTable) {
                     used = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_used[lane] : 0u);
                     squares = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_sq[lane] : 0u);
                     repeats = used <= kRangeUsed &&
-                              (most || 2 * (squares - nl * nl / kRangeSubs) > kRangeRepeat2 * nl);
+                              (sm.most || 2 * (squares - nl * nl / kRangeSubs) > kRangeRepeat2 * nl);
                 }
                 crun += __reduce_add_sync(0xFFFFFFFFu, lane < wid ? sm.warp_tot[lane] : 0u);
 #pragma unroll
