@@ -229,13 +229,17 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
                            sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used) {
     const bool pairs = dPairs != nullptr;
     const bool enumerate = pairs || (h->cfg.flags & SJBG_F_XOR);
+    h->by_ranges = false;
     if (h->cfg.algorithm == SJBG_ALG_HJ && !enumerate) {
         bool done = false;
         *part_used = SJBG_PART_NONE;
         if (int rc = hj_raw_batch(h, dL, dR, wins, n, hAcc, &done)) return rc;
         if (done) return SJBG_OK;
     }
-    if (n && h->cfg.algorithm != SJBG_ALG_NLJ && range_join_pays(h, wins, n, enumerate)) {
+    const bool ranges = range_join_pays(h, wins, n, enumerate);
+    h->by_ranges = ranges && h->use_ranges;
+    h->held_back |= ranges && !h->use_ranges;
+    if (h->by_ranges) {
         *part_used = h->cfg.algorithm == SJBG_ALG_HJ ? SJBG_PART_RADIX : SJBG_PART_NONE;
         return range_join_batch(h, dL, dR, wins, n, dPairs, hAcc, enumerate, h->cfg.algorithm == SJBG_ALG_HJ);
     }
@@ -255,13 +259,12 @@ int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, 
     return stage_copy(h, hAcc, acc, sizeof(WinAcc) * (n + 1));
 }
 
-int run_lazy_watched(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
-                     sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used) {
+int run_lazy_watched(sjbg_handle *h, RangeScope &ranges, const sjbg_tuple *dL, const sjbg_tuple *dR,
+                     const WinHost *wins, uint32_t n, sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used) {
     for (;;) {
         if (int rc = run_lazy_device(h, dL, dR, wins, n, dPairs, hAcc, part_used)) return rc;
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
-        if (!(hAcc[n].info & kErrRegroup) || h->regrouped) return SJBG_OK;
-        h->regrouped = true;   // (from now on, on this handle)
+        if (!ranges.missed(hAcc[n].info)) return SJBG_OK;
     }
 }
 
@@ -300,12 +303,12 @@ static void fill_result(const sjbg_handle *h, const WinAcc &a, const WinHost &w,
 // workspace) and is then captured with private pinned staging buffers; later
 // identical ones replay it.  done is recorded behind the pass, whose results
 // and status word will be in *out.
-constexpr size_t kGraphKeyRegrouped = 11;   // regrouped's place in a graph's key
-static int lazy_graph_pass(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
+constexpr size_t kGraphKeyRanges = 11;   // use_ranges' place in a graph's key
+static int lazy_graph_pass(sjbg_handle *h, RangeScope &ranges, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                            sjbg_pair *dPairs, cudaEvent_t done, WinAcc **out, uint32_t *part_used) {
     std::vector<uint64_t> key = {h->cfg.algorithm, h->cfg.partitioner, h->tune.partitioner, h->cfg.flags, h->cfg.result_mode,
                                  (uint64_t)(uintptr_t)dL, (uint64_t)(uintptr_t)dR, (uint64_t)(uintptr_t)dPairs, n,
-                                 h->tune.bucket_target, (uint64_t)h->tune.persistent_join, (uint64_t)h->regrouped,
+                                 h->tune.bucket_target, (uint64_t)h->tune.persistent_join, (uint64_t)h->use_ranges,
                                  (uint64_t)(uintptr_t)h->stream};
     for (uint32_t w = 0; w < n; w++) {
         const WinHost &x = wins[w];
@@ -318,16 +321,18 @@ static int lazy_graph_pass(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tupl
         h->launches += g->kernels;   // the replay runs every captured kernel again
         *out = static_cast<WinAcc *>(g->pinned[3].p);
         *part_used = g->part_used;
+        h->by_ranges = g->by_ranges;
+        h->held_back |= g->held_back;
         return SJBG_OK;
     }
     WinAcc *hAcc = static_cast<WinAcc *>(pinned_get(h, 3, sizeof(WinAcc) * (n + 1)));
     if (!hAcc) return fail(h, SJBG_E_NOMEM, "result staging");
     *out = hAcc;
-    if (int rc = run_lazy_watched(h, dL, dR, wins, n, dPairs, hAcc, part_used)) return rc;   // warm-up: sizes every buffer
+    if (int rc = run_lazy_watched(h, ranges, dL, dR, wins, n, dPairs, hAcc, part_used)) return rc;   // warm-up: sizes every buffer
     SJBG_CK(h, cudaEventRecord(done, h->stream));
     SJBG_CK(h, cudaStreamSynchronize(h->stream));
     profile_collect(h);
-    key[kGraphKeyRegrouped] = (uint64_t)h->regrouped;   // (it may have been met just now)
+    key[kGraphKeyRanges] = (uint64_t)h->use_ranges;   // (they may have missed just now)
     auto e = std::make_unique<sjbg_handle::GraphEntry>();
     e->key = key;
     e->part_used = *part_used;
@@ -353,6 +358,9 @@ static int lazy_graph_pass(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tupl
     cudaError_t ce2 = cudaStreamEndCapture(h->stream, &graph);
     h->capturing = false;
     e->kernels = h->launches - launches_before;
+    e->by_ranges = h->by_ranges;
+    e->held_back = h->held_back;
+    h->by_ranges = false;          // (the pass itself has been looked at)
     h->launches = launches_before;   // capture runs nothing
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], e->pinned[i]);
     if (rc2 == SJBG_OK && ce == cudaSuccess && ce2 == cudaSuccess && graph) {
@@ -381,13 +389,12 @@ static int lazy_graph(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR
     cudaEvent_t e0 = event_get(h), e1 = event_get(h);
     WinAcc *hAcc = nullptr;
     uint32_t part_used = SJBG_PART_NONE;
+    RangeScope ranges(h, wins, n);
     SJBG_CK(h, cudaEventRecord(e0, h->stream));
-    for (;;) {
-        if (int rc = lazy_graph_pass(h, dL, dR, wins, n, dPairs, e1, &hAcc, &part_used)) return rc;
+    do {   // (a replay may meet keys that do not fit: the general path's graph)
+        if (int rc = lazy_graph_pass(h, ranges, dL, dR, wins, n, dPairs, e1, &hAcc, &part_used)) return rc;
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
-        if (!(hAcc[n].info & kErrRegroup) || h->regrouped) break;
-        h->regrouped = true;   // a replay met keys that do not fit: the general path's graph
-    }
+    } while (ranges.missed(hAcc[n].info));
     float ms = 0.f;   // (of both passes, when it took two)
     cudaEventElapsedTime(&ms, e0, e1);
     h->event_pool.push_back(e0);
@@ -467,7 +474,8 @@ static int lazy_host_pipelined(sjbg_handle *h, const sjbg_tuple *L, const sjbg_t
         SJBG_CK(h, cudaStreamWaitEvent(h->stream, landed[g], 0));
         uint32_t pu = SJBG_PART_NONE;
         // (waited for: the staging buffers (pinned plan uploads, accumulators) are reused by the next group)
-        int rc = run_lazy_watched(h, sL, sR, wins + w0, m, dP, hAcc, &pu);
+        RangeScope ranges(h, wins + w0, m);
+        int rc = run_lazy_watched(h, ranges, sL, sR, wins + w0, m, dP, hAcc, &pu);
         if (rc) {
             cudaStreamSynchronize(h->copy_stream);
             release();
@@ -546,12 +554,13 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
             if (!dP) return fail(h, SJBG_E_NOMEM, "pair staging");
         }
     }
+    RangeScope ranges(h, wins, n);
     // CountKernel mode: an exact count first; refuse instead of truncating
     if (want && h->cfg.result_mode == SJBG_RESULT_COUNT_KERNEL) {
         WinAcc *hp = static_cast<WinAcc *>(pinned_get(h, 4, sizeof(WinAcc) * (n + 1)));
         if (!hp) return fail(h, SJBG_E_NOMEM, "count staging");
         uint32_t pu;
-        int rc = run_lazy_watched(h, dL, dR, wins, n, nullptr, hp, &pu);
+        int rc = run_lazy_watched(h, ranges, dL, dR, wins, n, nullptr, hp, &pu);
         if (rc) return rc;
         if (int se = device_status_error(h, hp[n].info)) return se;
         for (uint32_t w = 0; w < n; w++)
@@ -562,7 +571,7 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     if (!hAcc) return fail(h, SJBG_E_NOMEM, "result staging");
     uint32_t part_used = SJBG_PART_NONE;
     if (mem == SJBG_MEM_HOST && want) {
-        if (int rc = run_lazy_watched(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
+        if (int rc = run_lazy_watched(h, ranges, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
         if (int se = device_status_error(h, hAcc[n].info)) return se;
         // copy back each window's written pairs
         for (uint32_t w = 0; w < n; w++) {
@@ -576,9 +585,8 @@ int lazy_common(sjbg_handle *h, const sjbg_tuple *L, const sjbg_tuple *R, uint32
     }
     SJBG_CK(h, cudaEventRecord(e1, h->stream));
     SJBG_CK(h, cudaStreamSynchronize(h->stream));
-    if ((hAcc[n].info & kErrRegroup) && !h->regrouped) {   // (pairs written so far are written over)
-        h->regrouped = true;
-        if (int rc = run_lazy_watched(h, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
+    if (ranges.missed(hAcc[n].info)) {   // (pairs written so far are written over)
+        if (int rc = run_lazy_watched(h, ranges, dL, dR, wins, n, dP, hAcc, &part_used)) return rc;
         SJBG_CK(h, cudaEventRecord(e1, h->stream));
         SJBG_CK(h, cudaStreamSynchronize(h->stream));
     }

@@ -591,9 +591,10 @@ int sjbg_eager_run(sjbg_handle *h, const sjbg_tuple *left, const sjbg_tuple *rig
     }
     uint32_t windows = 0;
     const WinAcc *hw = nullptr;
-    // by buckets first, then, if the key groups were too large, by sorting (as
-    // every later stream of a handle that has met such a one)
-    for (bool grouped = !h->eager->few_keys;; grouped = false) {
+    // by buckets first, then, if the key groups were too large, by sorting
+    RouteTry &route = h->eager->groups;
+    const bool open = route.open();
+    for (bool grouped = open;; grouped = false) {
         rc = eager_run_batched(h, dl, dr, n_batches, eager_enumerates(h), grouped, dCounts, dWin, &windows);
         if (rc) return rc;
         const size_t outB = cntB + sizeof(WinAcc) * (windows + 1);
@@ -604,9 +605,11 @@ int sjbg_eager_run(sjbg_handle *h, const sjbg_tuple *left, const sjbg_tuple *rig
         hw = reinterpret_cast<const WinAcc *>(hOut + cntB);
         if (!(hw[windows].info & kErrRegroup)) {
             if (batch_counts && n_batches) std::memcpy(batch_counts, hOut, 8 * 2 * n_batches);
+            if (grouped) route.hit();
+            else if (!open) route.passed();
             break;
         }
-        h->eager->few_keys = true;
+        route.miss();
     }
     profile_collect(h);
     if (int se = device_status_error(h, hw[windows].info)) return se;

@@ -33,7 +33,7 @@ struct EagerState {
     uint32_t table_bits = 0;
     WinAcc *acc = nullptr;     // current window totals (device)
     unsigned long long *batch_count = nullptr;   // matches and finished CTAs of the batch in flight (zero between batches)
-    bool few_keys = false;     // a recorded stream had too few distinct keys to go by buckets (eager_run.cu)
+    RouteTry groups;           // recorded streams by buckets, which too few distinct keys do not fit (eager_run.cu)
     int host_direct = -1;      // whether kernels read pageable host memory in place (-1: not asked yet)
     sjbg_pair *pairs = nullptr;   // current window's pairs (device), pairs_cap entries
     uint64_t pairs_cap = 0;

@@ -22,8 +22,8 @@
 // the left words of each key in arrival order and counts, for every word, the
 // other side's earlier ones (egroup_*; the batch counts and the window totals
 // in one pass).  A bucket that does not fit (few distinct keys) sets
-// kErrRegroup: the call is made again by the sort below, which the handle then
-// keeps to.  2^20 tuples per window, 768 batches of 4,096: 478 us by the sort,
+// kErrRegroup: the call is made again by the sort below, as the handle's next
+// ones are for a while (RouteTry).  2^20 tuples per window, 768 batches of 4,096: 478 us by the sort,
 // 167 by buckets.
 // By the sort (also pair enumeration and xor): the window's keys in arrival
 // order are sorted (sort.cu) with each tuple's arrival position as payload, so

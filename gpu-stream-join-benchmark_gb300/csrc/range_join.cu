@@ -824,8 +824,39 @@ constexpr uint64_t kHashLeast = 1u << 17, kHashMost = 1u << 25;
 // costs decide, and the ranges' are lower (pairs, 128 of 1,000: 67 against 86).
 constexpr uint64_t kHashMean = 6144;   // tuples of both sides per window
 
+RouteTry &range_route(sjbg_handle *h, const WinHost *wins, uint32_t n) {
+    uint64_t most = 0;
+    for (uint32_t w = 0; w < n; w++) most = std::max({most, wins[w].n_left, wins[w].n_right});
+    uint32_t bits = 0;
+    for (; most; most >>= 1) bits++;
+    return h->range_try[bits];
+}
+
+RangeScope::RangeScope(sjbg_handle *handle, const WinHost *wins, uint32_t n) : h(handle), t(range_route(handle, wins, n)) {
+    h->use_ranges = t.open();
+    h->by_ranges = h->held_back = false;
+}
+
+RangeScope::~RangeScope() {
+    if (h->held_back && !once_missed) t.passed();
+    h->use_ranges = h->by_ranges = h->held_back = false;
+}
+
+bool RangeScope::missed(unsigned long long status) {
+    if (!h->by_ranges) return false;
+    h->by_ranges = false;
+    if (!(status & kErrRegroup)) {
+        t.hit();
+        return false;
+    }
+    t.miss();
+    once_missed = true;
+    h->use_ranges = false;
+    return true;
+}
+
 bool range_join_pays(const sjbg_handle *h, const WinHost *wins, uint32_t n, bool enumerate) {
-    if (h->regrouped || h->unwatched) return false;
+    if (n == 0 || h->cfg.algorithm == SJBG_ALG_NLJ) return false;
     if (h->cfg.algorithm == SJBG_ALG_HJ) {
         if (h->cfg.partitioner != SJBG_PART_AUTO || h->tune.partitioner) return false;
         uint64_t tuples = 0;

@@ -37,7 +37,7 @@ struct RingSlot {
     cudaEvent_t done = nullptr;
     DevBuf pinned[6];                    // private staging of this window's join
     uint32_t part_used = 0;
-    bool again = false;                  // its join was made a second time
+    bool by_ranges = false;              // its join may not have fitted (range_join.cu)
     int last_side = 0;                   // the side whose copy completed the window last
 };
 
@@ -74,15 +74,18 @@ static RingState *rs(sjbg_handle *h) { return h->ring.get(); }
 
 // Enqueue the join of the window in slot s (both sides are in the slot until it
 // is harvested), with the window's own staging.
-static int ring_join(sjbg_handle *h, RingState &st, RingSlot &s) {
+static int ring_join(sjbg_handle *h, RingState &st, RingSlot &s, bool ranges) {
     const uint64_t off = (s.id % st.depth) * st.W;
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], s.pinned[i]);
     WinHost wh{0, st.W, 0, st.W, 0, 0};
+    RangeScope scope(h, &wh, 1);
+    h->use_ranges &= ranges;
     WinAcc *hacc = static_cast<WinAcc *>(pinned_get(h, 3, 2 * sizeof(WinAcc)));   // window + status word
     const int rc = hacc ? run_lazy_device(h, st.buf[0] + off, st.buf[1] + off, &wh, 1, nullptr, hacc, &s.part_used)
                         : fail(h, SJBG_E_NOMEM, "window staging");
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], s.pinned[i]);
     if (rc) return rc;
+    s.by_ranges = h->by_ranges;
     SJBG_CK(h, cudaEventRecord(s.done, h->stream));
     return SJBG_OK;
 }
@@ -97,13 +100,17 @@ static int ring_harvest(sjbg_handle *h, RingState &st, bool wait) {
             cudaGetLastError();
             break;
         }
-        if (!s.again && (static_cast<const WinAcc *>(s.pinned[3].p)[1].info & kErrRegroup)) {
-            // the join could not finish by ranges (range_join.cu): by the general path,
-            // as every later one, and reported when that is done
-            h->regrouped = true;
-            if (int rc = ring_join(h, st, s)) return rc;
-            s.again = true;
-            continue;
+        if (s.by_ranges) {
+            const WinHost wh{0, st.W, 0, st.W, 0, 0};
+            RouteTry &route = range_route(h, &wh, 1);
+            if (static_cast<const WinAcc *>(s.pinned[3].p)[1].info & kErrRegroup) {
+                // the keys did not fit their ranges (range_join.cu): joined by the general
+                // path, and reported when that is done
+                if (int rc = ring_join(h, st, s, false)) return rc;
+                route.miss();
+                continue;
+            }
+            route.hit();
         }
         const WinAcc *a = static_cast<const WinAcc *>(s.pinned[3].p);
         sjbg_stream_window r;
@@ -138,7 +145,6 @@ static int ring_harvest(sjbg_handle *h, RingState &st, bool wait) {
         st.ready.push_back(r);
         st.joined += 2 * st.W;
         s.state = 0;
-        s.again = false;
         s.filled[0] = s.filled[1] = false;
         st.harvested++;
     }
@@ -149,7 +155,7 @@ static int ring_harvest(sjbg_handle *h, RingState &st, bool wait) {
 static int ring_launch(sjbg_handle *h, RingState &st, RingSlot &s) {
     SJBG_CK(h, cudaStreamWaitEvent(h->stream, s.copied[0], 0));
     SJBG_CK(h, cudaStreamWaitEvent(h->stream, s.copied[1], 0));
-    if (int rc = ring_join(h, st, s)) return rc;
+    if (int rc = ring_join(h, st, s, true)) return rc;
     s.state = 1;
     st.launched++;
     return SJBG_OK;

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <map>
 #include <memory>
 #include <string>
@@ -37,6 +38,23 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// Whether calls of one kind take a route that may turn out not to fit their
+// keys, when the call is made again another way.  After a miss the next calls
+// leave the route out: 16 of them, twice as many after the next miss with no
+// hit between, at most 256.  So one hot window costs the calls after it little,
+// and a stream that never fits one second try in 256 calls.
+struct RouteTry {
+    uint32_t wait = 0, span = 0;
+    bool open() const { return wait == 0; }
+    void passed() { if (wait) wait--; }   // a call that left it out
+    void hit() { span = 0; }
+    void miss() {
+        if (wait) return;   // (of a call enqueued before the last miss was seen)
+        span = span ? std::min(2 * span, 256u) : 16u;
+        wait = span;
+    }
+};
+
 struct EagerState;
 struct StreamState;
 struct RingState;   // device-resident ingest ring (ring.cu)
@@ -68,8 +86,11 @@ struct sjbg_handle {
     std::vector<double> kms;
     uint64_t launches = 0;
     bool capturing = false;
-    bool regrouped = false;       // a join's ranges did not fit: the handle's joins take the general path (range_join.cu)
-    bool unwatched = false;       // the call being enqueued is not waited for: it must not need a second try
+    // joins by ranges (range_join.cu), by the bit length of a call's largest window
+    sjbg::RouteTry range_try[65];
+    bool use_ranges = false;      // the call being enqueued may go by ranges (it is watched: RangeScope)
+    bool by_ranges = false;       // it did
+    bool held_back = false;       // it would have, but for use_ranges
 
     // tunables (the autotuner picks them per workload shape)
     struct Tune {
@@ -86,6 +107,7 @@ struct sjbg_handle {
         sjbg::DevBuf pinned[6];
         uint32_t part_used = 0;
         uint64_t kernels = 0;   // kernel launches captured: counted again on every replay
+        bool by_ranges = false, held_back = false;   // as of the handle, for the captured call
     };
     std::vector<std::unique_ptr<GraphEntry>> graphs;
     std::map<std::string, Tune> tuned;   // autotuner decisions by workload shape
@@ -211,10 +233,28 @@ int autotune_lazy(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
 // then the call's device status word in hAcc[n].info (kErr* bits).
 int run_lazy_device(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
                     sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used);
-// run_lazy_device, waited for, and made again with the full sort when a
-// sort-merge join's key ranges did not fit.
-int run_lazy_watched(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, const WinHost *wins, uint32_t n,
-                     sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used);
+// Lets the call enqueued in its scope go by ranges, unless calls of its size
+// lately did not fit them.  Only for calls whose status is looked at.
+class RangeScope {
+public:
+    RangeScope(sjbg_handle *h, const WinHost *wins, uint32_t n);
+    ~RangeScope();
+    RangeScope(const RangeScope &) = delete;
+    RangeScope &operator=(const RangeScope &) = delete;
+    // With the status word of a finished pass: whether its ranges did not fit,
+    // and the pass has to be made again (by the general path, in this scope).
+    bool missed(unsigned long long status);
+
+private:
+    sjbg_handle *h;
+    RouteTry &t;
+    bool once_missed = false;
+};
+RouteTry &range_route(sjbg_handle *h, const WinHost *wins, uint32_t n);
+// run_lazy_device, waited for, and made again by the general path when the
+// ranges did not fit.
+int run_lazy_watched(sjbg_handle *h, RangeScope &ranges, const sjbg_tuple *dL, const sjbg_tuple *dR,
+                     const WinHost *wins, uint32_t n, sjbg_pair *dPairs, WinAcc *hAcc, uint32_t *part_used);
 // SJBG_OK, or the error a device status word reports (recorded on the handle).
 int device_status_error(sjbg_handle *h, unsigned long long bits);
 

@@ -151,11 +151,9 @@ static int launch_join(sjbg_handle *h, StreamState &st, StreamWin *w, cudaStream
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], w->pinned[i]);
     WinHost wh{0, w->n[0], 0, w->n[1], 0, 0};
     WinAcc *hacc = static_cast<WinAcc *>(pinned_get(h, 3, 2 * sizeof(WinAcc)));   // window + status
-    h->unwatched = true;
     int rc = hacc ? run_lazy_device(h, w->buf[0] ? w->buf[0] : nullptr, w->buf[1] ? w->buf[1] : nullptr, &wh, 1,
                                     nullptr, hacc, &w->part_used)
                   : fail(h, SJBG_E_NOMEM, "window staging");
-    h->unwatched = false;
     for (int i = 0; i < 6; i++) std::swap(h->pinned[i], w->pinned[i]);
     if (rc) return rc;
     SJBG_CK(h, cudaEventRecord(w->ev_done, h->stream));
