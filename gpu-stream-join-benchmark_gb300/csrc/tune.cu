@@ -4,8 +4,9 @@
 // enumeration, log2 of the tuples and of the windows) not seen before, the
 // candidate settings - left tuples per bucket (which sets the partition
 // fan-out), persistent vs one-CTA-per-bucket joins and, for SJBG_PART_AUTO
-// handles, one HBM table per window vs radix partitioning - are each run on the
-// batch itself, timed with CUDA events, and the fastest is kept.  Decisions
+// handles, one HBM table per window vs radix partitioning vs the untuned choice
+// (which may go by hash ranges) - are each run on the batch itself, timed with
+// CUDA events, and the fastest is kept.  Decisions
 // are persisted as JSON lines in $SJBG_TUNE_CACHE (default
 // ~/.cache/sjbg_tune.json) and reloaded by later handles.
 #include <cstdio>
@@ -94,27 +95,33 @@ int autotune_lazy(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     sjbg_handle::Tune best;
     best.ms = 1e30f;
     // partitioners tried: the configured one, or for SJBG_PART_AUTO the HBM
-    // table and radix partitioning
+    // table, radix partitioning and, with its defaults, the untuned choice (AUTO)
+    const bool choose = h->cfg.partitioner == SJBG_PART_AUTO;
     std::vector<uint32_t> parts;
-    if (h->cfg.partitioner == SJBG_PART_AUTO) parts = {SJBG_PART_NONE, SJBG_PART_RADIX};
-    else parts = {0u};
+    if (choose) parts = {SJBG_PART_AUTO, SJBG_PART_NONE, SJBG_PART_RADIX};
+    else parts = {SJBG_PART_AUTO};
     for (uint32_t part : parts)
     for (uint32_t target : {2048u, 4096u, 8192u}) {
         for (bool persistent : {false, true}) {
-            if (enumerate && persistent) continue;   // chain-building joins run one CTA per bucket
+            const bool untuned = choose && part == SJBG_PART_AUTO;
+            if (untuned && (target != 4096u || !persistent)) continue;
+            if (enumerate && persistent && !untuned) continue;   // chain-building joins run one CTA per bucket
             if (part == SJBG_PART_NONE && (target != 4096u || !persistent)) continue;   // no buckets to tune
             h->tune.partitioner = part;
             h->tune.bucket_target = target;
             h->tune.persistent_join = persistent;
+            RangeScope ranges(h, wins, n);
             uint32_t pu;
             int rc = run_lazy_device(h, dL, dR, wins, n, nullptr, hAcc, &pu);   // warm-up (sizes buffers)
             if (rc) return rc;
             SJBG_CK(h, cudaStreamSynchronize(h->stream));
+            if (ranges.missed(hAcc[n].info)) continue;   // not for these keys
             SJBG_CK(h, cudaEventRecord(e0, h->stream));
             rc = run_lazy_device(h, dL, dR, wins, n, nullptr, hAcc, &pu);
             if (rc) return rc;
             SJBG_CK(h, cudaEventRecord(e1, h->stream));
             SJBG_CK(h, cudaStreamSynchronize(h->stream));
+            ranges.missed(hAcc[n].info);   // (the same keys: it fitted)
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
             if (ms < best.ms) {
