@@ -309,6 +309,17 @@ static int eager_clear(sjbg_handle *h) {
     return SJBG_OK;
 }
 
+// Through the host's page tables: pageable access alone may also mean that the
+// driver moves the pages it faults on.
+bool reads_host_pages(int device) {
+    int coherent = 0;
+    if (cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return coherent != 0;
+}
+
 // The address at which kernels may read a caller's batch in place, or null: a
 // 16-byte aligned device batch, or a host batch in pinned memory or, where the
 // device reads pageable host memory coherently, in any.  (The call waits for
@@ -317,14 +328,7 @@ static const sjbg_tuple *batch_in_place(sjbg_handle *h, const sjbg_tuple *batch,
     if (reinterpret_cast<uintptr_t>(batch) & 15u) return nullptr;
     if (!from_host) return batch;
     EagerState &st = *h->eager;
-    if (st.host_direct < 0) {
-        int pageable = 0;
-        if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, h->device) != cudaSuccess) {
-            cudaGetLastError();
-            pageable = 0;
-        }
-        st.host_direct = pageable;
-    }
+    if (st.host_direct < 0) st.host_direct = reads_host_pages(h->device);
     if (st.host_direct) return batch;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, batch) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)

@@ -62,6 +62,8 @@ uint32_t nlj_left_tile();   // left tuples per nested-loop CTA
 int eager_run_batched(sjbg_handle *h, const sjbg_tuple *dl, const sjbg_tuple *dr, uint64_t n_batches, bool enumerate,
                       bool grouped, unsigned long long *dCounts, WinAcc *dWin, uint32_t *n_windows);
 
+// Whether the device reads pageable host memory where it lies, coherently.
+bool reads_host_pages(int device);
 int eager_init(sjbg_handle *h);
 int eager_init_and_clear(sjbg_handle *h);
 

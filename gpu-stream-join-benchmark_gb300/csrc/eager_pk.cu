@@ -744,12 +744,7 @@ static int pk_init(sjbg_handle *h) {
     // the slots of 4 per SM, and every CTA joins each grid barrier)
     const int per_sm = h->cfg.algorithm == SJBG_ALG_SMJ ? 4 : 2;
     pk->grid = h->cfg.algorithm == SJBG_ALG_HJ ? std::min(16, h->num_sms) : std::min(occ, per_sm) * h->num_sms;
-    int pageable = 0;
-    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, h->device) != cudaSuccess) {
-        cudaGetLastError();
-        pageable = 0;
-    }
-    pk->host_direct = pageable != 0;
+    pk->host_direct = reads_host_pages(h->device);
     pk->count.assign(pk->Q, 0);
     pk->status.assign(pk->Q, 0);
     pk->snap.assign(pk->Q, WinAcc{0, 0, 0, 0, 0});
