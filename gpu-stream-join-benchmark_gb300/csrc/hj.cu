@@ -1484,12 +1484,11 @@ struct KeyRange {
     uint32_t lo, hi;
 };
 
-// Loads the first tile of a build run (kJoinPer tuples per thread) and returns
-// the run's smallest and largest keys to every thread; ends with a barrier, its only one after the CTA's first call (turn 0): the calls take the
-// two result slots in turn and leave the other one reset.
-template <bool kRaw>
-__device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
-                                               uint32_t &turn) {
+// The smallest lo and the largest hi of the CTA's threads, to every thread; its
+// only barrier ends it after the CTA's first call (turn 0): the calls take the
+// two result slots in turn and leave the other one reset.  (Not a template: raw
+// and partitioned items of a CTA use the same slots.)
+__device__ __forceinline__ KeyRange cta_key_range(uint32_t lo, uint32_t hi, uint32_t &turn) {
     __shared__ uint32_t min_s[2], max_s[2];
     if (turn == 0) {
         if (threadIdx.x == 0) {
@@ -1500,6 +1499,25 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
     }
     const uint32_t slot = turn & 1u;
     turn = slot + 1;
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    if (lane_id() == 0) {
+        atomicMin(&min_s[slot], lo);
+        atomicMax(&max_s[slot], hi);
+    }
+    SJBG_BARRIER();
+    if (threadIdx.x == 0) {
+        min_s[slot ^ 1u] = 0xFFFFFFFFu;
+        max_s[slot ^ 1u] = 0;
+    }
+    return KeyRange{min_s[slot], max_s[slot]};
+}
+
+// Loads the first tile of a build run (kJoinPer tuples per thread) and returns
+// the run's smallest and largest keys to every thread.
+template <bool kRaw>
+__device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
+                                               uint32_t &turn) {
     uint32_t lo = 0xFFFFFFFFu, hi = 0;
 #pragma unroll
     for (int k = 0; k < kJoinPer; k++) {
@@ -1518,18 +1536,7 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
         lo = min(lo, key);
         hi = max(hi, key);
     }
-    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
-    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
-    if (lane_id() == 0) {
-        atomicMin(&min_s[slot], lo);
-        atomicMax(&max_s[slot], hi);
-    }
-    SJBG_BARRIER();
-    if (threadIdx.x == 0) {
-        min_s[slot ^ 1u] = 0xFFFFFFFFu;
-        max_s[slot ^ 1u] = 0;
-    }
-    return KeyRange{min_s[slot], max_s[slot]};
+    return cta_key_range(lo, hi, turn);
 }
 
 // e: the build run's first tile (build_head), when loaded.
