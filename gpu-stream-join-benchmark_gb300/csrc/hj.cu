@@ -1351,8 +1351,8 @@ constexpr uint32_t kPlaceRepeat2 = 7;   // twice the tuples that share a tuple's
 constexpr uint32_t kPlaceMost = 32;
 constexpr size_t kPlaceBytes = sizeof(uint64_t) * kPlaceCap + sizeof(uint32_t) * (kPlacesMax + 1);
 
-// Adds the matches to count and prod; false, with nothing added and e still the
-// build run's first tile (build_head), when the run's keys repeat (nB <= kPlaceCap).
+// Adds the matches to count and prod; false, with nothing added, when the run's
+// keys repeat (nB <= kPlaceCap).  e: the build run's first tile (build_head).
 template <bool kRaw>
 __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
                                                   unsigned long long &count, unsigned long long &prod) {
@@ -1398,7 +1398,6 @@ __device__ __forceinline__ bool join_count_places(const JoinItem &ji, const Join
     const bool most = __syncthreads_or(largest > kPlaceMost);
     squares = __reduce_add_sync(0xFFFFFFFFu, lane_id() < kJoinThreads / 32 ? warp_sq[lane_id()] : 0u);
     if (most || 2 * (squares - (nB * nB >> bits)) > kPlaceRepeat2 * nB) {   // (the same for the whole CTA)
-        if (nB > tile) load(0);
         SJBG_BARRIER();   // the places are read before the next table's entries
         return false;
     }
@@ -1539,11 +1538,9 @@ __device__ __forceinline__ KeyRange build_head(const JoinItem &ji, const JoinRun
     return cta_key_range(lo, hi, turn);
 }
 
-// e: the build run's first tile (build_head), when loaded.
 template <bool kRaw>
-__device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const JoinRuns &jr, uint64_t (&e)[kJoinPer],
-                                                  bool loaded, uint32_t cap, unsigned long long &count,
-                                                  unsigned long long &prod) {
+__device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const JoinRuns &jr, uint32_t cap,
+                                                  unsigned long long &count, unsigned long long &prod) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ uint32_t novf;
     const uint32_t nB = ji.nB, nP = ji.nP;
@@ -1561,6 +1558,7 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
     t.max_probe = nB < C ? C : kMaxProbe;
     constexpr uint32_t tile = kJoinPer * kJoinThreads;
 
+    uint64_t e[kJoinPer];
     uint32_t n = nB;
     for (;;) {
         for (uint32_t i = threadIdx.x; i <= C; i += kJoinThreads) {
@@ -1572,15 +1570,12 @@ __device__ __forceinline__ void join_count_bucket(const JoinItem &ji, const Join
         SJBG_BARRIER();
         // build: kJoinPer independent loads per thread, then insert them
         for (uint32_t base = 0; base < n; base += tile) {
-            if (!loaded) {
 #pragma unroll
-                for (int k = 0; k < kJoinPer; k++) {
-                    const uint32_t i = base + k * kJoinThreads + threadIdx.x;
-                    e[k] = i < n ? run_load<kRaw>(jr.b, i) : 0ull;
-                }
-                SJBG_BARRIER();   // every read of this tile precedes any overflow write
+            for (int k = 0; k < kJoinPer; k++) {
+                const uint32_t i = base + k * kJoinThreads + threadIdx.x;
+                e[k] = i < n ? run_load<kRaw>(jr.b, i) : 0ull;
             }
-            loaded = false;
+            SJBG_BARRIER();   // every read of this tile precedes any overflow write
 #pragma unroll
             for (int k = 0; k < kJoinPer; k++) {
                 const uint32_t i = base + k * kJoinThreads + threadIdx.x;
@@ -1936,9 +1931,8 @@ struct JoinSums {
 };
 template <bool kRaw>
 __device__ __noinline__ JoinSums join_count_rest(const JoinItem ji, const JoinRuns jr, uint32_t cap) {
-    uint64_t e[kJoinPer];
     JoinSums r{0, 0};
-    join_count_bucket<kRaw>(ji, jr, e, false, cap, r.count, r.prod);
+    join_count_bucket<kRaw>(ji, jr, cap, r.count, r.prod);
     return r;
 }
 
@@ -1947,15 +1941,15 @@ __device__ __noinline__ JoinSums join_count_rest(const JoinItem ji, const JoinRu
 template <bool kRaw, bool kModels>
 __device__ __forceinline__ void join_item(const JoinItem &ji, const JoinRuns &jr, uint32_t cap, uint32_t &clean,
                                           uint32_t &turn, unsigned long long &count, unsigned long long &prod) {
-    uint64_t e[kJoinPer];
     // a learned bucket's light keys are a range (no direct table) and repeat, up
     // to the heavy cut: the hash table, which aggregates them (z = 1.5, 8 x 2^24:
     // 54 us, by places 130)
     if (kModels && (ji.flags & kItemModel)) {
-        join_count_bucket<kRaw>(ji, jr, e, false, cap, count, prod);
+        join_count_bucket<kRaw>(ji, jr, cap, count, prod);
         clean = 0;
         return;
     }
+    uint64_t e[kJoinPer];
     if (ji.nB <= kPlaceCap) {
         const KeyRange kr = build_head<kRaw>(ji, jr, e, turn);
         if (const uint32_t passes = direct_passes(ji, kr)) {
@@ -2226,7 +2220,11 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
     SJBG_BARRIER();
     while (valid_s & 1u) {
         const uint32_t c = cur_s, v = valid_s;
-        const JoinItem ji = slot_s[c];
+        // learned calls read the record in shared memory as they go (z = 0.5, 2 x 4 M:
+        // 76 us with it in registers, 74 without); for the others it is the other way
+        // round (2 x 2^24 dense tuples: 129 and 139)
+        using Item = std::conditional_t<kModels, const JoinItem &, const JoinItem>;
+        Item ji = slot_s[c];
         const uint32_t c1 = c == 2 ? 0u : c + 1u, c2 = c1 == 2 ? 0u : c1 + 1u;
         uint32_t claim_next = 0;
         if (threadIdx.x == 0) {
