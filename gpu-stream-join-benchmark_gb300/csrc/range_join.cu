@@ -44,7 +44,10 @@ constexpr int kRangeWarps = kRangeThreads / 32;
 constexpr uint32_t kRangeCap = 4096;            // left words of a range (shared memory)
 constexpr uint32_t kRangeWords = 8192;          // words of both sides
 constexpr uint32_t kRangeTarget = 3328;         // left words per range, and half the words of both: uneven ranges still fit
-constexpr uint32_t kRangeTargetMost = 3456;     // the same, when it saves a second wave of CTAs
+// Fuller ranges, when they save a second wave of CTAs: up to here a range of
+// keys with four tuples each has five standard deviations (sqrt(4 * 3,500) =
+// 118) of room below kRangeCap, so some 304 ranges hardly ever miss.
+constexpr uint32_t kRangeTargetMost = 3500;
 constexpr uint32_t kRangesMax = 1024;           // more ranges: runs of under 4 words per tile
 constexpr uint32_t kRangeTilesMax = 1536;       // tiles of both sides of a window
 constexpr uint32_t kRangeDigit = 7;             // bits per shared-memory sorting pass
@@ -766,9 +769,16 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
         }
     };
     plan(kRangeTarget);
-    if (hash && nb > slots) {   // somewhat fuller ranges, if they make it one wave
-        plan(kRangeTargetMost);
-        if (nb > slots) plan(kRangeTarget);
+    if (hash && nb > slots) {   // the least full ranges that make it one wave, if any do
+        uint32_t no = kRangeTarget, yes = kRangeTargetMost;
+        plan(yes);
+        if (nb > slots) yes = kRangeTarget;
+        while (yes > no + 1) {
+            const uint32_t mid = (no + yes) / 2;
+            plan(mid);
+            (nb > slots ? no : yes) = mid;
+        }
+        plan(yes);
     }
     if (tiles > 0x7FFFFFFFull || nb > 0x7FFFFFFFull) return fail(h, SJBG_E_CAPACITY, "batch has too many tiles");
     if (nb == 0) {

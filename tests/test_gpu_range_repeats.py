@@ -73,3 +73,26 @@ def test_pairs_of_repeated_keys_by_hash_ranges(lib, oracle, per):
                 else:
                     assert len(np.unique(have)) == len(have) and np.isin(have, sorted_pairs(w["pairs"])).all()
         assert "range_join" in j.kernel_stats()
+
+
+@pytest.mark.parametrize("per", [1, 4])
+@pytest.mark.parametrize("sizes", [[(1 << 20, 1 << 20)], [(1_063_000, 900_000)], [(1_064_500, 1_000_000)], [(65_536, 65_536)] * 16,
+                                   [(66_400, 66_400)] * 16])
+def test_one_wave_of_ranges(lib, oracle, sizes, per):
+    """Sizes around those whose ranges are filled up to make one wave of CTAs."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(47)
+    lefts = [keys_of(per, 0, False, nl, rng) for nl, _ in sizes]
+    rights = [keys_of(per, 0, False, nr, rng) for _, nr in sizes]
+    descs, lo, ro = [], 0, 0
+    for nl, nr in sizes:
+        descs.append((lo, nl, ro, nr, 0, 0))
+        lo, ro = lo + nl, ro + nr
+    left, right = make_tuples(np.concatenate(lefts)), make_tuples(np.concatenate(rights))
+    want, _ = oracle.join_windows(left, right, descs, enumerate_pairs=False)
+    dl, dr = torch.from_numpy(left.view(np.uint8)).cuda(), torch.from_numpy(right.view(np.uint8)).cuda()
+    with lib.Joiner(lib.ALG_HJ, lib.LAZY, flags=lib.F_PROFILE, max_tuples_per_window=1 << 21) as j:
+        got = j.lazy_execute_batch(dl, dr, descs, mem=lib.MEM_DEVICE)
+        assert "range_join" in j.kernel_stats()
+    for d, g, w in zip(descs, got, want):
+        assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
