@@ -28,8 +28,8 @@
 // Hash joins of calls in the middle of the size range (hj.cu) take the same
 // steps with ranges of a multiplicative hash of the key: no sample, two
 // launches for the partitioning and the join, where counting, scanning and
-// scattering first need five; a range whose keys
-// repeat adds them up in a table.
+// scattering first need five.  Counting, they add up the words of repeated keys
+// in a table.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -60,17 +60,24 @@ constexpr uint32_t kRangeSubs = 2048;           // subranges of a range
 // the range (13 us; at a limit of 16 for every subrange, one range in 300 of
 // keys with two duplicates each was sorted).
 constexpr uint32_t kRangeCrowd = 16, kRangeCrowdMost = 128;
-// By the hash, words of one subrange are mostly words of one key: when keys
-// repeat, counting joins add up the left words of each key in a table of
-// kRangeSubs slots in the words' space.  The rule is that of the bucket joins'
-// places (hj.cu): more than 3.5 left words that share a word's key on average,
-// by the squares of the subranges' numbers, or a subrange of more than
-// kRangeMost; and few enough keys that the table is not full, by the subranges
-// in use (kRangeUsed of 2,048: some 1,580 keys).  8 windows of 2^20 with 1 / 2 /
-// 4 / 8 / 16 / 64 tuples per key: lists and sort 238 / 253 / 281 / 335 / 449 /
-// 627 us, with the table 240 / 255 / 249 / 230 / 221 / 214; a kRangeMost of 16
-// takes ranges of two tuples per key too (289), 64 measures the same as 32.
-constexpr uint32_t kRangeRepeat2 = 7, kRangeMost = 32, kRangeUsed = 1100;
+// By the hash, words of one subrange are mostly words of one key, so counting
+// joins keep no list of a hot subrange, one with more than kRangeHot left words:
+// they add up the words of each of its keys in a table behind the lists, in the
+// words' space, and a probe looks there.  When keys repeat throughout, every
+// subrange is hot: with more than 3.5 left words that share a word's key on
+// average, by the squares of the subranges' numbers (the rule of the bucket
+// joins' places, hj.cu), and few enough keys for the table, by the subranges in
+// use (kRangeUsed of 2,048: some 1,580 keys).
+// 8 windows of 2^20, 1 / 2 / 4 / 8 / 16 / 64 tuples per key: lists, and a sort of
+// crowded ranges, 238 / 253 / 281 / 335 / 449 / 627 us; hot subranges without the
+// rule 246 / 261 / 293 / 348 / 370 / 222; with it 246 / 263 / 251 / 234 / 226 /
+// 221.  Dense keys, z = 0.4 / 0.5: lists and sort 322 / 427, rule without hot
+// subranges 322 / 430, both 276 / 295 (direct tables after radix partitioning 251
+// / 252).  A kRangeHot of 4 / 8 / 12 / 20: distinct keys 392 / 287 / 250 / 246,
+// z = 0.5 335 / 292 / 293 / 303.  One window of 1,000,003 distinct keys pays 1 us of 57.
+constexpr uint32_t kRangeHot = 16;
+constexpr uint32_t kRangeRepeat2 = 7, kRangeUsed = 1100;
+constexpr uint32_t kRangeHotBit = 1u << 31;   // of a subrange's first word: no list
 constexpr uint32_t kRangeProbe = 64;   // slots of the table looked at for a key
 
 struct RangeWin {
@@ -191,15 +198,15 @@ range_tiles_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restric
 }
 
 struct RangeTable {
-    unsigned long long sum[kRangeSubs];   // of fr
-    uint32_t key[kRangeSubs], cnt[kRangeSubs];
+    unsigned long long *sum;   // of fr
+    uint32_t *key, *cnt;
+    uint32_t slots;
 };
 
 struct RangeSmem {
     union {
         uint64_t word[kRangeCap];                   // left words by subrange
         uint32_t buf[2][2][kRangeCap];              // sorting: keys and vals, before and after a pass; then F in the free pair
-        RangeTable tab;                             // repeated keys
     };
     union {
         uint32_t sub[kRangeSubs + 1];               // first left word of each subrange, and their number
@@ -210,28 +217,29 @@ struct RangeSmem {
     uint16_t owner[kRangeWords];                    // tile of the range's i-th word
     uint32_t warp_tot[32], warp_used[32], warp_sq[32];
     unsigned long long wsum[32], base;
-    uint32_t lo, hi, crowd, most, n_left, next, stop, refused;
+    uint32_t lo, hi, crowd, n_left, next, stop, refused;
 };
-static_assert(sizeof(RangeTable) <= sizeof(uint64_t) * kRangeCap, "the table takes the words' space");
 
-// The slot of the table that holds the key or is the first free one after its
-// home; kRangeSubs: neither among kRangeProbe slots.
-__device__ __forceinline__ uint32_t range_slot(const RangeTable &t, uint32_t key, uint32_t home) {
+// The slot of the table that holds the key or is the first free one from its
+// home on; t.slots: neither among kRangeProbe slots.
+__device__ __forceinline__ uint32_t range_slot(const RangeTable &t, uint32_t key) {
+    uint32_t s = __umulhi(place_hash(key), t.slots);
     for (uint32_t p = 0; p < kRangeProbe; p++) {
-        const uint32_t s = (home + p) & (kRangeSubs - 1), k = *(volatile const uint32_t *)&t.key[s];
+        const uint32_t k = *(volatile const uint32_t *)&t.key[s];
         if (k == key || k == kEmptyKey) return s;
+        s = s + 1 == t.slots ? 0u : s + 1;
     }
-    return kRangeSubs;
+    return t.slots;
 }
 
 // Adds a left word to the table; false: no slot for its key (or the key is the
 // mark of free slots).
-__device__ __forceinline__ bool range_add(RangeTable &t, uint64_t word, uint32_t home) {
+__device__ __forceinline__ bool range_add(const RangeTable &t, uint64_t word) {
     const uint32_t key = (uint32_t)word;
     if (key == kEmptyKey) return false;
     for (;;) {   // (a slot lost to another key is taken for good: at most kRangeProbe times)
-        const uint32_t s = range_slot(t, key, home);
-        if (s == kRangeSubs) return false;
+        const uint32_t s = range_slot(t, key);
+        if (s == t.slots) return false;
         const uint32_t was = atomicCAS(&t.key[s], kEmptyKey, key);
         if (was != kEmptyKey && was != key) continue;
         atomicAdd(&t.cnt[s], 1u);
@@ -379,7 +387,7 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
             claim = gridDim.x + atomicAdd(queue, 1u);   // stored once this range is done
             sm.stop = *(volatile uint32_t *)status & kErrRegroup;
             sm.lo = 0xFFFFFFFFu;
-            sm.hi = sm.crowd = sm.most = sm.refused = 0;
+            sm.hi = sm.crowd = sm.refused = 0;
         }
         uint32_t wlo = 0, whi = nwin;   // the range's window
         while (whi - wlo > 1) {
@@ -479,17 +487,25 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
             // of them either way (8 windows of 2^20, 16 tuples per key: 670 us, sorted 701;
             // written, the pairs of a sorted range take 1,013, else 1,069)
             constexpr bool kVisit = kHash && kEnum && !kPairs;
-            bool crowded = false, repeats = false;
+            bool crowded = false;
+            [[maybe_unused]] RangeTable tab;
             {
                 constexpr uint32_t kPer = kRangeSubs / kRangeThreads;
-                uint32_t c[kPer], csum = 0, used = 0, squares = 0, largest = 0;   // (squares of at most kRangeCap words: 2^24)
+                uint32_t c[kPer], csum = 0, largest = 0, hot = 0;   // hot: bit q
+                uint32_t used = 0, squares = 0;                     // (squares of at most kRangeCap words: 2^24)
 #pragma unroll
                 for (uint32_t q = 0; q < kPer; q++) {
                     c[q] = sm.sub[threadIdx.x * kPer + q];
-                    csum += c[q];
-                    used += c[q] != 0;
-                    squares += c[q] * c[q];
                     largest = max(largest, c[q]);
+                    if (kTable) {
+                        used += c[q] != 0;
+                        squares += c[q] * c[q];
+                        if (c[q] > kRangeHot) {
+                            hot |= 1u << q;
+                            c[q] = 0;
+                        }
+                    }
+                    csum += c[q];
                 }
                 uint32_t ctot;
                 uint32_t crun = warp_excl_scan(csum, &ctot);
@@ -504,22 +520,43 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                         sm.warp_sq[wid] = squares;
                     }
                 }
-                if (largest > kRangeCrowdMost) sm.crowd = 1;
-                if (kTable && largest > kRangeMost) sm.most = 1;
-                crowded = __syncthreads_count(largest > (kVisit ? kRangeCrowdMost : kRangeCrowd)) > kRangeThreads / 10 || sm.crowd;
+                if (kTable) {
+                    SJBG_BARRIER();
+                } else {
+                    if (largest > kRangeCrowdMost) sm.crowd = 1;
+                    crowded = __syncthreads_count(largest > (kVisit ? kRangeCrowdMost : kRangeCrowd)) > kRangeThreads / 10 || sm.crowd;
+                }
+                uint32_t v = lane < kRangeWarps ? sm.warp_tot[lane] : 0u;
                 if (kTable) {
                     used = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_used[lane] : 0u);
                     squares = __reduce_add_sync(0xFFFFFFFFu, lane < kRangeWarps ? sm.warp_sq[lane] : 0u);
-                    repeats = used <= kRangeUsed &&
-                              (sm.most || 2 * (squares - nl * nl / kRangeSubs) > kRangeRepeat2 * nl);
+                    if (used <= kRangeUsed && 2 * (squares - nl * nl / kRangeSubs) > kRangeRepeat2 * nl) {   // no lists at all
+                        hot = (1u << kPer) - 1;
+                        v = crun = 0;
+#pragma unroll
+                        for (uint32_t q = 0; q < kPer; q++) c[q] = 0;
+                    }
                 }
-                crun += __reduce_add_sync(0xFFFFFFFFu, lane < wid ? sm.warp_tot[lane] : 0u);
+                crun += __reduce_add_sync(0xFFFFFFFFu, lane < wid ? v : 0u);
 #pragma unroll
                 for (uint32_t q = 0; q < kPer; q++) {
-                    sm.sub[threadIdx.x * kPer + q] = crun;
+                    sm.sub[threadIdx.x * kPer + q] = crun | (hot >> q & 1u ? kRangeHotBit : 0u);
                     crun += c[q];
                 }
                 if (threadIdx.x == kRangeThreads - 1) sm.sub[kRangeSubs] = crun;
+                if constexpr (kTable) {
+                    // the hot words' table: a slot for each of them, if there is room (half a slot there always is)
+                    const uint32_t listed = __reduce_add_sync(0xFFFFFFFFu, v);
+                    tab.slots = min(min(kRangeSubs, (kRangeCap - listed) / 2), max(nl - listed, 64u));
+                    tab.sum = reinterpret_cast<unsigned long long *>(sm.word + listed);
+                    tab.key = reinterpret_cast<uint32_t *>(tab.sum + tab.slots);
+                    tab.cnt = tab.key + tab.slots;
+                    for (uint32_t i = threadIdx.x; listed < nl && i < tab.slots; i += kRangeThreads) {
+                        tab.key[i] = kEmptyKey;
+                        tab.cnt[i] = 0;
+                        tab.sum[i] = 0;
+                    }
+                }
             }
             unsigned long long count = 0, prod = 0, xr = 0;
             // the right words one by one: first(x, j, end) gives the left words [j, end)
@@ -568,48 +605,24 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                     }
                 }
             };
-            bool done = false;   // (the same for the whole CTA)
-            if constexpr (kTable) {
-                if (repeats) {   // a table of the keys' numbers and sums
-                    for (uint32_t i = threadIdx.x; i < kRangeSubs; i += kRangeThreads) {
-                        sm.tab.key[i] = kEmptyKey;
-                        sm.tab.cnt[i] = 0;
-                        sm.tab.sum[i] = 0;
-                    }
-                    SJBG_BARRIER();
+            if (!crowded) {
+                SJBG_BARRIER();
 #pragma unroll
-                    for (uint32_t k = 0; k < kItems; k++) {
-                        if (threadIdx.x + k * kRangeThreads < nl && !range_add(sm.tab, e[k], sub_of((uint32_t)e[k])))
-                            sm.refused = 1;
-                        __syncwarp();
-                    }
-                    SJBG_BARRIER();
-                    done = sm.refused == 0;
-                    for (uint32_t i = nl + threadIdx.x; done && i < n; i += 4 * kRangeThreads) {
-                        uint64_t x[4];
-#pragma unroll
-                        for (uint32_t q = 0; q < 4; q++)
-                            x[q] = i + q * kRangeThreads < n ? word(i + q * kRangeThreads) : 0ull;
-#pragma unroll
-                        for (uint32_t q = 0; q < 4; q++) {
-                            const uint32_t key = (uint32_t)x[q];
-                            if (i + q * kRangeThreads >= n || key < lo || key > hi) continue;
-                            const uint32_t s = range_slot(sm.tab, key, sub_of(key));
-                            if (s == kRangeSubs || sm.tab.key[s] != key) continue;
-                            count += sm.tab.cnt[s];
-                            prod += sm.tab.sum[s] * sjbg_gs((uint32_t)(x[q] >> 32));
+                for (uint32_t k = 0; k < kItems; k++) {
+                    if (threadIdx.x + k * kRangeThreads < nl) {
+                        const uint32_t at = sm.sub[sub_of((uint32_t)e[k])];
+                        if (kTable && (at & kRangeHotBit)) {
+                            if (!range_add(tab, e[k])) sm.refused = 1;
+                        } else {
+                            sm.word[at + rank[k]] = e[k];
                         }
                     }
+                    if (kTable) __syncwarp();
                 }
+                SJBG_BARRIER();
+                if (kTable) crowded = sm.refused != 0;   // (sorted after all)
             }
-            if (done) {
-                // (by the table)
-            } else if (!crowded) {
-                SJBG_BARRIER();
-#pragma unroll
-                for (uint32_t k = 0; k < kItems; k++)
-                    if (threadIdx.x + k * kRangeThreads < nl) sm.word[sm.sub[sub_of((uint32_t)e[k])] + rank[k]] = e[k];
-                SJBG_BARRIER();
+            if (!crowded) {
                 if constexpr (kEnum) {
                     enumerate(
                         [&](uint64_t x, uint32_t &j, uint32_t &end) {
@@ -634,10 +647,17 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                         for (uint32_t q = 0; q < 4; q++) {
                             const uint32_t key = (uint32_t)e[q];
                             if (i + q * kRangeThreads >= n || key < lo || key > hi) continue;
-                            const uint32_t b = sub_of(key), end = sm.sub[b + 1];
+                            const uint32_t b = sub_of(key), first = sm.sub[b], end = sm.sub[b + 1] & ~kRangeHotBit;
                             uint32_t c = 0;
                             unsigned long long f = 0;
-                            for (uint32_t j = sm.sub[b]; j < end; j++) {
+                            if (kTable && (first & kRangeHotBit)) {
+                                const uint32_t s = range_slot(tab, key);
+                                if (s != tab.slots && tab.key[s] == key) {
+                                    c = tab.cnt[s];
+                                    f = tab.sum[s];
+                                }
+                            }
+                            for (uint32_t j = first; j < end; j++) {   // (a hot subrange's first word is past any end)
                                 const uint64_t x = sm.word[j];
                                 if ((uint32_t)x == key) {
                                     c++;
@@ -768,18 +788,25 @@ int range_join_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR,
             pmax = std::max(pmax, r.P);
         }
     };
-    plan(kRangeTarget);
-    if (hash && nb > slots) {   // the least full ranges that make it one wave, if any do
-        uint32_t no = kRangeTarget, yes = kRangeTargetMost;
-        plan(yes);
-        if (nb > slots) yes = kRangeTarget;
-        while (yes > no + 1) {
-            const uint32_t mid = (no + yes) / 2;
-            plan(mid);
-            (nb > slots ? no : yes) = mid;
+    // ranges of a target (sides of at most kRangeTarget * kRangesMax tuples: 32 bits)
+    auto ranges = [&](uint32_t target) {
+        uint64_t sum = 0;
+        for (uint32_t w = 0; w < n; w++) {
+            const uint32_t l = (uint32_t)wins[w].n_left, r = (uint32_t)wins[w].n_right;
+            if (l && r) sum += std::max({(l + target - 1) / target, (l + r + 2 * target - 1) / (2 * target), 1u});
         }
-        plan(yes);
+        return sum;
+    };
+    uint32_t target = kRangeTarget;
+    if (hash && ranges(target) > slots && ranges(kRangeTargetMost) <= slots) {
+        // about the least full ranges that make it one wave
+        uint32_t no = target;
+        for (target = kRangeTargetMost; target - no > 32;) {
+            const uint32_t mid = (no + target) / 2;
+            (ranges(mid) > slots ? no : target) = mid;
+        }
     }
+    plan(target);
     if (tiles > 0x7FFFFFFFull || nb > 0x7FFFFFFFull) return fail(h, SJBG_E_CAPACITY, "batch has too many tiles");
     if (nb == 0) {
         std::memset(hAcc, 0, sizeof(WinAcc) * (n + 1));

@@ -96,3 +96,27 @@ def test_one_wave_of_ranges(lib, oracle, sizes, per):
         assert "range_join" in j.kernel_stats()
     for d, g, w in zip(descs, got, want):
         assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
+
+
+@pytest.mark.parametrize("hot", [16, 17, 40, 1500, 3900])
+@pytest.mark.parametrize("keys", [1, 3, 60])
+def test_hot_subranges(lib, oracle, keys, hot):
+    """Some keys of `hot` tuples each among distinct ones: lists, and a table behind
+    them that the fullest ranges leave little room for."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(hot + keys)
+    W = 70_000
+    sides = []
+    for _ in range(2):
+        k = rng.permutation(np.arange(1, 1 << 20, dtype=np.uint32))[:W]
+        if keys * hot <= W:
+            k[: keys * hot] = np.repeat(np.arange(keys, dtype=np.uint32) * np.uint32(9973) + np.uint32(1 << 21), hot)
+        sides.append(make_tuples(rng.permutation(k * np.uint32(0x9E3779B1))))
+    left, right = sides
+    want = oracle.join(left, right, enumerate_pairs=False)
+    dl, dr = torch.from_numpy(left.view(np.uint8)).cuda(), torch.from_numpy(right.view(np.uint8)).cuda()
+    with lib.Joiner(lib.ALG_HJ, lib.LAZY, flags=lib.F_PROFILE, max_tuples_per_window=1 << 17) as j:
+        for _ in range(2):
+            got = j.lazy_execute_batch(dl, dr, [(0, W, 0, W, 0, 0)], mem=lib.MEM_DEVICE)[0]
+            assert (got["count"], got["prod"]) == (want["count"], want["prod"])
+        assert "range_join" in j.kernel_stats()
