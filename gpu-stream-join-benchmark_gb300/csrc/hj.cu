@@ -2528,9 +2528,10 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     // set-up of each CTA is paid over many tiles.  A share has at least
     // kHistTiles tiles with a model (whose copy and heavy-key sums each CTA sets
     // up), and for radix windows at least as many as make flushing the P
-    // counters cheap (2, or P / 256): a call of few tiles otherwise leaves most
-    // SMs idle (one window of 2^20 tuples per side, 490 tiles: 32 CTAs of 16
-    // tiles took 17.5 us).
+    // counters cheap (2, or P / 256, up to kHistTiles): a call of few tiles
+    // otherwise leaves most SMs idle (one window of 2^20 tuples per side, 490
+    // tiles: 32 CTAs of 16 tiles took 17.5 us; 2^21 per side in 2^14 buckets, 16
+    // CTAs of 64 tiles 156 us, 64 of 16 50).
     // When many sides are smaller than a share (uneven batches), shares of an
     // eighth of that keep the CTAs small enough to balance the SMs.
     uint32_t join_chunk;
@@ -2543,7 +2544,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             return fail(h, SJBG_E_CUDA, "counting pass occupancy");
         const uint64_t slots = (uint64_t)std::max(per_sm, 1) * (uint64_t)std::max(h->num_sms, 1);
         const uint64_t T = (uint64_t)tileL[n] + tileR[n];
-        const uint64_t least = learned ? kHistTiles : std::max<uint64_t>(2, maxP / 256);
+        const uint64_t least = learned ? kHistTiles : std::min<uint64_t>(kHistTiles, std::max<uint64_t>(2, maxP / 256));
         uint64_t share = std::max<uint64_t>(least, (T + slots - 1) / slots);
         uint64_t ctas = 0;
         for (uint32_t w = 0; w < n; w++)
