@@ -1353,16 +1353,16 @@ constexpr uint32_t kPlacesMax = 4096;
 // places a probe pays for every match, with a hash of the match's value.  The
 // squares of the places' tuple numbers tell how many build tuples share a
 // tuple's key on average: distinct keys give about nB + nB^2 / places, a key of
-// k tuples k^2.  64 windows of 2^20, keys spread over 32 bits, 1 / 2 / 3 / 4 / 8
-// tuples per key (a tuple then shares its key with 2 / 3 / 4 / 5 / 9): by places
-// 1.93 / 2.12 / 2.28 / 2.42 / 2.90 ms, by the table 2.40 / 2.71 / 2.31 / 2.12 /
-// 1.64, so the line is at 3.5.  A few hot keys among distinct ones hold up
-// their probes' warps before the mean shows them: a place of more than
-// kPlaceMost decides too (1,024 windows of 30,000, z = 0.5: no limit 1.54 ms,
-// 64 1.30, 32 1.16, 20 1.10; 64 of 2^20, z = 0.4: 64 2.47, 32 2.52, 20 2.86; one of
-// 65,536, z = 0.6: 32 48 us, 24 58).
+// k tuples k^2.  64 windows of 2^20, scattered keys, 1 / 2 / 3 / 4 / 8 tuples per
+// key (a tuple then shares its key with 2 / 3 / 4 / 5 / 9): by places 1.91 / 2.09
+// / 2.28 / 2.42 / 2.90 ms, by the table 2.39 / 2.08 / 1.97 / 1.90 / 1.80, so the
+// line is at 3.5 (the try costs the table 1 to 4 %).  A few hot keys among
+// distinct ones hold up their probes' warps before the mean shows them: a place
+// of more than kPlaceMost decides too (z = 0.5: 64 windows of 2^20 without a
+// limit 2.47, 32 2.38, 20 2.31, by the table alone 2.23; 1,024 of 30,000 1.54,
+// 1.20, 1.13, 1.13; z = 0.25 64 of 2^20: 32 1.97, 20 1.98, 16 2.01, table 2.36).
 constexpr uint32_t kPlaceRepeat2 = 7;   // twice the tuples that share a tuple's key
-constexpr uint32_t kPlaceMost = 32;
+constexpr uint32_t kPlaceMost = 20;
 constexpr size_t kPlaceBytes = sizeof(uint64_t) * kPlaceCap + sizeof(uint32_t) * (kPlacesMax + 1);
 
 // Adds the matches to count and prod; false, with nothing added, when the run's

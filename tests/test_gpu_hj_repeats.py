@@ -24,7 +24,7 @@ def keys_of(kind, n, rng):
 
 @pytest.mark.parametrize("part", ["PART_AUTO", "PART_RADIX"])
 @pytest.mark.parametrize("sizes", [SMALL, LARGE, SMALL + LARGE], ids=["small", "large", "both"])
-@pytest.mark.parametrize("kind", [1, 2, 3, 4, 5, 9, 40, 700, "hot31", "hot32", "hot33", "hot300"])
+@pytest.mark.parametrize("kind", [1, 2, 3, 4, 5, 9, 40, 700, "hot19", "hot20", "hot21", "hot32", "hot300"])
 def test_repeated_keys(lib, oracle, kind, sizes, part):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(17)
