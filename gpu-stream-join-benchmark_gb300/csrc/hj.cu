@@ -620,9 +620,16 @@ struct JoinGrid {
 // one piece, whose refused keys are compacted in place (only one CTA may do
 // that); beyond, both runs are cut, into at most kHotSplit pieces each, or one
 // CTA would join millions of tuples alone (8 x 2^24, z = 1.5, one hot key in
-// the buckets: 6.1 ms).
-constexpr uint32_t kHotRuns = 8, kHotSplit = 16;
-__host__ __device__ __forceinline__ JoinGrid join_grid(uint32_t nB, uint32_t nP, uint32_t chunk, uint32_t cap) {
+// the buckets: 6.1 ms).  With s pieces of each run a bucket costs s times its
+// tuples, spread over s^2 CTAs: s is the root of kHotFactor times the CTAs'
+// number times the bucket's share of the call's tuples (its tuples / hot_unit); at
+// a factor of 1 and with equal hot buckets one piece takes as long as an even
+// share of all of them, and buckets differ.  Whole calls, s = 16 / factor 1 / 2 /
+// 4 / one piece: 32 windows of 2^20, z = 1.25 1.59 / 1.55 / 1.32 / 1.29 / 1.43 ms,
+// z = 1.5 2.46 / 1.58 / 1.49 / 1.53 / 1.80; one of 2^22, z = 1.5 708 / 542 / 534 /
+// 580 / 2,590 us; 128 of 2^18, z = 1.5 1.30 / 1.28 / 1.25 / 1.16 / 1.19 ms.
+constexpr uint32_t kHotRuns = 8, kHotSplit = 16, kHotFactor = 4;
+__device__ __forceinline__ JoinGrid join_grid(uint32_t nB, uint32_t nP, uint32_t chunk, uint32_t cap, uint32_t hot_unit) {
     JoinGrid g{1, 1};
     if (nB < cap) {
         const uint32_t per = chunk > nB ? chunk : nB;
@@ -630,8 +637,9 @@ __host__ __device__ __forceinline__ JoinGrid join_grid(uint32_t nB, uint32_t nP,
         if (g.np == 0) g.np = 1;
     } else if (nB > kHotRuns * cap && nP > kHotRuns * cap) {
         const uint32_t per = kHotRuns / 2 * cap, kb = nB / per, kp = nP / per;   // at least 2 of each
-        g.nb = kb < kHotSplit ? kb : kHotSplit;
-        g.np = kp < kHotSplit ? kp : kHotSplit;
+        const uint32_t s = min(kHotSplit, max(1u, (uint32_t)(sqrtf(((float)nB + (float)nP) / (float)hot_unit) + 0.5f)));
+        g.nb = min(kb, s);
+        g.np = min(kp, s);
     }
     return g;
 }
@@ -675,7 +683,7 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
                      const uint32_t *__restrict__ baseR, const uint32_t *__restrict__ cnt,
                      uint32_t *__restrict__ start, uint32_t *__restrict__ cursor, uint32_t B,
                      const LearnedModel *__restrict__ models, JoinItem *__restrict__ items,
-                     uint32_t *__restrict__ jn, uint32_t chunk, uint32_t cap, bool either,
+                     uint32_t *__restrict__ jn, uint32_t chunk, uint32_t cap, uint32_t hot_unit, bool either,
                      const uint32_t *__restrict__ ccnt) {
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry_s;
@@ -685,7 +693,7 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
         const uint32_t nL = (uint32_t)wp.n_left, nR = (uint32_t)wp.n_right;
         const bool swap = either && nR < nL;
         const uint32_t nB = swap ? nR : nL, nP = swap ? nL : nR;
-        const JoinGrid g = join_grid(nB, nP, chunk, cap);   // (the build side is below cap)
+        const JoinGrid g = join_grid(nB, nP, chunk, cap, hot_unit);   // (the build side is below cap)
         const uint32_t k = g.items();
         if (threadIdx.x == 0) carry_s = atomicAdd(jn, k);
         SJBG_BARRIER();
@@ -746,7 +754,7 @@ part_scan_win_kernel(const WinPlan *__restrict__ wins, const uint32_t *__restric
         const uint32_t nL = i < P ? cnt[b] : 0u, nR = i < P ? cnt[B + b] : 0u;
         const bool swap = either && nR < nL;
         const uint32_t nB = swap ? nR : nL, nP = swap ? nL : nR;
-        const JoinGrid g = join_grid(nB, nP, chunk, cap);
+        const JoinGrid g = join_grid(nB, nP, chunk, cap, hot_unit);
         const uint32_t k = (nL != 0u && nR != 0u) ? g.items() : 0u;
         uint32_t tot;
         const uint32_t ex = warp_excl_scan(k, &tot);
@@ -2575,6 +2583,8 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
             kJoinChunk, std::max<uint64_t>(enumerate ? kJoinChunkEnum : kJoinChunkMin,
                                            (totL + totR) / (4 * (uint64_t)std::max(h->num_sms, 1))));
     }
+    // (two CTAs per SM)
+    const uint32_t hot_unit = (uint32_t)std::max<uint64_t>(1, (totL + totR) / (kHotFactor * 2 * (uint64_t)std::max(h->num_sms, 1)));
     const uint64_t max_items = join_items_bound(B, totL + totR, join_chunk, enumerate ? 0x0FFFFFFFu : cap);
     if (max_items > 0x7FFFFFFFull) return fail(h, SJBG_E_CAPACITY, "hash join batch has too many join items");
 
@@ -2659,7 +2669,7 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     auto scan = [&]() {
         return launch(h, "part_scan", part_scan_win_kernel, dim3(n), dim3(1024), 0, (const WinPlan *)dPlan, dPbL, dPbR,
                       (const uint32_t *)dCnt, dStart, dCur, (uint32_t)B, dModels, dJlist, dJn, join_chunk,
-                      enumerate ? 0x0FFFFFFFu : cap, !enumerate, (const uint32_t *)dCcnt);
+                      enumerate ? 0x0FFFFFFFu : cap, hot_unit, !enumerate, (const uint32_t *)dCcnt);
     };
     if (!tiles && any_raw) SJBG_CK(h, scan());
     if (tiles) {

@@ -63,3 +63,19 @@ def test_counting_pass_of_many_buckets(lib):
                 assert got["count"] == n
             ms[bits] = j.kernel_stats()["part_hist"][1]
     assert ms[14] < 2 * ms[12]
+
+
+@pytest.mark.parametrize("windows,n", [(1, 600_000), (3, 250_000), (40, 60_000)])
+def test_hot_buckets_in_pieces(lib, oracle, windows, n):
+    """One hot bucket of a call in many pieces, many of them in few or one."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(windows)
+    left, right = [make_tuples(np.concatenate([keys_of("hot", n, rng) for _ in range(windows)])) for _ in range(2)]
+    descs = [(w * n, n, w * n, n, 0, 0) for w in range(windows)]
+    want, _ = oracle.join_windows(left, right, descs, enumerate_pairs=False)
+    dl, dr = torch.from_numpy(left.view(np.uint8)).cuda(), torch.from_numpy(right.view(np.uint8)).cuda()
+    for bits in (0, 2):
+        with lib.Joiner(lib.ALG_HJ, lib.LAZY, partitioner=lib.PART_RADIX, radix_bits=bits, max_tuples_per_window=n) as j:
+            got = j.lazy_execute_batch(dl, dr, descs, mem=lib.MEM_DEVICE)
+            for d, g, w in zip(descs, got, want):
+                assert (g["count"], g["prod"]) == (w["count"], w["prod"]), d
