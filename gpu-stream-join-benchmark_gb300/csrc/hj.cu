@@ -2420,8 +2420,10 @@ int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, con
     }
     // Any cut of the two runs will do (the sums are over pairs of tuples).  The
     // smallest square pieces that make one wave of CTAs; windows that need more
-    // are taken when every build side fits a table, in pieces that cost the SMs
-    // about equal shares.
+    // are taken when every build side fits a table, whole build sides with pieces of
+    // the probes that cost the SMs about equal shares.  (With the build sides cut to
+    // a share too, every probe piece met several: 32 windows of 20,000 and 5,000
+    // tuples 85 us instead of 35, 2 of 500,000 and 5,000 94 instead of 39.)
     uint32_t piece = 0, chunk = 0;
     for (uint32_t s = kRawPiece; s <= kRawPieceMost && s < cap && piece == 0; s += kRawPiece / 2) {
         uint64_t items = 0;
@@ -2432,7 +2434,7 @@ int hj_raw_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, con
     if (piece == 0) {
         if (!small) return SJBG_OK;
         const uint64_t share = tuples / (2 * slots);
-        piece = (uint32_t)std::min<uint64_t>(cap - 1, std::max<uint64_t>(kRawPiece, share));
+        piece = cap - 1;
         chunk = (uint32_t)std::min<uint64_t>(kJoinChunk, std::max<uint64_t>(kRawPiece, share));
     }
     std::vector<RawItem> list;
