@@ -62,21 +62,24 @@ constexpr uint32_t kRangeSubs = 2048;           // subranges of a range
 constexpr uint32_t kRangeCrowd = 16, kRangeCrowdMost = 128;
 // By the hash, words of one subrange are mostly words of one key, so counting
 // joins keep no list of a hot subrange, one with more than kRangeHot left words:
-// they add up the words of each of its keys in a table behind the lists, in the
-// words' space, and a probe looks there.  When keys repeat throughout, every
-// subrange is hot: with more than 3.5 left words that share a word's key on
-// average, by the squares of the subranges' numbers (the rule of the bucket
-// joins' places, hj.cu), and few enough keys for the table, by the subranges in
-// use (kRangeUsed of 2,048: some 1,580 keys).
+// they add up the words of each of its keys in a table behind the lists (with
+// room for kRangeSubs words more than the lists need), and a probe looks there.
+// When keys repeat throughout, every subrange is hot: with more than 3.5 left
+// words that share a word's key on average, by the squares of the subranges'
+// numbers (the rule of the bucket joins' places, hj.cu), and few enough keys for
+// the table, by the subranges in use (kRangeUsed of 2,048: some 1,690 keys).
 // 8 windows of 2^20, 1 / 2 / 4 / 8 / 16 / 64 tuples per key: lists, and a sort of
 // crowded ranges, 238 / 253 / 281 / 335 / 449 / 627 us; hot subranges without the
-// rule 246 / 261 / 293 / 348 / 370 / 222; with it 246 / 263 / 251 / 234 / 226 /
+// rule 246 / 261 / 293 / 348 / 370 / 222; with it 247 / 266 / 241 / 232 / 227 /
 // 221.  Dense keys, z = 0.4 / 0.5: lists and sort 322 / 427, rule without hot
-// subranges 322 / 430, both 276 / 295 (direct tables after radix partitioning 251
+// subranges 322 / 430, both 277 / 297 (direct tables after radix partitioning 251
 // / 252).  A kRangeHot of 4 / 8 / 12 / 20: distinct keys 392 / 287 / 250 / 246,
-// z = 0.5 335 / 292 / 293 / 303.  One window of 1,000,003 distinct keys pays 1 us of 57.
+// z = 0.5 335 / 292 / 293 / 303.  A kRangeUsed of 1,350: one window of 1,000,003,
+// z = 0.4 61 -> 82.  No room behind full lists, kRangeUsed 1,100: 500 windows of
+// 20,000, z = 0.5 / 0.6 391 / 377 -> 456 / 543.  One window of 1,000,003 distinct
+// keys pays 1 us of 57 for the rule and the table.
 constexpr uint32_t kRangeHot = 16;
-constexpr uint32_t kRangeRepeat2 = 7, kRangeUsed = 1100;
+constexpr uint32_t kRangeRepeat2 = 7, kRangeUsed = 1150;
 constexpr uint32_t kRangeHotBit = 1u << 31;   // of a subrange's first word: no list
 constexpr uint32_t kRangeProbe = 64;   // slots of the table looked at for a key
 
@@ -205,7 +208,7 @@ struct RangeTable {
 
 struct RangeSmem {
     union {
-        uint64_t word[kRangeCap];                   // left words by subrange
+        uint64_t word[kRangeCap + kRangeSubs];      // left words by subrange, and room for a table behind them
         uint32_t buf[2][2][kRangeCap];              // sorting: keys and vals, before and after a pass; then F in the free pair
     };
     union {
@@ -547,7 +550,7 @@ range_join_kernel(const uint64_t *__restrict__ words, const uint16_t *__restrict
                 if constexpr (kTable) {
                     // the hot words' table: a slot for each of them, if there is room (half a slot there always is)
                     const uint32_t listed = __reduce_add_sync(0xFFFFFFFFu, v);
-                    tab.slots = min(min(kRangeSubs, (kRangeCap - listed) / 2), max(nl - listed, 64u));
+                    tab.slots = min((kRangeCap + kRangeSubs - listed) / 2, max(nl - listed, 64u));
                     tab.sum = reinterpret_cast<unsigned long long *>(sm.word + listed);
                     tab.key = reinterpret_cast<uint32_t *>(tab.sum + tab.slots);
                     tab.cnt = tab.key + tab.slots;
