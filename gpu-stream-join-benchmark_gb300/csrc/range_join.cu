@@ -53,6 +53,13 @@ constexpr uint32_t kRangeTilesMax = 1536;       // tiles of both sides of a wind
 constexpr uint32_t kRangeDigit = 7;             // bits per shared-memory sorting pass
 constexpr uint32_t kRangeDigits = 1u << kRangeDigit;
 constexpr uint32_t kRangeSample = 8192;         // sampled keys per side
+// The key map goes this many mean distances between sampled keys beyond the
+// sample at each end.  Keys outside it fall into the end ranges, which have room
+// for three such distances (of up to 256 left tuples each) above their share: one
+// distance left out four in a hundred windows of 2^20 beside a small one, and 6
+// in 60 draws of 128 windows of 2^10 to 2^20 took the sort, 1,640 us for 545.
+// With eight none of 60 did; the other ranges get at most 1.6 % fuller.
+constexpr uint32_t kRangeBeyond = 8;
 constexpr uint32_t kRangeSubs = 2048;           // subranges of a range
 // A range is crowded when one subrange holds more than kRangeCrowdMost left
 // words or more than one thread in ten owns a subrange of more than
@@ -149,9 +156,9 @@ range_sample_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restri
         m.lo = 0;
         uint64_t span = 1;
         if (lo_s <= hi_s) {
-            // the keys go a little beyond the sample's: by about span / sample at each end
+            // the keys go a little beyond the sample's
             const uint64_t sampled = max(max(range_samples(w.n[0]), range_samples(w.n[1])), (uint64_t)64);
-            const uint32_t more = (uint32_t)(((uint64_t)hi_s - lo_s) / sampled);
+            const uint32_t more = (uint32_t)min(((uint64_t)hi_s - lo_s) * kRangeBeyond / sampled, (uint64_t)0xFFFFFFFFu);
             m.lo = lo_s > more ? lo_s - more : 0u;
             span = (uint64_t)(hi_s < 0xFFFFFFFFu - more ? hi_s + more : 0xFFFFFFFFu) - m.lo + 1;
         }
