@@ -2179,6 +2179,22 @@ __device__ __forceinline__ void rows_join(const RowsJoin &rj, const WinPlan *__r
 // shared memory, from the index claimed during item k-1).  So no step of a
 // bucket waits on the queue, the list or the first loads of its runs.
 // kModels: the call has learned buckets (and no raw windows).
+// A CTA's place in the grid when the items are too few for two per SM: the first
+// CTAs of the SMs in front, in the order in which they ask, the others from the
+// end back.  A grid of two CTAs per SM does not come to the SMs quite in turn:
+// the second CTAs of some are started before the first of others, and with their
+// buckets these end last (128 buckets of 16,384 tuples per side: 604 us a call by
+// position, 519 so).  n, zeroed: first ones, others, CTAs seen on each SM.
+constexpr uint32_t kSpreadSms = 256;
+constexpr size_t kQueueBytes = 32 + sizeof(uint32_t) * (2 + kSpreadSms) + 8;   // the queues, then n (whole 16 bytes)
+static_assert(kQueueBytes % 16 == 0, "the heavy sums follow");
+__device__ __noinline__ uint32_t spread_cta(uint32_t *n) {
+    uint32_t sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    if (atomicAdd(&n[2 + sm % kSpreadSms], 1u) == 0) return atomicAdd(&n[0], 1u);
+    return gridDim.x - 1 - atomicAdd(&n[1], 1u);
+}
+
 template <bool kModels>
 __global__ void __launch_bounds__(kJoinThreads, 2)
 bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__restrict__ R,
@@ -2231,8 +2247,8 @@ bucket_join_count_kernel(const sjbg_tuple *__restrict__ L, const sjbg_tuple *__r
     __shared__ uint32_t cur_s, valid_s;   // slot of item k; bit q: slot (cur + q) % 3 holds an item
     uint32_t claim = 0;                   // thread 0: index claimed for item k+2
     if (threadIdx.x == 0) {
-        // the first two items are the CTA's by position; the queue hands out the rest
-        const uint32_t i0 = blockIdx.x, i1 = gridDim.x + blockIdx.x;
+        // the first two items are the CTA's by its place; the queue hands out the rest
+        const uint32_t i0 = nitems <= gridDim.x / 2 ? spread_cta(queue + 8) : blockIdx.x, i1 = gridDim.x + blockIdx.x;
         claim = 2 * gridDim.x + atomicAdd(queue, 1u);
         if (i0 < nitems) slot_s[0] = items[i0];
         if (i1 < nitems) slot_s[1] = items[i1];
@@ -2612,10 +2628,10 @@ int hj_lazy_batch(sjbg_handle *h, const sjbg_tuple *dL, const sjbg_tuple *dR, co
     // what starts from zero is zeroed by the same launch as the upload, with no
     // clears between the kernels later: the bucket counters; per window side its
     // compacted light tuples, then the join list's length; the join's queues
-    // (join items, then, 16 bytes on, the buckets joined from sorted tiles); the
-    // heavy keys' sums
+    // (join items, then, 16 bytes on, the buckets joined from sorted tiles) and the
+    // join CTAs' places; the heavy keys' sums
     const size_t ccntOff = sizeof(uint32_t) * 2 * B;
-    const size_t queueOff = (ccntOff + sizeof(uint32_t) * (2 * n + 1) + 15) & ~(size_t)15, heavyOff = queueOff + 32;
+    const size_t queueOff = (ccntOff + sizeof(uint32_t) * (2 * n + 1) + 15) & ~(size_t)15, heavyOff = queueOff + kQueueBytes;
     const size_t zeroB = heavyOff + (learned ? sizeof(HeavyAcc) * kMaxHeavy * n : 0);
     uint8_t *dZero = static_cast<uint8_t *>(ws_get(h, WS_BUCKET_CNT, zeroB));
     if (!dZero) return fail(h, SJBG_E_NOMEM, "partition buffers");
