@@ -52,7 +52,7 @@
 namespace sjbg {
 
 constexpr int kTile = 4096;          // tuples per partitioning tile
-constexpr uint32_t kHistTiles = 16;  // tiles per counting CTA at least (amortises its set-up)
+constexpr uint32_t kHistTiles = 16;  // tiles per counting CTA at least with a model (amortises its set-up)
 constexpr int kPartThreads = 512;
 constexpr int kJoinThreads = 512;
 constexpr uint32_t kMaxBucketsLog2 = 14;

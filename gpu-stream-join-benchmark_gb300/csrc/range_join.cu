@@ -84,7 +84,7 @@ constexpr uint32_t kRangeCrowd = 16, kRangeCrowdMost = 128;
 // z = 0.5 335 / 292 / 293 / 303.  A kRangeUsed of 1,350: one window of 1,000,003,
 // z = 0.4 61 -> 82.  No room behind full lists, kRangeUsed 1,100: 500 windows of
 // 20,000, z = 0.5 / 0.6 391 / 377 -> 456 / 543.  One window of 1,000,003 distinct
-// keys pays 1 us of 57 for the rule and the table.
+// keys pays 1 to 2 us of 57 for the rule and the table.
 constexpr uint32_t kRangeHot = 16;
 constexpr uint32_t kRangeRepeat2 = 7, kRangeUsed = 1150;
 constexpr uint32_t kRangeHotBit = 1u << 31;   // of a subrange's first word: no list

@@ -154,8 +154,8 @@ typedef struct sjbg_window_result {
     uint64_t n_pairs;          /* pairs written to the caller's buffer */
     uint32_t status;           /* SJBG_OK or SJBG_E_* for this window */
     uint32_t flags;            /* SJBG_WR_* */
-    uint32_t partitioner_used; /* SJBG_PART_* actually used */
-    float ms;                  /* device time of the call that produced it */
+    uint32_t partitioner_used; /* SJBG_PART_* actually used; with SJBG_PART_AUTO it may follow from the handle's earlier calls */
+    float ms;                  /* device time of the call that produced it, a second try at its join included */
 } sjbg_window_result;
 
 /* One window of a batched call: spans into the left / right arrays and into
